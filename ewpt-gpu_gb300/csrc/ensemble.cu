@@ -186,7 +186,7 @@ static int ens_view(ewpt_ens* e, int32_t m, ewpt_ctx** out, bool join = true) {
     v->p.precision = EWPT_FP64;
     if (join) {
         const ewpt_ctx* c = e->mem[m];
-        int rc = ens_cuda(e, launch_fp32_join(v->g, c->lay, c->y32, v->y, e->st), "ensemble view");
+        int rc = ens_cuda(e, launch_fp32_join(v->g, c->lay, c->y32, arrays36(v->y, v->g.S), e->st), "ensemble view");
         if (rc) return rc;
     }
     *out = v;
@@ -198,13 +198,18 @@ int ewpt_ensemble_set_state(ewpt_ens* e, int32_t m, const double* packed, int32_
     if (rc) return rc;
     if (!packed) return ens_fail(e, EWPT_ERR_ARG, "state is NULL");
     cudaSetDevice(e->device);
-    ewpt_ctx* v;
-    rc = ens_view(e, m, &v, false);
-    if (rc) return rc;
     ewpt_ctx* c = e->mem[m];
-    cudaError_t ce = cudaMemcpyAsync(v->y, packed, (size_t)36 * c->g.S * 8,
-                                     on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, e->st);
-    if (ce == cudaSuccess) ce = launch_fp32_split(c->g, c->lay, v->y, c->y32, e->st);
+    cudaError_t ce = cudaSuccess;
+    const double* src = packed;
+    if (!on_device || !ewpt_kernel_reads(packed, e->device)) {
+        ewpt_ctx* v;
+        rc = ens_view(e, m, &v, false);
+        if (rc) return rc;
+        ce = cudaMemcpyAsync(v->y, packed, (size_t)36 * c->g.S * 8,
+                             on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, e->st);
+        src = v->y;
+    }
+    if (ce == cudaSuccess) ce = launch_fp32_split(c->g, c->lay, arrays36(src, c->g.S), c->y32, e->st, false);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->st);
     return ens_cuda(e, ce, "ensemble set_state");
 }
@@ -214,11 +219,17 @@ int ewpt_ensemble_get_state(ewpt_ens* e, int32_t m, double* packed, int32_t on_d
     if (rc) return rc;
     if (!packed) return ens_fail(e, EWPT_ERR_ARG, "state is NULL");
     cudaSetDevice(e->device);
-    ewpt_ctx* v;
-    rc = ens_view(e, m, &v);
-    if (rc) return rc;
-    cudaError_t ce = cudaMemcpyAsync(packed, v->y, (size_t)36 * e->mem[m]->g.S * 8,
-                                     on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, e->st);
+    cudaError_t ce;
+    if (on_device && ewpt_kernel_reads(packed, e->device)) {
+        const ewpt_ctx* c = e->mem[m];
+        ce = launch_fp32_join(c->g, c->lay, c->y32, arrays36(packed, c->g.S), e->st);
+    } else {
+        ewpt_ctx* v;
+        rc = ens_view(e, m, &v);
+        if (rc) return rc;
+        ce = cudaMemcpyAsync(packed, v->y, (size_t)36 * e->mem[m]->g.S * 8,
+                             on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, e->st);
+    }
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->st);
     return ens_cuda(e, ce, "ensemble get_state");
 }
@@ -313,7 +324,7 @@ static int ens_thermal(ewpt_ens* e, int32_t m, double T, double mH, double mW, u
     rc = ewpt_thermal_fill(v->g, v->p, T, mH, mW, seed, v->y, e->st, &err, gauss_iters);
     if (rc) return ens_fail(e, rc, ("init_thermal: " + err).c_str());
     ewpt_ctx* c = e->mem[m];
-    cudaError_t ce = launch_fp32_split(c->g, c->lay, v->y, c->y32, e->st);
+    cudaError_t ce = launch_fp32_split(c->g, c->lay, arrays36((const double*)v->y, c->g.S), c->y32, e->st, false);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->st);
     return ens_cuda(e, ce, "ensemble init_thermal");
 }

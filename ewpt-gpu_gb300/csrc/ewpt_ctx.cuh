@@ -65,6 +65,9 @@ int ewpt_ensure_scratch64(ewpt_ctx* c);
 // context's form (FP32 split with ghost faces, DF64 pairs), on c->st.
 extern "C" int ewpt_staging64(ewpt_ctx* c, double** out, bool in);
 extern "C" cudaError_t ewpt_commit_staged(ewpt_ctx* c, const double* staged);
+// Whether a kernel on `device` may take p's memory as it is (memory of that
+// device, 8-byte aligned); other memory goes through a copy.
+bool ewpt_kernel_reads(const void* p, int device);
 // Interior of a slab context <-> a packed [36][nx ny nz] buffer (slab.cu).
 cudaError_t ewpt_slab_copy(ewpt_ctx* c, double* packed, bool to_dev, int32_t on_device);
 // Thermal IC (thermal.cu) into an FP64 [36][S] device state y, synchronous

@@ -185,8 +185,9 @@ cudaError_t launch_rates_fp64_order(const Grid& g, const Ptr36& in, const MPtr36
 // DF64 form (stage_dd.cu): y, yn, xa, xb hold float pairs (hi, lo).
 cudaError_t launch_step_dd(const Grid& g, const Tiling& t, double* y, double* yn, double* xa, double* xb,
                            double* cur, const ewpt_params& p, double Jex, double gam, cudaStream_t st);
-cudaError_t launch_to_dd(int64_t n, double* v, cudaStream_t st);  // in place: double -> (hi, lo)
-cudaError_t launch_from_dd(int64_t n, const double* src, double* dst, cudaStream_t st);
+// 36 FP64 arrays of S values <-> [36][S] float pairs (src = the pairs' own buffer: in place)
+cudaError_t launch_to_dd(int64_t S, const Ptr36& src, double* pairs, cudaStream_t st);
+cudaError_t launch_from_dd(int64_t S, const double* pairs, const MPtr36& dst, cudaStream_t st);
 cudaError_t launch_step_fp32(const Grid& g, const Layout& L, const Tiling& t, Fp32State y, Fp32Work w,
                              const ewpt_params& p, double Jex, double gam, cudaStream_t st);
 // comp: the compensated mode (gauge Laplacians and auxiliary gradients compensated, stage_pair.cu)
@@ -195,6 +196,19 @@ cudaError_t launch_step_fp32_pair(const Grid& g, const Layout& L, const Tiling& 
 // Copy the face sites of all 36 arrays of a ghosted buffer into their
 // periodic images (stage.cu); the x faces only if xfaces.
 cudaError_t launch_ghost_fill(const Grid& g, const Layout& L, float* buf, cudaStream_t st, bool xfaces);
-// FP64 [36][S] <-> FP32 hi/lo in layout L (the ghost images of hi refreshed on split).
-cudaError_t launch_fp32_split(const Grid& g, const Layout& L, const double* src, Fp32State dst, cudaStream_t st);
-cudaError_t launch_fp32_join(const Grid& g, const Layout& L, Fp32State src, double* dst, cudaStream_t st);
+// 36 FP64 arrays <-> FP32 hi/lo in layout L (the ghost images of hi refreshed
+// on split, the x faces only if xfaces).
+cudaError_t launch_fp32_split(const Grid& g, const Layout& L, const Ptr36& src, Fp32State dst, cudaStream_t st,
+                              bool xfaces);
+cudaError_t launch_fp32_join(const Grid& g, const Layout& L, Fp32State src, const MPtr36& dst, cudaStream_t st);
+// the arrays of a packed [36][S] FP64 buffer
+inline Ptr36 arrays36(const double* y, int64_t S) {
+    Ptr36 P;
+    for (int a = 0; a < 36; ++a) P.p[a] = y + a * S;
+    return P;
+}
+inline MPtr36 arrays36(double* y, int64_t S) {
+    MPtr36 P;
+    for (int a = 0; a < 36; ++a) P.p[a] = y + a * S;
+    return P;
+}

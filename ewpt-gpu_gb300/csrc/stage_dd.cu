@@ -7,7 +7,10 @@
 // yn accumulation order, main_rk4.jl:6146-6437), each value stored as the
 // float pair (hi, lo).  State I/O converts from / to FP64 exactly
 // representable splits (hi = fl(v), lo = fl(v - hi)).
+#include <algorithm>
+
 #include "accessors.cuh"
+#include "convert.cuh"
 #include "dd.cuh"
 
 namespace {
@@ -148,18 +151,33 @@ __global__ void __launch_bounds__(DdBudget<REG>::kThreads, DdBudget<REG>::kMinBl
     site_rates<dd, BETA, DdAcc, DdSink<STAGE>, PART>(A, pc, out);
 }
 
-__global__ void k_to_dd(int64_t n, double* __restrict__ v) {
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x)
-        reinterpret_cast<float2*>(v)[q] = dd(v[q]).f2();
-}
-
-__global__ void k_from_dd(int64_t n, const double* __restrict__ src, double* __restrict__ dst) {
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x) {
-        const float2 v = reinterpret_cast<const float2*>(src)[q];
-        dst[q] = (double)v.x + (double)v.y;
+// FP64 arrays <-> float pairs (convert.cuh), array blockIdx.y; in place when
+// the pairs lie over the array itself, each element by one thread.  Bound by
+// memory: 1.2 GB at 128^3; with C casts k_to_dd / k_from_dd took 557 / 411 us
+// there, the time of their FP64-pipe instructions.
+__global__ void __launch_bounds__(256) k_to_dd(int64_t S, const __grid_constant__ Ptr36 src, float2* pairs) {
+    const double* v = reinterpret_cast<const double*>(src.p[blockIdx.y]);
+    float2* out = pairs + blockIdx.y * S;
+#pragma unroll 4
+    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < S; q += (int64_t)gridDim.x * blockDim.x) {
+        float2 f;
+        split_f64(v[q], f.x, f.y);
+        out[q] = f;
     }
 }
 
+__global__ void __launch_bounds__(256) k_from_dd(int64_t S, const float2* __restrict__ pairs,
+                                                 const __grid_constant__ MPtr36 dst) {
+    const float2* in = pairs + blockIdx.y * S;
+    double* out = reinterpret_cast<double*>(dst.p[blockIdx.y]);
+#pragma unroll 4
+    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < S; q += (int64_t)gridDim.x * blockDim.x) {
+        const float2 v = __ldg(in + q);
+        out[q] = join_f64(v.x, v.y);
+    }
+}
+
+dim3 pair_grid(int64_t S) { return dim3((unsigned)std::min<int64_t>((S + 1023) / 1024, 4096), 36); }
 
 // One stage: the whole stage with beta terms, else its three parts.
 template <int STAGE, bool BETA, int REG>
@@ -211,12 +229,12 @@ cudaError_t launch_step_dd(const Grid& g, const Tiling& t, double* y, double* yn
     return cudaGetLastError();
 }
 
-cudaError_t launch_to_dd(int64_t n, double* v, cudaStream_t st) {
-    k_to_dd<<<1216, 256, 0, st>>>(n, v);
+cudaError_t launch_to_dd(int64_t S, const Ptr36& src, double* pairs, cudaStream_t st) {
+    k_to_dd<<<pair_grid(S), 256, 0, st>>>(S, src, reinterpret_cast<float2*>(pairs));
     return cudaGetLastError();
 }
 
-cudaError_t launch_from_dd(int64_t n, const double* src, double* dst, cudaStream_t st) {
-    k_from_dd<<<1216, 256, 0, st>>>(n, src, dst);
+cudaError_t launch_from_dd(int64_t S, const double* pairs, const MPtr36& dst, cudaStream_t st) {
+    k_from_dd<<<pair_grid(S), 256, 0, st>>>(S, reinterpret_cast<const float2*>(pairs), dst);
     return cudaGetLastError();
 }
