@@ -62,8 +62,8 @@ TRAFFIC_FP32 = 2973
 # own per-site templates with an operator-counting scalar type
 # (tests/test_devphys.py checks these figures against that count): FLOPs with
 # an FMA as 2, and FP64 pipe instructions with single-use products fused.
-FLOPS_FP64 = 7300
-FP64_INST_EST = 4976
+FLOPS_FP64 = 6820
+FP64_INST_EST = 4704
 # FP64 instructions per site-update the stage kernels execute (ncu
 # smsp__sass_thread_inst_executed_op_{dadd,dmul,dfma}_pred_on.sum over the 4
 # launches at 80^3, per site): 3 x (454 + 126 + 604) + (454 + 126 + 568).

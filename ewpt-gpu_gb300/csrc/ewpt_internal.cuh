@@ -20,6 +20,9 @@ struct Grid {
     // FP64 stage launches over a window of z planes: the launch's block z
     // index b covers plane k0 + b (0 for whole-lattice launches)
     int k0 = 0;
+    // FP64 stage launches: > 0 = a 1-D launch over this many sites, x fastest,
+    // then y, then the planes from k0 on; 0 = tiles over x-y, one plane per block
+    int flat = 0;
 };
 
 // Storage of one FP32-form [36][.] array set: element (i, j, k) of array a
@@ -125,6 +128,36 @@ PhysCoef<T> make_phys(const ewpt_params& p, double Jex, double gam) {
     c.gamh = (T)(gam / (0.5 * p.gw));
     c.ryw = (T)(p.gy / p.gw);
     c.igw = (T)(1.0 / p.gw);
+    c.hgw_d = c.hgw;
+    c.gw_d = c.gw;
+    c.omgp2_d = c.omgp2;
+    c.it = c.t = c.hgw_o = c.gw_o = c.gy_o = c.lap_h = c.lap_w = c.lap_y = T(0);
+    return c;
+}
+
+// Coefficients for an accessor with scaled stencils (physics.cuh): first
+// derivatives in units of t = 1/(60 dx), Laplacians of 1/(180 dx^2).
+inline PhysCoef<double> make_phys_scaled(const ewpt_params& p, double Jex, double gam) {
+    PhysCoef<double> c = make_phys<double>(p, Jex, gam);
+    const double T = 60.0 * p.dx, iU = 1.0 / (180.0 * p.dx * p.dx);
+    c.it = T;
+    c.t = 1.0 / T;
+    c.hgw_d = T * c.hgw;
+    c.gw_d = T * c.gw;
+    c.omgp2_d = c.omgp2 / T;
+    c.lam2h *= T;
+    c.hJexh *= T;
+    c.gamh *= T;
+    c.hgw_o = c.hgw / T;
+    c.gw_o = c.gw / T;
+    c.gy_o = c.gy / T;
+    c.lap_h = iU / c.hgw_o;
+    c.lap_w = iU / c.gw_o;
+    c.lap_y = iU;
+    c.bW /= T;
+    c.bY /= T;
+    c.bW2 /= T;
+    c.bY2 /= T;
     return c;
 }
 
@@ -160,8 +193,11 @@ cudaError_t launch_rates_fp64(const Grid& g, const Ptr36& in, const MPtr36& out,
 struct Tiling {
     int bx, by, reg;
     int pair;  // FP32 form: 1 = two x-adjacent sites per thread (stage_pair.cu), needs nx even
+    // 1 until ewpt_set_tiling: the launchers pick a shape for the lattice
+    // that gives the same bits as this one
+    int pick = 0;
 };
-constexpr Tiling kDefaultTiling{32, 4, 0, 0};
+constexpr Tiling kDefaultTiling{32, 4, 0, 0, 1};
 int tiling_max_threads(int reg);
 
 cudaError_t launch_step_fp64(const Grid& g, const Tiling& t, double* y, double* yn, double* xa, double* xb,

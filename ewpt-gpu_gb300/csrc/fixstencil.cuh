@@ -1,0 +1,214 @@
+// fixstencil.cuh -- 6th-order FP64 stencils in exact integer arithmetic.
+//
+// GB300 issues one FP64 warp instruction per 64 cycles and SM quarter, 64
+// times fewer than 32-bit integer or FP32 instructions, and the stencils are
+// 736 of the ~1180 FP64 instructions of a site and stage.  Here a stencil's
+// doubles are aligned to the largest exponent among them as 64-bit integers
+// (56 bits below the largest value's binade: 3 bits more than FP64), summed
+// exactly with the integer weights 45, -9, 1 (60 dx times the derivative) and
+// 270, -27, 2 (180 dx^2 times the Laplacian, on differences from the centre
+// value), and each finished sum is rounded once to FP64; the factors stay in
+// the coefficients of the physics.  A derivative carries that rounding and
+// the bits below 2^-55 of the largest value of its stencil, where the
+// floating-point evaluation rounds every partial sum at 2^-53 and every
+// weight (3/20, 1/90, 49/6 ... are no FP64 numbers) once.
+//
+// A value goes to an integer by bit operations (about 12), the sums are
+// add/multiply pairs, a finished sum goes back by a count of leading zeros
+// and shifts (about 20): some 450 integer instructions for a gradient with
+// Laplacian, against 37 FP64 instructions (2368 issue slots).  A step of the
+// FP64 form at 256^3 went from 144.4 to 76.1 ms (64^3: 2.41 to 1.20) with
+// these stencils, the factored physics and 16 warps per SM; ncu at 96^3: 501
+// FP64 instructions per warp and stage (1046 before), FP64 pipe 66% busy,
+// instruction fetch and fixed latencies the largest stalls.
+//
+// Stencils whose largest magnitude lies outside [2^-895, 2^977] (denormals,
+// infinities and NaN among them) take the floating-point evaluation, a
+// stencil of zeros gives zero.
+#pragma once
+#include "accessors.cuh"
+
+namespace fix {
+
+__device__ __forceinline__ int64_t i64(uint32_t lo, uint32_t hi) { return (int64_t)(((uint64_t)hi << 32) | lo); }
+
+// exponent field of v, in place
+__device__ __forceinline__ uint32_t exp20(double v) { return (uint32_t)__double2hiint(v) & 0x7ff00000u; }
+
+// the exponents e20 (largest of a stencil) that the integer path covers
+__device__ __forceinline__ bool covered(uint32_t e20) { return e20 - (128u << 20) < (1872u << 20); }
+
+// zeros (either sign): the arrays a run starts without, away from what feeds them
+__device__ __forceinline__ bool zero_bits(double v) {
+    return (((uint32_t)__double2hiint(v) << 1) | (uint32_t)__double2loint(v)) == 0u;
+}
+__device__ __forceinline__ bool zero_bits(const double (&f)[3][6]) {
+    bool z = true;
+#pragma unroll
+    for (int ax = 0; ax < 3; ++ax)
+#pragma unroll
+        for (int k = 0; k < 6; ++k) z = z && zero_bits(f[ax][k]);
+    return z;
+}
+
+// v in units of 2^(E - 1023 - 55), rounded towards minus infinity (a
+// negative value one unit lower: stencil weights sum to zero, and the unit is
+// an eighth of the largest value's last place); e20p = e20 + (7 << 20)
+__device__ __forceinline__ int64_t align(double v, uint32_t e20p) {
+    const uint32_t h = (uint32_t)__double2hiint(v), l = (uint32_t)__double2loint(v);
+    const uint32_t s = (uint32_t)((int32_t)h >> 31);
+    const uint32_t sh = (e20p - (h & 0x7ff00000u)) >> 20;  // 7 + the distance to the largest exponent
+    // 1.mantissa at bits 62..10
+    const uint32_t mh = ((__funnelshift_l(l, h, 10) & 0x3fffffffu) | 0x40000000u) ^ s;
+    const uint32_t ml = (l << 10) ^ s;
+    return i64(ml, mh) >> min(sh, 63u);
+}
+
+// V * 2^(E - 1023 - 55 + up) rounded to nearest, |V| < 2^63
+__device__ __forceinline__ double to_double(int64_t V, uint32_t e20, int up) {
+    const int64_t s = V >> 63;
+    uint64_t u = (uint64_t)((V ^ s) - s);
+    const int n = __clzll((long long)u);
+    u <<= (n - 1) & 63;  // leading one at bit 62
+    u += 0x200u;
+    const uint32_t hi = (uint32_t)(u >> 42), lo = (uint32_t)(u >> 10);  // leading one at bit 52 of (hi, lo): adds 1 to the exponent field
+    // |V| in [2^(63 - n), 2^(64 - n)): exponent E - 55 + up + 63 - n
+    const uint32_t e = e20 + (uint32_t)((8 - 1 + up) - n) * (1u << 20);
+    const uint32_t r = (hi + e) | ((uint32_t)(s >> 32) & 0x80000000u);
+    return V == 0 ? 0.0 : __hiloint2double((int)r, (int)lo);
+}
+
+// 45 d1 - 9 d2 + d3, |d| <= 2^57
+__device__ __forceinline__ int64_t weigh_grad(int64_t d1, int64_t d2, int64_t d3) { return 45 * d1 - 9 * d2 + d3; }
+
+// (270 t1 - 27 t2 + 2 t3) >> 6, |t| < 2^60, without overflow
+__device__ __forceinline__ int64_t weigh_lap(int64_t t1, int64_t t2, int64_t t3) {
+    const int64_t lo = (int64_t)((uint64_t)(uint32_t)t1 * 270u + (uint64_t)(uint32_t)t3 * 2u) -
+                       (int64_t)((uint64_t)(uint32_t)t2 * 27u);
+    const int64_t hi = (int64_t)(int32_t)(t1 >> 32) * 270 + (int64_t)(int32_t)(t3 >> 32) * 2 -
+                       (int64_t)(int32_t)(t2 >> 32) * 27 + (lo >> 32);
+    return (hi << 26) | (int64_t)((uint32_t)lo >> 6);
+}
+
+}  // namespace fix
+
+// SiteAcc's FP64 stencils on the integer pipes.  The routines are out-of-line
+// calls: inlined 24 times they would be far larger than the instruction cache.
+struct FixAcc : SiteAcc<double, double, SrcPtr36<double>> {
+    using Base = SiteAcc<double, double, SrcPtr36<double>>;
+    static constexpr bool kScaledStencils = true;  // 60 dx grad and div, 180 dx^2 lap
+    double T, U;                                   // 60 dx, 180 dx^2 (the floating-point evaluation)
+
+    __device__ __noinline__ void grad_lap(int a, double& gx, double& gy, double& gz, double& lap) const {
+        const double* p = src.arr(a) + c;
+        double f[3][6];
+        const double f0 = __ldg(p);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            f[0][k] = __ldg(p + ox[k]);
+            f[1][k] = __ldg(p + oy[k]);
+            f[2][k] = __ldg(p + oz[k]);
+        }
+        uint32_t e = fix::exp20(f0);
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax)
+#pragma unroll
+            for (int k = 0; k < 6; ++k) e = max(e, fix::exp20(f[ax][k]));
+        if (!fix::covered(e)) {
+            if (e == 0 && fix::zero_bits(f0) && fix::zero_bits(f))
+                gx = gy = gz = lap = 0.0;
+            else {
+                Base::grad_lap(a, gx, gy, gz, lap);
+                gx *= T;
+                gy *= T;
+                gz *= T;
+                lap *= U;
+            }
+            return;
+        }
+        const uint32_t ep = e + (7u << 20);
+        const int64_t i0 = fix::align(f0, ep);
+        int64_t T[3] = {-6 * i0, -6 * i0, -6 * i0};
+        double g[3];
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax) {
+            int64_t D[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const int64_t u = fix::align(f[ax][k], ep), w = fix::align(f[ax][k + 3], ep);
+                D[k] = u - w;
+                T[k] += u + w;
+            }
+            g[ax] = fix::to_double(fix::weigh_grad(D[0], D[1], D[2]), e, 0);
+        }
+        gx = g[0];
+        gy = g[1];
+        gz = g[2];
+        lap = fix::to_double(fix::weigh_lap(T[0], T[1], T[2]), e, 6);
+    }
+
+    __device__ __noinline__ void grad(int a, double& gx, double& gy, double& gz) const {
+        const double* p = src.arr(a) + c;
+        double f[3][6];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            f[0][k] = __ldg(p + ox[k]);
+            f[1][k] = __ldg(p + oy[k]);
+            f[2][k] = __ldg(p + oz[k]);
+        }
+        uint32_t e = 0;
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax)
+#pragma unroll
+            for (int k = 0; k < 6; ++k) e = max(e, fix::exp20(f[ax][k]));
+        if (!fix::covered(e)) {
+            if (e == 0 && fix::zero_bits(f))
+                gx = gy = gz = 0.0;
+            else {
+                Base::grad(a, gx, gy, gz);
+                gx *= T;
+                gy *= T;
+                gz *= T;
+            }
+            return;
+        }
+        const uint32_t ep = e + (7u << 20);
+        double g[3];
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax) {
+            int64_t D[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) D[k] = fix::align(f[ax][k], ep) - fix::align(f[ax][k + 3], ep);
+            g[ax] = fix::to_double(fix::weigh_grad(D[0], D[1], D[2]), e, 0);
+        }
+        gx = g[0];
+        gy = g[1];
+        gz = g[2];
+    }
+
+    __device__ __noinline__ double div3(int a) const {
+        double f[3][6];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            f[0][k] = __ldg(src.arr(a) + c + ox[k]);
+            f[1][k] = __ldg(src.arr(a + 1) + c + oy[k]);
+            f[2][k] = __ldg(src.arr(a + 2) + c + oz[k]);
+        }
+        uint32_t e = 0;
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax)
+#pragma unroll
+            for (int k = 0; k < 6; ++k) e = max(e, fix::exp20(f[ax][k]));
+        if (!fix::covered(e)) return e == 0 && fix::zero_bits(f) ? 0.0 : T * Base::div3(a);
+        const uint32_t ep = e + (7u << 20);
+        int64_t V = 0;  // three axes: two bits more than one derivative
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax) {
+            int64_t D[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) D[k] = fix::align(f[ax][k], ep) - fix::align(f[ax][k + 3], ep);
+            V += fix::weigh_grad(D[0], D[1], D[2]) >> 2;
+        }
+        return fix::to_double(V, e, 2);
+    }
+};

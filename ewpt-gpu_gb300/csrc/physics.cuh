@@ -59,6 +59,15 @@ struct CompGauge : std::false_type {};
 template <class A>
 struct CompGauge<A, std::void_t<decltype(A::kCompGauge)>> : std::integral_constant<bool, A::kCompGauge> {};
 
+// Accessors that declare kScaledStencils = true return 60 dx times a first
+// derivative or divergence and 180 dx^2 times a Laplacian (FixAcc,
+// fixstencil.cuh); the coefficients of make_phys_scaled absorb the factors.
+template <class A, class = void>
+struct ScaledStencils : std::false_type {};
+template <class A>
+struct ScaledStencils<A, std::void_t<decltype(A::kScaledStencils)>>
+    : std::integral_constant<bool, A::kScaledStencils> {};
+
 template <typename T>
 struct PhysCoef {
     T gw, gy, hgw, hgy;  // g, g', g/2, g'/2
@@ -70,19 +79,25 @@ struct PhysCoef {
     T gg, ggy;           // gp2*g, gp2*g'
     T lam2h, hJexh, gamh;// 2*lambda, Jex/2 and gamma over g/2
     T ryw, igw;          // g'/g, 1/g
+    // couplings where a product meets a derivative: hgw, gw and omgp2, or with
+    // scaled stencils (derivatives in units of t = 1/(60 dx)) hgw/t, gw/t, omgp2 t
+    T hgw_d, gw_d, omgp2_d;
+    // scaled stencils only: 1/t, t, then the factors that end a rate (t g/2,
+    // t g, t g') and those of a Laplacian in its sum
+    T it, t, hgw_o, gw_o, gy_o, lap_h, lap_w, lap_y;
 };
 
 // Covariant derivatives D_i phi_a (cov_derivs_temporal.jl:23-130) along one
-// axis with gauge components W1 = W_1_i, W2 = W_2_i, W3 = W_3_i and the
-// hypercharge component in units of g: Yr = (g'/g) Y_i, so that
-// D = d + (g/2) (W terms + Yr terms).
+// axis with gauge components W1 = W_1_i, W2 = W_2_i and the sums Zp = W_3_i +
+// Yr, Zm = W_3_i - Yr with the hypercharge component in units of g, Yr =
+// (g'/g) Y_i, so that D = d + (g/2) (W terms + Yr terms).
 template <typename T>
-EWPT_ARITH void cov_deriv_s(T d1, T d2, T d3, T d4, T p1, T p2, T p3, T p4, T W1, T W2, T W3, T Yr, T hgw, T& D1,
+EWPT_ARITH void cov_deriv_s(T d1, T d2, T d3, T d4, T p1, T p2, T p3, T p4, T W1, T W2, T Zp, T Zm, T hgw, T& D1,
                             T& D2, T& D3, T& D4) {
-    D1 = d1 + hgw * (W1 * p4 - W2 * p3 + W3 * p2 + Yr * p2);
-    D2 = d2 - hgw * (W1 * p3 + W2 * p4 + W3 * p1 + Yr * p1);
-    D3 = d3 + hgw * (W1 * p2 + W2 * p1 - W3 * p4 + Yr * p4);
-    D4 = d4 - hgw * (W1 * p1 - W2 * p2 - W3 * p3 + Yr * p3);
+    D1 = d1 + hgw * (W1 * p4 - W2 * p3 + Zp * p2);
+    D2 = d2 - hgw * (W1 * p3 + W2 * p4 + Zp * p1);
+    D3 = d3 + hgw * (W1 * p2 + W2 * p1 - Zm * p4);
+    D4 = d4 - hgw * (W1 * p1 - W2 * p2 - Zm * p3);
 }
 
 // The same with Y_i and g'/2 apart (the diagnostics).
@@ -103,7 +118,10 @@ EWPT_ARITH void site_rates(const Acc& A, const PhysCoef<T>& c, Sink& out) {
     // compensated gauge stencils: kt W^a_i = (lap W^a_i - d_i Gamma^a) + g Q^a_i and
     // kt Y_i = (lap Y_i - d_i Sigma) + g' jY_i with each bracket formed before rounding
     constexpr bool kComp = CompGauge<Acc>::value;
-    const T gw = c.gw, gy = c.gy, hgw = c.hgw;
+    // derivatives in units of t = 1/(60 dx): every sum below that holds one is
+    // then in units of t too, and the last factor of its rate restores it
+    constexpr bool kScaled = ScaledStencils<Acc>::value;
+    const T hgw = c.hgw_d, gw_d = c.gw_d;
     const T p1 = A.v(0), p2 = A.v(1), p3 = A.v(2), p4 = A.v(3);
     T W[3][3];  // W[a][i] = W_{a+1}_{i+2}
 #pragma unroll
@@ -111,8 +129,13 @@ EWPT_ARITH void site_rates(const Acc& A, const PhysCoef<T>& c, Sink& out) {
 #pragma unroll
         for (int i = 0; i < 3; ++i) W[a][i] = A.v(4 + 3 * a + i);
     const T Y2 = A.v(13), Y3 = A.v(14), Y4 = A.v(15);
-    const T G[3] = {A.v(16), A.v(17), A.v(18)};
-    const T S = A.v(19);
+    T G[3] = {A.v(16), A.v(17), A.v(18)};
+    T S = A.v(19);
+    if constexpr (kScaled) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) G[a] = G[a] * c.it;
+        S = S * c.it;
+    }
     const T pt1 = A.v(20), pt2 = A.v(21), pt3 = A.v(22), pt4 = A.v(23);
 
     // ---- k_field = momentum (main_rk4.jl:585-600)
@@ -128,6 +151,7 @@ EWPT_ARITH void site_rates(const Acc& A, const PhysCoef<T>& c, Sink& out) {
         for (int a = 0; a < 3; ++a)
 #pragma unroll
             for (int i = 0; i < 3; ++i) Wt[a][i] = A.v(24 + 3 * a + i);
+        const T q12 = p1 * pt2 - p2 * pt1, q34 = p3 * pt4 - p4 * pt3;  // of charge 3 and the hypercharge
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
             const int b = (a + 1) % 3, cc = (a + 2) % 3;
@@ -135,12 +159,12 @@ EWPT_ARITH void site_rates(const Acc& A, const PhysCoef<T>& c, Sink& out) {
             T q;
             if (a == 0) q = p1 * pt4 - p4 * pt1 + p3 * pt2 - p2 * pt3;
             else if (a == 1) q = p3 * pt1 - p1 * pt3 + p4 * pt2 - p2 * pt4;
-            else q = p1 * pt2 - p2 * pt1 + p4 * pt3 - p3 * pt4;
+            else q = q12 - q34;
             q = q - W[b][0] * Wt[cc][0] + W[cc][0] * Wt[b][0] - W[b][1] * Wt[cc][1] + W[cc][1] * Wt[b][1] -
                 W[b][2] * Wt[cc][2] + W[cc][2] * Wt[b][2];
-            out(16 + a, c.omgp2 * A.div3(24 + 3 * a) + c.gg * q);
+            out(16 + a, c.omgp2_d * A.div3(24 + 3 * a) + c.gg * q);
         }
-        out(19, c.omgp2 * A.div3(33) + c.ggy * (p1 * pt2 - p2 * pt1 + p3 * pt4 - p4 * pt3));
+        out(19, c.omgp2_d * A.div3(33) + c.ggy * (q12 + q34));
     }
 
     // ---- Higgs block: gradients, covariant derivatives, kt_phi (main_rk4.jl:337-407)
@@ -169,18 +193,26 @@ EWPT_ARITH void site_rates(const Acc& A, const PhysCoef<T>& c, Sink& out) {
         A.grad_lap(2, d3[0], d3[1], d3[2], l3);
         A.grad_lap(3, d4[0], d4[1], d4[2], l4);
         const T Yr[3] = {c.ryw * Y2, c.ryw * Y3, c.ryw * Y4};  // (g'/g) Y_i
+        // W^3 and Y act alike on (phi_1, phi_2) and oppositely on (phi_3, phi_4)
+        T Zp[3], Zm[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            Zp[i] = W[2][i] + Yr[i];
+            Zm[i] = W[2][i] - Yr[i];
+        }
         T D1[3], D2[3], D3[3], D4[3];
 #pragma unroll
         for (int i = 0; i < 3; ++i)
-            cov_deriv_s(d1[i], d2[i], d3[i], d4[i], p1, p2, p3, p4, W[0][i], W[1][i], W[2][i], Yr[i], hgw, D1[i],
+            cov_deriv_s(d1[i], d2[i], d3[i], d4[i], p1, p2, p3, p4, W[0][i], W[1][i], Zp[i], Zm[i], hgw, D1[i],
                         D2[i], D3[i], D4[i]);
         // Higgs currents of kt_W (main_rk4.jl:415,432,449,...) and kt_Y (:563), over g and g'
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
             jW[0][i] = p1 * D4[i] - p2 * D3[i] + p3 * D2[i] - p4 * D1[i];
             jW[1][i] = -p1 * D3[i] - p2 * D4[i] + p3 * D1[i] + p4 * D2[i];
-            jW[2][i] = p1 * D2[i] - p2 * D1[i] - p3 * D4[i] + p4 * D3[i];
-            jY[i] = p1 * D2[i] - p2 * D1[i] + p3 * D4[i] - p4 * D3[i];
+            const T j12 = p1 * D2[i] - p2 * D1[i], j34 = p3 * D4[i] - p4 * D3[i];
+            jW[2][i] = j12 - j34;
+            jY[i] = j12 + j34;
         }
         if constexpr (PART == 1) {
 #pragma unroll
@@ -213,94 +245,102 @@ EWPT_ARITH void site_rates(const Acc& A, const PhysCoef<T>& c, Sink& out) {
         const T damp = c.gamh / mag;
         const T q12 = G[2] + c.ryw * S, q34 = c.ryw * S - G[2];
         T a1 = W[0][0] * d4[0] + W[0][1] * d4[1] + W[0][2] * d4[2] - W[1][0] * d3[0] - W[1][1] * d3[1] -
-               W[1][2] * d3[2] + W[2][0] * d2[0] + W[2][1] * d2[1] + W[2][2] * d2[2] + Yr[0] * d2[0] +
-               Yr[1] * d2[1] + Yr[2] * d2[2] + q12 * p2 - G[1] * p3 + G[0] * p4 - potg * p1 - damp * p1 * (p1 * pt1);
-        ktp1 = l1 + hgw * a1;
+               W[1][2] * d3[2] + Zp[0] * d2[0] + Zp[1] * d2[1] + Zp[2] * d2[2] + q12 * p2 - G[1] * p3 + G[0] * p4 -
+               potg * p1 - damp * p1 * (p1 * pt1);
         T a2 = -W[0][0] * d3[0] - W[0][1] * d3[1] - W[0][2] * d3[2] - W[1][0] * d4[0] - W[1][1] * d4[1] -
-               W[1][2] * d4[2] - W[2][0] * d1[0] - W[2][1] * d1[1] - W[2][2] * d1[2] - Yr[0] * d1[0] -
-               Yr[1] * d1[1] - Yr[2] * d1[2] - q12 * p1 - G[0] * p3 - G[1] * p4 - potg * p2 - damp * p2 * (p2 * pt2);
-        ktp2 = l2 + hgw * a2;
+               W[1][2] * d4[2] - Zp[0] * d1[0] - Zp[1] * d1[1] - Zp[2] * d1[2] - q12 * p1 - G[0] * p3 - G[1] * p4 -
+               potg * p2 - damp * p2 * (p2 * pt2);
         T a3 = W[0][0] * d2[0] + W[0][1] * d2[1] + W[0][2] * d2[2] + W[1][0] * d1[0] + W[1][1] * d1[1] +
-               W[1][2] * d1[2] - W[2][0] * d4[0] - W[2][1] * d4[1] - W[2][2] * d4[2] + Yr[0] * d4[0] +
-               Yr[1] * d4[1] + Yr[2] * d4[2] + q34 * p4 + G[1] * p1 + G[0] * p2 - potg * p3 - damp * p3 * (p3 * pt3);
-        ktp3 = l3 + hgw * a3;
+               W[1][2] * d1[2] - Zm[0] * d4[0] - Zm[1] * d4[1] - Zm[2] * d4[2] + q34 * p4 + G[1] * p1 + G[0] * p2 -
+               potg * p3 - damp * p3 * (p3 * pt3);
         T a4 = -W[0][0] * d1[0] - W[0][1] * d1[1] - W[0][2] * d1[2] + W[1][0] * d2[0] + W[1][1] * d2[1] +
-               W[1][2] * d2[2] + W[2][0] * d3[0] + W[2][1] * d3[1] + W[2][2] * d3[2] - Yr[0] * d3[0] -
-               Yr[1] * d3[1] - Yr[2] * d3[2] - q34 * p3 - G[0] * p1 + G[1] * p2 - potg * p4 - damp * p4 * (p4 * pt4);
-        ktp4 = l4 + hgw * a4;
+               W[1][2] * d2[2] + Zm[0] * d3[0] + Zm[1] * d3[1] + Zm[2] * d3[2] - q34 * p3 - G[0] * p1 + G[1] * p2 -
+               potg * p4 - damp * p4 * (p4 * pt4);
+        if constexpr (kScaled) {
+            ktp1 = c.hgw_o * (a1 + l1 * c.lap_h);
+            ktp2 = c.hgw_o * (a2 + l2 * c.lap_h);
+            ktp3 = c.hgw_o * (a3 + l3 * c.lap_h);
+            ktp4 = c.hgw_o * (a4 + l4 * c.lap_h);
+        } else {
+            ktp1 = l1 + hgw * a1;
+            ktp2 = l2 + hgw * a2;
+            ktp3 = l3 + hgw * a3;
+            ktp4 = l4 + hgw * a4;
+        }
     }
 
     // ---- SU(2) block, one colour at a time (field_strengths.jl:34-224)
-    //   kt W^a_i = lap W^a_i - d_i Gamma^a + g Q^a_i, Q accumulated over g
+    //   kt W^a_i = lap W^a_i - d_i Gamma^a + g Q^a_i, Q accumulated over g.
+    // The terms of colour b's derivatives and field strength in the other two
+    // colours share their factors W_j, so they enter as E_ij = F^b_ij - d_j W^b_i:
+    //   Q^{b-1}_i += sum_j W^{b+1}_j E_ij,   Q^{b+1}_i -= sum_j W^{b-1}_j E_ij
     T ktW[3][3];
-    T F[3][3];  // F[b][0] = F^b_xy (W_b_23), [1] = F^b_xz (W_b_24), [2] = F^b_yz (W_b_34)
+    T F[3][3];  // beta terms only: F[b][0] = F^b_xy (W_b_23), [1] = F^b_xz (W_b_24), [2] = F^b_yz (W_b_34)
     if constexpr (kSU2) {
-    T Q[3][3];
+        T Q[3][3];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        const int b = (a + 1) % 3, cc = (a + 2) % 3;
+        for (int a = 0; a < 3; ++a) {
+            const int b = (a + 1) % 3, cc = (a + 2) % 3;
 #pragma unroll
-        for (int i = 0; i < 3; ++i) Q[a][i] = jW[a][i] - W[b][i] * G[cc] + W[cc][i] * G[b];
-    }
+            for (int i = 0; i < 3; ++i) Q[a][i] = jW[a][i] - W[b][i] * G[cc] + W[cc][i] * G[b];
+        }
 #pragma unroll
-    for (int b = 0; b < 3; ++b) {
-        T dW[3][3];  // dW[i][j] = d_j W^b_i
-        if constexpr (kComp) {
-            T Gh[3], Gl[3];
-            A.grad_c(16 + b, Gh, Gl);
+        for (int b = 0; b < 3; ++b) {
+            T dW[3][3];  // dW[i][j] = d_j W^b_i
+            if constexpr (kComp) {
+                T Gh[3], Gl[3];
+                A.grad_c(16 + b, Gh, Gl);
 #pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                T lh, ll;
-                A.grad_lap_c(4 + 3 * b + i, dW[i][0], dW[i][1], dW[i][2], lh, ll);
-                Q[b][i] = Q[b][i] + A.comp_diff(lh, ll, Gh[i], Gl[i]) * c.igw;
+                for (int i = 0; i < 3; ++i) {
+                    T lh, ll;
+                    A.grad_lap_c(4 + 3 * b + i, dW[i][0], dW[i][1], dW[i][2], lh, ll);
+                    Q[b][i] = Q[b][i] + A.comp_diff(lh, ll, Gh[i], Gl[i]) * c.igw;
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    T lap;
+                    A.grad_lap(4 + 3 * b + i, dW[i][0], dW[i][1], dW[i][2], lap);
+                    Q[b][i] = Q[b][i] + lap * (kScaled ? c.lap_w : c.igw);
+                }
             }
-        } else {
+            const int b1 = (b + 1) % 3, b2 = (b + 2) % 3;
 #pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                T lap;
-                A.grad_lap(4 + 3 * b + i, dW[i][0], dW[i][1], dW[i][2], lap);
-                Q[b][i] = Q[b][i] + lap * c.igw;
+            for (int i = 0; i < 3; ++i) {  // E_ii = -d_i W^b_i
+                Q[b2][i] = Q[b2][i] - W[b1][i] * dW[i][i];
+                Q[b1][i] = Q[b1][i] + W[b2][i] * dW[i][i];
+            }
+#pragma unroll
+            for (int m = 0; m < 3; ++m) {
+                const int i = m == 2 ? 1 : 0, j = m == 0 ? 1 : 2;
+                const T Fij = dW[j][i] - dW[i][j] + gw_d * (W[b1][i] * W[b2][j] - W[b1][j] * W[b2][i]);
+                if (BETA) F[b][m] = Fij;
+                const T Eij = Fij - dW[i][j], mEji = Fij + dW[j][i];  // E_ij and -E_ji
+                Q[b2][i] = Q[b2][i] + W[b1][j] * Eij;
+                Q[b1][i] = Q[b1][i] - W[b2][j] * Eij;
+                Q[b2][j] = Q[b2][j] - W[b1][i] * mEji;
+                Q[b1][j] = Q[b1][j] + W[b2][i] * mEji;
             }
         }
-        const int b1 = (b + 1) % 3, b2 = (b + 2) % 3;
-        F[b][0] = dW[1][0] - dW[0][1] + gw * (W[b1][0] * W[b2][1] - W[b1][1] * W[b2][0]);
-        F[b][1] = dW[2][0] - dW[0][2] + gw * (W[b1][0] * W[b2][2] - W[b1][2] * W[b2][0]);
-        F[b][2] = dW[2][1] - dW[1][2] + gw * (W[b1][1] * W[b2][2] - W[b1][2] * W[b2][1]);
-        // d_j W^b_i enters Q^{b-1}_i with -W^{b+1}_j and Q^{b+1}_i with +W^{b-1}_j
+        // the coupling and the auxiliary gradient
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            Q[b2][i] = Q[b2][i] - dW[i][0] * W[b1][0] - dW[i][1] * W[b1][1] - dW[i][2] * W[b1][2];
-            Q[b1][i] = Q[b1][i] + dW[i][0] * W[b2][0] + dW[i][1] * W[b2][1] + dW[i][2] * W[b2][2];
+        for (int a = 0; a < 3; ++a) {
+            if constexpr (kComp) {  // the gradient is in Q already
+#pragma unroll
+                for (int i = 0; i < 3; ++i) ktW[a][i] = c.gw * Q[a][i];
+            } else {
+                T g[3];
+                A.grad(16 + a, g[0], g[1], g[2]);
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    if constexpr (kScaled)
+                        ktW[a][i] = c.gw_o * (Q[a][i] - g[i] * c.igw);
+                    else
+                        ktW[a][i] = c.gw * Q[a][i] - g[i];
+                }
+            }
         }
     }
-    // -sum_j (W^b_j F^c_ij - W^c_j F^b_ij) with F_ij antisymmetric
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        const int b = (a + 1) % 3, cc = (a + 2) % 3;
-        // i = x: j = y (F_xy), z (F_xz)
-        Q[a][0] = Q[a][0] - W[b][1] * F[cc][0] + W[cc][1] * F[b][0] - W[b][2] * F[cc][1] + W[cc][2] * F[b][1];
-        // i = y: j = x (F_yx = -F_xy), z (F_yz)
-        Q[a][1] = Q[a][1] - W[cc][0] * F[b][0] + W[b][0] * F[cc][0] - W[b][2] * F[cc][2] + W[cc][2] * F[b][2];
-        // i = z: j = x (F_zx = -F_xz), y (F_zy = -F_yz)
-        Q[a][2] = Q[a][2] - W[cc][0] * F[b][1] + W[b][0] * F[cc][1] - W[cc][1] * F[b][2] + W[b][1] * F[cc][2];
-    }
-    // the coupling and the auxiliary gradient
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        if constexpr (kComp) {  // the gradient is in Q already
-            ktW[a][0] = gw * Q[a][0];
-            ktW[a][1] = gw * Q[a][1];
-            ktW[a][2] = gw * Q[a][2];
-        } else {
-            T gx, gy_, gz;
-            A.grad(16 + a, gx, gy_, gz);
-            ktW[a][0] = gw * Q[a][0] - gx;
-            ktW[a][1] = gw * Q[a][1] - gy_;
-            ktW[a][2] = gw * Q[a][2] - gz;
-        }
-    }
-
-    }  // SU(2) block
 
     // ---- U(1) block (field_strengths.jl:281-311, main_rk4.jl:562-581)
     T ktY[3], FY[3];
@@ -323,15 +363,18 @@ EWPT_ARITH void site_rates(const Acc& A, const PhysCoef<T>& c, Sink& out) {
         FY[1] = dY[2][0] - dY[0][2];
         FY[2] = dY[2][1] - dY[1][2];
         if constexpr (kComp) {
-            ktY[0] = lap[0] + gy * jY[0];
-            ktY[1] = lap[1] + gy * jY[1];
-            ktY[2] = lap[2] + gy * jY[2];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) ktY[i] = lap[i] + c.gy * jY[i];
         } else {
-            T gx, gy_, gz;
-            A.grad(19, gx, gy_, gz);
-            ktY[0] = lap[0] + gy * jY[0] - gx;
-            ktY[1] = lap[1] + gy * jY[1] - gy_;
-            ktY[2] = lap[2] + gy * jY[2] - gz;
+            T g[3];
+            A.grad(19, g[0], g[1], g[2]);
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                if constexpr (kScaled)
+                    ktY[i] = c.lap_y * lap[i] + c.gy_o * jY[i] - c.t * g[i];
+                else
+                    ktY[i] = lap[i] + c.gy * jY[i] - g[i];
+            }
         }
     }
 
