@@ -34,7 +34,7 @@ struct ewpt_ens {
     std::vector<ewpt_params> mp;
     std::vector<ewpt_ctx*> mem;      // one FP32-form context per member
     std::vector<double> jex, gam;    // per-member drive (default 0, 0)
-    Tiling tile{16, 8, 2, 0};
+    Tiling tile{16, 8, 2, 0, 1};
     bool dirty = true;               // the step graph must be captured again
     cudaEvent_t fork = nullptr;
     std::vector<cudaEvent_t> join;
@@ -71,10 +71,10 @@ static int ens_capture(ewpt_ens* e) {
             ewpt_ctx* c = e->mem[m];
             le = cudaStreamWaitEvent(c->st, e->fork, 0);
             if (le == cudaSuccess)
-                le = c->tile.pair ? launch_step_fp32_pair(c->g, c->lay, c->tile, c->y32, c->w32, c->p, e->jex[m],
-                                                          e->gam[m], c->st)
-                                  : launch_step_fp32(c->g, c->lay, c->tile, c->y32, c->w32, c->p, e->jex[m],
-                                                     e->gam[m], c->st);
+                le = fp32_pairs(c->g, c->tile) ? launch_step_fp32_pair(c->g, c->lay, c->tile, c->y32, c->w32, c->p,
+                                                                       e->jex[m], e->gam[m], c->st)
+                                               : launch_step_fp32(c->g, c->lay, c->tile, c->y32, c->w32, c->p,
+                                                                  e->jex[m], e->gam[m], c->st);
             if (le == cudaSuccess) le = cudaEventRecord(e->join[m], c->st);
             if (le == cudaSuccess) le = cudaStreamWaitEvent(e->st, e->join[m], 0);
         }
@@ -109,7 +109,7 @@ int ewpt_ensemble_create(int32_t n, const ewpt_params* members, ewpt_ens** out) 
     e->mp.assign(members, members + n);
     e->jex.assign(n, 0.0);
     e->gam.assign(n, 0.0);
-    e->tile = Tiling{16, 8, 2, all_even ? 1 : 0};
+    e->tile = Tiling{16, 8, 2, all_even ? 1 : 0, 1};
     cudaError_t ce = cudaSetDevice(e->device);
     if (ce == cudaSuccess) ce = cudaStreamCreateWithFlags(&e->st, cudaStreamNonBlocking);
     if (ce == cudaSuccess) ce = cudaEventCreateWithFlags(&e->fork, cudaEventDisableTiming);

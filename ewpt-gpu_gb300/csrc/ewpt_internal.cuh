@@ -103,6 +103,33 @@ __device__ __forceinline__ void chunk_walk(int b, int nbx, int nby, int nz, int 
 }
 
 
+// Which thread of the FP32-form kernels evolves which site (or pair): tiles
+// in the order of chunk_walk, or (flat > 0: rows per chunk) the block's threads
+// along the rows of a chunk, nbx blocks per plane of a full chunk, then the
+// planes, then the chunks.
+struct Walk {
+    int nbx, nby, ycb, flat;
+    // position of this thread in rows of n; false: none
+    __device__ __forceinline__ bool site(int n, int ny, int nz, int& i, int& j, int& k) const {
+        if (flat == 0) {
+            int bx, by;
+            chunk_walk(blockIdx.x, nbx, nby, nz, ycb, bx, by, k);
+            i = bx * blockDim.x + threadIdx.x;
+            j = by * blockDim.y + threadIdx.y;
+            return i < n && j < ny;
+        }
+        const int T = blockDim.x * blockDim.y;
+        const int c = blockIdx.x / (nbx * nz), rem = blockIdx.x - c * nbx * nz;
+        const int rows = min(flat, ny - c * flat), nb = rows == flat ? nbx : (rows * n + T - 1) / T;
+        k = rem / nb;
+        const int q = (rem - k * nb) * T + threadIdx.y * blockDim.x + threadIdx.x;
+        const int r = q / n;
+        i = q - r * n;
+        j = c * flat + r;
+        return r < rows;
+    }
+};
+
 template <typename T>
 PhysCoef<T> make_phys(const ewpt_params& p, double Jex, double gam) {
     PhysCoef<T> c;
@@ -200,6 +227,40 @@ struct Tiling {
 constexpr Tiling kDefaultTiling{32, 4, 0, 0, 1};
 int tiling_max_threads(int reg);
 
+// Two sites per thread?  As the caller chose, or (t.pick) wherever the row
+// allows and the lattice has more sites than the 384 threads per SM that run
+// at once: 24^3 0.051 ms per step with one site and 0.068 with two, 48^3 0.123
+// and 0.111.
+inline bool fp32_pairs(const Grid& g, const Tiling& t) {
+    return g.nx % 2 == 0 && (t.pair || (t.pick && g.S > 152 * 384));
+}
+
+// Launch of the FP32-form kernels over rows of n threads (sites or pairs).
+// The caller's tile, or (t.pick) 64 x 2 threads.  A tile that leaves more than
+// an eighth of its lanes without a site is laid along the rows instead
+// (Walk::flat), paired kernel, ms per step: 160^3 (80 pairs a row) 2.30 against
+// 2.96 for 64 x 2 and 2.43 for 16 x 8 tiles, 96^3 0.594 against 0.606 for
+// 16 x 8, 48^3 0.111 against 0.116 for 8 x 16.
+inline Walk fp32_walk(int n, int ny, int nz, const Tiling& t, dim3& gr, dim3& bl) {
+    Walk w{};
+    int bx = t.bx, by = t.by;
+    if (t.pick) bx = 64, by = 2;
+    const int64_t padded = (int64_t)((n + bx - 1) / bx * bx) * ((ny + by - 1) / by * by);
+    bl = dim3(bx, by);
+    if (8 * padded > 9 * (int64_t)n * ny) {
+        const int T = bx * by, rows = ny < kChunkRows ? ny : kChunkRows, full = ny / rows, last = ny - full * rows;
+        w.flat = rows;
+        w.nbx = (rows * n + T - 1) / T;
+        gr = dim3((unsigned)(full * w.nbx + (last * n + T - 1) / T) * (unsigned)nz);
+        return w;
+    }
+    w.nbx = (n + bx - 1) / bx;
+    w.nby = (ny + by - 1) / by;
+    w.ycb = kChunkRows / by > 1 ? kChunkRows / by : 1;
+    gr = dim3((unsigned)(w.nbx * w.nby) * (unsigned)nz);
+    return w;
+}
+
 cudaError_t launch_step_fp64(const Grid& g, const Tiling& t, double* y, double* yn, double* xa, double* xb,
                              const ewpt_params& p, double Jex, double gam, cudaStream_t st);
 // One stage (1..4) of that step (z-slabs exchange ghost planes between stages).
@@ -232,6 +293,9 @@ cudaError_t launch_step_fp32_pair(const Grid& g, const Layout& L, const Tiling& 
 // Copy the face sites of all 36 arrays of a ghosted buffer into their
 // periodic images (stage.cu); the x faces only if xfaces.
 cudaError_t launch_ghost_fill(const Grid& g, const Layout& L, float* buf, cudaStream_t st, bool xfaces);
+// The y and z faces that the one-site and paired kernels read, of a buffer
+// whose arrays 20-35 may lie in another one (mom + a*P).
+cudaError_t launch_ghost_fill_yz(const Grid& g, const Layout& L, float* fld, float* mom, cudaStream_t st);
 // 36 FP64 arrays <-> FP32 hi/lo in layout L (the ghost images of hi refreshed
 // on split, the x faces only if xfaces).
 cudaError_t launch_fp32_split(const Grid& g, const Layout& L, const Ptr36& src, Fp32State dst, cudaStream_t st,

@@ -17,7 +17,8 @@
 //   stage 1:     kacc = k1;           X2 = y_hi + k1 dt/2
 //   stage 2, 3:  kacc += 2 k_s;       X3 = y_hi + k2 dt/2,  X4 = y_hi + k3 dt
 //   stage 4:     (y_hi, y_lo) += dt/6 (kacc + k4), compensated, in place
-// (X_1 is y_hi itself).  Bytes per site-update: FP64 4608, FP32 2736.
+// (X_1 is y_hi itself; kacc of the fields is not stored, see Fp32Bufs).
+// Bytes per site-update: FP64 4608, FP32 2480.
 #include <algorithm>
 
 #include "accessors.cuh"
@@ -122,12 +123,19 @@ __global__ void __launch_bounds__(RegBudget<REG>::kThreads, RegBudget<REG>::kMin
 // ------------------------------------------------------------- FP32 stage
 // All five FP32 buffers use the ghosted layout L.  After each stage the
 // ghost images of what it wrote (the next stage input, or the state high
-// part after stage 4) are refreshed by k_ghost_fill, so every stencil reads
-// its neighbours with no wrap.
+// part after stage 4) are refreshed by k_ghost_fill_yz, so every stencil
+// reads its neighbours with no wrap.
+//
+// The rate of a field (arrays 0-15) is its momentum, so k1, k2, k3 of a field
+// are the momenta of the stage inputs y_hi, X2, X3 and no rate sum is stored
+// for it: stage 4 forms k1 + 2 k2 + 2 k3 from them (the same roundings).  For
+// that X2's momenta outlive stage 3, which writes X4's (arrays 20-35) into
+// the unused arrays 0-15 of the rate sum instead of over X2's.  A step moves
+// 2480 bytes per site instead of 2736.
 struct Fp32Bufs {
     float* yhi;  // [36][P] state, high part (also the stage-1 stencil input)
     float* ylo;  // [36][P] state, low part
-    float* kacc; // [36][P] RK4-weighted rate sum: k1, then k1 + 2 k2, then k1 + 2 k2 + 2 k3
+    float* kacc; // [36][P] arrays 16-35: rate sum k1, k1 + 2 k2, k1 + 2 k2 + 2 k3; 0-15: X4's momenta
 };
 
 template <int STAGE>
@@ -135,20 +143,27 @@ struct Fp32Sink {
     const GlobalAcc<float, float>& A;
     const Layout& L;
     Fp32Bufs b;
-    float* __restrict__ xn;
+    float* xn;
     float h, w6;
+    const float *x2, *x3;  // stage 4: the inputs of stages 2 and 3
     __device__ __forceinline__ void operator()(int a, float r) const {
         const int64_t q = a * L.P + A.c;
-        if (STAGE == 1) {
-            b.kacc[q] = r;
-            xn[q] = A.v(a) + h * r;  // X1 == y_hi
-        } else if (STAGE < 4) {
+        if (STAGE < 4) {
             // kacc[q], yhi[q], ylo[q] are read and then written by this thread
             // only: the read-only path lets the loads issue ahead of stores
-            b.kacc[q] = __ldg(b.kacc + q) + 2.f * r;
-            xn[q] = __ldg(b.yhi + q) + h * r;
+            if (a >= 16) b.kacc[q] = STAGE == 1 ? r : __ldg(b.kacc + q) + 2.f * r;
+            float* x = STAGE == 3 && a >= 20 ? b.kacc - 20 * L.P : xn;  // X4's momenta
+            x[q] = (STAGE == 1 ? A.v(a) : __ldg(b.yhi + q)) + h * r;    // X1 == y_hi
         } else {
-            const float s = __ldg(b.kacc + q) + r;
+            float k;
+            if (a < 16) {
+                const int64_t m = q + 20 * L.P;
+                k = __ldg(b.yhi + m) + 2.f * __ldg(x2 + m);
+                k = k + 2.f * __ldg(x3 + m);
+            } else {
+                k = __ldg(b.kacc + q);
+            }
+            const float s = k + r;
             float hi = __ldg(b.yhi + q), lo = __ldg(b.ylo + q);
             acc_hilo(hi, lo, w6 * s);
             b.yhi[q] = hi;
@@ -160,17 +175,14 @@ struct Fp32Sink {
 template <int STAGE, bool BETA, int REG>
 __global__ void __launch_bounds__(RegBudget<REG>::kThreads, RegBudget<REG>::kMinBlocks)
     k_stage_fp32(const __grid_constant__ Grid g, const __grid_constant__ Layout L, const __grid_constant__ Ptr36 X,
-                 Fp32Bufs b, float* __restrict__ xn, PhysCoef<float> pc, StencilCoef<float> sc, float h, float w6,
-                 int nbx, int nby, int ycb) {
-    int bx, by, k;
-    chunk_walk(blockIdx.x, nbx, nby, g.nz, ycb, bx, by, k);
-    const int i = bx * blockDim.x + threadIdx.x;
-    const int j = by * blockDim.y + threadIdx.y;
-    if (i >= g.nx || j >= g.ny) return;
+                 Fp32Bufs b, float* xn, const float* x2, const float* x3, PhysCoef<float> pc, StencilCoef<float> sc,
+                 float h, float w6, Walk walk) {
+    int i, j, k;
+    if (!walk.site(g.nx, g.ny, g.nz, i, j, k)) return;
     GlobalAcc<float, float> A{{X}};
     A.place_ghost(i, j, k, g.nx, L);
     A.s = sc;
-    Fp32Sink<STAGE> out{A, L, b, xn, h, w6};
+    Fp32Sink<STAGE> out{A, L, b, xn, h, w6, x2, x3};
     site_rates<float, BETA>(A, pc, out);
 }
 
@@ -223,15 +235,15 @@ __global__ void __launch_bounds__(kConvThreads) k_join(Grid g, Layout L, const f
 // Ghost images of a ghosted buffer, one warp per work item over a grid of a
 // few blocks per SM: first the y- and z-face rows (a warp copies one row of
 // nx sites into one of the 3 + 3 ghost rows of an x-y plane, or into a row
-// of one of the 3 + 3 ghost planes), then, if asked, the x faces (a warp
-// serves 4 rows, 8 cells each: the 4 ghost cells before the row and the 4
-// after it).  The x faces cost most of the time (16-byte pieces of every
-// row, 0.86 GB of DRAM reads per launch at 256^3 with them against ~0.12 GB
-// without), so only the TMA-staged kernel, whose boxes read them, keeps
-// them; the other FP32 kernels wrap x in their neighbour offsets.  Every
+// of one of the 3 + 3 ghost planes), then the x faces (a warp serves 4 rows,
+// 8 cells each: the 4 ghost cells before the row and the 4 after it).  The x
+// faces cost most of the time (16-byte pieces of every row, 0.86 GB of DRAM
+// reads per launch at 256^3), so only the TMA-staged kernel, whose boxes read
+// them, has them filled; the other FP32 kernels wrap x in their neighbour
+// offsets and take k_ghost_fill_yz.  Every
 // cell copies the site it is the periodic image of; the box edges and
 // corners are left alone (no axis-aligned stencil reaches them).
-__global__ void __launch_bounds__(256) k_ghost_fill(Grid g, Layout L, float* __restrict__ buf, int xfaces) {
+__global__ void __launch_bounds__(256) k_ghost_fill(Grid g, Layout L, float* __restrict__ buf) {
     const int nx = g.nx, ny = g.ny, nz = g.nz;
     const int px = L.px, pxy = L.px * L.py;
     const int lane = threadIdx.x & 31;
@@ -252,7 +264,6 @@ __global__ void __launch_bounds__(256) k_ghost_fill(Grid g, Layout L, float* __r
         }
         for (int i = lane; i < nx; i += 32) arr[doff + i] = arr[soff + i];
     }
-    if (!xfaces) return;
     const int rows = ny * nz, quads = (36 * rows + 3) / 4;
     const int xg = lane & 7;
     const int di = xg < 4 ? xg - 4 : nx + xg - 4, si = xg < 4 ? nx + xg - 4 : xg - 4;
@@ -265,12 +276,39 @@ __global__ void __launch_bounds__(256) k_ghost_fill(Grid g, Layout L, float* __r
     }
 }
 
+// The same without the x faces, and only the arrays some stencil reads along
+// the face's axis: the 20 fields and, along y or z, the gauge momentum of that
+// component (the Gauss-law divergence).  One row per warp.  Array a lies at
+// fld + a*P for a < 20, at mom + a*P from 20 on.
+__global__ void __launch_bounds__(256) k_ghost_fill_yz(Grid g, Layout L, float* __restrict__ fld,
+                                                       float* __restrict__ mom) {
+    const int nx = g.nx, ny = g.ny, nz = g.nz;
+    const int px = L.px, pxy = L.px * L.py;
+    const int lane = threadIdx.x & 31;
+    int r = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
+    const int per_a = 6 * (ny + nz);
+    if (r >= 24 * per_a) return;
+    const int q = r / per_a;
+    r -= q * per_a;
+    const bool yface = r < 6 * nz;
+    if (!yface) r -= 6 * nz;
+    const int gh = r % 6, line = r / 6;
+    const int a = q < 20 ? q : 20 + 3 * (q - 19) + (yface ? 2 : 3);
+    float* arr = (a < 20 ? fld : mom) + a * L.P + L.o0;  // site (0, 0, 0)
+    const int n = yface ? ny : nz, step = yface ? px : pxy, base = line * (yface ? pxy : px);
+    const int doff = base + (gh < 3 ? gh - 3 : n + gh - 3) * step;
+    const int soff = base + (gh < 3 ? n + gh - 3 : gh - 3) * step;
+#pragma unroll 4
+    for (int i = lane; i < nx; i += 32) arr[doff + i] = arr[soff + i];
+}
+
 inline dim3 grid_of(const Grid& g, const Tiling& t) {
     return dim3((g.nx + t.bx - 1) / t.bx, (g.ny + t.by - 1) / t.by, g.nz);
 }
 
-// Launch of an FP64 kernel over nzl planes: the caller's tile, or (t.pick)
-// the shape for the lattice.
+// Launch of an FP64 kernel over nzl planes: the caller's tile (laid along
+// the sites if it left more than an eighth of its lanes without one), or
+// (t.pick) the shape for the lattice.
 //  * Tiles of 32 x 4 sites where they fit x and y to 3%, else a 1-D launch
 //    over the sites: a lane without a site costs the FP64 pipe as much as one
 //    with.
@@ -286,24 +324,17 @@ struct Shape {
 };
 Shape shape_fp64(const Grid& g, const Tiling& t, int nzl) {
     Shape s{};
-    if (!t.pick) {
+    const int64_t sites = (int64_t)g.nx * g.ny * g.nz, plane = (int64_t)g.nx * g.ny;
+    const int64_t padded = (int64_t)((g.nx + t.bx - 1) / t.bx * t.bx) * ((g.ny + t.by - 1) / t.by * t.by);
+    s.reg = !t.pick ? t.reg : sites > 152 * 8 * 32 ? 1 : 0;
+    if (t.pick ? 33 * padded <= 34 * plane && sites > 152 * 4 * 128 : 8 * padded <= 9 * plane) {
         s.gr = grid_of(g, t);
         s.gr.z = nzl;
         s.bl = dim3(t.bx, t.by);
-        s.reg = t.reg;
         return s;
     }
-    const int64_t sites = (int64_t)g.nx * g.ny * g.nz;
-    const int64_t padded = (int64_t)((g.nx + 31) / 32 * 32) * ((g.ny + 3) / 4 * 4);
-    s.reg = sites > 152 * 8 * 32 ? 1 : 0;
-    if (33 * padded <= 34 * (int64_t)g.nx * g.ny && sites > 152 * 4 * 128) {
-        s.gr = grid_of(g, t);
-        s.gr.z = nzl;
-        s.bl = dim3(32, 4);
-        return s;
-    }
-    const int64_t n = (int64_t)g.nx * g.ny * nzl;
-    const int b = sites > 152 * 4 * 32 ? 128 : 32;
+    const int64_t n = plane * nzl;
+    const int b = !t.pick ? t.bx * t.by : sites > 152 * 4 * 32 ? 128 : 32;
     s.flat = (int)n;
     s.gr = dim3((unsigned)((n + b - 1) / b));
     s.bl = dim3(b);
@@ -394,28 +425,29 @@ cudaError_t launch_step_fp64(const Grid& g, const Tiling& t, double* y, double* 
 template <bool BETA, int REG>
 static void step_fp32(const Grid& g, const Layout& L, const Tiling& t, Fp32Bufs b, float* xa, float* xb,
                       const PhysCoef<float>& pc, const StencilCoef<float>& sc, double dt, cudaStream_t st) {
-    const int nbx = (g.nx + t.bx - 1) / t.bx, nby = (g.ny + t.by - 1) / t.by;
-    const int ycb = std::max(1, kChunkRows / t.by);
-    const dim3 gr(nbx * nby * g.nz), bl(t.bx, t.by);
+    dim3 gr, bl;
+    const Walk walk = fp32_walk(g.nx, g.ny, g.nz, t, gr, bl);
     const float h2 = (float)(dt / 2.), h1 = (float)dt, w6 = (float)(dt / 6.);
-#define EWPT_WALK nbx, nby, ycb
-    k_stage_fp32<1, BETA, REG><<<gr, bl, 0, st>>>(g, L, pack(b.yhi, L.P, 4), b, xa, pc, sc, h2, w6, EWPT_WALK);
-    launch_ghost_fill(g, L, xa, st, false);
-    k_stage_fp32<2, BETA, REG><<<gr, bl, 0, st>>>(g, L, pack(xa, L.P, 4), b, xb, pc, sc, h2, w6, EWPT_WALK);
-    launch_ghost_fill(g, L, xb, st, false);
-    k_stage_fp32<3, BETA, REG><<<gr, bl, 0, st>>>(g, L, pack(xb, L.P, 4), b, xa, pc, sc, h1, w6, EWPT_WALK);
-    launch_ghost_fill(g, L, xa, st, false);
-    k_stage_fp32<4, BETA, REG><<<gr, bl, 0, st>>>(g, L, pack(xa, L.P, 4), b, nullptr, pc, sc, 0.f, w6, EWPT_WALK);
-    launch_ghost_fill(g, L, b.yhi, st, false);
-#undef EWPT_WALK
+    float* x4m = b.kacc - 20 * L.P;  // X4's momenta
+    Ptr36 X4 = pack(xa, L.P, 4);
+    for (int a = 20; a < 36; ++a) X4.p[a] = x4m + a * L.P;
+    const float* no = nullptr;
+    k_stage_fp32<1, BETA, REG><<<gr, bl, 0, st>>>(g, L, pack(b.yhi, L.P, 4), b, xa, no, no, pc, sc, h2, w6, walk);
+    launch_ghost_fill_yz(g, L, xa, xa, st);
+    k_stage_fp32<2, BETA, REG><<<gr, bl, 0, st>>>(g, L, pack(xa, L.P, 4), b, xb, no, no, pc, sc, h2, w6, walk);
+    launch_ghost_fill_yz(g, L, xb, xb, st);
+    k_stage_fp32<3, BETA, REG><<<gr, bl, 0, st>>>(g, L, pack(xb, L.P, 4), b, xa, no, no, pc, sc, h1, w6, walk);
+    launch_ghost_fill_yz(g, L, xa, x4m, st);
+    k_stage_fp32<4, BETA, REG><<<gr, bl, 0, st>>>(g, L, X4, b, nullptr, xa, xb, pc, sc, 0.f, w6, walk);
+    launch_ghost_fill_yz(g, L, b.yhi, b.yhi, st);
 }
 
 template <bool BETA>
 static void step_fp32_r(const Grid& g, const Layout& L, const Tiling& t, Fp32Bufs b, float* xa, float* xb,
                         const PhysCoef<float>& pc, const StencilCoef<float>& sc, double dt, cudaStream_t st) {
-    if (t.reg == 1)
+    if (t.reg == 1 && !t.pick)
         step_fp32<BETA, 1>(g, L, t, b, xa, xb, pc, sc, dt, st);
-    else if (t.reg == 2)
+    else if (t.reg == 2 || t.pick)
         step_fp32<BETA, 2>(g, L, t, b, xa, xb, pc, sc, dt, st);
     else
         step_fp32<BETA, 0>(g, L, t, b, xa, xb, pc, sc, dt, st);
@@ -436,7 +468,14 @@ cudaError_t launch_step_fp32(const Grid& g, const Layout& L, const Tiling& t, Fp
 
 cudaError_t launch_ghost_fill(const Grid& g, const Layout& L, float* buf, cudaStream_t st, bool xfaces) {
     if (L.gx == 0) return cudaSuccess;
-    k_ghost_fill<<<152 * 8, 256, 0, st>>>(g, L, buf, xfaces ? 1 : 0);
+    if (!xfaces) return launch_ghost_fill_yz(g, L, buf, buf, st);
+    k_ghost_fill<<<152 * 8, 256, 0, st>>>(g, L, buf);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_ghost_fill_yz(const Grid& g, const Layout& L, float* fld, float* mom, cudaStream_t st) {
+    const int64_t rows = (int64_t)24 * 6 * (g.ny + g.nz);
+    k_ghost_fill_yz<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(g, L, fld, mom);
     return cudaGetLastError();
 }
 

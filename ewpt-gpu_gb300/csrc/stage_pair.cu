@@ -31,28 +31,36 @@ struct PairBufs {
     float* kacc;
 };
 
+// The scheme of Fp32Sink (stage.cu): no stored rate sum for the fields.
 template <int STAGE, class Acc>
 struct PairSink {
     const Acc& A;
     const Layout& L;
     PairBufs b;
-    float* __restrict__ xn;
+    float* xn;
     f2 h, w6;
+    const float *x2, *x3;  // stage 4: the inputs of stages 2 and 3
     __device__ __forceinline__ static float2* at(float* base, int64_t q) { return reinterpret_cast<float2*>(base + q); }
     __device__ __forceinline__ static float2 rd(const float* base, int64_t q) {
         return __ldg(reinterpret_cast<const float2*>(base + q));
     }
     __device__ __forceinline__ void operator()(int a, f2 r) const {
         const int64_t q = a * L.P + A.c;
-        if (STAGE == 1) {
-            *at(b.kacc, q) = r.v;
-            *at(xn, q) = (A.v(a) + h * r).v;
-        } else if (STAGE < 4) {
+        if (STAGE < 4) {
             // read then written by this thread only: read-only path is safe
-            *at(b.kacc, q) = (f2(rd(b.kacc, q)) + f2(2.f) * r).v;
-            *at(xn, q) = (f2(rd(b.yhi, q)) + h * r).v;
+            if (a >= 16) *at(b.kacc, q) = STAGE == 1 ? r.v : (f2(rd(b.kacc, q)) + f2(2.f) * r).v;
+            float* x = STAGE == 3 && a >= 20 ? b.kacc - 20 * L.P : xn;  // X4's momenta
+            *at(x, q) = ((STAGE == 1 ? A.v(a) : f2(rd(b.yhi, q))) + h * r).v;
         } else {
-            const f2 s = f2(rd(b.kacc, q)) + r;
+            f2 k;
+            if (a < 16) {
+                const int64_t m = q + 20 * L.P;
+                k = f2(rd(b.yhi, m)) + f2(2.f) * f2(rd(x2, m));
+                k = k + f2(2.f) * f2(rd(x3, m));
+            } else {
+                k = f2(rd(b.kacc, q));
+            }
+            const f2 s = k + r;
             f2 hi(rd(b.yhi, q)), lo(rd(b.ylo, q));
             acc_hilo(hi, lo, f2(w6 * s));
             *at(b.yhi, q) = hi.v;
@@ -68,14 +76,11 @@ __device__ __forceinline__ void prefetch_l2(const float* p) { asm volatile("pref
 template <int STAGE, bool BETA, int REG, bool COMP = false>
 __global__ void __launch_bounds__(PairBudget<REG>::kThreads, PairBudget<REG>::kMinBlocks)
     k_stage_fp32x2(const __grid_constant__ Grid g, const __grid_constant__ Layout L, const __grid_constant__ Ptr36 X,
-                   PairBufs b, float* __restrict__ xn, PhysCoef<f2> pc, StencilCoef<f2> sc, f2 h, f2 w6, int nbx,
-                   int nby, int ycb, StencilCoef<f2> scl) {
-    int bx, by, k;
-    chunk_walk(blockIdx.x, nbx, nby, g.nz, ycb, bx, by, k);
-    const int ip = bx * blockDim.x + threadIdx.x;  // pair index along x
-    const int j = by * blockDim.y + threadIdx.y;
+                   PairBufs b, float* xn, const float* x2, const float* x3, PhysCoef<f2> pc, StencilCoef<f2> sc,
+                   f2 h, f2 w6, Walk walk, StencilCoef<f2> scl) {
+    int ip, j, k;  // pair index along x
+    if (!walk.site(g.nx >> 1, g.ny, g.nz, ip, j, k)) return;
     const int i0 = 2 * ip;
-    if (i0 >= g.nx || j >= g.ny) return;
     PairAcc<SrcPtr36<float>, COMP> A{{X}};
     A.place_ghost(i0, j, k, g.nx, L);
     A.s = sc;
@@ -88,24 +93,32 @@ __global__ void __launch_bounds__(PairBudget<REG>::kThreads, PairBudget<REG>::kM
     // tile: 10.19 ms per step without, 9.75 with these prefetches; the stage
     // input at k+1 or k+3 instead of k+2: 9.80, at k+4: 9.91, two planes:
     // 10.02-10.15; the stage input alone (k+3): 9.96; the epilogue operands
-    // alone: 3% slower than none.  Only full warps of one row prefetch: a
-    // warp's 64 sites x 36 arrays are 72 lines of 128 bytes per buffer, two
+    // alone: 3% slower than none.  Only full warps prefetch, the lines of
+    // their lanes 0 and 16 (a warp's 64 sites where it lies in one row, its two
+    // rows of 32 in tiles 16 wide): 72 lines of 128 bytes per buffer, two
     // or three per lane.  Plane k+2 <= nz+1 lies inside the ghosted box.
-    if ((blockDim.x & 31) == 0 && i0 - 2 * (int)(threadIdx.x & 31) + 64 <= g.nx) {
-        const int lane = threadIdx.x & 31;
-        const int cw = A.c - 2 * lane;  // first site of the warp's 64-site segment
+    if (blockDim.x >= 16 && __activemask() == 0xffffffffu) {
+        const int lane = (threadIdx.y * blockDim.x + threadIdx.x) & 31;
+        const int cl = __shfl_sync(0xffffffffu, A.c, 0), cu = __shfl_sync(0xffffffffu, A.c, 16);
         const int kz = 2 * L.px * L.py;
         for (int q = lane; q < 72; q += 32) {
-            const int64_t o = (q >> 1) * L.P + cw + 32 * (q & 1);
+            const bool upper = q & 1;
+            const int64_t o = (q >> 1) * L.P + (upper ? cu : cl);
             if (STAGE > 1) {
-                prefetch_l2(b.kacc + o);
+                if (q >= 32) prefetch_l2(b.kacc + o);
                 prefetch_l2(b.yhi + o);
             }
-            if (STAGE == 4) prefetch_l2(b.ylo + o);
-            prefetch_l2(reinterpret_cast<const float*>(X.p[q >> 1]) + cw + kz + 32 * (q & 1));
+            if (STAGE == 4) {
+                prefetch_l2(b.ylo + o);
+                if (q >= 40) {
+                    prefetch_l2(x2 + o);
+                    prefetch_l2(x3 + o);
+                }
+            }
+            prefetch_l2(reinterpret_cast<const float*>(X.p[q >> 1]) + (upper ? cu : cl) + kz);
         }
     }
-    PairSink<STAGE, PairAcc<SrcPtr36<float>, COMP>> out{A, L, b, xn, h, w6};
+    PairSink<STAGE, PairAcc<SrcPtr36<float>, COMP>> out{A, L, b, xn, h, w6, x2, x3};
     site_rates<f2, BETA>(A, pc, out);
 }
 
@@ -119,21 +132,21 @@ template <bool BETA, int REG, bool COMP = false>
 void step_pair(const Grid& g, const Layout& L, const Tiling& t, PairBufs b, float* xa, float* xb,
                const PhysCoef<f2>& pc, const StencilCoef<f2>& sc, const StencilCoef<f2>& scl, double dt,
                cudaStream_t st) {
-    const int npx = g.nx / 2;
-    const int nbx = (npx + t.bx - 1) / t.bx, nby = (g.ny + t.by - 1) / t.by;
-    const int ycb = std::max(1, kChunkRows / t.by);
-    const dim3 gr(nbx * nby * g.nz), bl(t.bx, t.by);
+    dim3 gr, bl;
+    const Walk walk = fp32_walk(g.nx / 2, g.ny, g.nz, t, gr, bl);
     const f2 h2((float)(dt / 2.)), h1((float)dt), w6((float)(dt / 6.)), z(0.f);
-#define EWPT_PAIR_ARGS nbx, nby, ycb, scl
-    k_stage_fp32x2<1, BETA, REG, COMP><<<gr, bl, 0, st>>>(g, L, pack4(b.yhi, L.P), b, xa, pc, sc, h2, w6, EWPT_PAIR_ARGS);
-    launch_ghost_fill(g, L, xa, st, false);
-    k_stage_fp32x2<2, BETA, REG, COMP><<<gr, bl, 0, st>>>(g, L, pack4(xa, L.P), b, xb, pc, sc, h2, w6, EWPT_PAIR_ARGS);
-    launch_ghost_fill(g, L, xb, st, false);
-    k_stage_fp32x2<3, BETA, REG, COMP><<<gr, bl, 0, st>>>(g, L, pack4(xb, L.P), b, xa, pc, sc, h1, w6, EWPT_PAIR_ARGS);
-    launch_ghost_fill(g, L, xa, st, false);
-    k_stage_fp32x2<4, BETA, REG, COMP><<<gr, bl, 0, st>>>(g, L, pack4(xa, L.P), b, nullptr, pc, sc, z, w6, EWPT_PAIR_ARGS);
-    launch_ghost_fill(g, L, b.yhi, st, false);
-#undef EWPT_PAIR_ARGS
+    float* x4m = b.kacc - 20 * L.P;  // X4's momenta
+    Ptr36 X4 = pack4(xa, L.P);
+    for (int a = 20; a < 36; ++a) X4.p[a] = x4m + a * L.P;
+    const float* no = nullptr;
+    k_stage_fp32x2<1, BETA, REG, COMP><<<gr, bl, 0, st>>>(g, L, pack4(b.yhi, L.P), b, xa, no, no, pc, sc, h2, w6, walk, scl);
+    launch_ghost_fill_yz(g, L, xa, xa, st);
+    k_stage_fp32x2<2, BETA, REG, COMP><<<gr, bl, 0, st>>>(g, L, pack4(xa, L.P), b, xb, no, no, pc, sc, h2, w6, walk, scl);
+    launch_ghost_fill_yz(g, L, xb, xb, st);
+    k_stage_fp32x2<3, BETA, REG, COMP><<<gr, bl, 0, st>>>(g, L, pack4(xb, L.P), b, xa, no, no, pc, sc, h1, w6, walk, scl);
+    launch_ghost_fill_yz(g, L, xa, x4m, st);
+    k_stage_fp32x2<4, BETA, REG, COMP><<<gr, bl, 0, st>>>(g, L, X4, b, nullptr, xa, xb, pc, sc, z, w6, walk, scl);
+    launch_ghost_fill_yz(g, L, b.yhi, b.yhi, st);
 }
 
 template <bool BETA>
@@ -142,9 +155,9 @@ void step_pair_r(const Grid& g, const Layout& L, const Tiling& t, PairBufs b, fl
                  double dt, cudaStream_t st) {
     if (comp)  // one register budget (<= 168) for the compensated mode
         step_pair<BETA, 2, true>(g, L, t, b, xa, xb, pc, sc, scl, dt, st);
-    else if (t.reg == 1)
+    else if (t.reg == 1 && !t.pick)
         step_pair<BETA, 1>(g, L, t, b, xa, xb, pc, sc, scl, dt, st);
-    else if (t.reg == 2)
+    else if (t.reg == 2 || t.pick)
         step_pair<BETA, 2>(g, L, t, b, xa, xb, pc, sc, scl, dt, st);
     else
         step_pair<BETA, 0>(g, L, t, b, xa, xb, pc, sc, scl, dt, st);
