@@ -10,6 +10,7 @@
 #include <cmath>
 
 #include "ewpt_ctx.cuh"
+#include "fixstencil.cuh"
 #include "stencil_n.cuh"
 
 namespace {
@@ -20,6 +21,7 @@ struct DiagCoef {
     double gw, gy, hgw, hgy, lambda, vev2, sw, cw, bcoef;  // bcoef = 4 sin(th)/(gw vev^2)
     double four_sw_gw;                                      // 4 sin(th)/gw (B_2)
     double a[6];                                            // first-derivative weights / dx (radius R)
+    double t;  // what a derivative of the accessor is multiplied by: 1, or 1 / (60 dx) (FixDiff)
 };
 
 // Neighbour access on an FP64 [36][S] buffer, stencil radius R.
@@ -38,9 +40,25 @@ struct DAcc {
         for (int d = 1; d < R; ++d) r = r + a[d] * (ld(q, o[d]) - ld(q, o[R + d]));
         return r;
     }
-    __device__ __forceinline__ double dx(int a) const { return d1(a, ox); }
-    __device__ __forceinline__ double dy(int a) const { return d1(a, oy); }
-    __device__ __forceinline__ double dz(int a) const { return d1(a, oz); }
+    __device__ __forceinline__ const int* off(int ax) const { return ax == 0 ? ox : (ax == 1 ? oy : oz); }
+    __device__ __forceinline__ void grad(int q, double& gx, double& gy, double& gz) const {
+        gx = d1(q, ox);
+        gy = d1(q, oy);
+        gz = d1(q, oz);
+    }
+    __device__ __forceinline__ double curl(int q, int ax, int r, int bx) const {
+        return d1(q, off(ax)) - d1(r, off(bx));
+    }
+    __device__ __forceinline__ double div(int q) const { return d1(q, ox) + d1(q + 1, oy) + d1(q + 2, oz); }
+};
+// the accessor of a stencil radius: the 6th order on the integer pipes
+template <int R>
+struct DiagAcc {
+    using type = DAcc<R>;
+};
+template <>
+struct DiagAcc<3> {
+    using type = FixDiff;
 };
 
 // All snapshot densities of one site.
@@ -59,19 +77,17 @@ __device__ __forceinline__ void site_diag(const DA& A, const DiagCoef& k, SiteDi
     const double W32 = A.v(10), W33 = A.v(11), W34 = A.v(12);
     const double Y2 = A.v(13), Y3 = A.v(14), Y4 = A.v(15);
     const double t1 = A.v(20), t2 = A.v(21), t3 = A.v(22), t4 = A.v(23);
-    const double gw = k.gw, gy = k.gy;
+    const double gw = k.gw, gy = k.gy, t = k.t;
     double D[3][4];
     {
         const double W1[3] = {W12, W13, W14}, W2[3] = {W22, W23, W24}, W3[3] = {W32, W33, W34}, Y[3] = {Y2, Y3, Y4};
+        double d[4][3];
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            const double d1 = i == 0 ? A.dx(0) : (i == 1 ? A.dy(0) : A.dz(0));
-            const double d2 = i == 0 ? A.dx(1) : (i == 1 ? A.dy(1) : A.dz(1));
-            const double d3 = i == 0 ? A.dx(2) : (i == 1 ? A.dy(2) : A.dz(2));
-            const double d4 = i == 0 ? A.dx(3) : (i == 1 ? A.dy(3) : A.dz(3));
-            cov_deriv(d1, d2, d3, d4, p1, p2, p3, p4, W1[i], W2[i], W3[i], Y[i], k.hgw, k.hgy, D[i][0], D[i][1],
-                      D[i][2], D[i][3]);
-        }
+        for (int a = 0; a < 4; ++a) A.grad(a, d[a][0], d[a][1], d[a][2]);
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+            cov_deriv(t * d[0][i], t * d[1][i], t * d[2][i], t * d[3][i], p1, p2, p3, p4, W1[i], W2[i], W3[i], Y[i],
+                      k.hgw, k.hgy, D[i][0], D[i][1], D[i][2], D[i][3]);
     }
     const double mag = p1 * p1 + p2 * p2 + p3 * p3 + p4 * p4;
     const double dev = mag - k.vev2;
@@ -85,22 +101,22 @@ __device__ __forceinline__ void site_diag(const DA& A, const DiagCoef& k, SiteDi
 #pragma unroll
     for (int a = 24; a < 33; ++a) eew += A.v(a) * A.v(a);
     o.eew = 0.5 * eew;
-    const double F1_23 = A.dx(5) - A.dy(4) + gw * (W22 * W33 - W23 * W32);
-    const double F1_24 = A.dx(6) - A.dz(4) + gw * (W22 * W34 - W24 * W32);
-    const double F1_34 = A.dy(6) - A.dz(5) + gw * (W23 * W34 - W24 * W33);
-    const double F2_23 = A.dx(8) - A.dy(7) + gw * (W32 * W13 - W33 * W12);
-    const double F2_24 = A.dx(9) - A.dz(7) + gw * (W32 * W14 - W34 * W12);
-    const double F2_34 = A.dy(9) - A.dz(8) + gw * (W33 * W14 - W34 * W13);
-    const double F3_23 = A.dx(11) - A.dy(10) + gw * (W12 * W23 - W13 * W22);
-    const double F3_24 = A.dx(12) - A.dz(10) + gw * (W12 * W24 - W14 * W22);
-    const double F3_34 = A.dy(12) - A.dz(11) + gw * (W13 * W24 - W14 * W23);
+    const double F1_23 = t * A.curl(5, 0, 4, 1) + gw * (W22 * W33 - W23 * W32);
+    const double F1_24 = t * A.curl(6, 0, 4, 2) + gw * (W22 * W34 - W24 * W32);
+    const double F1_34 = t * A.curl(6, 1, 5, 2) + gw * (W23 * W34 - W24 * W33);
+    const double F2_23 = t * A.curl(8, 0, 7, 1) + gw * (W32 * W13 - W33 * W12);
+    const double F2_24 = t * A.curl(9, 0, 7, 2) + gw * (W32 * W14 - W34 * W12);
+    const double F2_34 = t * A.curl(9, 1, 8, 2) + gw * (W33 * W14 - W34 * W13);
+    const double F3_23 = t * A.curl(11, 0, 10, 1) + gw * (W12 * W23 - W13 * W22);
+    const double F3_24 = t * A.curl(12, 0, 10, 2) + gw * (W12 * W24 - W14 * W22);
+    const double F3_34 = t * A.curl(12, 1, 11, 2) + gw * (W13 * W24 - W14 * W23);
     o.mew = 0.5 * (F1_23 * F1_23 + F1_24 * F1_24 + F1_34 * F1_34 + F2_23 * F2_23 + F2_24 * F2_24 +
                    F2_34 * F2_34 + F3_23 * F3_23 + F3_24 * F3_24 + F3_34 * F3_34);   // compute_MEW! :1978
     const double Yt2 = A.v(33), Yt3 = A.v(34), Yt4 = A.v(35);
     o.eey = 0.5 * (Yt2 * Yt2 + Yt3 * Yt3 + Yt4 * Yt4);             // compute_EEY! :2139
-    const double Y_23 = A.dx(14) - A.dy(13);
-    const double Y_24 = A.dx(15) - A.dz(13);
-    const double Y_34 = A.dy(15) - A.dz(14);
+    const double Y_23 = t * A.curl(14, 0, 13, 1);
+    const double Y_24 = t * A.curl(15, 0, 13, 2);
+    const double Y_34 = t * A.curl(15, 1, 14, 2);
     o.mey = 0.5 * (Y_23 * Y_23 + Y_24 * Y_24 + Y_34 * Y_34);       // compute_MEY! :2298
 
     // EM fields: n^a = Phi^dag sigma^a Phi / |Phi|^2 (main_rk4.jl:2455-2467)
@@ -144,19 +160,28 @@ __device__ __forceinline__ void site_diag(const DA& A, const DiagCoef& k, SiteDi
     const double q3 = gw * (-(W12 * Wt22 - W22 * Wt12) - (W13 * Wt23 - W23 * Wt13) - (W14 * Wt24 - W24 * Wt14)) +
                       gw * (p1 * t2 - p2 * t1 + p4 * t3 - p3 * t4);
     const double qY = gy * (p1 * t2 - p2 * t1 + p3 * t4 - p4 * t3);
-    o.gw1 = (A.dx(24) + A.dy(25) + A.dz(26)) - q1;
-    o.gw2 = (A.dx(27) + A.dy(28) + A.dz(29)) - q2;
-    o.gw3 = (A.dx(30) + A.dy(31) + A.dz(32)) - q3;
-    o.gy_ = (A.dx(33) + A.dy(34) + A.dz(35)) - qY;
-    o.cw1 = A.v(16) - (A.dx(4) + A.dy(5) + A.dz(6));
-    o.cw2 = A.v(17) - (A.dx(7) + A.dy(8) + A.dz(9));
-    o.cw3 = A.v(18) - (A.dx(10) + A.dy(11) + A.dz(12));
-    o.cy = A.v(19) - (A.dx(13) + A.dy(14) + A.dz(15));
+    o.gw1 = t * A.div(24) - q1;
+    o.gw2 = t * A.div(27) - q2;
+    o.gw3 = t * A.div(30) - q3;
+    o.gy_ = t * A.div(33) - qY;
+    o.cw1 = A.v(16) - t * A.div(4);
+    o.cw2 = A.v(17) - t * A.div(7);
+    o.cw3 = A.v(18) - t * A.div(10);
+    o.cy = A.v(19) - t * A.div(13);
 }
 
 // Reduction slots
 enum { R_PE = 0, R_KE, R_GE, R_EEW, R_MEW, R_EEY, R_MEY, R_BX, R_BY, R_BZ, R_B2X, R_B2Y, R_B2Z,
        R_MOD, R_HEL, R_GW, R_GY, R_CW, R_CY, NSUM, R_MIN = NSUM, R_MAXGW, R_MAXGY, NRED };
+
+__device__ __forceinline__ double fold(int q, double v, double u) {
+    return q < NSUM ? v + u : (q == R_MIN ? fmin(v, u) : fmax(v, u));
+}
+__device__ __forceinline__ double fold_warp(int q, double v) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v = fold(q, v, __shfl_down_sync(0xffffffffu, v, off));
+    return v;
+}
 
 template <int R>
 __device__ __forceinline__ void make_dacc(const Grid& g, const double* y, const DiagCoef& kc, int i, int j, int k,
@@ -171,115 +196,96 @@ __device__ __forceinline__ void make_dacc(const Grid& g, const double* y, const 
     for (int d = 0; d < R; ++d) A.a[d] = kc.a[d];
 }
 
-template <int R>
-__global__ void __launch_bounds__(DT) k_diag_partial(Grid g, const double* __restrict__ y, DiagCoef kc,
-                                                     double* __restrict__ part) {
-    double acc[NRED];
+__device__ __forceinline__ void make_dacc(const Grid& g, const double* y, const DiagCoef& kc, int i, int j, int k,
+                                          FixDiff& A) {
+    A.y = y;
+    A.S = g.S;
+    A.c = i + g.nx * (j + g.ny * k);
+    axis_offsets(i, g.nx, 1, A.o[0]);
+    axis_offsets(j, g.ny, g.nx, A.o[1]);
+    axis_offsets(k, g.nz, g.nx * g.ny, A.o[2]);
 #pragma unroll
-    for (int q = 0; q < NSUM; ++q) acc[q] = 0.0;
-    acc[R_MIN] = INFINITY;
-    acc[R_MAXGW] = 0.0;
-    acc[R_MAXGY] = 0.0;
+    for (int d = 0; d < 3; ++d) A.s[d] = kc.a[d];
+    A.T = 1.0 / kc.t;
+}
+
+template <int R>
+__global__ void __launch_bounds__(DT, R == 3 ? 3 : 1) k_diag_partial(Grid g, const double* __restrict__ y, DiagCoef kc,
+                                                     double* __restrict__ part) {
+    // the sums of each thread live in shared memory: 22 doubles less per
+    // thread in registers during the stencils
+    __shared__ double acc[NRED][DT];
+    const int t = threadIdx.y * DX_ + threadIdx.x;
+#pragma unroll
+    for (int q = 0; q < NRED; ++q) acc[q][t] = q == R_MIN ? (double)INFINITY : 0.0;
     const int i = blockIdx.x * DX_ + threadIdx.x;
     const int j = blockIdx.y * DY_ + threadIdx.y;
     if (i < g.nx && j < g.ny) {
         for (int k = blockIdx.z; k < g.nz; k += gridDim.z) {
-            DAcc<R> A;
-            make_dacc<R>(g, y, kc, i, j, k, A);
+            typename DiagAcc<R>::type A;
+            make_dacc(g, y, kc, i, j, k, A);
             SiteDiag o;
             site_diag(A, kc, o);
-            acc[R_PE] += o.pe;
-            acc[R_KE] += o.ke;
-            acc[R_GE] += o.ge;
-            acc[R_EEW] += o.eew;
-            acc[R_MEW] += o.mew;
-            acc[R_EEY] += o.eey;
-            acc[R_MEY] += o.mey;
-            acc[R_BX] += o.bx * o.bx;
-            acc[R_BY] += o.by * o.by;
-            acc[R_BZ] += o.bz * o.bz;
-            acc[R_B2X] += o.b2x * o.b2x;
-            acc[R_B2Y] += o.b2y * o.b2y;
-            acc[R_B2Z] += o.b2z * o.b2z;
-            acc[R_MOD] += o.modphi;
-            acc[R_HEL] += o.b2x * o.ax + o.b2y * o.ay + o.b2z * o.az;
-            acc[R_GW] += o.gw1 * o.gw1 + o.gw2 * o.gw2 + o.gw3 * o.gw3;
-            acc[R_GY] += o.gy_ * o.gy_;
-            acc[R_CW] += o.cw1 * o.cw1 + o.cw2 * o.cw2 + o.cw3 * o.cw3;
-            acc[R_CY] += o.cy * o.cy;
-            acc[R_MIN] = fmin(acc[R_MIN], o.modphi);
-            acc[R_MAXGW] = fmax(acc[R_MAXGW], fmax(fabs(o.gw1), fmax(fabs(o.gw2), fabs(o.gw3))));
-            acc[R_MAXGY] = fmax(acc[R_MAXGY], fabs(o.gy_));
+            acc[R_PE][t] += o.pe;
+            acc[R_KE][t] += o.ke;
+            acc[R_GE][t] += o.ge;
+            acc[R_EEW][t] += o.eew;
+            acc[R_MEW][t] += o.mew;
+            acc[R_EEY][t] += o.eey;
+            acc[R_MEY][t] += o.mey;
+            acc[R_BX][t] += o.bx * o.bx;
+            acc[R_BY][t] += o.by * o.by;
+            acc[R_BZ][t] += o.bz * o.bz;
+            acc[R_B2X][t] += o.b2x * o.b2x;
+            acc[R_B2Y][t] += o.b2y * o.b2y;
+            acc[R_B2Z][t] += o.b2z * o.b2z;
+            acc[R_MOD][t] += o.modphi;
+            acc[R_HEL][t] += o.b2x * o.ax + o.b2y * o.ay + o.b2z * o.az;
+            acc[R_GW][t] += o.gw1 * o.gw1 + o.gw2 * o.gw2 + o.gw3 * o.gw3;
+            acc[R_GY][t] += o.gy_ * o.gy_;
+            acc[R_CW][t] += o.cw1 * o.cw1 + o.cw2 * o.cw2 + o.cw3 * o.cw3;
+            acc[R_CY][t] += o.cy * o.cy;
+            acc[R_MIN][t] = fmin(acc[R_MIN][t], o.modphi);
+            acc[R_MAXGW][t] = fmax(acc[R_MAXGW][t], fmax(fabs(o.gw1), fmax(fabs(o.gw2), fabs(o.gw3))));
+            acc[R_MAXGY][t] = fmax(acc[R_MAXGY][t], fabs(o.gy_));
         }
     }
-    // warp shuffle reduction
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-#pragma unroll
-        for (int q = 0; q < NSUM; ++q) acc[q] += __shfl_down_sync(0xffffffffu, acc[q], off);
-        acc[R_MIN] = fmin(acc[R_MIN], __shfl_down_sync(0xffffffffu, acc[R_MIN], off));
-        acc[R_MAXGW] = fmax(acc[R_MAXGW], __shfl_down_sync(0xffffffffu, acc[R_MAXGW], off));
-        acc[R_MAXGY] = fmax(acc[R_MAXGY], __shfl_down_sync(0xffffffffu, acc[R_MAXGY], off));
-    }
-    __shared__ double sh[DT / 32][NRED];
-    const int lane = threadIdx.x & 31, warp = (threadIdx.y * DX_ + threadIdx.x) >> 5;
-    if (lane == 0)
-#pragma unroll
-        for (int q = 0; q < NRED; ++q) sh[warp][q] = acc[q];
     __syncthreads();
-    const int t = threadIdx.y * DX_ + threadIdx.x;
-    if (t < NRED) {
-        double v = sh[0][t];
-        for (int w = 1; w < DT / 32; ++w) {
-            const double u = sh[w][t];
-            v = t < NSUM ? v + u : (t == R_MIN ? fmin(v, u) : fmax(v, u));
-        }
-        const int64_t b = blockIdx.x + (int64_t)gridDim.x * (blockIdx.y + (int64_t)gridDim.y * blockIdx.z);
-        part[b * NRED + t] = v;
+    // one warp per slot: four values per lane, then a shuffle reduction
+    const int64_t b = blockIdx.x + (int64_t)gridDim.x * (blockIdx.y + (int64_t)gridDim.y * blockIdx.z);
+    for (int q = threadIdx.y; q < NRED; q += DT / 32) {
+        double v = acc[q][threadIdx.x];
+        for (int w = 1; w < DT / 32; ++w) v = fold(q, v, acc[q][threadIdx.x + 32 * w]);
+        v = fold_warp(q, v);
+        if (threadIdx.x == 0) part[b * NRED + q] = v;
     }
 }
 
-__global__ void k_diag_final(const double* __restrict__ part, int nb, double* __restrict__ out) {
-    __shared__ double sh[256];
-    for (int q = 0; q < NRED; ++q) {
-        double v = q < NSUM ? 0.0 : (q == R_MIN ? INFINITY : 0.0);
-        for (int b = threadIdx.x; b < nb; b += blockDim.x) {
-            const double u = part[(int64_t)b * NRED + q];
-            v = q < NSUM ? v + u : (q == R_MIN ? fmin(v, u) : fmax(v, u));
-        }
-        sh[threadIdx.x] = v;
-        __syncthreads();
-        for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-            if (threadIdx.x < s) {
-                const double u = sh[threadIdx.x + s];
-                double& w = sh[threadIdx.x];
-                w = q < NSUM ? w + u : (q == R_MIN ? fmin(w, u) : fmax(w, u));
-            }
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) out[q] = sh[0];
-        __syncthreads();
-    }
+// One warp per slot folds the partial rows (one block of NRED warps).
+__global__ void __launch_bounds__(32 * NRED) k_diag_final(const double* __restrict__ part, int nb,
+                                                          double* __restrict__ out) {
+    const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double v = q == R_MIN ? (double)INFINITY : 0.0;
+#pragma unroll 8
+    for (int b = lane; b < nb; b += 32) v = fold(q, v, part[(int64_t)b * NRED + q]);
+    v = fold_warp(q, v);
+    if (lane == 0) out[q] = v;
 }
 
 // Writes one real field per component: which = 0 -> B (compute_Bx/By/Bz!),
 // 1 -> B_2 (compute_B_2_*!), 2 -> Higgs phi_1..4, 3 -> the seven energy
 // densities (compute_PE! .. compute_MEY!).
-template <int R>
-__global__ void __launch_bounds__(DT) k_fields(Grid g, const double* __restrict__ y, DiagCoef kc, int which,
-                                               double* __restrict__ f) {
+// A kernel per field: what the others alone need is not computed.
+template <int R, int which>
+__global__ void __launch_bounds__(DT, R == 3 && which != 2 ? 3 : 1) k_fields(Grid g, const double* __restrict__ y,
+                                                                             DiagCoef kc, double* __restrict__ f) {
     const int i = blockIdx.x * DX_ + threadIdx.x;
     const int j = blockIdx.y * DY_ + threadIdx.y;
     if (i >= g.nx || j >= g.ny) return;
     for (int k = blockIdx.z; k < g.nz; k += gridDim.z) {
         const int64_t c = i + (int64_t)g.nx * (j + (int64_t)g.ny * k);
-        if (which == 2) {
-#pragma unroll
-            for (int a = 0; a < 4; ++a) f[a * g.S + c] = y[a * g.S + c];
-            continue;
-        }
-        DAcc<R> A;
-        make_dacc<R>(g, y, kc, i, j, k, A);
+        typename DiagAcc<R>::type A;
+        make_dacc(g, y, kc, i, j, k, A);
         SiteDiag o;
         site_diag(A, kc, o);
         if (which == 3) {
@@ -308,6 +314,7 @@ DiagCoef diag_coef(const ewpt_params& p) {
     k.four_sw_gw = 4. * k.sw / p.gw;
     const int R = stencil_radius(p.stencil_order);
     for (int d = 0; d < 6; ++d) k.a[d] = 0.0;
+    k.t = 1.0;
     switch (R) {
         case 1: { const auto s = make_stencil_n<double, 1>(p.dx); for (int d = 0; d < 1; ++d) k.a[d] = s.a[d]; break; }
         case 4: { const auto s = make_stencil_n<double, 4>(p.dx); for (int d = 0; d < 4; ++d) k.a[d] = s.a[d]; break; }
@@ -318,6 +325,7 @@ DiagCoef diag_coef(const ewpt_params& p) {
             k.a[0] = s.a1;
             k.a[1] = s.a2;
             k.a[2] = s.a3;
+            k.t = s.a3;  // 1 / (60 dx)
         }
     }
     return k;
@@ -346,12 +354,28 @@ dim3 diag_grid(const Grid& g) {
 
 }  // namespace
 
+cudaError_t launch_fields(const Grid& g, const ewpt_params& p, const double* y, int which, double* f,
+                          cudaStream_t st);
+
 int ewpt_ensure_scratch64(ewpt_ctx* c) {
     if (c->scratch64) return EWPT_OK;
     return ewpt_cuda_check(c, cudaMalloc(&c->scratch64, (size_t)36 * c->g.S * 8), "scratch64");
 }
 
-int ewpt_state64(ewpt_ctx* c, const double** out) {
+int ewpt_higgs64(ewpt_ctx* c, double* out) {
+    if (c->slab || c->p.precision == EWPT_FP64) {
+        const double* y;
+        const int rc = ewpt_state64(c, &y, 4);
+        return rc ? rc : ewpt_cuda_check(c, launch_fields(c->g, c->p, y, 2, out, c->st), "higgs");
+    }
+    MPtr36 dst{};
+    for (int a = 0; a < 4; ++a) dst.p[a] = out + a * c->g.S;
+    if (c->p.precision == EWPT_DF64) return ewpt_cuda_check(c, launch_from_dd(c->g.S, c->y, dst, c->st, 4), "join");
+    const int rc = ewpt_tma_check(c);
+    return rc ? rc : ewpt_cuda_check(c, launch_fp32_join(c->g, c->lay, c->y32, dst, c->st, 4), "join");
+}
+
+int ewpt_state64(ewpt_ctx* c, const double** out, int arrays) {
     if (c->slab)
         return ewpt_fail(c, EWPT_ERR_STATE, "a slab holds part of a lattice: gather the state (ewpt_slabs_get_state)");
     if (c->p.precision == EWPT_FP64) {
@@ -361,11 +385,11 @@ int ewpt_state64(ewpt_ctx* c, const double** out) {
     int rc = ewpt_ensure_scratch64(c);
     if (rc) return rc;
     if (c->p.precision == EWPT_DF64) {
-        rc = ewpt_cuda_check(c, launch_from_dd(c->g.S, c->y, arrays36(c->scratch64, c->g.S), c->st), "join");
+        rc = ewpt_cuda_check(c, launch_from_dd(c->g.S, c->y, arrays36(c->scratch64, c->g.S), c->st, arrays), "join");
     } else {
         rc = ewpt_tma_check(c);
         if (rc) return rc;
-        rc = ewpt_cuda_check(c, launch_fp32_join(c->g, c->lay, c->y32, arrays36(c->scratch64, c->g.S), c->st), "join");
+        rc = ewpt_cuda_check(c, launch_fp32_join(c->g, c->lay, c->y32, arrays36(c->scratch64, c->g.S), c->st, arrays), "join");
     }
     if (rc) return rc;
     *out = c->scratch64;
@@ -397,7 +421,7 @@ cudaError_t launch_diag(const Grid& g, const ewpt_params& p, const double* y, do
                         cudaStream_t st) {
     const dim3 gr = diag_grid(g);
     launch_partial(stencil_radius(p.stencil_order), gr, g, y, diag_coef(p), part, st);
-    k_diag_final<<<1, 256, 0, st>>>(part, gr.x * gr.y * gr.z, dres);
+    k_diag_final<<<1, 32 * NRED, 0, st>>>(part, gr.x * gr.y * gr.z, dres);
     return cudaGetLastError();
 }
 
@@ -424,22 +448,33 @@ cudaError_t launch_diag_bounded(const Grid& g, const ewpt_params& p, const doubl
     if (bz < 1) bz = 1;
     gr.z = (unsigned)bz;
     launch_partial(stencil_radius(p.stencil_order), gr, g, y, diag_coef(p), part, st);
-    k_diag_final<<<1, 256, 0, st>>>(part, gr.x * gr.y * gr.z, dres);
+    k_diag_final<<<1, 32 * NRED, 0, st>>>(part, gr.x * gr.y * gr.z, dres);
     return cudaGetLastError();
 }
 
 void diag_finish_row(const ewpt_params& p, int64_t S, const double* r, double* out) { finish_row(p, S, r, out); }
 
+template <int R>
+static void fields_of(const Grid& g, const DiagCoef& kc, const double* y, int which, double* f, cudaStream_t st) {
+    const dim3 gr = diag_grid(g), bl(DX_, DY_);
+    switch (which) {
+        case 0: k_fields<R, 0><<<gr, bl, 0, st>>>(g, y, kc, f); break;
+        case 1: k_fields<R, 1><<<gr, bl, 0, st>>>(g, y, kc, f); break;
+        default: k_fields<R, 3><<<gr, bl, 0, st>>>(g, y, kc, f);
+    }
+}
+
 cudaError_t launch_fields(const Grid& g, const ewpt_params& p, const double* y, int which, double* f,
                           cudaStream_t st) {
-    const dim3 gr = diag_grid(g), bl(DX_, DY_);
+    if (which == 2)  // phi_1..4 as stored
+        return cudaMemcpyAsync(f, y, (size_t)4 * g.S * 8, cudaMemcpyDeviceToDevice, st);
     const DiagCoef kc = diag_coef(p);
     switch (stencil_radius(p.stencil_order)) {
-        case 1: k_fields<1><<<gr, bl, 0, st>>>(g, y, kc, which, f); break;
-        case 4: k_fields<4><<<gr, bl, 0, st>>>(g, y, kc, which, f); break;
-        case 5: k_fields<5><<<gr, bl, 0, st>>>(g, y, kc, which, f); break;
-        case 6: k_fields<6><<<gr, bl, 0, st>>>(g, y, kc, which, f); break;
-        default: k_fields<3><<<gr, bl, 0, st>>>(g, y, kc, which, f);
+        case 1: fields_of<1>(g, kc, y, which, f, st); break;
+        case 4: fields_of<4>(g, kc, y, which, f, st); break;
+        case 5: fields_of<5>(g, kc, y, which, f, st); break;
+        case 6: fields_of<6>(g, kc, y, which, f, st); break;
+        default: fields_of<3>(g, kc, y, which, f, st);
     }
     return cudaGetLastError();
 }
@@ -461,7 +496,7 @@ extern "C" int ewpt_fields(ewpt_ctx* c, int32_t field, double* out, int32_t on_d
     if (!out) return ewpt_fail(c, EWPT_ERR_ARG, "out is NULL");
     cudaSetDevice(c->p.device);
     const double* y;
-    int rc = ewpt_state64(c, &y);
+    int rc = ewpt_state64(c, &y, field == EWPT_FIELD_HIGGS ? 4 : field == EWPT_FIELD_DENSITY ? 36 : 16);
     if (rc) return rc;
     const size_t bytes = (size_t)ncomp * c->g.S * 8;
     double* f = out;

@@ -162,10 +162,10 @@ static int ens_member_check(ewpt_ens* e, int32_t m) {
     return EWPT_OK;
 }
 
-// FP64 view of member m's size holding its state (joined after the steps
-// queued on the ensemble's stream); the view's work runs on the ensemble's
-// stream too.
-static int ens_view(ewpt_ens* e, int32_t m, ewpt_ctx** out, bool join = true) {
+// FP64 view of member m's size holding the first `join` arrays of its state
+// (joined after the steps queued on the ensemble's stream); the view's work
+// runs on the ensemble's stream too.
+static int ens_view(ewpt_ens* e, int32_t m, ewpt_ctx** out, int join = 36) {
     const ewpt_params& p = e->mp[m];
     const auto key = std::make_tuple(p.nx, p.ny, p.nz);
     auto it = e->views.find(key);
@@ -184,9 +184,10 @@ static int ens_view(ewpt_ens* e, int32_t m, ewpt_ctx** out, bool join = true) {
     }
     v->p = p;  // couplings / dt / theta_w of this member
     v->p.precision = EWPT_FP64;
-    if (join) {
+    if (join > 0) {
         const ewpt_ctx* c = e->mem[m];
-        int rc = ens_cuda(e, launch_fp32_join(v->g, c->lay, c->y32, arrays36(v->y, v->g.S), e->st), "ensemble view");
+        int rc = ens_cuda(e, launch_fp32_join(v->g, c->lay, c->y32, arrays36(v->y, v->g.S), e->st, join),
+                         "ensemble view");
         if (rc) return rc;
     }
     *out = v;
@@ -203,7 +204,7 @@ int ewpt_ensemble_set_state(ewpt_ens* e, int32_t m, const double* packed, int32_
     const double* src = packed;
     if (!on_device || !ewpt_kernel_reads(packed, e->device)) {
         ewpt_ctx* v;
-        rc = ens_view(e, m, &v, false);
+        rc = ens_view(e, m, &v, 0);
         if (rc) return rc;
         ce = cudaMemcpyAsync(v->y, packed, (size_t)36 * c->g.S * 8,
                              on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, e->st);
@@ -318,7 +319,7 @@ static int ens_thermal(ewpt_ens* e, int32_t m, double T, double mH, double mW, u
     if (rc) return ens_fail(e, rc, ewpt_last_error(nullptr));
     cudaSetDevice(e->device);
     ewpt_ctx* v;
-    rc = ens_view(e, m, &v, false);
+    rc = ens_view(e, m, &v, 0);
     if (rc) return rc;
     std::string err;
     rc = ewpt_thermal_fill(v->g, v->p, T, mH, mW, seed, v->y, e->st, &err, gauss_iters);
@@ -358,7 +359,7 @@ int ewpt_ensemble_spectrum(ewpt_ens* e, int32_t m, int32_t field, int32_t mode, 
     if (rc) return rc;
     cudaSetDevice(e->device);
     ewpt_ctx* v;
-    rc = ens_view(e, m, &v);
+    rc = ens_view(e, m, &v, field == EWPT_FIELD_HIGGS ? 4 : 16);
     if (rc) return rc;
     rc = ewpt_spectrum(v, field, mode, nbins, k, sum, count, mean, nbins_out);
     if (rc) e->err = v->err;

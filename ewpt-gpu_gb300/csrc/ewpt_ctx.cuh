@@ -46,7 +46,8 @@ struct ewpt_ctx {
     void* fft_out = nullptr;    // complex half-spectrum buffers
     int fft_plan = 0;           // cufftHandle
     int fft_ready = 0;
-    double* shell = nullptr;    // per-shell accumulators
+    double* shell = nullptr;    // shell sums (spectrum.cu)
+    size_t shell_doubles = 0;
     std::string err;
 };
 
@@ -56,9 +57,11 @@ int ewpt_validate_params(const ewpt_params* p, ewpt_ctx* ctx);
 // FP64 context holding only the state buffer, for diagnostics and spectra of
 // a state that lives elsewhere (ensemble members).
 extern "C" int ewpt_create_view(const ewpt_params* p, ewpt_ctx** out);
-// FP64 view of the current state: c->y for FP64 contexts; for FP32 contexts
-// the state joined into c->scratch64.
-int ewpt_state64(ewpt_ctx* c, const double** out);
+// FP64 view of the current state: c->y for FP64 contexts; for the others the
+// first `arrays` arrays joined into c->scratch64 (the rest is undefined).
+int ewpt_state64(ewpt_ctx* c, const double** out, int arrays = 36);
+// phi_1..4 of the current state in FP64, [4][S] device memory, on c->st
+int ewpt_higgs64(ewpt_ctx* c, double* out);
 int ewpt_ensure_scratch64(ewpt_ctx* c);
 // FP64 [36][S] buffer to write a whole state into (c->y, or the FP32 form's
 // scratch64), and the conversion of a state written there into the

@@ -284,7 +284,7 @@ cudaError_t launch_step_dd(const Grid& g, const Tiling& t, double* y, double* yn
                            double* cur, const ewpt_params& p, double Jex, double gam, cudaStream_t st);
 // 36 FP64 arrays of S values <-> [36][S] float pairs (src = the pairs' own buffer: in place)
 cudaError_t launch_to_dd(int64_t S, const Ptr36& src, double* pairs, cudaStream_t st);
-cudaError_t launch_from_dd(int64_t S, const double* pairs, const MPtr36& dst, cudaStream_t st);
+cudaError_t launch_from_dd(int64_t S, const double* pairs, const MPtr36& dst, cudaStream_t st, int arrays = 36);
 cudaError_t launch_step_fp32(const Grid& g, const Layout& L, const Tiling& t, Fp32State y, Fp32Work w,
                              const ewpt_params& p, double Jex, double gam, cudaStream_t st);
 // comp: the compensated mode (gauge Laplacians and auxiliary gradients compensated, stage_pair.cu)
@@ -297,10 +297,11 @@ cudaError_t launch_ghost_fill(const Grid& g, const Layout& L, float* buf, cudaSt
 // whose arrays 20-35 may lie in another one (mom + a*P).
 cudaError_t launch_ghost_fill_yz(const Grid& g, const Layout& L, float* fld, float* mom, cudaStream_t st);
 // 36 FP64 arrays <-> FP32 hi/lo in layout L (the ghost images of hi refreshed
-// on split, the x faces only if xfaces).
+// on split, the x faces only if xfaces; joins of the first `arrays` arrays).
 cudaError_t launch_fp32_split(const Grid& g, const Layout& L, const Ptr36& src, Fp32State dst, cudaStream_t st,
                               bool xfaces);
-cudaError_t launch_fp32_join(const Grid& g, const Layout& L, Fp32State src, const MPtr36& dst, cudaStream_t st);
+cudaError_t launch_fp32_join(const Grid& g, const Layout& L, Fp32State src, const MPtr36& dst, cudaStream_t st,
+                             int arrays = 36);
 // the arrays of a packed [36][S] FP64 buffer
 inline Ptr36 arrays36(const double* y, int64_t S) {
     Ptr36 P;

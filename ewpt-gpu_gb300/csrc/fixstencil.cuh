@@ -212,3 +212,89 @@ struct FixAcc : SiteAcc<double, double, SrcPtr36<double>> {
         return fix::to_double(V, e, 2);
     }
 };
+
+// First derivatives of an FP64 [36][S] buffer for the diagnostics, 60 dx times
+// their value; one conversion per derivative, curl component or divergence.
+struct FixDiff {
+    const double* y;
+    int64_t S;
+    int c;
+    int o[3][6];  // [+1, +2, +3, -1, -2, -3] along x, y, z
+    double T;     // 60 dx
+    double s[3];  // 45, -9, 1 over 60 dx (the floating-point evaluation)
+
+    __device__ __forceinline__ double v(int q) const { return __ldg(y + q * S + c); }
+    __device__ __forceinline__ double d1(int q, int ax) const {
+        const double* p = y + q * S + c;
+        double r = 0.0;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) r += s[k] * (__ldg(p + o[ax][k]) - __ldg(p + o[ax][k + 3]));
+        return r;
+    }
+    __device__ __forceinline__ static int64_t weighed(const double* f, uint32_t ep) {
+        int64_t D[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) D[k] = fix::align(f[k], ep) - fix::align(f[k + 3], ep);
+        return fix::weigh_grad(D[0], D[1], D[2]);
+    }
+    __device__ __noinline__ void grad(int q, double& gx, double& gy, double& gz) const {
+        double f[3][6];
+        uint32_t e = 0;
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax)
+#pragma unroll
+            for (int k = 0; k < 6; ++k) f[ax][k] = __ldg(y + q * S + c + o[ax][k]);
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax)
+#pragma unroll
+            for (int k = 0; k < 6; ++k) e = max(e, fix::exp20(f[ax][k]));
+        if (fix::covered(e)) {
+            const uint32_t ep = e + (7u << 20);
+            gx = fix::to_double(weighed(f[0], ep), e, 0);
+            gy = fix::to_double(weighed(f[1], ep), e, 0);
+            gz = fix::to_double(weighed(f[2], ep), e, 0);
+        } else if (e == 0 && fix::zero_bits(f)) {
+            gx = gy = gz = 0.0;
+        } else {
+            gx = T * d1(q, 0);
+            gy = T * d1(q, 1);
+            gz = T * d1(q, 2);
+        }
+    }
+    // d_a q - d_b r
+    __device__ __noinline__ double curl(int q, int a, int r, int b) const {
+        double f[3][6];
+        uint32_t e = 0;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            f[0][k] = __ldg(y + q * S + c + o[a][k]);
+            f[1][k] = __ldg(y + r * S + c + o[b][k]);
+            f[2][k] = 0.0;
+        }
+#pragma unroll
+        for (int k = 0; k < 6; ++k) e = max(e, max(fix::exp20(f[0][k]), fix::exp20(f[1][k])));
+        if (fix::covered(e)) {
+            const uint32_t ep = e + (7u << 20);
+            return fix::to_double((weighed(f[0], ep) >> 1) - (weighed(f[1], ep) >> 1), e, 1);
+        }
+        return e == 0 && fix::zero_bits(f) ? 0.0 : T * (d1(q, a) - d1(r, b));
+    }
+    // dx q + dy (q + 1) + dz (q + 2)
+    __device__ __noinline__ double div(int q) const {
+        double f[3][6];
+        uint32_t e = 0;
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax)
+#pragma unroll
+            for (int k = 0; k < 6; ++k) f[ax][k] = __ldg(y + (q + ax) * S + c + o[ax][k]);
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax)
+#pragma unroll
+            for (int k = 0; k < 6; ++k) e = max(e, fix::exp20(f[ax][k]));
+        if (fix::covered(e)) {
+            const uint32_t ep = e + (7u << 20);
+            return fix::to_double((weighed(f[0], ep) >> 2) + (weighed(f[1], ep) >> 2) + (weighed(f[2], ep) >> 2), e, 2);
+        }
+        return e == 0 && fix::zero_bits(f) ? 0.0 : T * (d1(q, 0) + d1(q + 1, 1) + d1(q + 2, 2));
+    }
+};

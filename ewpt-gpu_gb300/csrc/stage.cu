@@ -479,17 +479,18 @@ cudaError_t launch_ghost_fill_yz(const Grid& g, const Layout& L, float* fld, flo
     return cudaGetLastError();
 }
 
-static unsigned conv_grid(const Grid& g) {
-    return (unsigned)((g.nx * g.ny + kConvPiece - 1) / kConvPiece) * 36u * (unsigned)g.nz;
+static unsigned conv_grid(const Grid& g, int arrays) {
+    return (unsigned)((g.nx * g.ny + kConvPiece - 1) / kConvPiece) * (unsigned)arrays * (unsigned)g.nz;
 }
 
 cudaError_t launch_fp32_split(const Grid& g, const Layout& L, const Ptr36& src, Fp32State dst, cudaStream_t st,
                               bool xfaces) {
-    k_split<<<conv_grid(g), kConvThreads, 0, st>>>(g, L, src, dst.hi, dst.lo);
+    k_split<<<conv_grid(g, 36), kConvThreads, 0, st>>>(g, L, src, dst.hi, dst.lo);
     return launch_ghost_fill(g, L, dst.hi, st, xfaces);
 }
 
-cudaError_t launch_fp32_join(const Grid& g, const Layout& L, Fp32State src, const MPtr36& dst, cudaStream_t st) {
-    k_join<<<conv_grid(g), kConvThreads, 0, st>>>(g, L, src.hi, src.lo, dst);
+cudaError_t launch_fp32_join(const Grid& g, const Layout& L, Fp32State src, const MPtr36& dst, cudaStream_t st,
+                             int arrays) {
+    k_join<<<conv_grid(g, arrays), kConvThreads, 0, st>>>(g, L, src.hi, src.lo, dst);
     return cudaGetLastError();
 }

@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(256) k_from_dd(int64_t S, const float2* __rest
     }
 }
 
-dim3 pair_grid(int64_t S) { return dim3((unsigned)std::min<int64_t>((S + 1023) / 1024, 4096), 36); }
+dim3 pair_grid(int64_t S, int arrays) { return dim3((unsigned)std::min<int64_t>((S + 1023) / 1024, 4096), arrays); }
 
 // One stage: the whole stage with beta terms, else its three parts.
 template <int STAGE, bool BETA, int REG>
@@ -230,11 +230,11 @@ cudaError_t launch_step_dd(const Grid& g, const Tiling& t, double* y, double* yn
 }
 
 cudaError_t launch_to_dd(int64_t S, const Ptr36& src, double* pairs, cudaStream_t st) {
-    k_to_dd<<<pair_grid(S), 256, 0, st>>>(S, src, reinterpret_cast<float2*>(pairs));
+    k_to_dd<<<pair_grid(S, 36), 256, 0, st>>>(S, src, reinterpret_cast<float2*>(pairs));
     return cudaGetLastError();
 }
 
-cudaError_t launch_from_dd(int64_t S, const double* pairs, const MPtr36& dst, cudaStream_t st) {
-    k_from_dd<<<pair_grid(S), 256, 0, st>>>(S, reinterpret_cast<const float2*>(pairs), dst);
+cudaError_t launch_from_dd(int64_t S, const double* pairs, const MPtr36& dst, cudaStream_t st, int arrays) {
+    k_from_dd<<<pair_grid(S, arrays), 256, 0, st>>>(S, reinterpret_cast<const float2*>(pairs), dst);
     return cudaGetLastError();
 }
