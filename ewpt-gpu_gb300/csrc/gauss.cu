@@ -18,13 +18,20 @@
 //      kernel, then a one-sided Jacobi SVD of the <= 32 x 32 system on the
 //      host, the minimum-norm solution as numpy's lstsq gives it);
 //   2. project: per group (the three SU(2) colours and U(1)), with rho taken
-//      before the iteration, E <- E - grad chi with d.d chi = d.E - rho solved
-//      in Fourier space with the derivative's symbol
+//      before the iteration, E <- E - grad chi with d.d chi = d.E - rho: the
+//      divergence and the gradient are the stencils, and chi comes from one
+//      forward and one backward real FFT of the source with the squared symbol
 //      s(theta) = (90 sin theta - 18 sin 2 theta + 2 sin 3 theta) / (60 dx)
 //      (cuFFT D2Z / Z2D); modes with |s|^2 <= 1e-12 max |s|^2 are left alone.
 // The rho^a of the next iteration sees the projected E (the SU(2) charge
-// depends on E), so the residual falls by iterations.  This is the device
-// version of ewpt/ic.py gauss_project (same steps, same order).
+// depends on E), so the residual falls by iterations.  ewpt/ic.py
+// gauss_project does the same steps on the host, with step 2 wholly in Fourier
+// space (E and rho transformed, E transformed back).
+//
+// Bound by the FP64 pipe: the FFTs (96^3: 0.11 ms each, 8 per iteration; 28
+// when E itself is transformed), then the charges.  20 iterations at 96^3 on
+// a thermal state took 110 ms with 28 FFTs, the symbol's nine sines per mode
+// and the moments in shared-memory atomics.
 #include <cufft.h>
 
 #include <cmath>
@@ -32,144 +39,191 @@
 #include <vector>
 
 #include "ewpt_ctx.cuh"
+#include "fixstencil.cuh"
 
 namespace {
 
 constexpr int kNQ = 20;  // moments per parity class: 4 charges, then 16 generator overlaps
+// what the device sums of them: the 4 charges, |phi|^2 and the overlaps of the
+// SU(2) generators with the U(1) generator.  The SU(2) generators turn phi into
+// three orthogonal vectors of its length, so the other overlaps are |phi|^2 or 0.
+constexpr int kND = 8;
 
-// charge generators M_a (a = 0, 1, 2: SU(2); 3: U(1)): M[i][j] = 1, M[j][i] = -1 per pair
-__constant__ int kPairs[4][2][2] = {{{0, 3}, {2, 1}}, {{2, 0}, {3, 1}}, {{0, 1}, {3, 2}}, {{0, 1}, {2, 3}}};
-
-// u = M_b^T phi
+// u = M_b^T phi of the charge generators M_b (b = 0, 1, 2: SU(2); 3: U(1))
 __device__ __forceinline__ void gen_t(int b, const double* ph, double* u) {
-    u[0] = u[1] = u[2] = u[3] = 0.0;
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-        const int i = kPairs[b][q][0], j = kPairs[b][q][1];
-        u[j] += ph[i];
-        u[i] -= ph[j];
+    switch (b) {
+        case 0: u[0] = -ph[3], u[1] = ph[2], u[2] = -ph[1], u[3] = ph[0]; break;
+        case 1: u[0] = ph[2], u[1] = ph[3], u[2] = -ph[0], u[3] = -ph[1]; break;
+        case 2: u[0] = -ph[1], u[1] = ph[0], u[2] = ph[3], u[3] = -ph[2]; break;
+        default: u[0] = -ph[1], u[1] = ph[0], u[2] = -ph[3], u[3] = ph[2];
     }
 }
 
-// rho^1..3 and rho_Y at site c of an FP64 [36][S] state
-__device__ __forceinline__ void site_charges(const double* __restrict__ y, int64_t S, int64_t c, double gw, double gy,
-                                             double* rho) {
-    double ph[4], pi[4], u[4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-        ph[a] = y[a * S + c];
-        pi[a] = y[(20 + a) * S + c];
-    }
+// rho^1..3 and rho_Y at site c of an FP64 [36][S] state with Higgs field ph
+// and momentum pi
+__device__ __forceinline__ void site_charges(const double* __restrict__ y, int64_t S, int64_t c, const double* ph,
+                                             const double* pi, double gw, double gy, double* rho) {
+    double u[4];
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
         gen_t(a, ph, u);  // phi^T M_a pi = (M_a^T phi) . pi
         double h = u[0] * pi[0] + u[1] * pi[1] + u[2] * pi[2] + u[3] * pi[3];
         if (a < 3) {
             const int b = (a + 1) % 3, cc = (a + 2) % 3;
-            double q = 0.0;
 #pragma unroll
             for (int i = 0; i < 3; ++i)
-                q -= y[(4 + 3 * b + i) * S + c] * y[(24 + 3 * cc + i) * S + c] -
+                h -= y[(4 + 3 * b + i) * S + c] * y[(24 + 3 * cc + i) * S + c] -
                      y[(4 + 3 * cc + i) * S + c] * y[(24 + 3 * b + i) * S + c];
-            rho[a] = gw * q + gw * h;
+            rho[a] = gw * h;
         } else {
             rho[a] = gy * h;
         }
     }
 }
 
-__global__ void k_charges(Grid g, const double* __restrict__ y, double gw, double gy, double* __restrict__ rho) {
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < g.S; q += (int64_t)gridDim.x * blockDim.x) {
-        double r[4];
-        site_charges(y, g.S, q, gw, gy, r);
-#pragma unroll
-        for (int a = 0; a < 4; ++a) rho[a * g.S + q] = r[a];
-    }
-}
+constexpr int kMomentBlocks = 4 * 152, kMomentWarps = 8;
 
-__device__ __forceinline__ int parity_class(const Grid& g, int64_t q) {
-    const int i = (int)(q % g.nx), j = (int)((q / g.nx) % g.ny), k = (int)(q / ((int64_t)g.nx * g.ny));
-    return (k & 1) * 4 + (j & 1) * 2 + (i & 1);
-}
-
-// per-block sums over each parity class of the 4 charges and of the 16
-// coup_a (M_a^T phi).(M_b^T phi); part[block][class][kNQ]
-__global__ void __launch_bounds__(256) k_class_moments(Grid g, const double* __restrict__ y, double gw, double gy,
-                                                       double* __restrict__ part) {
-    __shared__ double sh[8 * kNQ];
-    for (int t = threadIdx.x; t < 8 * kNQ; t += blockDim.x) sh[t] = 0.0;
-    __syncthreads();
-    const double coup[4] = {gw, gw, gw, gy};
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < g.S; q += (int64_t)gridDim.x * blockDim.x) {
-        double v[kNQ], ph[4], u[4][4];
-        site_charges(y, g.S, q, gw, gy, v);
+// Sums over each parity class of the kND quantities.  Block b takes the rows
+// whose (j, k) have the parities of b % 4, a warp a row at a time, a lane the
+// sites of its own parity, so every thread sums one class in registers.
+// part[block][parity of i][kND].
+__global__ void __launch_bounds__(32 * kMomentWarps) k_class_moments(Grid g, const double* __restrict__ y, double gw,
+                                                                     double gy, double* __restrict__ part) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int pj = blockIdx.x & 1, pk = (blockIdx.x >> 1) & 1;
+    const int nj = (g.ny + 1 - pj) / 2, nk = (g.nz + 1 - pk) / 2;
+    double s[kND] = {};
+    for (int r = (blockIdx.x >> 2) * kMomentWarps + warp; r < nj * nk; r += (kMomentBlocks / 4) * kMomentWarps) {
+        const int j = 2 * (r % nj) + pj, k = 2 * (r / nj) + pk;
+        const int64_t row = (int64_t)g.nx * (j + (int64_t)g.ny * k);
+        for (int i = lane; i < g.nx; i += 32) {
+            const int64_t q = row + i;
+            double rho[4], ph[4], pi[4], uy[4], u[4];
 #pragma unroll
-        for (int a = 0; a < 4; ++a) ph[a] = y[a * g.S + q];
+            for (int a = 0; a < 4; ++a) {
+                ph[a] = y[a * g.S + q];
+                pi[a] = y[(20 + a) * g.S + q];
+            }
+            site_charges(y, g.S, q, ph, pi, gw, gy, rho);
+            gen_t(3, ph, uy);
 #pragma unroll
-        for (int b = 0; b < 4; ++b) gen_t(b, ph, u[b]);
+            for (int a = 0; a < 4; ++a) s[a] += rho[a];
+            s[4] += ph[0] * ph[0] + ph[1] * ph[1] + ph[2] * ph[2] + ph[3] * ph[3];
 #pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int b = 0; b < 4; ++b)
-                v[4 + 4 * a + b] =
-                    coup[a] * (u[a][0] * u[b][0] + u[a][1] * u[b][1] + u[a][2] * u[b][2] + u[a][3] * u[b][3]);
-        double* s = sh + parity_class(g, q) * kNQ;
-#pragma unroll
-        for (int t = 0; t < kNQ; ++t) atomicAdd(s + t, v[t]);
-    }
-    __syncthreads();
-    for (int t = threadIdx.x; t < 8 * kNQ; t += blockDim.x) part[(int64_t)blockIdx.x * 8 * kNQ + t] = sh[t];
-}
-
-// pi += table[b][class(x)] M_b^T phi
-__global__ void k_shift_momenta(Grid g, double* __restrict__ y, const double* __restrict__ table) {
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < g.S; q += (int64_t)gridDim.x * blockDim.x) {
-        const int cls = parity_class(g, q);
-        double ph[4], u[4], d[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-        for (int a = 0; a < 4; ++a) ph[a] = y[a * g.S + q];
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            gen_t(b, ph, u);
-            const double t = table[b * 8 + cls];
-#pragma unroll
-            for (int a = 0; a < 4; ++a) d[a] += t * u[a];
+            for (int a = 0; a < 3; ++a) {
+                gen_t(a, ph, u);
+                s[5 + a] += u[0] * uy[0] + u[1] * uy[1] + u[2] * uy[2] + u[3] * uy[3];
+            }
         }
+    }
+    __shared__ double sh[kMomentWarps][2][kND];
 #pragma unroll
-        for (int a = 0; a < 4; ++a) y[(20 + a) * g.S + q] += d[a];
+    for (int t = 0; t < kND; ++t) {
+        for (int off = 16; off > 1; off >>= 1) s[t] += __shfl_down_sync(0xffffffffu, s[t], off);
+        if (lane < 2) sh[warp][lane][t] = s[t];
+    }
+    __syncthreads();
+    if (threadIdx.x < 2 * kND) {
+        double v = 0.0;
+        for (int w = 0; w < kMomentWarps; ++w) v += (&sh[w][0][0])[threadIdx.x];
+        part[blockIdx.x * 2 * kND + threadIdx.x] = v;
     }
 }
 
-__device__ __forceinline__ double deriv_symbol(double th, double dx) {
-    return (90.0 * sin(th) - 18.0 * sin(2.0 * th) + 2.0 * sin(3.0 * th)) / (60.0 * dx);
+// out[class][kND]: one warp per sum
+__global__ void __launch_bounds__(1024) k_fold_moments(const double* __restrict__ part, double* __restrict__ out) {
+    const int lane = threadIdx.x & 31;
+    for (int q = threadIdx.x >> 5; q < 8 * kND; q += 32) {
+        const int cls = q / kND, t = q % kND;  // class = pk*4 + pj*2 + pi
+        double v = 0.0;
+        for (int b = (cls >> 1) + 4 * lane; b < kMomentBlocks; b += 128) v += part[b * 2 * kND + (cls & 1) * kND + t];
+        for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+        if (lane == 0) out[q] = v;
+    }
 }
 
-// half spectrum (x: 0..nx/2): C0..C2 = FFT(E_x, E_y, E_z), C3 = FFT(rho);
-// C_j <- (C_j - i s_j chi) / S, chi = (i s.C - C3) / (-|s|^2) where |s|^2 > cut
-__global__ void k_project_modes(Grid g, double dx, double cut, cufftDoubleComplex* __restrict__ c0,
-                                cufftDoubleComplex* __restrict__ c1, cufftDoubleComplex* __restrict__ c2,
-                                const cufftDoubleComplex* __restrict__ c3) {
+// difference operator over a [.][S] buffer at the site of this thread
+__device__ __forceinline__ bool site_of(const Grid& g, const double* y, double t, FixDiff& A, int* parity) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if ((int64_t)blockIdx.x * blockDim.x + threadIdx.x >= g.S) return false;
+    const int row = q / g.nx, i = q - row * g.nx, k = row / g.ny, j = row - k * g.ny;
+    A.y = y;
+    A.S = g.S;
+    A.c = q;
+    axis_offsets(i, g.nx, 1, A.o[0]);
+    axis_offsets(j, g.ny, g.nx, A.o[1]);
+    axis_offsets(k, g.nz, g.nx * g.ny, A.o[2]);
+    A.T = 1.0 / t;
+    A.s[0] = 45.0 * t;
+    A.s[1] = -9.0 * t;
+    A.s[2] = t;
+    if (parity) *parity = (k & 1) * 4 + (j & 1) * 2 + (i & 1);
+    return true;
+}
+
+struct Table32 {
+    double t[32];
+};
+
+// pi += table[b][class(x)] M_b^T phi, then src[a] = d_i E^a_i - rho^a
+__global__ void __launch_bounds__(128, 4) k_source(Grid g, double* __restrict__ y, const __grid_constant__ Table32 tab,
+                                                   double gw, double gy, double t, double* __restrict__ src, int64_t Sp) {
+    FixDiff A;
+    int cls;
+    if (!site_of(g, y, t, A, &cls)) return;
+    const int64_t q = A.c;
+    double ph[4], pi[4], u[4], rho[4], d[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int a = 0; a < 4; ++a) ph[a] = y[a * g.S + q];
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+        gen_t(b, ph, u);
+        const double w = tab.t[b * 8 + cls];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) d[a] += w * u[a];
+    }
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        pi[a] = y[(20 + a) * g.S + q] + d[a];
+        y[(20 + a) * g.S + q] = pi[a];
+    }
+    site_charges(y, g.S, q, ph, pi, gw, gy, rho);
+#pragma unroll
+    for (int a = 0; a < 4; ++a) src[a * Sp + q] = t * A.div(24 + 3 * a) - rho[a];
+}
+
+// half spectrum (x: 0..nx/2) of the source -> of chi: times -1 / (S |s|^2),
+// zero where |s|^2 <= cut; the tables hold each axis' s^2
+__global__ void __launch_bounds__(256) k_solve(Grid g, const double* __restrict__ sx, const double* __restrict__ sy,
+                                               const double* __restrict__ sz, double cut,
+                                               cufftDoubleComplex* __restrict__ C) {
     const int hx = g.nx / 2 + 1;
     const int64_t H = (int64_t)hx * g.ny * g.nz;
-    const double inv = 1.0 / (double)g.S, two_pi = 6.283185307179586;
+    const double inv = 1.0 / (double)g.S;
     for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < H; q += (int64_t)gridDim.x * blockDim.x) {
-        const int i = (int)(q % hx), j = (int)((q / hx) % g.ny), k = (int)(q / ((int64_t)hx * g.ny));
-        const double sx = deriv_symbol(two_pi * i / g.nx, dx), sy = deriv_symbol(two_pi * j / g.ny, dx),
-                     sz = deriv_symbol(two_pi * k / g.nz, dx);
-        const double s2 = sx * sx + sy * sy + sz * sz;
-        const cufftDoubleComplex a = c0[q], b = c1[q], c = c2[q], r = c3[q];
-        double chr = 0.0, chi = 0.0;
-        if (s2 > cut) {
-            // res = i (s . C) - rho_hat
-            const double re = -(sx * a.y + sy * b.y + sz * c.y) - r.x;
-            const double im = (sx * a.x + sy * b.x + sz * c.x) - r.y;
-            chr = -re / s2;
-            chi = -im / s2;
+        const int row = (int)(q / hx), i = (int)(q - (int64_t)row * hx), k = row / g.ny, j = row - k * g.ny;
+        const double s2 = sx[i] + sy[j] + sz[k];
+        const double f = s2 > cut ? -inv / s2 : 0.0;
+        const cufftDoubleComplex v = C[q];
+        C[q] = make_cuDoubleComplex(f * v.x, f * v.y);
+    }
+}
+
+// E^a_i -= d_i chi^a
+__global__ void __launch_bounds__(128, 4) k_subtract(Grid g, double* __restrict__ y, const double* __restrict__ chi,
+                                                     int64_t Sp, double t) {
+    FixDiff A;
+    if (!site_of(g, chi, t, A, nullptr)) return;
+    A.S = Sp;
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        double d[3];
+        A.grad(a, d[0], d[1], d[2]);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            double* e = y + (24 + 3 * a + i) * g.S + A.c;
+            *e = fma(-t, d[i], *e);
         }
-        // C_j - i s_j chi: (x + i y) - i s (u + i v) = (x + s v) + i (y - s u)
-        c0[q] = make_cuDoubleComplex((a.x + sx * chi) * inv, (a.y - sx * chr) * inv);
-        c1[q] = make_cuDoubleComplex((b.x + sy * chi) * inv, (b.y - sy * chr) * inv);
-        c2[q] = make_cuDoubleComplex((c.x + sz * chi) * inv, (c.y - sz * chr) * inv);
     }
 }
 
@@ -196,16 +250,20 @@ double moment(const double* s, int stride, int e) {
 // Minimum-norm least-squares solution of A x = b (m x n, row-major), by a
 // one-sided Jacobi SVD (Hestenes); singular values below
 // eps * max(m, n) * sigma_max are dropped, as numpy's lstsq does by default.
-std::vector<double> lstsq(std::vector<double> A, int m, int n, const std::vector<double>& b) {
-    std::vector<double> V((size_t)n * n, 0.0);
+std::vector<double> lstsq(const std::vector<double>& rows, int m, int n, const std::vector<double>& b) {
+    // columns of A and V back to back: the rotations run over whole columns
+    std::vector<double> A((size_t)n * m), V((size_t)n * n, 0.0);
+    for (int i = 0; i < m; ++i)
+        for (int j = 0; j < n; ++j) A[(size_t)j * m + i] = rows[(size_t)i * n + j];
     for (int i = 0; i < n; ++i) V[(size_t)i * n + i] = 1.0;
     for (int sweep = 0; sweep < 60; ++sweep) {
         double off = 0.0;
         for (int p = 0; p < n - 1; ++p)
             for (int q = p + 1; q < n; ++q) {
                 double al = 0.0, be = 0.0, ga = 0.0;
+                double *ap = &A[(size_t)p * m], *aq = &A[(size_t)q * m], *vp = &V[(size_t)p * n], *vq = &V[(size_t)q * n];
                 for (int i = 0; i < m; ++i) {
-                    const double x = A[(size_t)i * n + p], y = A[(size_t)i * n + q];
+                    const double x = ap[i], y = aq[i];
                     al += x * x;
                     be += y * y;
                     ga += x * y;
@@ -216,14 +274,14 @@ std::vector<double> lstsq(std::vector<double> A, int m, int n, const std::vector
                 const double t = (zeta >= 0 ? 1.0 : -1.0) / (std::fabs(zeta) + std::sqrt(1.0 + zeta * zeta));
                 const double c = 1.0 / std::sqrt(1.0 + t * t), s = c * t;
                 for (int i = 0; i < m; ++i) {
-                    const double x = A[(size_t)i * n + p], y = A[(size_t)i * n + q];
-                    A[(size_t)i * n + p] = c * x - s * y;
-                    A[(size_t)i * n + q] = s * x + c * y;
+                    const double x = ap[i], y = aq[i];
+                    ap[i] = c * x - s * y;
+                    aq[i] = s * x + c * y;
                 }
                 for (int i = 0; i < n; ++i) {
-                    const double x = V[(size_t)i * n + p], y = V[(size_t)i * n + q];
-                    V[(size_t)i * n + p] = c * x - s * y;
-                    V[(size_t)i * n + q] = s * x + c * y;
+                    const double x = vp[i], y = vq[i];
+                    vp[i] = c * x - s * y;
+                    vq[i] = s * x + c * y;
                 }
             }
         if (off < 1e-15) break;
@@ -232,7 +290,7 @@ std::vector<double> lstsq(std::vector<double> A, int m, int n, const std::vector
     double smax = 0.0;
     for (int k = 0; k < n; ++k) {
         double s = 0.0;
-        for (int i = 0; i < m; ++i) s += A[(size_t)i * n + k] * A[(size_t)i * n + k];
+        for (int i = 0; i < m; ++i) s += A[(size_t)k * m + i] * A[(size_t)k * m + i];
         sig[k] = std::sqrt(s);
         smax = std::fmax(smax, sig[k]);
     }
@@ -240,9 +298,9 @@ std::vector<double> lstsq(std::vector<double> A, int m, int n, const std::vector
     for (int k = 0; k < n; ++k) {
         if (!(sig[k] > tol)) continue;
         double ub = 0.0;  // u_k . b, u_k = A[:, k] / sigma_k
-        for (int i = 0; i < m; ++i) ub += A[(size_t)i * n + k] * b[i];
+        for (int i = 0; i < m; ++i) ub += A[(size_t)k * m + i] * b[i];
         const double w = ub / (sig[k] * sig[k]);
-        for (int j = 0; j < n; ++j) x[j] += V[(size_t)j * n + k] * w;
+        for (int j = 0; j < n; ++j) x[j] += V[(size_t)k * n + j] * w;
     }
     return x;
 }
@@ -254,7 +312,6 @@ std::vector<double> lstsq(std::vector<double> A, int m, int n, const std::vector
 int ewpt_gauss_project_fp64(const Grid& g, const ewpt_params& p, double* y, int iters, cudaStream_t st,
                             std::string* err) {
     if (iters <= 0) return EWPT_OK;
-    const int nb = 1216, nt = 256;
     const int hx = g.nx / 2 + 1;
     const int64_t H = (int64_t)hx * g.ny * g.nz;
     cufftHandle fwd = 0, inv = 0;
@@ -266,35 +323,56 @@ int ewpt_gauss_project_fp64(const Grid& g, const ewpt_params& p, double* y, int 
     }
     cufftSetStream(fwd, st);
     cufftSetStream(inv, st);
-    double *rho = nullptr, *part = nullptr, *table = nullptr;
-    cufftDoubleComplex* C = nullptr;
-    cudaError_t e = cudaMallocAsync(&rho, (size_t)4 * g.S * 8, st);
-    if (e == cudaSuccess) e = cudaMallocAsync(&C, (size_t)4 * H * sizeof(cufftDoubleComplex), st);
-    if (e == cudaSuccess) e = cudaMallocAsync(&part, (size_t)nb * 8 * kNQ * 8, st);
-    if (e == cudaSuccess) e = cudaMallocAsync(&table, 32 * 8, st);
-    // |s|^2 cut: 1e-12 of its largest value (the sum of each axis' largest)
-    double smax = 0.0;
+    // squared symbol per axis; |s|^2 cut: 1e-12 of its largest value (the sum
+    // of each axis' largest)
     const int N[3] = {g.nx, g.ny, g.nz};
-    for (int d = 0; d < 3; ++d) {
+    std::vector<double> sym((size_t)g.nx + g.ny + g.nz);
+    double smax = 0.0;
+    for (int d = 0, o = 0; d < 3; o += N[d++]) {
         double m = 0.0;
-        for (int n = 0; n < N[d]; ++n) m = std::fmax(m, std::pow(host_symbol(6.283185307179586 * n / N[d], p.dx), 2));
+        for (int n = 0; n < N[d]; ++n) {
+            sym[o + n] = std::pow(host_symbol(6.283185307179586 * n / N[d], p.dx), 2);
+            m = std::fmax(m, sym[o + n]);
+        }
         smax += m;
     }
-    const double cut = 1e-12 * smax;
+    const double cut = 1e-12 * smax, t = 1.0 / (60.0 * p.dx);
+    // src [4][Sp] (the source, then chi), one half spectrum, the symbol's tables, the moments
+    const size_t npart = (size_t)kMomentBlocks * 2 * kND;
+    double *src = nullptr, *tab = nullptr;
+    cufftDoubleComplex* C = nullptr;
+    const int64_t Sp = (g.S + 1) / 2 * 2;  // array stride: cuFFT wants its arrays aligned to a complex number
+    cudaError_t e = cudaMallocAsync(&src, (size_t)4 * Sp * 8, st);
+    if (e == cudaSuccess) e = cudaMallocAsync(&C, (size_t)H * sizeof(cufftDoubleComplex), st);
+    if (e == cudaSuccess) e = cudaMallocAsync(&tab, (sym.size() + npart + 8 * kND) * 8, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(tab, sym.data(), sym.size() * 8, cudaMemcpyHostToDevice, st);
+    double* const part = tab + sym.size();
     const std::vector<int> es = null_vectors(g);
     const int ne = (int)es.size(), n = 4 * ne;
-    std::vector<double> hp((size_t)nb * 8 * kNQ), sums(8 * kNQ);
+    const unsigned sites = (unsigned)((g.S + 127) / 128);
+    const double coup[4] = {p.gw, p.gw, p.gw, p.gy};
     bool fft_ok = true;
     for (int it = 0; it < iters && e == cudaSuccess && fft_ok; ++it) {
         // 1. neutralise the charges' null-mode components
-        k_class_moments<<<nb, nt, 0, st>>>(g, y, p.gw, p.gy, part);
+        double hs[8 * kND], sums[8 * kNQ] = {};
+        k_class_moments<<<kMomentBlocks, 32 * kMomentWarps, 0, st>>>(g, y, p.gw, p.gy, part);
+        k_fold_moments<<<1, 1024, 0, st>>>(part, part + npart);
         e = cudaGetLastError();
-        if (e == cudaSuccess) e = cudaMemcpyAsync(hp.data(), part, hp.size() * 8, cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(hs, part + npart, sizeof hs, cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) break;
-        std::fill(sums.begin(), sums.end(), 0.0);
-        for (int b = 0; b < nb; ++b)
-            for (int t = 0; t < 8 * kNQ; ++t) sums[t] += hp[(size_t)b * 8 * kNQ + t];
+        for (int c = 0; c < 8; ++c) {
+            double* v = sums + c * kNQ;
+            const double* h = hs + c * kND;
+            for (int a = 0; a < 4; ++a) {
+                v[a] = h[a];
+                v[4 + 4 * a + a] = coup[a] * h[4];
+            }
+            for (int a = 0; a < 3; ++a) {
+                v[4 + 4 * a + 3] = coup[a] * h[5 + a];
+                v[4 + 4 * 3 + a] = coup[3] * h[5 + a];
+            }
+        }
         std::vector<double> A((size_t)n * n), Q(n);
         for (int a = 0; a < 4; ++a) {
             for (int i = 0; i < ne; ++i) Q[a * ne + i] = -moment(&sums[a], kNQ, es[i]);
@@ -304,31 +382,31 @@ int ewpt_gauss_project_fp64(const Grid& g, const ewpt_params& p, double* y, int 
                         A[(size_t)(a * ne + i) * n + b * ne + j] = moment(&sums[4 + 4 * a + b], kNQ, es[i] ^ es[j]);
         }
         const std::vector<double> alpha = lstsq(A, n, n, Q);
-        double tab[32];
+        Table32 shift;
         for (int b = 0; b < 4; ++b)
             for (int c = 0; c < 8; ++c) {
-                double t = 0.0;
-                for (int j = 0; j < ne; ++j) t += alpha[b * ne + j] * (__builtin_popcount(c & es[j]) & 1 ? -1.0 : 1.0);
-                tab[b * 8 + c] = t;
+                double w = 0.0;
+                for (int j = 0; j < ne; ++j) w += alpha[b * ne + j] * (__builtin_popcount(c & es[j]) & 1 ? -1.0 : 1.0);
+                shift.t[b * 8 + c] = w;
             }
-        e = cudaMemcpyAsync(table, tab, sizeof tab, cudaMemcpyHostToDevice, st);
-        if (e == cudaSuccess) k_shift_momenta<<<nb, nt, 0, st>>>(g, y, table);
-        // 2. charges of this iteration, then each group's projection
-        if (e == cudaSuccess) k_charges<<<nb, nt, 0, st>>>(g, y, p.gw, p.gy, rho);
-        if (e == cudaSuccess) e = cudaGetLastError();
+        // 2. sources of this iteration, then each group's projection
+        k_source<<<sites, 128, 0, st>>>(g, y, shift, p.gw, p.gy, t, src, Sp);
+        e = cudaGetLastError();
         for (int grp = 0; grp < 4 && e == cudaSuccess && fft_ok; ++grp) {
-            double* E = y + (size_t)(grp < 3 ? 24 + 3 * grp : 33) * g.S;
-            for (int i = 0; i < 3 && fft_ok; ++i) fft_ok = cufftExecD2Z(fwd, E + (size_t)i * g.S, C + i * H) == CUFFT_SUCCESS;
-            if (fft_ok) fft_ok = cufftExecD2Z(fwd, rho + (size_t)grp * g.S, C + 3 * H) == CUFFT_SUCCESS;
+            double* f = src + (size_t)grp * Sp;
+            fft_ok = cufftExecD2Z(fwd, f, C) == CUFFT_SUCCESS;
             if (!fft_ok) break;
-            k_project_modes<<<nb, nt, 0, st>>>(g, p.dx, cut, C, C + H, C + 2 * H, C + 3 * H);
+            k_solve<<<1216, 256, 0, st>>>(g, tab, tab + g.nx, tab + g.nx + g.ny, cut, C);
             e = cudaGetLastError();
-            for (int i = 0; i < 3 && fft_ok && e == cudaSuccess; ++i)
-                fft_ok = cufftExecZ2D(inv, C + i * H, E + (size_t)i * g.S) == CUFFT_SUCCESS;
+            if (e == cudaSuccess) fft_ok = cufftExecZ2D(inv, C, f) == CUFFT_SUCCESS;
+        }
+        if (e == cudaSuccess && fft_ok) {
+            k_subtract<<<sites, 128, 0, st>>>(g, y, src, Sp, t);
+            e = cudaGetLastError();
         }
     }
-    const cudaError_t ef[4] = {rho ? cudaFreeAsync(rho, st) : cudaSuccess, C ? cudaFreeAsync(C, st) : cudaSuccess,
-                               part ? cudaFreeAsync(part, st) : cudaSuccess, table ? cudaFreeAsync(table, st) : cudaSuccess};
+    const cudaError_t ef[3] = {src ? cudaFreeAsync(src, st) : cudaSuccess, C ? cudaFreeAsync(C, st) : cudaSuccess,
+                               tab ? cudaFreeAsync(tab, st) : cudaSuccess};
     for (cudaError_t x : ef)
         if (e == cudaSuccess) e = x;
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);

@@ -26,6 +26,7 @@
 
 #include <cmath>
 #include <string>
+#include <vector>
 
 #include "ewpt_ctx.cuh"
 #include "stencil_n.cuh"
@@ -96,37 +97,72 @@ __device__ __forceinline__ double amplitude(double k2, double m, double T, doubl
     return mom ? sqrt(occupation(w, T) * w / vol) : sqrt(occupation(w, T) / (w * vol));
 }
 
-__global__ void k_modes_scalar(Grid g, double dx, double T, double m, double vol, uint64_t key, int stream,
-                               cufftDoubleComplex* __restrict__ z, int mom) {
+// What a mode's spectrum needs of its wave vector, from tables: per axis the
+// lattice momentum 2 sin(theta / 2) / dx and 2 (1 - cos theta) / dx^2 of each
+// index, and per octant mode (|n_x|, |n_y|, |n_z|) the amplitude and 1 / |k|.
+// Sines, cosines, expm1 and the divisions of every mode were two fifths of the
+// FP64 instructions of k_modes_transverse, which is bound by that pipe.
+struct ModeTables {
+    const double* kv[3];  // [n_axis]
+    const double* k2[3];
+    double *amp, *ik;     // [ox * oy * oz]
+    int ox, oy, oz;       // octant sides n / 2 + 1
+    __device__ __forceinline__ int64_t octant(int i, int j, int k, const Grid& g) const {
+        i = min(i, g.nx - i);
+        j = min(j, g.ny - j);
+        k = min(k, g.nz - k);
+        return i + (int64_t)ox * (j + (int64_t)oy * k);
+    }
+};
+
+__global__ void k_mode_tables(Grid g, ModeTables t, double T, double m, double vol, int empty_k0, int mom) {
+    const int64_t n = (int64_t)t.ox * t.oy * t.oz;
+    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x) {
+        const int row = (int)(q / t.ox), i = (int)(q - (int64_t)row * t.ox), k = row / t.oy, j = row - k * t.oy;
+        const double k2 = t.k2[0][i] + t.k2[1][j] + t.k2[2][k];
+        t.amp[q] = amplitude(k2, m, T, vol, empty_k0 != 0, mom != 0);
+        t.ik[q] = k2 > 0.0 ? 1.0 / sqrt(k2) : 1.0;
+    }
+}
+
+__device__ __forceinline__ void mode_index(const Grid& g, int64_t q, int& i, int& j, int& k) {
+    const int row = (int)(q / g.nx);
+    i = (int)(q - (int64_t)row * g.nx);
+    k = row / g.ny;
+    j = row - k * g.ny;
+}
+
+__global__ void k_modes_scalar(Grid g, ModeTables t, uint64_t key, int stream, cufftDoubleComplex* __restrict__ z) {
     for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < g.S; q += (int64_t)gridDim.x * blockDim.x) {
-        const ModeGeom mg = mode_geom(g, dx, q);
-        const double amp = amplitude(mg.k2, m, T, vol, false, mom != 0);
+        int i, j, k;
+        mode_index(g, q, i, j, k);
+        const double amp = t.amp[t.octant(i, j, k, g)];
         double a, b;
         normal_pair(key, stream, q, a, b);
         z[q] = make_cuDoubleComplex(amp * a, amp * b);
     }
 }
 
-__global__ void k_modes_transverse(Grid g, double dx, double T, double m, double vol, uint64_t key, int stream,
-                                   cufftDoubleComplex* __restrict__ z0, cufftDoubleComplex* __restrict__ z1,
-                                   cufftDoubleComplex* __restrict__ z2, int mom) {
+__global__ void k_modes_transverse(Grid g, ModeTables t, uint64_t key, int stream, cufftDoubleComplex* __restrict__ z0,
+                                   cufftDoubleComplex* __restrict__ z1, cufftDoubleComplex* __restrict__ z2) {
     for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < g.S; q += (int64_t)gridDim.x * blockDim.x) {
-        const ModeGeom mg = mode_geom(g, dx, q);
-        const double* kv = mg.kv;
+        int i, j, k;
+        mode_index(g, q, i, j, k);
+        const int64_t oc = t.octant(i, j, k, g);
+        const double amp = t.amp[oc], ik = t.ik[oc];
+        const double kv[3] = {t.kv[0][i], t.kv[1][j], t.kv[2][k]};
         double r[4], x[4];
         normal_pair(key, stream, q, r[0], r[1]);
         normal_pair(key, stream + 1, q, r[2], r[3]);
         normal_pair(key, stream + 2, q, x[0], x[1]);
         normal_pair(key, stream + 3, q, x[2], x[3]);
         double e1[3] = {r[1] * kv[2] - r[2] * kv[1], r[2] * kv[0] - r[0] * kv[2], r[0] * kv[1] - r[1] * kv[0]};
-        double n1 = sqrt(e1[0] * e1[0] + e1[1] * e1[1] + e1[2] * e1[2]);
-        n1 = n1 == 0.0 ? 1.0 : n1;
-        for (int d = 0; d < 3; ++d) e1[d] /= n1;
-        double e2[3] = {e1[1] * kv[2] - e1[2] * kv[1], e1[2] * kv[0] - e1[0] * kv[2], e1[0] * kv[1] - e1[1] * kv[0]};
-        double n2 = sqrt(e2[0] * e2[0] + e2[1] * e2[1] + e2[2] * e2[2]);
-        n2 = n2 == 0.0 ? 1.0 : n2;
-        for (int d = 0; d < 3; ++d) e2[d] /= n2;
-        const double amp = amplitude(mg.k2, m, T, vol, true, mom != 0);
+        const double n2 = e1[0] * e1[0] + e1[1] * e1[1] + e1[2] * e1[2];
+        const double n1 = n2 == 0.0 ? 1.0 : 1.0 / sqrt(n2);
+        for (int d = 0; d < 3; ++d) e1[d] *= n1;
+        // e1 is a unit vector normal to k: |e1 x k| = |k|
+        const double e2[3] = {(e1[1] * kv[2] - e1[2] * kv[1]) * ik, (e1[2] * kv[0] - e1[0] * kv[2]) * ik,
+                              (e1[0] * kv[1] - e1[1] * kv[0]) * ik};
         // x1 + i x3 on e1, x2 + i x4 on e2 (thermal_initializer_gauge!)
         cufftDoubleComplex* out[3] = {z0, z1, z2};
 #pragma unroll
@@ -238,6 +274,30 @@ int ewpt_thermal_fill(const Grid& g, const ewpt_params& p, double T, double mH, 
     cufftDoubleComplex* z = nullptr;
     cudaError_t e = cudaMemsetAsync(y, 0, (size_t)36 * g.S * 8, st);
     if (e == cudaSuccess) e = cudaMallocAsync(&z, (size_t)3 * g.S * sizeof(cufftDoubleComplex), st);
+    // per-axis and octant tables of the modes
+    const int N[3] = {g.nx, g.ny, g.nz};
+    const size_t nax = (size_t)g.nx + g.ny + g.nz;
+    std::vector<double> axes(2 * nax);
+    for (int d = 0, o = 0; d < 3; o += N[d++])
+        for (int i = 0; i < N[d]; ++i) {
+            const double th = kTwoPi * (i < (N[d] + 1) / 2 ? i : i - N[d]) / N[d];
+            axes[o + i] = 2.0 * std::sin(0.5 * th) / p.dx;
+            axes[nax + o + i] = 2.0 * (1.0 - std::cos(th)) / (p.dx * p.dx);
+        }
+    double* dtab = nullptr;
+    ModeTables mt{};
+    mt.ox = g.nx / 2 + 1;
+    mt.oy = g.ny / 2 + 1;
+    mt.oz = g.nz / 2 + 1;
+    const size_t noct = (size_t)mt.ox * mt.oy * mt.oz;
+    if (e == cudaSuccess) e = cudaMallocAsync(&dtab, (2 * nax + 2 * noct) * 8, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(dtab, axes.data(), 2 * nax * 8, cudaMemcpyHostToDevice, st);
+    for (int d = 0, o = 0; d < 3; o += N[d++]) {
+        mt.kv[d] = dtab + o;
+        mt.k2[d] = dtab + nax + o;
+    }
+    mt.amp = dtab + 2 * nax;
+    mt.ik = mt.amp + noct;
     const uint64_t key = splitmix64(seed);
     const int nb = 1216, nt = 256;
     bool fft_ok = true;
@@ -250,39 +310,32 @@ int ewpt_thermal_fill(const Grid& g, const ewpt_params& p, double T, double mH, 
     };
     // Higgs phi_1..4: streams 0..3
     const bool mom = gauss_iters >= 0;
-    for (int a = 0; a < 4 && e == cudaSuccess; ++a) {
-        k_modes_scalar<<<nb, nt, 0, st>>>(g, p.dx, T, mH, vol, key, a, z, 0);
-        e = cudaGetLastError();
-        to_real(z, a);
-        if (mom && e == cudaSuccess && fft_ok) {
-            k_modes_scalar<<<nb, nt, 0, st>>>(g, p.dx, T, mH, vol, key, 4 + a, z, 1);
+    for (int pi = 0; pi <= (mom ? 1 : 0) && e == cudaSuccess && fft_ok; ++pi) {
+        k_mode_tables<<<nb, nt, 0, st>>>(g, mt, T, mH, vol, 0, pi);
+        for (int a = 0; a < 4 && fft_ok; ++a) {
+            k_modes_scalar<<<nb, nt, 0, st>>>(g, mt, key, 4 * pi + a, z);
             e = cudaGetLastError();
-            to_real(z, 20 + a);
+            to_real(z, 20 * pi + a);
+            if (e != cudaSuccess) break;
         }
     }
     // W^a (arrays 4 + 3a + i), streams 8 + 4a .. ; Y (13 + i), streams 20 ..;
     // their momenta (24 + 3a + i, 33 + i) streams 24 + 4 c
-    for (int c = 0; c < 4 && e == cudaSuccess && fft_ok; ++c) {
-        const bool is_y = c == 3;
-        k_modes_transverse<<<nb, nt, 0, st>>>(g, p.dx, T, is_y ? 0.0 : mW, vol, key, 8 + 4 * c, z, z + g.S,
-                                              z + 2 * g.S, 0);
-        e = cudaGetLastError();
-        const int base = is_y ? 13 : 4 + 3 * c;
-        for (int i = 0; i < 3; ++i) to_real(z + (size_t)i * g.S, base + i);
-        if (mom && e == cudaSuccess && fft_ok) {
-            k_modes_transverse<<<nb, nt, 0, st>>>(g, p.dx, T, is_y ? 0.0 : mW, vol, key, 24 + 4 * c, z, z + g.S,
-                                                  z + 2 * g.S, 1);
+    for (int pi = 0; pi <= (mom ? 1 : 0); ++pi)
+        for (int c = 0; c < 4 && e == cudaSuccess && fft_ok; ++c) {
+            const bool is_y = c == 3;
+            if (c == 0 || is_y) k_mode_tables<<<nb, nt, 0, st>>>(g, mt, T, is_y ? 0.0 : mW, vol, 1, pi);
+            k_modes_transverse<<<nb, nt, 0, st>>>(g, mt, key, (pi ? 24 : 8) + 4 * c, z, z + g.S, z + 2 * g.S);
             e = cudaGetLastError();
-            for (int i = 0; i < 3; ++i) to_real(z + (size_t)i * g.S, 20 + base + i);
+            const int base = 20 * pi + (is_y ? 13 : 4 + 3 * c);
+            for (int i = 0; i < 3; ++i) to_real(z + (size_t)i * g.S, base + i);
         }
-    }
     // Gamma^a = div W^a (arrays 16..18), Sigma = div Y (19)
     if (e == cudaSuccess && fft_ok) e = divergence(g, p.stencil_order, p.dx, y + (size_t)4 * g.S, 3, y + (size_t)16 * g.S, st);
     if (e == cudaSuccess && fft_ok) e = divergence(g, p.stencil_order, p.dx, y + (size_t)13 * g.S, 1, y + (size_t)19 * g.S, st);
-    if (z) {
-        const cudaError_t ef = cudaFreeAsync(z, st);
-        if (e == cudaSuccess) e = ef;
-    }
+    const cudaError_t ef[2] = {z ? cudaFreeAsync(z, st) : cudaSuccess, dtab ? cudaFreeAsync(dtab, st) : cudaSuccess};
+    for (cudaError_t x : ef)
+        if (e == cudaSuccess) e = x;
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     cufftDestroy(plan);
     if (!fft_ok) {
