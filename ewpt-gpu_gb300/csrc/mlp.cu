@@ -11,6 +11,11 @@
 // FP32.  This network has no counterpart in the reference: it maps early-time
 // spectra of the evolution to late-time magnetic spectra for parameter
 // sweeps, and the evolution itself stays the fallback and the reference answer.
+//
+// Networks whose operands fit shared memory (width a multiple of 16 and at
+// most 512, n_in <= 512, n_out <= 128; training batches <= 512), the surrogate's
+// among them, run the layer kernels of mlp_layers.cuh; others the general
+// GEMM with element-wise kernels.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -195,6 +200,12 @@ __device__ __forceinline__ float gelu_grad(float x) {
     return 0.5f * (1.f + erff(x * 0.70710678118654752f)) + x * 0.39894228040143268f * expf(-0.5f * x * x);
 }
 
+}  // namespace
+
+#include "mlp_layers.cuh"
+
+namespace {
+
 // z += bias (in place, z keeps the pre-activation); act = bf16(gelu(z)) or bf16(z)
 __global__ void k_bias_act(float* z, const float* __restrict__ bias, __nv_bfloat16* act, int B, int N, int apply) {
     for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < (int64_t)B * N;
@@ -290,6 +301,20 @@ struct ewpt_mlp {
     float* loss = nullptr;
     int64_t t = 0;
     std::string err;
+    // layer kernels (mlp_layers.cuh): operand images in one allocation, and
+    // mapped page-locked memory for the call's inputs, outputs and status
+    bool layers = false;
+    int K1 = 0, N3 = 0, Bt = 0;  // n_in and n_out padded, columns of the batch images
+    void* images = nullptr;
+    __nv_bfloat16 *W1i = nullptr, *W2i = nullptr, *W2t = nullptr, *W3i = nullptr, *W3t = nullptr;
+    __nv_bfloat16 *a1i = nullptr, *a2i = nullptr, *dz3i = nullptr, *dz2i = nullptr;
+    __nv_bfloat16 *x0T = nullptr, *a1T = nullptr, *a2T = nullptr, *dz1T = nullptr, *dz2T = nullptr, *dz3T = nullptr;
+    float *dz1 = nullptr, *dz2 = nullptr, *dz3 = nullptr, *lpart = nullptr;
+    int* flag = nullptr;
+    int gen = 0;
+    float* host = nullptr;  // [0] loss, [1] status, then x, y, z3
+    float *hx = nullptr, *hy = nullptr, *hz = nullptr;
+    float* mapped = nullptr;  // device address of host
 };
 
 namespace {
@@ -374,6 +399,154 @@ cudaError_t backward(ewpt_mlp* n, int B) {
     return cudaGetLastError();
 }
 
+// ---- layer kernels
+constexpr int kMappedHead = 32;  // floats before x in the mapped buffer
+
+bool layers_fit(const ewpt_mlp* n) {
+    return n->width % LN == 0 && n->width <= kLayerMaxK && n->nin <= kLayerMaxK && n->nout <= LM;
+}
+
+cudaError_t layers_alloc(ewpt_mlp* n) {
+    const int W = n->width;
+    n->K1 = round_up(n->nin, 16);
+    n->N3 = round_up(n->nout, LN);
+    n->Bt = round_up(std::min(n->maxb, kLayerMaxK), 16);
+    const int64_t Mp = round_up(n->maxb, LM), Wm = round_up(W, LM);
+    // bf16 images, then the FP32 arrays and the flag; every piece a multiple of 128 bytes
+    struct Piece {
+        void** p;
+        int64_t bytes;
+    } pieces[] = {{(void**)&n->W1i, (int64_t)W * n->K1 * 2},
+                  {(void**)&n->W2i, (int64_t)W * W * 2},
+                  {(void**)&n->W2t, (int64_t)W * W * 2},
+                  {(void**)&n->W3i, (int64_t)n->N3 * W * 2},
+                  {(void**)&n->W3t, (int64_t)W * n->N3 * 2},
+                  {(void**)&n->a1i, Mp * W * 2},
+                  {(void**)&n->a2i, Mp * W * 2},
+                  {(void**)&n->dz3i, Mp * n->N3 * 2},
+                  {(void**)&n->dz2i, Mp * W * 2},
+                  {(void**)&n->x0T, (int64_t)round_up(n->nin, LN) * n->Bt * 2},
+                  {(void**)&n->a1T, (int64_t)W * n->Bt * 2},
+                  {(void**)&n->a2T, (int64_t)W * n->Bt * 2},
+                  {(void**)&n->dz1T, Wm * n->Bt * 2},
+                  {(void**)&n->dz2T, Wm * n->Bt * 2},
+                  {(void**)&n->dz3T, (int64_t)LM * n->Bt * 2},
+                  {(void**)&n->dz1, (int64_t)n->maxb * W * 4},
+                  {(void**)&n->dz2, (int64_t)n->maxb * W * 4},
+                  {(void**)&n->dz3, (int64_t)n->maxb * n->nout * 4},
+                  {(void**)&n->lpart, Mp / LM * (n->N3 / LN) * (LT / 32) * 4},
+                  {(void**)&n->flag, 4}};
+    int64_t total = 0;
+    for (const Piece& q : pieces) total += (q.bytes + 127) / 128 * 128;
+    cudaError_t e = cudaMalloc(&n->images, total);
+    if (e == cudaSuccess) e = cudaMemsetAsync(n->images, 0, total, n->st);  // the padding stays zero
+    int64_t off = 0;
+    for (const Piece& q : pieces) {
+        *q.p = static_cast<char*>(n->images) + off;
+        off += (q.bytes + 127) / 128 * 128;
+    }
+    const int64_t rows = n->maxb;
+    if (e == cudaSuccess)
+        e = cudaHostAlloc((void**)&n->host, (kMappedHead + rows * (n->nin + 2 * n->nout)) * 4, cudaHostAllocMapped);
+    if (e == cudaSuccess) e = cudaHostGetDevicePointer((void**)&n->mapped, n->host, 0);
+    n->hx = n->host + kMappedHead;
+    n->hy = n->hx + rows * n->nin;
+    n->hz = n->hy + rows * n->nout;
+    const int smem = (LM + LN) * kLayerMaxK * 2;
+    const void* kernels[] = {(const void*)k_layer<kForward>, (const void*)k_layer<kOutput>,
+                             (const void*)k_layer<kBackward>, (const void*)k_weights};
+    for (const void* k : kernels)
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    return e;
+}
+
+// set_params: the weight images
+cudaError_t layers_pack(ewpt_mlp* n) {
+    const int W = n->width;
+    k_pack<<<152, 256, 0, n->st>>>(n->p + n->oW1, W, n->nin, n->W1i, n->K1, nullptr, 0);
+    k_pack<<<152, 256, 0, n->st>>>(n->p + n->oW2, W, W, n->W2i, W, n->W2t, W);
+    k_pack<<<152, 256, 0, n->st>>>(n->p + n->oW3, n->nout, W, n->W3i, W, n->W3t, n->N3);
+    return cudaGetLastError();
+}
+
+// dependent: the kernel may start before the previous one of the stream ends
+template <class Args>
+cudaError_t launch(const ewpt_mlp* n, void (*k)(Args), dim3 grid, int smem, const Args& a, bool dependent) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = dim3(LT);
+    c.dynamicSmemBytes = smem;
+    c.stream = n->st;
+    c.attrs = &at;
+    c.numAttrs = dependent ? 1 : 0;
+    return cudaLaunchKernelEx(&c, k, a);
+}
+
+// The layers on the batch in the mapped buffer; train: loss and weight
+// gradients into n->g, or (adam) one AdamW step instead.
+cudaError_t layers_run(ewpt_mlp* n, int B, bool train, bool adam, float lr, float wd, float c1, float c2) {
+    const int W = n->width, I = n->nin, O = n->nout, Bp = round_up(B, 16);
+    const unsigned my = (unsigned)((B + LM - 1) / LM);
+    n->host[0] = 0.f;
+    reinterpret_cast<int*>(n->host)[1] = 0;
+    ++n->gen;
+    const Status st{reinterpret_cast<volatile int*>(n->mapped) + 1, n->flag, n->gen,
+                    n->wait_polls < 0 ? kTcSpin : (long)n->wait_polls};
+    LayerArgs b{};
+    b.batch = B;
+    b.nin = I;
+    b.Bp = Bp;
+    b.train = train;
+    b.st = st;
+    LayerArgs f1 = b, f2 = b, f3 = b, b2 = b, b1 = b;
+    f1.x = n->mapped + kMappedHead;
+    f1.W = n->W1i, f1.bias = n->p + n->ob1, f1.N = W, f1.Kp = n->K1, f1.z = n->z1, f1.out = n->a1i, f1.outK = W;
+    f2.A = n->a1i, f2.W = n->W2i, f2.bias = n->p + n->ob2, f2.N = W, f2.Kp = W, f2.z = n->z2, f2.out = n->a2i, f2.outK = W;
+    f3.A = n->a2i, f3.W = n->W3i, f3.bias = n->p + n->ob3, f3.N = O, f3.Kp = W, f3.zo = n->z3;
+    if (train) {
+        f1.xT = n->x0T, f1.outT = n->a1T, f2.outT = n->a2T;
+        f3.y = n->mapped + (n->hy - n->host), f3.scale = 1.f / ((float)B * O), f3.loss = n->lpart, f3.dz = n->dz3;
+        f3.out = n->dz3i, f3.outK = n->N3, f3.outT = n->dz3T;
+    }
+    auto smem = [](int K) { return (LM + LN) * K * 2; };
+    cudaError_t e = launch(n, k_layer<kForward>, dim3(W / LN, my), smem(f1.Kp), f1, false);
+    if (e == cudaSuccess) e = launch(n, k_layer<kForward>, dim3(W / LN, my), smem(W), f2, true);
+    if (e == cudaSuccess) e = launch(n, k_layer<kOutput>, dim3(n->N3 / LN, my), smem(W), f3, true);
+    if (!train || e != cudaSuccess) return e;
+    b2.A = n->dz3i, b2.W = n->W3t, b2.N = W, b2.Kp = n->N3, b2.z = n->z2, b2.dz = n->dz2, b2.out = n->dz2i, b2.outK = W;
+    b2.outT = n->dz2T;
+    b1.A = n->dz2i, b1.W = n->W2t, b1.N = W, b1.Kp = W, b1.z = n->z1, b1.dz = n->dz1, b1.outT = n->dz1T;
+    e = launch(n, k_layer<kBackward>, dim3(W / LN, my), smem(n->N3), b2, true);
+    if (e == cudaSuccess) e = launch(n, k_layer<kBackward>, dim3(W / LN, my), smem(W), b1, true);
+    WeightArgs w{};
+    const int tw = round_up(W, LM) / LM, n1 = round_up(I, LN) / LN, nW = W / LN;
+    w.w[0] = WeightGrad{n->dz2T, n->a1T, n->dz2, W, W, nW, 0, n->oW2, n->ob2, n->W2i, n->W2t, W, W};
+    w.w[1] = WeightGrad{n->dz1T, n->x0T, n->dz1, W, I, n1, tw * nW, n->oW1, n->ob1, n->W1i, nullptr, n->K1, 0};
+    w.w[2] = WeightGrad{n->dz3T, n->a2T, n->dz3, O, W, nW, tw * (nW + n1), n->oW3, n->ob3, n->W3i, n->W3t, W, n->N3};
+    w.batch = B, w.Bp = Bp, w.adam = adam, w.nloss = (int)my * (n->N3 / LN) * (LT / 32), w.loss_part = n->lpart;
+    w.loss = n->mapped;
+    w.p = n->p, w.g = n->g, w.m = n->m, w.v = n->v, w.pb = n->pb;
+    w.lr = lr, w.b1 = 0.9f, w.b2 = 0.999f, w.eps = 1e-8f, w.wd = wd, w.c1 = c1, w.c2 = c2;
+    w.st = st;
+    if (e == cudaSuccess)
+        e = launch(n, k_weights, dim3(tw * (nW + n1) + nW), std::max(smem(Bp), LM * (LN + 1) * 4), w, true);
+    return e;
+}
+
+// after the stream has been waited for
+int layers_done(ewpt_mlp* n, cudaError_t e, const char* what) {
+    if (e != cudaSuccess) {
+        std::string s = std::string(what) + ": " + cudaGetErrorString(e);
+        return mlp_fail(n, e == cudaErrorMemoryAllocation ? EWPT_ERR_OOM : EWPT_ERR_CUDA, s.c_str());
+    }
+    if (reinterpret_cast<volatile int*>(n->host)[1])
+        return mlp_fail(n, EWPT_ERR_TIMEOUT, "a tensor-core wait in the MLP layers ran out (results invalid)");
+    return EWPT_OK;
+}
+
 int check_batch(ewpt_mlp* n, int B) {
     if (!n) return ewpt_fail(nullptr, EWPT_ERR_ARG, "mlp is NULL");
     if (B < 1 || B > n->maxb) return mlp_fail(n, EWPT_ERR_ARG, "batch size out of range (1..max_batch)");
@@ -432,6 +605,8 @@ int ewpt_mlp_create(int32_t n_in, int32_t width, int32_t n_out, int32_t max_batc
     A((void**)&n->dzb, (size_t)max_batch * wa * 2);
     A((void**)&n->part, 64 * 4);
     A((void**)&n->loss, 4);
+    n->layers = layers_fit(n);
+    if (e == cudaSuccess && n->layers) e = layers_alloc(n);
     if (e == cudaSuccess) e = cudaStreamSynchronize(n->st);
     int rc = mlp_cuda(nullptr, e, "mlp allocation");
     if (rc) {
@@ -449,6 +624,8 @@ int ewpt_mlp_destroy(ewpt_mlp* n) {
     void* bufs[] = {n->p, n->g, n->m, n->v, n->pb, n->xf, n->yf, n->x0, n->z1, n->z2, n->z3,
                     n->a1, n->a2, n->da, n->dzf, n->dzb, n->part, n->loss};
     for (void* b : bufs) cudaFree(b);
+    cudaFree(n->images);
+    cudaFreeHost(n->host);
     if (n->st) cudaStreamDestroy(n->st);
     delete n;
     return EWPT_OK;
@@ -473,6 +650,7 @@ int ewpt_mlp_set_params(ewpt_mlp* n, const float* params) {
     if (e == cudaSuccess) e = cudaMemsetAsync(n->m, 0, n->np * 4, n->st);
     if (e == cudaSuccess) e = cudaMemsetAsync(n->v, 0, n->np * 4, n->st);
     if (e == cudaSuccess) e = refresh_bf16(n);
+    if (e == cudaSuccess && n->layers) e = layers_pack(n);
     if (e == cudaSuccess) e = cudaStreamSynchronize(n->st);
     n->t = 0;
     return mlp_cuda(n, e, "mlp set_params");
@@ -490,6 +668,16 @@ int ewpt_mlp_forward(ewpt_mlp* n, const float* x, int32_t batch, float* y) {
     int rc = check_batch(n, batch);
     if (rc) return rc;
     if (!x || !y) return mlp_fail(n, EWPT_ERR_ARG, "NULL argument");
+    if (n->layers) {
+        const size_t out = (size_t)batch * n->nout * 4;
+        std::memcpy(n->hx, x, (size_t)batch * n->nin * 4);
+        cudaError_t e = layers_run(n, batch, false, false, 0.f, 0.f, 1.f, 1.f);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(n->hz, n->z3, out, cudaMemcpyDeviceToHost, n->st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(n->st);
+        rc = layers_done(n, e, "mlp forward");
+        if (!rc) std::memcpy(y, n->hz, out);
+        return rc;
+    }
     cudaError_t e = upload(n, n->xf, x, (int64_t)batch * n->nin);
     if (e == cudaSuccess) e = forward(n, batch);
     if (e == cudaSuccess) e = cudaMemcpyAsync(y, n->z3, (size_t)batch * n->nout * 4, cudaMemcpyDeviceToHost, n->st);
@@ -501,6 +689,15 @@ int ewpt_mlp_gradients(ewpt_mlp* n, const float* x, const float* y, int32_t batc
     int rc = check_batch(n, batch);
     if (rc) return rc;
     if (!x || !y || !grads) return mlp_fail(n, EWPT_ERR_ARG, "NULL argument");
+    if (n->layers && batch <= kLayerMaxK) {
+        std::memcpy(n->hx, x, (size_t)batch * n->nin * 4);
+        std::memcpy(n->hy, y, (size_t)batch * n->nout * 4);
+        cudaError_t e = layers_run(n, batch, true, false, 0.f, 0.f, 1.f, 1.f);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(grads, n->g, n->np * 4, cudaMemcpyDeviceToHost, n->st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(n->st);
+        if (loss) *loss = n->host[0] / ((float)batch * n->nout);
+        return layers_done(n, e, "mlp gradients");
+    }
     cudaError_t e = upload(n, n->xf, x, (int64_t)batch * n->nin);
     if (e == cudaSuccess) e = upload(n, n->yf, y, (int64_t)batch * n->nout);
     if (e == cudaSuccess) e = forward(n, batch);
@@ -519,6 +716,16 @@ int ewpt_mlp_train_step(ewpt_mlp* n, const float* x, const float* y, int32_t bat
     if (rc) return rc;
     if (!x || !y) return mlp_fail(n, EWPT_ERR_ARG, "NULL argument");
     if (!std::isfinite(lr) || !std::isfinite(weight_decay)) return mlp_fail(n, EWPT_ERR_ARG, "non-finite lr/wd");
+    if (n->layers && batch <= kLayerMaxK) {
+        std::memcpy(n->hx, x, (size_t)batch * n->nin * 4);
+        std::memcpy(n->hy, y, (size_t)batch * n->nout * 4);
+        n->t += 1;
+        cudaError_t e = layers_run(n, batch, true, true, lr, weight_decay, 1.f - std::pow(0.9f, (float)n->t),
+                                   1.f - std::pow(0.999f, (float)n->t));
+        if (e == cudaSuccess) e = cudaStreamSynchronize(n->st);
+        if (loss) *loss = n->host[0] / ((float)batch * n->nout);
+        return layers_done(n, e, "mlp train_step");
+    }
     cudaError_t e = upload(n, n->xf, x, (int64_t)batch * n->nin);
     if (e == cudaSuccess) e = upload(n, n->yf, y, (int64_t)batch * n->nout);
     if (e == cudaSuccess) e = forward(n, batch);
@@ -531,6 +738,7 @@ int ewpt_mlp_train_step(ewpt_mlp* n, const float* x, const float* y, int32_t bat
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = refresh_bf16(n);
+    if (e == cudaSuccess && n->layers) e = layers_pack(n);
     float l = 0.f;
     if (e == cudaSuccess && loss) e = cudaMemcpyAsync(&l, n->loss, 4, cudaMemcpyDeviceToHost, n->st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(n->st);
