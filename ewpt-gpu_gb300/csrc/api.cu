@@ -397,7 +397,7 @@ static int do_steps(ewpt_ctx* c, int32_t nsteps, bool expl, double Jex, double g
         else if (c->tile.pair == 2)
             e = launch_step_fp32_tma(c, J, G);
         else
-            e = fp32_pairs(c->g, c->tile)
+            e = (c->tile.pair && c->g.nx % 2 == 0)
                     ? launch_step_fp32_pair(c->g, c->lay, c->tile, c->y32, c->w32, c->p, J, G, c->st, c->fp32_comp)
                     : launch_step_fp32(c->g, c->lay, c->tile, c->y32, c->w32, c->p, J, G, c->st);
         int rc = ewpt_cuda_check(c, e, "step launch");

@@ -71,10 +71,10 @@ static int ens_capture(ewpt_ens* e) {
             ewpt_ctx* c = e->mem[m];
             le = cudaStreamWaitEvent(c->st, e->fork, 0);
             if (le == cudaSuccess)
-                le = fp32_pairs(c->g, c->tile) ? launch_step_fp32_pair(c->g, c->lay, c->tile, c->y32, c->w32, c->p,
-                                                                       e->jex[m], e->gam[m], c->st)
-                                               : launch_step_fp32(c->g, c->lay, c->tile, c->y32, c->w32, c->p,
-                                                                  e->jex[m], e->gam[m], c->st);
+                le = c->tile.pair ? launch_step_fp32_pair(c->g, c->lay, c->tile, c->y32, c->w32, c->p, e->jex[m],
+                                                          e->gam[m], c->st)
+                                  : launch_step_fp32(c->g, c->lay, c->tile, c->y32, c->w32, c->p, e->jex[m],
+                                                     e->gam[m], c->st);
             if (le == cudaSuccess) le = cudaEventRecord(e->join[m], c->st);
             if (le == cudaSuccess) le = cudaStreamWaitEvent(e->st, e->join[m], 0);
         }

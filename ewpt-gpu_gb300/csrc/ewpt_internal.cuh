@@ -227,24 +227,16 @@ struct Tiling {
 constexpr Tiling kDefaultTiling{32, 4, 0, 0, 1};
 int tiling_max_threads(int reg);
 
-// Two sites per thread?  As the caller chose, or (t.pick) wherever the row
-// allows and the lattice has more sites than the 384 threads per SM that run
-// at once: 24^3 0.051 ms per step with one site and 0.068 with two, 48^3 0.123
-// and 0.111.
-inline bool fp32_pairs(const Grid& g, const Tiling& t) {
-    return g.nx % 2 == 0 && (t.pair || (t.pick && g.S > 152 * 384));
-}
-
 // Launch of the FP32-form kernels over rows of n threads (sites or pairs).
-// The caller's tile, or (t.pick) 64 x 2 threads.  A tile that leaves more than
+// The caller's tile, or (t.pick) 64 x 2 pairs, 32 x 4 sites.  A tile that leaves more than
 // an eighth of its lanes without a site is laid along the rows instead
 // (Walk::flat), paired kernel, ms per step: 160^3 (80 pairs a row) 2.30 against
 // 2.96 for 64 x 2 and 2.43 for 16 x 8 tiles, 96^3 0.594 against 0.606 for
 // 16 x 8, 48^3 0.111 against 0.116 for 8 x 16.
-inline Walk fp32_walk(int n, int ny, int nz, const Tiling& t, dim3& gr, dim3& bl) {
+inline Walk fp32_walk(int n, int ny, int nz, const Tiling& t, bool pairs, dim3& gr, dim3& bl) {
     Walk w{};
     int bx = t.bx, by = t.by;
-    if (t.pick) bx = 64, by = 2;
+    if (t.pick) bx = pairs ? 64 : 32, by = 128 / bx;
     const int64_t padded = (int64_t)((n + bx - 1) / bx * bx) * ((ny + by - 1) / by * by);
     bl = dim3(bx, by);
     if (8 * padded > 9 * (int64_t)n * ny) {

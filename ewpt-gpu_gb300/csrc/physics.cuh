@@ -50,15 +50,6 @@
 
 #include <type_traits>
 
-// Accessors that declare kCompGauge = true give the gauge fields'
-// Laplacians and the auxiliaries' gradients as compensated pairs
-// (grad_lap_c, grad_c; accessors.cuh PairAcc) and site_rates subtracts them
-// before rounding (comp_diff); every other accessor takes the plain path.
-template <class A, class = void>
-struct CompGauge : std::false_type {};
-template <class A>
-struct CompGauge<A, std::void_t<decltype(A::kCompGauge)>> : std::integral_constant<bool, A::kCompGauge> {};
-
 // Accessors that declare kScaledStencils = true return 60 dx times a first
 // derivative or divergence and 180 dx^2 times a Laplacian (FixAcc,
 // fixstencil.cuh); the coefficients of make_phys_scaled absorb the factors.
@@ -115,9 +106,6 @@ EWPT_ARITH void site_rates(const Acc& A, const PhysCoef<T>& c, Sink& out) {
     static_assert(PART == 0 || !BETA, "the beta terms couple every block: PART 0 only");
     constexpr bool kHiggs = PART == 0 || PART == 1, kSU2 = PART == 0 || PART == 2,
                    kRest = PART == 0 || PART == 3;
-    // compensated gauge stencils: kt W^a_i = (lap W^a_i - d_i Gamma^a) + g Q^a_i and
-    // kt Y_i = (lap Y_i - d_i Sigma) + g' jY_i with each bracket formed before rounding
-    constexpr bool kComp = CompGauge<Acc>::value;
     // derivatives in units of t = 1/(60 dx): every sum below that holds one is
     // then in units of t too, and the last factor of its rate restores it
     constexpr bool kScaled = ScaledStencils<Acc>::value;
@@ -287,22 +275,11 @@ EWPT_ARITH void site_rates(const Acc& A, const PhysCoef<T>& c, Sink& out) {
 #pragma unroll
         for (int b = 0; b < 3; ++b) {
             T dW[3][3];  // dW[i][j] = d_j W^b_i
-            if constexpr (kComp) {
-                T Gh[3], Gl[3];
-                A.grad_c(16 + b, Gh, Gl);
 #pragma unroll
-                for (int i = 0; i < 3; ++i) {
-                    T lh, ll;
-                    A.grad_lap_c(4 + 3 * b + i, dW[i][0], dW[i][1], dW[i][2], lh, ll);
-                    Q[b][i] = Q[b][i] + A.comp_diff(lh, ll, Gh[i], Gl[i]) * c.igw;
-                }
-            } else {
-#pragma unroll
-                for (int i = 0; i < 3; ++i) {
-                    T lap;
-                    A.grad_lap(4 + 3 * b + i, dW[i][0], dW[i][1], dW[i][2], lap);
-                    Q[b][i] = Q[b][i] + lap * (kScaled ? c.lap_w : c.igw);
-                }
+            for (int i = 0; i < 3; ++i) {
+                T lap;
+                A.grad_lap(4 + 3 * b + i, dW[i][0], dW[i][1], dW[i][2], lap);
+                Q[b][i] = Q[b][i] + lap * (kScaled ? c.lap_w : c.igw);
             }
             const int b1 = (b + 1) % 3, b2 = (b + 2) % 3;
 #pragma unroll
@@ -325,19 +302,14 @@ EWPT_ARITH void site_rates(const Acc& A, const PhysCoef<T>& c, Sink& out) {
         // the coupling and the auxiliary gradient
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            if constexpr (kComp) {  // the gradient is in Q already
+            T g[3];
+            A.grad(16 + a, g[0], g[1], g[2]);
 #pragma unroll
-                for (int i = 0; i < 3; ++i) ktW[a][i] = c.gw * Q[a][i];
-            } else {
-                T g[3];
-                A.grad(16 + a, g[0], g[1], g[2]);
-#pragma unroll
-                for (int i = 0; i < 3; ++i) {
-                    if constexpr (kScaled)
-                        ktW[a][i] = c.gw_o * (Q[a][i] - g[i] * c.igw);
-                    else
-                        ktW[a][i] = c.gw * Q[a][i] - g[i];
-                }
+            for (int i = 0; i < 3; ++i) {
+                if constexpr (kScaled)
+                    ktW[a][i] = c.gw_o * (Q[a][i] - g[i] * c.igw);
+                else
+                    ktW[a][i] = c.gw * Q[a][i] - g[i];
             }
         }
     }
@@ -346,35 +318,19 @@ EWPT_ARITH void site_rates(const Acc& A, const PhysCoef<T>& c, Sink& out) {
     T ktY[3], FY[3];
     if constexpr (kRest) {
         T dY[3][3], lap[3];
-        if constexpr (kComp) {
-            T Sh[3], Sl[3];
-            A.grad_c(19, Sh, Sl);
 #pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                T lh, ll;
-                A.grad_lap_c(13 + i, dY[i][0], dY[i][1], dY[i][2], lh, ll);
-                lap[i] = A.comp_diff(lh, ll, Sh[i], Sl[i]);  // lap Y_i - d_i Sigma
-            }
-        } else {
-#pragma unroll
-            for (int i = 0; i < 3; ++i) A.grad_lap(13 + i, dY[i][0], dY[i][1], dY[i][2], lap[i]);
-        }
+        for (int i = 0; i < 3; ++i) A.grad_lap(13 + i, dY[i][0], dY[i][1], dY[i][2], lap[i]);
         FY[0] = dY[1][0] - dY[0][1];
         FY[1] = dY[2][0] - dY[0][2];
         FY[2] = dY[2][1] - dY[1][2];
-        if constexpr (kComp) {
+        T g[3];
+        A.grad(19, g[0], g[1], g[2]);
 #pragma unroll
-            for (int i = 0; i < 3; ++i) ktY[i] = lap[i] + c.gy * jY[i];
-        } else {
-            T g[3];
-            A.grad(19, g[0], g[1], g[2]);
-#pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                if constexpr (kScaled)
-                    ktY[i] = c.lap_y * lap[i] + c.gy_o * jY[i] - c.t * g[i];
-                else
-                    ktY[i] = lap[i] + c.gy * jY[i] - g[i];
-            }
+        for (int i = 0; i < 3; ++i) {
+            if constexpr (kScaled)
+                ktY[i] = c.lap_y * lap[i] + c.gy_o * jY[i] - c.t * g[i];
+            else
+                ktY[i] = lap[i] + c.gy * jY[i] - g[i];
         }
     }
 

@@ -22,6 +22,7 @@
 #include <algorithm>
 
 #include "accessors.cuh"
+#include "physics_fp32.cuh"
 #include "convert.cuh"
 #include "fixstencil.cuh"
 
@@ -183,7 +184,7 @@ __global__ void __launch_bounds__(RegBudget<REG>::kThreads, RegBudget<REG>::kMin
     A.place_ghost(i, j, k, g.nx, L);
     A.s = sc;
     Fp32Sink<STAGE> out{A, L, b, xn, h, w6, x2, x3};
-    site_rates<float, BETA>(A, pc, out);
+    site_rates_fp32<float, BETA>(A, pc, out);
 }
 
 // FP64 arrays <-> (hi, lo) in layout L (ghost cells left to k_ghost_fill).
@@ -426,7 +427,7 @@ template <bool BETA, int REG>
 static void step_fp32(const Grid& g, const Layout& L, const Tiling& t, Fp32Bufs b, float* xa, float* xb,
                       const PhysCoef<float>& pc, const StencilCoef<float>& sc, double dt, cudaStream_t st) {
     dim3 gr, bl;
-    const Walk walk = fp32_walk(g.nx, g.ny, g.nz, t, gr, bl);
+    const Walk walk = fp32_walk(g.nx, g.ny, g.nz, t, false, gr, bl);
     const float h2 = (float)(dt / 2.), h1 = (float)dt, w6 = (float)(dt / 6.);
     float* x4m = b.kacc - 20 * L.P;  // X4's momenta
     Ptr36 X4 = pack(xa, L.P, 4);

@@ -13,6 +13,7 @@
 #include <algorithm>
 
 #include "accessors.cuh"
+#include "physics_fp32.cuh"
 
 namespace {
 
@@ -119,7 +120,7 @@ __global__ void __launch_bounds__(PairBudget<REG>::kThreads, PairBudget<REG>::kM
         }
     }
     PairSink<STAGE, PairAcc<SrcPtr36<float>, COMP>> out{A, L, b, xn, h, w6, x2, x3};
-    site_rates<f2, BETA>(A, pc, out);
+    site_rates_fp32<f2, BETA>(A, pc, out);
 }
 
 Ptr36 pack4(const void* base, int64_t S) {
@@ -133,7 +134,7 @@ void step_pair(const Grid& g, const Layout& L, const Tiling& t, PairBufs b, floa
                const PhysCoef<f2>& pc, const StencilCoef<f2>& sc, const StencilCoef<f2>& scl, double dt,
                cudaStream_t st) {
     dim3 gr, bl;
-    const Walk walk = fp32_walk(g.nx / 2, g.ny, g.nz, t, gr, bl);
+    const Walk walk = fp32_walk(g.nx / 2, g.ny, g.nz, t, true, gr, bl);
     const f2 h2((float)(dt / 2.)), h1((float)dt), w6((float)(dt / 6.)), z(0.f);
     float* x4m = b.kacc - 20 * L.P;  // X4's momenta
     Ptr36 X4 = pack4(xa, L.P);

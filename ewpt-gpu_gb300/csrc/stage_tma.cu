@@ -39,6 +39,7 @@
 #include <mutex>
 
 #include "accessors.cuh"
+#include "physics_fp32.cuh"
 #include "ewpt_ctx.cuh"
 
 namespace {
@@ -510,7 +511,7 @@ __global__ void __launch_bounds__(Cfg<TBY, TBZ>::NTHREADS, 1)
         const int i0 = R.x0 + lx, j = R.y0 + ly, k = R.z0 + lz;
         TmaAcc<C, NB> A{R, X, L.P, (int)L.at(i0, j, k), lx, ly, lz, sc};
         TmaSink<STAGE, C, NB> out{A, L, b, xn, h, w6, {0u, 0u, 0u}};
-        site_rates<f2, BETA>(A, pc, out);
+        site_rates_fp32<f2, BETA>(A, pc, out);
     }
 }
 

@@ -1,8 +1,7 @@
 """FP32-form launches laid along the rows (tiles that would leave more than an
 eighth of their lanes without a site): the same bits as tiles, for rows
 shorter and longer than a block, chunks of fewer rows, and one or two sites per
-thread; and the shape picked without ewpt_set_tiling agrees with them to
-FP32 rounding."""
+thread; and the shape picked without ewpt_set_tiling, too."""
 import pytest
 
 import ewpt
@@ -77,10 +76,8 @@ def test_single_rows(shape, flat, tile):
 
 @pytest.mark.parametrize("shape", [(24, 24, 24), (48, 48, 48), (64, 40, 36), (75, 61, 20)])
 def test_picked_shape(shape):
-    """Fields of order one after three steps: FP32 evaluations of the same
-    rates differ by a few roundings (2^-24 = 6e-8) of the terms of a rate
-    (at most ~500 |f|) times 3 dt."""
+    import torch
+
     p = ewpt.baseline_couplings(shape=shape, N=shape[0], precision=ewpt.FP32)
     y = state(shape, 5)
-    a, b = evolve(p, y, None), evolve(p, y, (32, 4, 0, 0))
-    assert float((a - b).abs().max()) < 8 * 2.0 ** -24 * 500 * 3 * p.dt * float(y.abs().max())
+    assert torch.equal(evolve(p, y, None), evolve(p, y, (4, 8, 0, 0)))
