@@ -297,7 +297,7 @@ int ewpt_set_state(ewpt_ctx* c, const double* const arrays[EWPT_NARR], int32_t o
         Ptr36 src;
         for (int a = 0; a < 36; ++a) src.p[a] = arrays[a];
         e = c->p.precision == EWPT_FP32 ? launch_fp32_split(c->g, c->lay, src, c->y32, c->st, c->tile.pair == 2)
-                                        : launch_to_dd(c->g.S, src, c->y, c->st);
+                                        : launch_to_dd(c->g.S, dd_in_pairs(c->g, c->p), src, c->y, c->st);
     } else {
         double* dst;
         int rc = ewpt_staging64(c, &dst, true);
@@ -312,7 +312,7 @@ int ewpt_set_state(ewpt_ctx* c, const double* const arrays[EWPT_NARR], int32_t o
 cudaError_t ewpt_commit_staged(ewpt_ctx* c, const double* staged) {
     if (c->p.precision == EWPT_FP32)  // only the TMA-staged kernels read x ghost cells
         return launch_fp32_split(c->g, c->lay, arrays36(staged, c->g.S), c->y32, c->st, c->tile.pair == 2);
-    if (c->p.precision == EWPT_DF64) return launch_to_dd(c->g.S, arrays36(staged, c->g.S), c->y, c->st);
+    if (c->p.precision == EWPT_DF64) return launch_to_dd(c->g.S, dd_in_pairs(c->g, c->p), arrays36(staged, c->g.S), c->y, c->st);
     return cudaSuccess;
 }
 
@@ -331,7 +331,7 @@ int ewpt_get_state(ewpt_ctx* c, double* const arrays[EWPT_NARR], int32_t on_devi
     for (int a = 0; a < 36; ++a) dst.p[a] = direct ? arrays[a] : src + a * c->g.S;
     cudaError_t e = cudaSuccess;
     if (c->p.precision == EWPT_FP32) e = launch_fp32_join(c->g, c->lay, c->y32, dst, c->st);
-    if (c->p.precision == EWPT_DF64) e = launch_from_dd(c->g.S, c->y, dst, c->st);
+    if (c->p.precision == EWPT_DF64) e = launch_from_dd(c->g.S, dd_in_pairs(c->g, c->p), c->y, dst, c->st);
     if (e == cudaSuccess && !direct) e = copy_runs(c, src, arrays, c->g.S, false, on_device);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->st);
     rc = ewpt_cuda_check(c, e, "get_state");

@@ -370,7 +370,7 @@ int ewpt_higgs64(ewpt_ctx* c, double* out) {
     }
     MPtr36 dst{};
     for (int a = 0; a < 4; ++a) dst.p[a] = out + a * c->g.S;
-    if (c->p.precision == EWPT_DF64) return ewpt_cuda_check(c, launch_from_dd(c->g.S, c->y, dst, c->st, 4), "join");
+    if (c->p.precision == EWPT_DF64) return ewpt_cuda_check(c, launch_from_dd(c->g.S, dd_in_pairs(c->g, c->p), c->y, dst, c->st, 4), "join");
     const int rc = ewpt_tma_check(c);
     return rc ? rc : ewpt_cuda_check(c, launch_fp32_join(c->g, c->lay, c->y32, dst, c->st, 4), "join");
 }
@@ -385,7 +385,7 @@ int ewpt_state64(ewpt_ctx* c, const double** out, int arrays) {
     int rc = ewpt_ensure_scratch64(c);
     if (rc) return rc;
     if (c->p.precision == EWPT_DF64) {
-        rc = ewpt_cuda_check(c, launch_from_dd(c->g.S, c->y, arrays36(c->scratch64, c->g.S), c->st, arrays), "join");
+        rc = ewpt_cuda_check(c, launch_from_dd(c->g.S, dd_in_pairs(c->g, c->p), c->y, arrays36(c->scratch64, c->g.S), c->st, arrays), "join");
     } else {
         rc = ewpt_tma_check(c);
         if (rc) return rc;

@@ -274,9 +274,12 @@ cudaError_t launch_rates_fp64_order(const Grid& g, const Ptr36& in, const MPtr36
 // DF64 form (stage_dd.cu): y, yn, xa, xb hold float pairs (hi, lo).
 cudaError_t launch_step_dd(const Grid& g, const Tiling& t, double* y, double* yn, double* xa, double* xb,
                            double* cur, const ewpt_params& p, double Jex, double gam, cudaStream_t st);
+// Whether a DF64 context evolves two sites per thread; its arrays then hold
+// (hi0, hi1, lo0, lo1) per site pair, else (hi, lo) per site.
+bool dd_in_pairs(const Grid& g, const ewpt_params& p);
 // 36 FP64 arrays of S values <-> [36][S] float pairs (src = the pairs' own buffer: in place)
-cudaError_t launch_to_dd(int64_t S, const Ptr36& src, double* pairs, cudaStream_t st);
-cudaError_t launch_from_dd(int64_t S, const double* pairs, const MPtr36& dst, cudaStream_t st, int arrays = 36);
+cudaError_t launch_to_dd(int64_t S, bool in_pairs, const Ptr36& src, double* pairs, cudaStream_t st);
+cudaError_t launch_from_dd(int64_t S, bool in_pairs, const double* pairs, const MPtr36& dst, cudaStream_t st, int arrays = 36);
 cudaError_t launch_step_fp32(const Grid& g, const Layout& L, const Tiling& t, Fp32State y, Fp32Work w,
                              const ewpt_params& p, double Jex, double gam, cudaStream_t st);
 // comp: the compensated mode (gauge Laplacians and auxiliary gradients compensated, stage_pair.cu)

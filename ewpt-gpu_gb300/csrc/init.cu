@@ -139,7 +139,7 @@ extern "C" int ewpt_init_bubbles(ewpt_ctx* c, int32_t nb, const double* bubbles,
                                    c->y32.lo, c->lay, c->st, &err);
     if (rc) return ewpt_fail(c, rc, "init_bubbles: %s", err.c_str());
     if (c->p.precision == EWPT_DF64) {
-        rc = ewpt_cuda_check(c, launch_to_dd(c->g.S, arrays36((const double*)c->y, c->g.S), c->y, c->st), "init_bubbles");
+        rc = ewpt_cuda_check(c, launch_to_dd(c->g.S, dd_in_pairs(c->g, c->p), arrays36((const double*)c->y, c->g.S), c->y, c->st), "init_bubbles");
         if (rc) return rc;
     }
     c->it = 0;

@@ -381,3 +381,46 @@ EWPT_ARITH void site_rates(const Acc& A, const PhysCoef<T>& c, Sink& out) {
         out(35, ktY[2]);
     }
 }
+
+// PART 1 axis by axis, for arithmetic types whose values take several
+// registers: the gradients of one axis at a time, each Laplacian at the end.
+// The same terms as in site_rates, summed in another order.  Accessor:
+// d1(a, i) and lap(a).
+template <typename T, class Acc, class Sink>
+EWPT_ARITH void higgs_rates_by_axis(const Acc& A, const PhysCoef<T>& c, Sink& out) {
+    const T p[4] = {A.v(0), A.v(1), A.v(2), A.v(3)};
+    T a[4];  // kt_phi over g/2, without the Laplacian
+    {
+        const T mag = p[0] * p[0] + p[1] * p[1] + p[2] * p[2] + p[3] * p[3];
+        const T potg = c.lam2h * (mag - c.vev2) + c.hJexh;
+        const T damp = c.gamh / mag;
+        const T G1 = A.v(16), G2 = A.v(17), G3 = A.v(18), S = c.ryw * A.v(19);
+        const T q12 = G3 + S, q34 = S - G3;
+        a[0] = q12 * p[1] - G2 * p[2] + G1 * p[3] - potg * p[0] - damp * p[0] * (p[0] * A.v(20));
+        a[1] = -q12 * p[0] - G1 * p[2] - G2 * p[3] - potg * p[1] - damp * p[1] * (p[1] * A.v(21));
+        a[2] = q34 * p[3] + G2 * p[0] + G1 * p[1] - potg * p[2] - damp * p[2] * (p[2] * A.v(22));
+        a[3] = -q34 * p[2] - G1 * p[0] + G2 * p[1] - potg * p[3] - damp * p[3] * (p[3] * A.v(23));
+    }
+#pragma unroll 1
+    for (int i = 0; i < 3; ++i) {
+        const T W1 = A.v(4 + i), W2 = A.v(7 + i), W3 = A.v(10 + i), Yr = c.ryw * A.v(13 + i);
+        const T Zp = W3 + Yr, Zm = W3 - Yr;
+        T d1 = A.d1(0, i), d2 = A.d1(1, i), d3 = A.d1(2, i), d4 = A.d1(3, i), D1, D2, D3, D4;
+        cov_deriv_s(d1, d2, d3, d4, p[0], p[1], p[2], p[3], W1, W2, Zp, Zm, c.hgw, D1, D2, D3, D4);
+        out.keep_current(i, p[0] * D4 - p[1] * D3 + p[2] * D2 - p[3] * D1);
+        out.keep_current(3 + i, -p[0] * D3 - p[1] * D4 + p[2] * D1 + p[3] * D2);
+        const T j12 = p[0] * D2 - p[1] * D1, j34 = p[2] * D4 - p[3] * D3;
+        out.keep_current(6 + i, j12 - j34);
+        out.keep_current(9 + i, j12 + j34);
+        d1 += D1;
+        d2 += D2;
+        d3 += D3;
+        d4 += D4;
+        a[0] += W1 * d4 - W2 * d3 + Zp * d2;
+        a[1] -= W1 * d3 + W2 * d4 + Zp * d1;
+        a[2] += W1 * d2 + W2 * d1 - Zm * d4;
+        a[3] -= W1 * d1 - W2 * d2 - Zm * d3;
+    }
+#pragma unroll 1
+    for (int b = 0; b < 4; ++b) out(20 + b, A.lap(b) + c.hgw * (b == 0 ? a[0] : b == 1 ? a[1] : b == 2 ? a[2] : a[3]));
+}

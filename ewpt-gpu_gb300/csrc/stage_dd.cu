@@ -12,6 +12,7 @@
 #include "accessors.cuh"
 #include "convert.cuh"
 #include "dd.cuh"
+#include "dd2.cuh"
 
 namespace {
 
@@ -19,6 +20,8 @@ template <int REG>
 struct DdBudget;
 template <>
 struct DdBudget<0> { static constexpr int kThreads = 128, kMinBlocks = 1; };
+template <>
+struct DdBudget<1> { static constexpr int kThreads = 128, kMinBlocks = 4; };
 template <>
 struct DdBudget<2> { static constexpr int kThreads = 128, kMinBlocks = 3; };
 
@@ -151,6 +154,202 @@ __global__ void __launch_bounds__(DdBudget<REG>::kThreads, DdBudget<REG>::kMinBl
     site_rates<dd, BETA, DdAcc, DdSink<STAGE>, PART>(A, pc, out);
 }
 
+// ------------------------------------------------- two sites per thread
+// Even rows without beta terms, lattices whose pairs fill the SMs (384 threads
+// each; 24^3 0.19 ms per step with one site per thread, 0.24 with two): thread = the x-adjacent sites (i0, i0 + 1), i0
+// even, on packed double-float pairs (dd2.cuh), three launches per stage as
+// above.  The arrays then hold a site pair as (hi0, hi1, lo0, lo1), one
+// 16-byte load; the conversions read and write that order.
+struct Dd2Acc {
+    const float4* x;  // [36][S / 2]
+    int64_t Sp;       // S / 2
+    int c;            // pair index
+    int ox[4];        // pairs at i0 - 4, i0 - 2, i0 + 2, i0 + 4
+    int oy[6], oz[6];
+    StencilCoef<dd2> s;
+
+    __device__ __forceinline__ dd2 at(const float4* p, int off) const { return dd2(__ldg(p + off)); }
+    __device__ __forceinline__ dd2 v(int a) const { return at(x + a * Sp + c, 0); }
+    __device__ __forceinline__ static dd2 odd(const dd2& l, const dd2& r) {
+        return dd2(make_float2(l.hi.y, r.hi.x), make_float2(l.lo.y, r.lo.x));
+    }
+    // neighbours +1, +2, +3, -1, -2, -3 along an axis
+    __device__ __forceinline__ void along(const float4* p, int ax, dd2* f) const {
+        if (ax == 0) {
+            const dd2 qm2 = at(p, ox[0]), qm1 = at(p, ox[1]), q0 = at(p, 0), qp1 = at(p, ox[2]), qp2 = at(p, ox[3]);
+            f[0] = odd(q0, qp1);
+            f[1] = qp1;
+            f[2] = odd(qp1, qp2);
+            f[3] = odd(qm1, q0);
+            f[4] = qm1;
+            f[5] = odd(qm2, qm1);
+        } else {
+            const int* o = ax == 1 ? oy : oz;
+#pragma unroll
+            for (int k = 0; k < 6; ++k) f[k] = at(p, o[k]);
+        }
+    }
+    __device__ __forceinline__ dd2 weigh(const dd2* f) const {
+        return mul2(s.a1, f[0] - f[3]) + mul2(s.a2, f[1] - f[4]) + mul2(s.a3, f[2] - f[5]);
+    }
+    __device__ __forceinline__ dd2 weigh_lap(const dd2& f0, const dd2* S) const {
+        return mul2(s.l0, f0) + mul2(s.l1, S[0]) + mul2(s.l2, S[1]) + mul2(s.l3, S[2]);
+    }
+    __device__ __noinline__ void grad_lap(int a, dd2& gx, dd2& gy, dd2& gz, dd2& lap) const {
+        const float4* p = x + a * Sp + c;
+        dd2 S[3], f[3][6];
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax) along(p, ax, f[ax]);
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax) {
+            (ax == 0 ? gx : (ax == 1 ? gy : gz)) = done2(weigh(f[ax]));
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const dd2 q = f[ax][k] + f[ax][k + 3];
+                S[k] = ax == 0 ? q : S[k] + q;
+            }
+        }
+        lap = done2(weigh_lap(at(p, 0), S));
+    }
+    __device__ __noinline__ dd2 lap(int a) const {
+        const float4* p = x + a * Sp + c;
+        dd2 S[3], f[3][6];
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax) along(p, ax, f[ax]);
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const dd2 q = f[ax][k] + f[ax][k + 3];
+                S[k] = ax == 0 ? q : S[k] + q;
+            }
+        }
+        return done2(weigh_lap(at(p, 0), S));
+    }
+    __device__ __noinline__ dd2 d1(int a, int ax) const {
+        dd2 f[6];
+        along(x + a * Sp + c, ax, f);
+        return done2(weigh(f));
+    }
+    __device__ __noinline__ void grad(int a, dd2& gx, dd2& gy, dd2& gz) const {
+        dd2 f[3][6];
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax) along(x + a * Sp + c, ax, f[ax]);
+        gx = done2(weigh(f[0]));
+        gy = done2(weigh(f[1]));
+        gz = done2(weigh(f[2]));
+    }
+    __device__ __noinline__ dd2 div3(int a) const {
+        dd2 f[3][6];
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax) along(x + (a + ax) * Sp + c, ax, f[ax]);
+        return done2(weigh(f[0]) + weigh(f[1]) + weigh(f[2]));
+    }
+
+    __device__ __forceinline__ void place(int ip, int j, int k, int npx, int ny, int nz) {
+        c = ip + npx * (j + ny * k);
+        ox[0] = ip >= 2 ? -2 : npx - 2;
+        ox[1] = ip >= 1 ? -1 : npx - 1;
+        ox[2] = ip + 1 < npx ? 1 : 1 - npx;
+        ox[3] = ip + 2 < npx ? 2 : 2 - npx;
+        axis_offsets(j, ny, npx, oy);
+        axis_offsets(k, nz, npx * ny, oz);
+    }
+};
+
+template <int STAGE>
+struct Dd2Sink {
+    const Dd2Acc& A;
+    const float4* __restrict__ y;
+    float4* yn;
+    float4* xn;
+    dd2 w, h;
+    float4* cur;  // [12][S / 2] Higgs currents, as DdSink::cur
+    __device__ __forceinline__ void keep_current(int q, const dd2& v) const { cur[q * A.Sp + A.c] = done2(v).f4(); }
+    __device__ __forceinline__ dd2 load_current(int q) const { return dd2(__ldg(cur + q * A.Sp + A.c)); }
+    __device__ __forceinline__ void operator()(int a, const dd2& rate) const {
+        const int64_t q = a * A.Sp + A.c;
+        const dd2 r = done2(rate);
+        if (STAGE < 4) {
+            // read then written by this thread only: read-only path is safe
+            const dd2 ya = STAGE == 1 ? A.v(a) : dd2(__ldg(y + q));  // X1 == y
+            yn[q] = done2((STAGE == 1 ? ya : dd2(__ldg(yn + q))) + w * r).f4();
+            xn[q] = done2(ya + h * r).f4();
+        } else {
+            xn[q] = done2(dd2(__ldg(yn + q)) + w * r).f4();  // the new y
+        }
+    }
+};
+
+template <int STAGE, int REG, int PART>
+__global__ void __launch_bounds__(DdBudget<REG>::kThreads, DdBudget<REG>::kMinBlocks)
+    k_stage_dd2(Grid g, const float4* __restrict__ X, const float4* __restrict__ y, float4* yn, float4* xn,
+                const __grid_constant__ PhysCoef<dd2> pc, const __grid_constant__ StencilCoef<dd2> sc, dd2 w, dd2 h,
+                float4* cur, Walk walk) {
+    int ip, j, k;
+    const int npx = g.nx >> 1;
+    if (!walk.site(npx, g.ny, g.nz, ip, j, k)) return;
+    Dd2Acc A;
+    A.x = X;
+    A.Sp = g.S >> 1;
+    A.place(ip, j, k, npx, g.ny, g.nz);
+    A.s = sc;
+    Dd2Sink<STAGE> out{A, y, yn, xn, w, h, cur};
+    if constexpr (PART == 1)
+        higgs_rates_by_axis<dd2>(A, pc, out);
+    else
+        site_rates<dd2, false, Dd2Acc, Dd2Sink<STAGE>, PART>(A, pc, out);
+}
+
+template <int STAGE, int REG>
+void stage_dd2(const Grid& g, const Tiling& t, cudaStream_t st, const double* X, double* y, double* yn, double* xn,
+               const PhysCoef<dd2>& pc, const StencilCoef<dd2>& sc, dd2 w, dd2 h, double* cur) {
+    dim3 gr, bl;
+    const Walk walk = fp32_walk(g.nx / 2, g.ny, g.nz, t, true, gr, bl);
+    auto f = [](const double* v) { return reinterpret_cast<float4*>(const_cast<double*>(v)); };
+    k_stage_dd2<STAGE, REG, 1><<<gr, bl, 0, st>>>(g, f(X), f(y), f(yn), f(xn), pc, sc, w, h, f(cur), walk);
+    k_stage_dd2<STAGE, REG, 2><<<gr, bl, 0, st>>>(g, f(X), f(y), f(yn), f(xn), pc, sc, w, h, f(cur), walk);
+    k_stage_dd2<STAGE, REG, 3><<<gr, bl, 0, st>>>(g, f(X), f(y), f(yn), f(xn), pc, sc, w, h, f(cur), walk);
+}
+
+template <int REG>
+void step_dd2(const Grid& g, const Tiling& t, double* y, double* yn, double* xa, double* xb, double* cur,
+              const ewpt_params& p, double Jex, double gam, cudaStream_t st) {
+    const PhysCoef<dd2> pc = make_phys<dd2>(p, Jex, gam);
+    const StencilCoef<dd2> sc = make_stencil<dd2>(p.dx);
+    const dd2 w6(p.dt / 6.), w3(p.dt / 3.), h2(p.dt / 2.), h1(p.dt), z(0.0);
+    stage_dd2<1, REG>(g, t, st, y, y, yn, xa, pc, sc, w6, h2, cur);
+    stage_dd2<2, REG>(g, t, st, xa, y, yn, xb, pc, sc, w3, h2, cur);
+    stage_dd2<3, REG>(g, t, st, xb, y, yn, xa, pc, sc, w3, h1, cur);
+    stage_dd2<4, REG>(g, t, st, xa, y, yn, y, pc, sc, w6, z, cur);
+}
+
+// The same conversions for arrays in site pairs: S even, a thread per pair.
+__global__ void __launch_bounds__(256) k_to_dd2(int64_t Sp, const __grid_constant__ Ptr36 src, float4* pairs) {
+    const double* v = reinterpret_cast<const double*>(src.p[blockIdx.y]);
+    float4* out = pairs + blockIdx.y * Sp;
+#pragma unroll 2
+    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < Sp; q += (int64_t)gridDim.x * blockDim.x) {
+        const double a = v[2 * q], b = v[2 * q + 1];
+        float4 f;
+        split_f64(a, f.x, f.z);
+        split_f64(b, f.y, f.w);
+        out[q] = f;
+    }
+}
+
+__global__ void __launch_bounds__(256) k_from_dd2(int64_t Sp, const float4* __restrict__ pairs,
+                                                  const __grid_constant__ MPtr36 dst) {
+    const float4* in = pairs + blockIdx.y * Sp;
+    double* out = reinterpret_cast<double*>(dst.p[blockIdx.y]);
+#pragma unroll 2
+    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < Sp; q += (int64_t)gridDim.x * blockDim.x) {
+        const float4 f = __ldg(in + q);
+        out[2 * q] = join_f64(f.x, f.z);
+        out[2 * q + 1] = join_f64(f.y, f.w);
+    }
+}
+
 // FP64 arrays <-> float pairs (convert.cuh), array blockIdx.y; in place when
 // the pairs lie over the array itself, each element by one thread.  Bound by
 // memory: 1.2 GB at 128^3; with C casts k_to_dd / k_from_dd took 557 / 411 us
@@ -219,6 +418,17 @@ void step_dd_r(const Grid& g, const Tiling& t, float2* y, float2* yn, float2* xa
 
 cudaError_t launch_step_dd(const Grid& g, const Tiling& t, double* y, double* yn, double* xa, double* xb,
                            double* cur, const ewpt_params& p, double Jex, double gam, cudaStream_t st) {
+    if (dd_in_pairs(g, p)) {
+        // 128 registers run fastest (256^3: 46.9 ms per step against 48.2 with
+        // 168 and 55.9 with 255)
+        if (t.reg == 0 && !t.pick)
+            step_dd2<0>(g, t, y, yn, xa, xb, cur, p, Jex, gam, st);
+        else if (t.reg == 2)
+            step_dd2<2>(g, t, y, yn, xa, xb, cur, p, Jex, gam, st);
+        else
+            step_dd2<1>(g, t, y, yn, xa, xb, cur, p, Jex, gam, st);
+        return cudaGetLastError();
+    }
     const PhysCoef<dd> pc = make_phys<dd>(p, Jex, gam);
     const StencilCoef<dd> sc = make_stencil<dd>(p.dx);
     auto f2p = [](double* v) { return reinterpret_cast<float2*>(v); };
@@ -229,12 +439,22 @@ cudaError_t launch_step_dd(const Grid& g, const Tiling& t, double* y, double* yn
     return cudaGetLastError();
 }
 
-cudaError_t launch_to_dd(int64_t S, const Ptr36& src, double* pairs, cudaStream_t st) {
-    k_to_dd<<<pair_grid(S, 36), 256, 0, st>>>(S, src, reinterpret_cast<float2*>(pairs));
+bool dd_in_pairs(const Grid& g, const ewpt_params& p) {
+    return g.nx % 2 == 0 && p.beta_w == 0.0 && p.beta_y == 0.0 && g.S > 152 * 768;
+}
+
+cudaError_t launch_to_dd(int64_t S, bool in_pairs, const Ptr36& src, double* pairs, cudaStream_t st) {
+    if (in_pairs)
+        k_to_dd2<<<pair_grid(S / 2, 36), 256, 0, st>>>(S / 2, src, reinterpret_cast<float4*>(pairs));
+    else
+        k_to_dd<<<pair_grid(S, 36), 256, 0, st>>>(S, src, reinterpret_cast<float2*>(pairs));
     return cudaGetLastError();
 }
 
-cudaError_t launch_from_dd(int64_t S, const double* pairs, const MPtr36& dst, cudaStream_t st, int arrays) {
-    k_from_dd<<<pair_grid(S, arrays), 256, 0, st>>>(S, reinterpret_cast<const float2*>(pairs), dst);
+cudaError_t launch_from_dd(int64_t S, bool in_pairs, const double* pairs, const MPtr36& dst, cudaStream_t st, int arrays) {
+    if (in_pairs)
+        k_from_dd2<<<pair_grid(S / 2, arrays), 256, 0, st>>>(S / 2, reinterpret_cast<const float4*>(pairs), dst);
+    else
+        k_from_dd<<<pair_grid(S, arrays), 256, 0, st>>>(S, reinterpret_cast<const float2*>(pairs), dst);
     return cudaGetLastError();
 }

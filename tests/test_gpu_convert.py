@@ -48,7 +48,7 @@ def bits(a):
 
 
 @pytest.mark.parametrize("form", [ewpt.FP32, ewpt.DF64])
-@pytest.mark.parametrize("shape", [(7, 7, 7), (33, 9, 11), (70, 64, 8)])
+@pytest.mark.parametrize("shape", [(7, 7, 7), (33, 9, 11), (70, 64, 8), (66, 62, 30)])
 def test_split_and_join_are_the_casts(form, shape):
     import torch
 
