@@ -391,7 +391,7 @@ static int do_steps(ewpt_ctx* c, int32_t nsteps, bool expl, double Jex, double g
         if (c->p.precision == EWPT_FP64 && c->p.stencil_order != 6)
             e = launch_step_fp64_order(c->g, c->tile, c->y, c->yn, c->xa, c->xb, c->p, J, G, c->st);
         else if (c->p.precision == EWPT_FP64)
-            e = launch_step_fp64(c->g, c->tile, c->y, c->yn, c->xa, c->xb, c->p, J, G, c->st);
+            e = launch_step_fp64(c->g, c->y, c->yn, c->xa, c->xb, c->p, J, G, c->st);
         else if (c->p.precision == EWPT_DF64)
             e = launch_step_dd(c->g, c->tile, c->y, c->yn, c->xa, c->xb, c->ddcur, c->p, J, G, c->st);
         else if (c->tile.pair == 2)
@@ -467,7 +467,7 @@ static int step_host_overlapped(ewpt_ctx* c, const double* in, double* out, int3
     };
     auto stage = [&](int s, int k0, int k1, double J, double G) {
         if (e == cudaSuccess)
-            e = launch_stage_fp64_planes(g, c->tile, s, k0, k1, c->y, c->yn, c->xa, c->xb, c->p, J, G, c->st);
+            e = launch_stage_fp64_planes(g, s, k0, k1, c->y, c->yn, c->xa, c->xb, c->p, J, G, c->st);
     };
     for (int32_t s = 0; s < nsteps && e == cudaSuccess; ++s) {
         const int64_t it = c->it + 1 + s;

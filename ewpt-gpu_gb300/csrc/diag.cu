@@ -204,9 +204,6 @@ __device__ __forceinline__ void make_dacc(const Grid& g, const double* y, const 
     axis_offsets(i, g.nx, 1, A.o[0]);
     axis_offsets(j, g.ny, g.nx, A.o[1]);
     axis_offsets(k, g.nz, g.nx * g.ny, A.o[2]);
-#pragma unroll
-    for (int d = 0; d < 3; ++d) A.s[d] = kc.a[d];
-    A.T = 1.0 / kc.t;
 }
 
 template <int R>

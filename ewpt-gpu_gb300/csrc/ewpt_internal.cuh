@@ -17,12 +17,8 @@ struct Grid {
     int nx, ny, nz;
     int64_t S;  // nx*ny*nz, or the padded array stride of a slab
     int zg = 0;
-    // FP64 stage launches over a window of z planes: the launch's block z
-    // index b covers plane k0 + b (0 for whole-lattice launches)
+    // FP64 stage launches over a window of z planes: the first of them
     int k0 = 0;
-    // FP64 stage launches: > 0 = a 1-D launch over this many sites, x fastest,
-    // then y, then the planes from k0 on; 0 = tiles over x-y, one plane per block
-    int flat = 0;
 };
 
 // Storage of one FP32-form [36][.] array set: element (i, j, k) of array a
@@ -155,36 +151,6 @@ PhysCoef<T> make_phys(const ewpt_params& p, double Jex, double gam) {
     c.gamh = (T)(gam / (0.5 * p.gw));
     c.ryw = (T)(p.gy / p.gw);
     c.igw = (T)(1.0 / p.gw);
-    c.hgw_d = c.hgw;
-    c.gw_d = c.gw;
-    c.omgp2_d = c.omgp2;
-    c.it = c.t = c.hgw_o = c.gw_o = c.gy_o = c.lap_h = c.lap_w = c.lap_y = T(0);
-    return c;
-}
-
-// Coefficients for an accessor with scaled stencils (physics.cuh): first
-// derivatives in units of t = 1/(60 dx), Laplacians of 1/(180 dx^2).
-inline PhysCoef<double> make_phys_scaled(const ewpt_params& p, double Jex, double gam) {
-    PhysCoef<double> c = make_phys<double>(p, Jex, gam);
-    const double T = 60.0 * p.dx, iU = 1.0 / (180.0 * p.dx * p.dx);
-    c.it = T;
-    c.t = 1.0 / T;
-    c.hgw_d = T * c.hgw;
-    c.gw_d = T * c.gw;
-    c.omgp2_d = c.omgp2 / T;
-    c.lam2h *= T;
-    c.hJexh *= T;
-    c.gamh *= T;
-    c.hgw_o = c.hgw / T;
-    c.gw_o = c.gw / T;
-    c.gy_o = c.gy / T;
-    c.lap_h = iU / c.hgw_o;
-    c.lap_w = iU / c.gw_o;
-    c.lap_y = iU;
-    c.bW /= T;
-    c.bY /= T;
-    c.bW2 /= T;
-    c.bY2 /= T;
     return c;
 }
 
@@ -253,19 +219,18 @@ inline Walk fp32_walk(int n, int ny, int nz, const Tiling& t, bool pairs, dim3& 
     return w;
 }
 
-cudaError_t launch_step_fp64(const Grid& g, const Tiling& t, double* y, double* yn, double* xa, double* xb,
-                             const ewpt_params& p, double Jex, double gam, cudaStream_t st);
+cudaError_t launch_step_fp64(const Grid& g, double* y, double* yn, double* xa, double* xb, const ewpt_params& p,
+                             double Jex, double gam, cudaStream_t st);
 // One stage (1..4) of that step (z-slabs exchange ghost planes between stages).
-cudaError_t launch_stage_fp64(const Grid& g, const Tiling& t, int stage, double* y, double* yn, double* xa,
-                              double* xb, const ewpt_params& p, double Jex, double gam, cudaStream_t st);
+cudaError_t launch_stage_fp64(const Grid& g, int stage, double* y, double* yn, double* xa, double* xb,
+                              const ewpt_params& p, double Jex, double gam, cudaStream_t st);
 // The same stage over the z planes [k0, k1) only: those sites' outputs are
 // what a whole-lattice launch writes for them, bit for bit, and no other
 // site is written.  Reads the stage input on planes [k0 - 3, k1 + 3)
 // (periodic).  Lets a host-to-host step start stage 1 on the planes already
 // uploaded and download the planes stage 4 has finished.
-cudaError_t launch_stage_fp64_planes(const Grid& g, const Tiling& t, int stage, int k0, int k1, double* y,
-                                     double* yn, double* xa, double* xb, const ewpt_params& p, double Jex,
-                                     double gam, cudaStream_t st);
+cudaError_t launch_stage_fp64_planes(const Grid& g, int stage, int k0, int k1, double* y, double* yn, double* xa,
+                                     double* xb, const ewpt_params& p, double Jex, double gam, cudaStream_t st);
 // FP64 stage and rates with the alternative stencil orders (stage_orders.cu)
 cudaError_t launch_step_fp64_order(const Grid& g, const Tiling& t, double* y, double* yn, double* xa, double* xb,
                                    const ewpt_params& p, double Jex, double gam, cudaStream_t st);

@@ -18,9 +18,8 @@
 // and shifts (about 20): some 450 integer instructions for a gradient with
 // Laplacian, against 37 FP64 instructions (2368 issue slots).  A step of the
 // FP64 form at 256^3 went from 144.4 to 76.1 ms (64^3: 2.41 to 1.20) with
-// these stencils, the factored physics and 16 warps per SM; ncu at 96^3: 501
-// FP64 instructions per warp and stage (1046 before), FP64 pipe 66% busy,
-// instruction fetch and fixed latencies the largest stalls.
+// these stencils and the factored physics, 1046 FP64 instructions per warp and
+// stage to 501, and to 68.4 (1.15) with four warps per 32 sites (stage_fp64.cu).
 //
 // Stencils whose largest magnitude lies outside [2^-895, 2^977] (denormals,
 // infinities and NaN among them) take the floating-point evaluation, a
@@ -92,12 +91,11 @@ __device__ __forceinline__ int64_t weigh_lap(int64_t t1, int64_t t2, int64_t t3)
 
 }  // namespace fix
 
-// SiteAcc's FP64 stencils on the integer pipes.  The routines are out-of-line
+// SiteAcc's FP64 stencils on the integer pipes, first derivatives and
+// divergences times 60 dx, Laplacians times 180 dx^2.  The routines are out-of-line
 // calls: inlined 24 times they would be far larger than the instruction cache.
 struct FixAcc : SiteAcc<double, double, SrcPtr36<double>> {
     using Base = SiteAcc<double, double, SrcPtr36<double>>;
-    static constexpr bool kScaledStencils = true;  // 60 dx grad and div, 180 dx^2 lap
-    double T, U;                                   // 60 dx, 180 dx^2 (the floating-point evaluation)
 
     __device__ __noinline__ void grad_lap(int a, double& gx, double& gy, double& gz, double& lap) const {
         const double* p = src.arr(a) + c;
@@ -119,10 +117,11 @@ struct FixAcc : SiteAcc<double, double, SrcPtr36<double>> {
                 gx = gy = gz = lap = 0.0;
             else {
                 Base::grad_lap(a, gx, gy, gz, lap);
+                const double T = 1.0 / s.a3;
                 gx *= T;
                 gy *= T;
                 gz *= T;
-                lap *= U;
+                lap *= 2.0 / s.l3;  // 180 dx^2
             }
             return;
         }
@@ -166,6 +165,7 @@ struct FixAcc : SiteAcc<double, double, SrcPtr36<double>> {
                 gx = gy = gz = 0.0;
             else {
                 Base::grad(a, gx, gy, gz);
+                const double T = 1.0 / s.a3;
                 gx *= T;
                 gy *= T;
                 gz *= T;
@@ -199,7 +199,7 @@ struct FixAcc : SiteAcc<double, double, SrcPtr36<double>> {
         for (int ax = 0; ax < 3; ++ax)
 #pragma unroll
             for (int k = 0; k < 6; ++k) e = max(e, fix::exp20(f[ax][k]));
-        if (!fix::covered(e)) return e == 0 && fix::zero_bits(f) ? 0.0 : T * Base::div3(a);
+        if (!fix::covered(e)) return e == 0 && fix::zero_bits(f) ? 0.0 : Base::div3(a) / s.a3;
         const uint32_t ep = e + (7u << 20);
         int64_t V = 0;  // three axes: two bits more than one derivative
 #pragma unroll
@@ -220,16 +220,14 @@ struct FixDiff {
     int64_t S;
     int c;
     int o[3][6];  // [+1, +2, +3, -1, -2, -3] along x, y, z
-    double T;     // 60 dx
-    double s[3];  // 45, -9, 1 over 60 dx (the floating-point evaluation)
 
     __device__ __forceinline__ double v(int q) const { return __ldg(y + q * S + c); }
+    // the floating-point evaluation
     __device__ __forceinline__ double d1(int q, int ax) const {
         const double* p = y + q * S + c;
-        double r = 0.0;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) r += s[k] * (__ldg(p + o[ax][k]) - __ldg(p + o[ax][k + 3]));
-        return r;
+        const int* n = o[ax];
+        return 45.0 * (__ldg(p + n[0]) - __ldg(p + n[3])) - 9.0 * (__ldg(p + n[1]) - __ldg(p + n[4])) +
+               (__ldg(p + n[2]) - __ldg(p + n[5]));
     }
     __device__ __forceinline__ static int64_t weighed(const double* f, uint32_t ep) {
         int64_t D[3];
@@ -256,9 +254,9 @@ struct FixDiff {
         } else if (e == 0 && fix::zero_bits(f)) {
             gx = gy = gz = 0.0;
         } else {
-            gx = T * d1(q, 0);
-            gy = T * d1(q, 1);
-            gz = T * d1(q, 2);
+            gx = d1(q, 0);
+            gy = d1(q, 1);
+            gz = d1(q, 2);
         }
     }
     // d_a q - d_b r
@@ -277,7 +275,7 @@ struct FixDiff {
             const uint32_t ep = e + (7u << 20);
             return fix::to_double((weighed(f[0], ep) >> 1) - (weighed(f[1], ep) >> 1), e, 1);
         }
-        return e == 0 && fix::zero_bits(f) ? 0.0 : T * (d1(q, a) - d1(r, b));
+        return e == 0 && fix::zero_bits(f) ? 0.0 : d1(q, a) - d1(r, b);
     }
     // dx q + dy (q + 1) + dz (q + 2)
     __device__ __noinline__ double div(int q) const {
@@ -295,6 +293,6 @@ struct FixDiff {
             const uint32_t ep = e + (7u << 20);
             return fix::to_double((weighed(f[0], ep) >> 2) + (weighed(f[1], ep) >> 2) + (weighed(f[2], ep) >> 2), e, 2);
         }
-        return e == 0 && fix::zero_bits(f) ? 0.0 : T * (d1(q, 0) + d1(q + 1, 1) + d1(q + 2, 2));
+        return e == 0 && fix::zero_bits(f) ? 0.0 : d1(q, 0) + d1(q + 1, 1) + d1(q + 2, 2);
     }
 };

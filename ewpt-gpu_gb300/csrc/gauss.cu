@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(1024) k_fold_moments(const double* __restrict_
 }
 
 // difference operator over a [.][S] buffer at the site of this thread
-__device__ __forceinline__ bool site_of(const Grid& g, const double* y, double t, FixDiff& A, int* parity) {
+__device__ __forceinline__ bool site_of(const Grid& g, const double* y, FixDiff& A, int* parity) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if ((int64_t)blockIdx.x * blockDim.x + threadIdx.x >= g.S) return false;
     const int row = q / g.nx, i = q - row * g.nx, k = row / g.ny, j = row - k * g.ny;
@@ -153,10 +153,6 @@ __device__ __forceinline__ bool site_of(const Grid& g, const double* y, double t
     axis_offsets(i, g.nx, 1, A.o[0]);
     axis_offsets(j, g.ny, g.nx, A.o[1]);
     axis_offsets(k, g.nz, g.nx * g.ny, A.o[2]);
-    A.T = 1.0 / t;
-    A.s[0] = 45.0 * t;
-    A.s[1] = -9.0 * t;
-    A.s[2] = t;
     if (parity) *parity = (k & 1) * 4 + (j & 1) * 2 + (i & 1);
     return true;
 }
@@ -170,7 +166,7 @@ __global__ void __launch_bounds__(128, 4) k_source(Grid g, double* __restrict__ 
                                                    double gw, double gy, double t, double* __restrict__ src, int64_t Sp) {
     FixDiff A;
     int cls;
-    if (!site_of(g, y, t, A, &cls)) return;
+    if (!site_of(g, y, A, &cls)) return;
     const int64_t q = A.c;
     double ph[4], pi[4], u[4], rho[4], d[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
@@ -213,7 +209,7 @@ __global__ void __launch_bounds__(256) k_solve(Grid g, const double* __restrict_
 __global__ void __launch_bounds__(128, 4) k_subtract(Grid g, double* __restrict__ y, const double* __restrict__ chi,
                                                      int64_t Sp, double t) {
     FixDiff A;
-    if (!site_of(g, chi, t, A, nullptr)) return;
+    if (!site_of(g, chi, A, nullptr)) return;
     A.S = Sp;
 #pragma unroll
     for (int a = 0; a < 4; ++a) {

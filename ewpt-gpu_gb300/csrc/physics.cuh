@@ -48,17 +48,6 @@
 #define EWPT_ARITH __device__ __forceinline__
 #endif
 
-#include <type_traits>
-
-// Accessors that declare kScaledStencils = true return 60 dx times a first
-// derivative or divergence and 180 dx^2 times a Laplacian (FixAcc,
-// fixstencil.cuh); the coefficients of make_phys_scaled absorb the factors.
-template <class A, class = void>
-struct ScaledStencils : std::false_type {};
-template <class A>
-struct ScaledStencils<A, std::void_t<decltype(A::kScaledStencils)>>
-    : std::integral_constant<bool, A::kScaledStencils> {};
-
 template <typename T>
 struct PhysCoef {
     T gw, gy, hgw, hgy;  // g, g', g/2, g'/2
@@ -70,12 +59,6 @@ struct PhysCoef {
     T gg, ggy;           // gp2*g, gp2*g'
     T lam2h, hJexh, gamh;// 2*lambda, Jex/2 and gamma over g/2
     T ryw, igw;          // g'/g, 1/g
-    // couplings where a product meets a derivative: hgw, gw and omgp2, or with
-    // scaled stencils (derivatives in units of t = 1/(60 dx)) hgw/t, gw/t, omgp2 t
-    T hgw_d, gw_d, omgp2_d;
-    // scaled stencils only: 1/t, t, then the factors that end a rate (t g/2,
-    // t g, t g') and those of a Laplacian in its sum
-    T it, t, hgw_o, gw_o, gy_o, lap_h, lap_w, lap_y;
 };
 
 // Covariant derivatives D_i phi_a (cov_derivs_temporal.jl:23-130) along one
@@ -106,10 +89,7 @@ EWPT_ARITH void site_rates(const Acc& A, const PhysCoef<T>& c, Sink& out) {
     static_assert(PART == 0 || !BETA, "the beta terms couple every block: PART 0 only");
     constexpr bool kHiggs = PART == 0 || PART == 1, kSU2 = PART == 0 || PART == 2,
                    kRest = PART == 0 || PART == 3;
-    // derivatives in units of t = 1/(60 dx): every sum below that holds one is
-    // then in units of t too, and the last factor of its rate restores it
-    constexpr bool kScaled = ScaledStencils<Acc>::value;
-    const T hgw = c.hgw_d, gw_d = c.gw_d;
+    const T hgw = c.hgw;
     const T p1 = A.v(0), p2 = A.v(1), p3 = A.v(2), p4 = A.v(3);
     T W[3][3];  // W[a][i] = W_{a+1}_{i+2}
 #pragma unroll
@@ -117,13 +97,7 @@ EWPT_ARITH void site_rates(const Acc& A, const PhysCoef<T>& c, Sink& out) {
 #pragma unroll
         for (int i = 0; i < 3; ++i) W[a][i] = A.v(4 + 3 * a + i);
     const T Y2 = A.v(13), Y3 = A.v(14), Y4 = A.v(15);
-    T G[3] = {A.v(16), A.v(17), A.v(18)};
-    T S = A.v(19);
-    if constexpr (kScaled) {
-#pragma unroll
-        for (int a = 0; a < 3; ++a) G[a] = G[a] * c.it;
-        S = S * c.it;
-    }
+    const T G[3] = {A.v(16), A.v(17), A.v(18)}, S = A.v(19);
     const T pt1 = A.v(20), pt2 = A.v(21), pt3 = A.v(22), pt4 = A.v(23);
 
     // ---- k_field = momentum (main_rk4.jl:585-600)
@@ -150,9 +124,9 @@ EWPT_ARITH void site_rates(const Acc& A, const PhysCoef<T>& c, Sink& out) {
             else q = q12 - q34;
             q = q - W[b][0] * Wt[cc][0] + W[cc][0] * Wt[b][0] - W[b][1] * Wt[cc][1] + W[cc][1] * Wt[b][1] -
                 W[b][2] * Wt[cc][2] + W[cc][2] * Wt[b][2];
-            out(16 + a, c.omgp2_d * A.div3(24 + 3 * a) + c.gg * q);
+            out(16 + a, c.omgp2 * A.div3(24 + 3 * a) + c.gg * q);
         }
-        out(19, c.omgp2_d * A.div3(33) + c.ggy * (q12 + q34));
+        out(19, c.omgp2 * A.div3(33) + c.ggy * (q12 + q34));
     }
 
     // ---- Higgs block: gradients, covariant derivatives, kt_phi (main_rk4.jl:337-407)
@@ -244,17 +218,10 @@ EWPT_ARITH void site_rates(const Acc& A, const PhysCoef<T>& c, Sink& out) {
         T a4 = -W[0][0] * d1[0] - W[0][1] * d1[1] - W[0][2] * d1[2] + W[1][0] * d2[0] + W[1][1] * d2[1] +
                W[1][2] * d2[2] + Zm[0] * d3[0] + Zm[1] * d3[1] + Zm[2] * d3[2] - q34 * p3 - G[0] * p1 + G[1] * p2 -
                potg * p4 - damp * p4 * (p4 * pt4);
-        if constexpr (kScaled) {
-            ktp1 = c.hgw_o * (a1 + l1 * c.lap_h);
-            ktp2 = c.hgw_o * (a2 + l2 * c.lap_h);
-            ktp3 = c.hgw_o * (a3 + l3 * c.lap_h);
-            ktp4 = c.hgw_o * (a4 + l4 * c.lap_h);
-        } else {
-            ktp1 = l1 + hgw * a1;
-            ktp2 = l2 + hgw * a2;
-            ktp3 = l3 + hgw * a3;
-            ktp4 = l4 + hgw * a4;
-        }
+        ktp1 = l1 + hgw * a1;
+        ktp2 = l2 + hgw * a2;
+        ktp3 = l3 + hgw * a3;
+        ktp4 = l4 + hgw * a4;
     }
 
     // ---- SU(2) block, one colour at a time (field_strengths.jl:34-224)
@@ -279,7 +246,7 @@ EWPT_ARITH void site_rates(const Acc& A, const PhysCoef<T>& c, Sink& out) {
             for (int i = 0; i < 3; ++i) {
                 T lap;
                 A.grad_lap(4 + 3 * b + i, dW[i][0], dW[i][1], dW[i][2], lap);
-                Q[b][i] = Q[b][i] + lap * (kScaled ? c.lap_w : c.igw);
+                Q[b][i] = Q[b][i] + lap * c.igw;
             }
             const int b1 = (b + 1) % 3, b2 = (b + 2) % 3;
 #pragma unroll
@@ -290,7 +257,7 @@ EWPT_ARITH void site_rates(const Acc& A, const PhysCoef<T>& c, Sink& out) {
 #pragma unroll
             for (int m = 0; m < 3; ++m) {
                 const int i = m == 2 ? 1 : 0, j = m == 0 ? 1 : 2;
-                const T Fij = dW[j][i] - dW[i][j] + gw_d * (W[b1][i] * W[b2][j] - W[b1][j] * W[b2][i]);
+                const T Fij = dW[j][i] - dW[i][j] + c.gw * (W[b1][i] * W[b2][j] - W[b1][j] * W[b2][i]);
                 if (BETA) F[b][m] = Fij;
                 const T Eij = Fij - dW[i][j], mEji = Fij + dW[j][i];  // E_ij and -E_ji
                 Q[b2][i] = Q[b2][i] + W[b1][j] * Eij;
@@ -305,12 +272,7 @@ EWPT_ARITH void site_rates(const Acc& A, const PhysCoef<T>& c, Sink& out) {
             T g[3];
             A.grad(16 + a, g[0], g[1], g[2]);
 #pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                if constexpr (kScaled)
-                    ktW[a][i] = c.gw_o * (Q[a][i] - g[i] * c.igw);
-                else
-                    ktW[a][i] = c.gw * Q[a][i] - g[i];
-            }
+            for (int i = 0; i < 3; ++i) ktW[a][i] = c.gw * Q[a][i] - g[i];
         }
     }
 
@@ -326,12 +288,7 @@ EWPT_ARITH void site_rates(const Acc& A, const PhysCoef<T>& c, Sink& out) {
         T g[3];
         A.grad(19, g[0], g[1], g[2]);
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            if constexpr (kScaled)
-                ktY[i] = c.lap_y * lap[i] + c.gy_o * jY[i] - c.t * g[i];
-            else
-                ktY[i] = lap[i] + c.gy * jY[i] - g[i];
-        }
+        for (int i = 0; i < 3; ++i) ktY[i] = lap[i] + c.gy * jY[i] - g[i];
     }
 
     // ---- beta (CP-odd) terms

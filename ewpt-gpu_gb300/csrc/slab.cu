@@ -104,7 +104,7 @@ int ewpt_slab_stage(ewpt_ctx* c, int32_t stage, double Jex, double gamma) {
     if (stage < 1 || stage > 4) return ewpt_fail(c, EWPT_ERR_ARG, "stage %d: 1..4", stage);
     if (!std::isfinite(Jex) || !std::isfinite(gamma)) return ewpt_fail(c, EWPT_ERR_ARG, "non-finite Jex/gamma");
     cudaSetDevice(c->p.device);
-    rc = ewpt_cuda_check(c, launch_stage_fp64(c->g, c->tile, stage, c->y, c->yn, c->xa, c->xb, c->p, Jex, gamma, c->st),
+    rc = ewpt_cuda_check(c, launch_stage_fp64(c->g, stage, c->y, c->yn, c->xa, c->xb, c->p, Jex, gamma, c->st),
                          "slab stage");
     if (rc == EWPT_OK && stage == 4) ++c->it;
     return rc;
@@ -202,7 +202,7 @@ int slabs_steps(ewpt_slabs* G, int32_t nsteps, bool expl, double Jex, double gam
             for (size_t m = 0; m < G->s.size() && e == cudaSuccess; ++m) {
                 ewpt_ctx* c = G->s[m];
                 cudaSetDevice(c->p.device);
-                e = launch_stage_fp64(c->g, c->tile, s, c->y, c->yn, c->xa, c->xb, c->p, J, D, c->st);
+                e = launch_stage_fp64(c->g, s, c->y, c->yn, c->xa, c->xb, c->p, J, D, c->st);
             }
             if (e != cudaSuccess) return slabs_fail(G, EWPT_ERR_CUDA, std::string("slab step: ") + cudaGetErrorString(e));
         }

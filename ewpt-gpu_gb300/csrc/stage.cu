@@ -8,11 +8,6 @@
 // stage by the previous launch; the periodic halo is a wrap of the neighbour
 // offsets inside the kernel (no ghost cells, no halo exchange).
 //
-// FP64 form (reference accumulation order, FMA contracted):
-//   stage 1: k = f(y);   yn = y  + k dt/6;  X2 = y + k dt/2
-//   stage 2: k = f(X2);  yn = yn + k dt/3;  X3 = y + k dt/2
-//   stage 3: k = f(X3);  yn = yn + k dt/3;  X4 = y + k dt
-//   stage 4: k = f(X4);  y  = yn + k dt/6
 // FP32 form (FP32 stencils and fluxes, compensated float hi/lo state):
 //   stage 1:     kacc = k1;           X2 = y_hi + k1 dt/2
 //   stage 2, 3:  kacc += 2 k_s;       X3 = y_hi + k2 dt/2,  X4 = y_hi + k3 dt
@@ -24,7 +19,6 @@
 #include "accessors.cuh"
 #include "physics_fp32.cuh"
 #include "convert.cuh"
-#include "fixstencil.cuh"
 
 namespace {
 
@@ -43,83 +37,6 @@ struct RegBudget<2> { static constexpr int kThreads = 128, kMinBlocks = 3; };
 
 template <typename TL, typename T>
 using GlobalAcc = SiteAcc<TL, T, SrcPtr36<TL>>;
-
-__device__ __forceinline__ bool make_acc(const Grid& g, const StencilCoef<double>& sc, FixAcc& A) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int j, k;
-    if (g.flat > 0) {
-        if ((unsigned)i >= (unsigned)g.flat) return false;
-        const int row = i / g.nx, pl = row / g.ny;
-        i -= row * g.nx;
-        j = row - pl * g.ny;
-        k = pl + g.k0;
-    } else {
-        j = blockIdx.y * blockDim.y + threadIdx.y;
-        k = blockIdx.z + g.k0;
-        if (i >= g.nx || j >= g.ny) return false;
-    }
-    A.place(i, j, k, g.nx, g.ny, g.nz, g.zg);
-    A.s = sc;
-    A.T = 1.0 / sc.a3;        // 60 dx
-    A.U = 1.0 / (0.5 * sc.l3);  // 180 dx^2
-    return true;
-}
-
-// ------------------------------------------------------------- rk4_step!
-struct RatesSink {
-    const MPtr36& R;
-    int c;
-    __device__ __forceinline__ void operator()(int a, double r) const { reinterpret_cast<double*>(R.p[a])[c] = r; }
-};
-
-template <bool BETA>
-__global__ void __launch_bounds__(256) k_rates_fp64(Grid g, const __grid_constant__ Ptr36 X,
-                                                       const __grid_constant__ MPtr36 R, PhysCoef<double> pc,
-                                                       StencilCoef<double> sc) {
-    FixAcc A{{{X}}};
-    if (!make_acc(g, sc, A)) return;
-    RatesSink out{R, A.c};
-    site_rates<double, BETA>(A, pc, out);
-}
-
-// ------------------------------------------------------------- FP64 stage
-template <int STAGE>
-struct Fp64Sink {
-    const FixAcc& A;
-    const double* __restrict__ y;
-    double* yn;
-    double* __restrict__ xn;
-    double* acc_out;
-    int64_t S;
-    double w, h;
-    __device__ __forceinline__ void operator()(int a, double r) const {
-        const int64_t q = a * S + A.c;
-        if (STAGE == 1) {
-            const double ya = A.v(a);  // X1 == y
-            yn[q] = fma(r, w, ya);
-            xn[q] = fma(r, h, ya);
-        } else if (STAGE < 4) {
-            // yn[q] is read and then written by this thread only: the
-            // read-only path lets these loads issue ahead of earlier stores
-            yn[q] = fma(r, w, __ldg(yn + q));
-            xn[q] = fma(r, h, __ldg(y + q));
-        } else {
-            acc_out[q] = fma(r, w, __ldg(yn + q));
-        }
-    }
-};
-
-template <int STAGE, bool BETA, int REG>
-__global__ void __launch_bounds__(RegBudget<REG>::kThreads, RegBudget<REG>::kMinBlocks) k_stage_fp64(Grid g, const __grid_constant__ Ptr36 X,
-                                                       const double* __restrict__ y, double* yn,
-                                                       double* __restrict__ xn, double* acc_out,
-                                                       PhysCoef<double> pc, StencilCoef<double> sc, double w,
-                                                       double h) {
-    FixAcc A{{{X}}};
-    if (!make_acc(g, sc, A)) return;
-    Fp64Sink<STAGE> out{A, y, yn, xn, acc_out, g.S, w, h};
-    site_rates<double, BETA>(A, pc, out);
-}
 
 // ------------------------------------------------------------- FP32 stage
 // All five FP32 buffers use the ghosted layout L.  After each stage the
@@ -303,45 +220,6 @@ __global__ void __launch_bounds__(256) k_ghost_fill_yz(Grid g, Layout L, float* 
     for (int i = lane; i < nx; i += 32) arr[doff + i] = arr[soff + i];
 }
 
-inline dim3 grid_of(const Grid& g, const Tiling& t) {
-    return dim3((g.nx + t.bx - 1) / t.bx, (g.ny + t.by - 1) / t.by, g.nz);
-}
-
-// Launch of an FP64 kernel over nzl planes: the caller's tile (laid along
-// the sites if it left more than an eighth of its lanes without one), or
-// (t.pick) the shape for the lattice.
-//  * Tiles of 32 x 4 sites where they fit x and y to 3%, else a 1-D launch
-//    over the sites: a lane without a site costs the FP64 pipe as much as one
-//    with.
-//  * 1-D blocks of one warp up to four warps per SM, so that the warps spread
-//    over all SMs; of four warps above.
-//  * <= 128 registers (16 warps per SM) once the lattice has more than the
-//    8 warps per SM that 255 registers allow: 64^3 1.33 against 1.61 ms per
-//    step, 256^3 81.4 against 100.8; below that the wide variant's shorter
-//    code wins (24 x 20 x 28: 0.186 against 0.195 ms).
-struct Shape {
-    dim3 gr, bl;
-    int flat, reg;
-};
-Shape shape_fp64(const Grid& g, const Tiling& t, int nzl) {
-    Shape s{};
-    const int64_t sites = (int64_t)g.nx * g.ny * g.nz, plane = (int64_t)g.nx * g.ny;
-    const int64_t padded = (int64_t)((g.nx + t.bx - 1) / t.bx * t.bx) * ((g.ny + t.by - 1) / t.by * t.by);
-    s.reg = !t.pick ? t.reg : sites > 152 * 8 * 32 ? 1 : 0;
-    if (t.pick ? 33 * padded <= 34 * plane && sites > 152 * 4 * 128 : 8 * padded <= 9 * plane) {
-        s.gr = grid_of(g, t);
-        s.gr.z = nzl;
-        s.bl = dim3(t.bx, t.by);
-        return s;
-    }
-    const int64_t n = plane * nzl;
-    const int b = !t.pick ? t.bx * t.by : sites > 152 * 4 * 32 ? 128 : 32;
-    s.flat = (int)n;
-    s.gr = dim3((unsigned)((n + b - 1) / b));
-    s.bl = dim3(b);
-    return s;
-}
-
 Ptr36 pack(const void* base, int64_t S, size_t elem) {
     Ptr36 P;
     for (int a = 0; a < 36; ++a) P.p[a] = static_cast<const char*>(base) + (size_t)a * S * elem;
@@ -351,76 +229,6 @@ Ptr36 pack(const void* base, int64_t S, size_t elem) {
 }  // namespace
 
 int tiling_max_threads(int reg) { return reg >= 0 && reg <= 2 ? 128 : 0; }
-
-cudaError_t launch_rates_fp64(const Grid& g, const Ptr36& in, const MPtr36& out, const ewpt_params& p,
-                              double Jex, double gam, cudaStream_t st) {
-    const PhysCoef<double> pc = make_phys_scaled(p, Jex, gam);
-    const StencilCoef<double> sc = make_stencil<double>(p.dx);
-    const bool beta = p.beta_w != 0.0 || p.beta_y != 0.0;
-    const Shape s = shape_fp64(g, kDefaultTiling, g.nz);
-    Grid gs = g;
-    gs.flat = s.flat;
-    if (beta)
-        k_rates_fp64<true><<<s.gr, s.bl, 0, st>>>(gs, in, out, pc, sc);
-    else
-        k_rates_fp64<false><<<s.gr, s.bl, 0, st>>>(gs, in, out, pc, sc);
-    return cudaGetLastError();
-}
-
-template <bool BETA, int REG>
-static void stage_fp64(const Grid& g, const Shape& s, int stage, double* y, double* yn, double* xa, double* xb,
-                       const PhysCoef<double>& pc, const StencilCoef<double>& sc, double dt, cudaStream_t st) {
-    const dim3 gr = s.gr, bl = s.bl;
-    switch (stage) {
-        case 1: k_stage_fp64<1, BETA, REG><<<gr, bl, 0, st>>>(g, pack(y, g.S, 8), y, yn, xa, nullptr, pc, sc, dt / 6., dt / 2.); break;
-        case 2: k_stage_fp64<2, BETA, REG><<<gr, bl, 0, st>>>(g, pack(xa, g.S, 8), y, yn, xb, nullptr, pc, sc, dt / 3., dt / 2.); break;
-        case 3: k_stage_fp64<3, BETA, REG><<<gr, bl, 0, st>>>(g, pack(xb, g.S, 8), y, yn, xa, nullptr, pc, sc, dt / 3., dt); break;
-        default: k_stage_fp64<4, BETA, REG><<<gr, bl, 0, st>>>(g, pack(xa, g.S, 8), y, yn, nullptr, y, pc, sc, dt / 6., 0.0);
-    }
-}
-
-template <bool BETA>
-static void stage_fp64_r(const Grid& g, const Shape& s, int stage, double* y, double* yn, double* xa, double* xb,
-                         const PhysCoef<double>& pc, const StencilCoef<double>& sc, double dt, cudaStream_t st) {
-    if (s.reg == 1)
-        stage_fp64<BETA, 1>(g, s, stage, y, yn, xa, xb, pc, sc, dt, st);
-    else if (s.reg == 2)
-        stage_fp64<BETA, 2>(g, s, stage, y, yn, xa, xb, pc, sc, dt, st);
-    else
-        stage_fp64<BETA, 0>(g, s, stage, y, yn, xa, xb, pc, sc, dt, st);
-}
-
-cudaError_t launch_stage_fp64(const Grid& g, const Tiling& t, int stage, double* y, double* yn, double* xa,
-                              double* xb, const ewpt_params& p, double Jex, double gam, cudaStream_t st) {
-    Grid gw = g;
-    gw.k0 = 0;
-    return launch_stage_fp64_planes(gw, t, stage, 0, g.nz, y, yn, xa, xb, p, Jex, gam, st);
-}
-
-cudaError_t launch_stage_fp64_planes(const Grid& g, const Tiling& t, int stage, int k0, int k1, double* y,
-                                     double* yn, double* xa, double* xb, const ewpt_params& p, double Jex,
-                                     double gam, cudaStream_t st) {
-    if (k0 < 0 || k1 > g.nz || k0 >= k1) return k0 == k1 ? cudaSuccess : cudaErrorInvalidValue;
-    const PhysCoef<double> pc = make_phys_scaled(p, Jex, gam);
-    const StencilCoef<double> sc = make_stencil<double>(p.dx);
-    const Shape s = shape_fp64(g, t, k1 - k0);
-    Grid gw = g;
-    gw.k0 = k0;
-    gw.flat = s.flat;
-    if (p.beta_w != 0.0 || p.beta_y != 0.0)
-        stage_fp64_r<true>(gw, s, stage, y, yn, xa, xb, pc, sc, p.dt, st);
-    else
-        stage_fp64_r<false>(gw, s, stage, y, yn, xa, xb, pc, sc, p.dt, st);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_step_fp64(const Grid& g, const Tiling& t, double* y, double* yn, double* xa, double* xb,
-                             const ewpt_params& p, double Jex, double gam, cudaStream_t st) {
-    cudaError_t e = cudaSuccess;
-    for (int stage = 1; stage <= 4 && e == cudaSuccess; ++stage)
-        e = launch_stage_fp64(g, t, stage, y, yn, xa, xb, p, Jex, gam, st);
-    return e;
-}
 
 // FP32 form: stage inputs ping-pong between xa and xb.
 template <bool BETA, int REG>

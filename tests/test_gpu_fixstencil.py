@@ -149,8 +149,8 @@ def test_values_outside_the_integer_range(special):
 @pytest.mark.parametrize("shape", [(24, 20, 28), (75, 31, 34), (75, 61, 90), (64, 64, 64), (33, 7, 9)])
 @pytest.mark.parametrize("beta", [0.0, 0.3])
 def test_picked_shape_gives_the_bits_of_the_default_tile(shape, beta):
-    """A context without ewpt_set_tiling runs the shape picked for its
-    lattice (tiles, or a 1-D launch with blocks of one or four warps)."""
+    """A tile set by ewpt_set_tiling changes no bit of the FP64 form (its
+    6th-order stages run four warps per 32 sites whatever the tile)."""
     import torch
 
     p = ewpt.baseline_couplings(shape=shape, N=shape[0], beta_w=beta)
