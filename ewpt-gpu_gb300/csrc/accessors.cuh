@@ -142,47 +142,48 @@ struct SiteAcc {
 // subtracts them (comp_diff) before rounding to FP32: for the longitudinal
 // gauge modes the two nearly cancel, and FP32 rounding of each would leak
 // into the transverse (magnetic) modes.
-template <class Src, bool COMP = false>
+template <class Src, bool COMP = false, class V = f2>
 struct PairAcc {
     static constexpr bool kCompGauge = COMP;
+    using Value = V;
     Src src;
     int c;      // linear index of site i0 (even)
     int ox[4];  // float offsets of the x pairs at i0-4, i0-2, i0+2, i0+4 (wrapped)
     int oy[6], oz[6];
-    StencilCoef<f2> s;
-    StencilCoef<f2> sl;  // low parts of the coefficients (COMP only)
+    StencilCoef<V> s;
+    StencilCoef<V> sl;  // low parts of the coefficients (COMP only)
 
     __device__ __forceinline__ float2 ld(int a, int off) const {
         return __ldg(reinterpret_cast<const float2*>(src.arr(a) + (c + off)));
     }
-    __device__ __forceinline__ f2 v(int a) const { return f2(ld(a, 0)); }
-    __device__ __forceinline__ void xpairs(int a, f2& p1, f2& p2, f2& p3, f2& m1, f2& m2, f2& m3) const {
+    __device__ __forceinline__ V v(int a) const { return V(ld(a, 0)); }
+    __device__ __forceinline__ void xpairs(int a, V& p1, V& p2, V& p3, V& m1, V& m2, V& m3) const {
         const float2 qm2 = ld(a, ox[0]), qm1 = ld(a, ox[1]), q0 = ld(a, 0), qp1 = ld(a, ox[2]), qp2 = ld(a, ox[3]);
-        p1 = f2(make_float2(q0.y, qp1.x));
-        p2 = f2(qp1);
-        p3 = f2(make_float2(qp1.y, qp2.x));
-        m1 = f2(make_float2(qm1.y, q0.x));
-        m2 = f2(qm1);
-        m3 = f2(make_float2(qm2.y, qm1.x));
+        p1 = V(make_float2(q0.y, qp1.x));
+        p2 = V(qp1);
+        p3 = V(make_float2(qp1.y, qp2.x));
+        m1 = V(make_float2(qm1.y, q0.x));
+        m2 = V(qm1);
+        m3 = V(make_float2(qm2.y, qm1.x));
     }
-    __device__ __forceinline__ f2 dx(int a) const {
-        f2 p1, p2, p3, m1, m2, m3;
+    __device__ __forceinline__ V dx(int a) const {
+        V p1, p2, p3, m1, m2, m3;
         xpairs(a, p1, p2, p3, m1, m2, m3);
         return s.a1 * (p1 - m1) + s.a2 * (p2 - m2) + s.a3 * (p3 - m3);
     }
-    __device__ __forceinline__ f2 d1(int a, const int* o) const {
-        return s.a1 * (f2(ld(a, o[0])) - f2(ld(a, o[3]))) + s.a2 * (f2(ld(a, o[1])) - f2(ld(a, o[4]))) +
-               s.a3 * (f2(ld(a, o[2])) - f2(ld(a, o[5])));
+    __device__ __forceinline__ V d1(int a, const int* o) const {
+        return s.a1 * (V(ld(a, o[0])) - V(ld(a, o[3]))) + s.a2 * (V(ld(a, o[1])) - V(ld(a, o[4]))) +
+               s.a3 * (V(ld(a, o[2])) - V(ld(a, o[5])));
     }
-    __device__ __forceinline__ void grad(int a, f2& gx, f2& gy, f2& gz) const {
+    __device__ __forceinline__ void grad(int a, V& gx, V& gy, V& gz) const {
         gx = dx(a);
         gy = d1(a, oy);
         gz = d1(a, oz);
     }
-    __device__ __forceinline__ void grad_lap(int a, f2& gx, f2& gy, f2& gz, f2& lap) const {
-        f2 s1, s2, s3;
+    __device__ __forceinline__ void grad_lap(int a, V& gx, V& gy, V& gz, V& lap) const {
+        V s1, s2, s3;
         {
-            f2 p1, p2, p3, m1, m2, m3;
+            V p1, p2, p3, m1, m2, m3;
             xpairs(a, p1, p2, p3, m1, m2, m3);
             gx = s.a1 * (p1 - m1) + s.a2 * (p2 - m2) + s.a3 * (p3 - m3);
             s1 = p1 + m1;
@@ -192,9 +193,9 @@ struct PairAcc {
 #pragma unroll
         for (int ax = 0; ax < 2; ++ax) {
             const int* o = ax == 0 ? oy : oz;
-            const f2 p1 = f2(ld(a, o[0])), p2 = f2(ld(a, o[1])), p3 = f2(ld(a, o[2]));
-            const f2 m1 = f2(ld(a, o[3])), m2 = f2(ld(a, o[4])), m3 = f2(ld(a, o[5]));
-            const f2 g = s.a1 * (p1 - m1) + s.a2 * (p2 - m2) + s.a3 * (p3 - m3);
+            const V p1 = V(ld(a, o[0])), p2 = V(ld(a, o[1])), p3 = V(ld(a, o[2]));
+            const V m1 = V(ld(a, o[3])), m2 = V(ld(a, o[4])), m3 = V(ld(a, o[5]));
+            const V g = s.a1 * (p1 - m1) + s.a2 * (p2 - m2) + s.a3 * (p3 - m3);
             if (ax == 0)
                 gy = g;
             else
@@ -205,7 +206,17 @@ struct PairAcc {
         }
         lap = s.l0 * v(a) + s.l1 * s1 + s.l2 * s2 + s.l3 * s3;
     }
-    __device__ __forceinline__ f2 div3(int a) const { return dx(a) + d1(a + 1, oy) + d1(a + 2, oz); }
+    __device__ __forceinline__ V div3(int a) const {
+        if constexpr (V::kFirst) {  // SiteAcc's one chain
+            V r = dx(a);
+            r = r + s.a1 * (V(ld(a + 1, oy[0])) - V(ld(a + 1, oy[3]))) +
+                s.a2 * (V(ld(a + 1, oy[1])) - V(ld(a + 1, oy[4]))) + s.a3 * (V(ld(a + 1, oy[2])) - V(ld(a + 1, oy[5])));
+            return r + s.a1 * (V(ld(a + 2, oz[0])) - V(ld(a + 2, oz[3]))) +
+                   s.a2 * (V(ld(a + 2, oz[1])) - V(ld(a + 2, oz[4]))) + s.a3 * (V(ld(a + 2, oz[2])) - V(ld(a + 2, oz[5])));
+        } else {
+            return dx(a) + d1(a + 1, oy) + d1(a + 2, oz);
+        }
+    }
 
     // ---- compensated stencils (COMP)
     // (sh, sl) += v
@@ -328,9 +339,9 @@ struct PairAcc {
     }
 };
 
-template <typename T>
-__host__ __device__ inline StencilCoef<f2> pair_stencil(const StencilCoef<T>& s) {
-    return StencilCoef<f2>{f2(s.a1), f2(s.a2), f2(s.a3), f2(s.l0), f2(s.l1), f2(s.l2), f2(s.l3)};
+template <class V = f2, typename T>
+__host__ __device__ inline StencilCoef<V> pair_stencil(const StencilCoef<T>& s) {
+    return StencilCoef<V>{V(s.a1), V(s.a2), V(s.a3), V(s.l0), V(s.l1), V(s.l2), V(s.l3)};
 }
 // the parts the FP32 coefficients miss: c - (float)c of the FP64 coefficients
 inline StencilCoef<f2> pair_stencil_lo(const StencilCoef<double>& d) {
@@ -339,8 +350,8 @@ inline StencilCoef<f2> pair_stencil_lo(const StencilCoef<double>& d) {
 }
 
 // Compensated accumulation (hi, lo) += p (TwoSum, then renormalise).
-template <typename T>
-__device__ __forceinline__ void acc_hilo(T& hi, T& lo, T p) {
+template <typename T, typename P>
+__device__ __forceinline__ void acc_hilo(T& hi, T& lo, P p) {
     const T s = hi + p;
     const T bp = s - hi;
     const T e = (hi - (s - bp)) + (p - bp);

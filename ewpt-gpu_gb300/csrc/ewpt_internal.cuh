@@ -248,6 +248,18 @@ cudaError_t launch_from_dd(int64_t S, bool in_pairs, const double* pairs, const 
 cudaError_t launch_step_fp32(const Grid& g, const Layout& L, const Tiling& t, Fp32State y, Fp32Work w,
                              const ewpt_params& p, double Jex, double gam, cudaStream_t st);
 // comp: the compensated mode (gauge Laplacians and auxiliary gradients compensated, stage_pair.cu)
+// The one-site kernel's step, bit for bit, with two sites per thread
+// (stage_pair.cu, s2): lattices with even nx, without beta terms (whose sums
+// the compiler orders otherwise), of more sites than one wave of the one-site
+// kernel (152 SMs x 12 warps).  Below that a step costs one thread's chain of
+// operations, which two sites lengthen.  ms per step, one site -> two: 32^3
+// 0.050 -> 0.068, 48^3 0.123 -> 0.113, 64^3 0.260 -> 0.250, 128^3 1.63 -> 1.28,
+// 256^3 12.6 -> 9.29.
+inline bool fp32_as_one(const Grid& g, const ewpt_params& p) {
+    return g.nx % 2 == 0 && g.S > 152 * 12 * 32 && p.beta_w == 0.0 && p.beta_y == 0.0;
+}
+cudaError_t launch_step_fp32_as_one(const Grid& g, const Layout& L, Fp32State y, Fp32Work w, const ewpt_params& p,
+                                    double Jex, double gam, cudaStream_t st);
 cudaError_t launch_step_fp32_pair(const Grid& g, const Layout& L, const Tiling& t, Fp32State y, Fp32Work w,
                                   const ewpt_params& p, double Jex, double gam, cudaStream_t st, bool comp = false);
 // Copy the face sites of all 36 arrays of a ghosted buffer into their

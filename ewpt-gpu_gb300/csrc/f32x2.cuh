@@ -9,60 +9,67 @@
 #pragma once
 #include <cuda_runtime.h>
 
-struct f2;
-struct Prod;
-
-struct f2 {
-    float2 v;
-    __host__ __device__ __forceinline__ f2() {}
-    __host__ __device__ __forceinline__ f2(float2 x) : v(x) {}
-    __host__ __device__ __forceinline__ explicit f2(float s) : v(make_float2(s, s)) {}
-    __host__ __device__ __forceinline__ explicit f2(double s) : v(make_float2((float)s, (float)s)) {}
-    __host__ __device__ __forceinline__ explicit f2(int s) : v(make_float2((float)s, (float)s)) {}
-    __device__ __forceinline__ f2(const Prod& p);
-    __device__ __forceinline__ f2& operator+=(const f2& b);
-    __device__ __forceinline__ f2& operator-=(const f2& b);
-    __device__ __forceinline__ f2& operator+=(const Prod& b);
-    __device__ __forceinline__ f2& operator-=(const Prod& b);
-};
-
-struct Prod {
+// Where two products meet, one of them is rounded first: the left one, with the
+// right one fused (f2, the paired kernels' own rounding), or with FIRST the
+// right one, as the scalar compiler contracts the one-site kernel's sums (s2:
+// two sites with the bits of one at a time; test_gpu_pairs_as_one.py).
+template <bool FIRST>
+struct Prod2 {
     float2 a, b;
     __device__ __forceinline__ float2 eval() const { return __fmul2_rn(a, b); }
 };
 
+template <bool FIRST>
+struct Pair2 {
+    static constexpr bool kFirst = FIRST;
+    using Prod = Prod2<FIRST>;
+    float2 v;
+    __host__ __device__ __forceinline__ Pair2() {}
+    __host__ __device__ __forceinline__ Pair2(float2 x) : v(x) {}
+    __host__ __device__ __forceinline__ explicit Pair2(float s) : v(make_float2(s, s)) {}
+    __host__ __device__ __forceinline__ explicit Pair2(double s) : v(make_float2((float)s, (float)s)) {}
+    __host__ __device__ __forceinline__ explicit Pair2(int s) : v(make_float2((float)s, (float)s)) {}
+    __device__ __forceinline__ Pair2(const Prod& p) : v(p.eval()) {}
+    __device__ __forceinline__ Pair2& operator+=(const Pair2& b) { return *this = *this + b; }
+    __device__ __forceinline__ Pair2& operator-=(const Pair2& b) { return *this = *this - b; }
+    __device__ __forceinline__ Pair2& operator+=(const Prod& b) { return *this = *this + b; }
+    __device__ __forceinline__ Pair2& operator-=(const Prod& b) { return *this = *this - b; }
+};
+using f2 = Pair2<false>;
+using s2 = Pair2<true>;
+
 __device__ __forceinline__ float2 neg2(float2 x) { return make_float2(-x.x, -x.y); }
 
-__device__ __forceinline__ f2::f2(const Prod& p) : v(p.eval()) {}
+#define PAIR2_OP template <bool F> __device__ __forceinline__
 
 // products
-__device__ __forceinline__ Prod operator*(const f2& a, const f2& b) { return Prod{a.v, b.v}; }
-__device__ __forceinline__ Prod operator*(const Prod& a, const f2& b) { return Prod{a.eval(), b.v}; }
-__device__ __forceinline__ Prod operator*(const f2& a, const Prod& b) { return Prod{a.v, b.eval()}; }
-__device__ __forceinline__ Prod operator*(const Prod& a, const Prod& b) { return Prod{a.eval(), b.eval()}; }
-__device__ __forceinline__ Prod operator-(const Prod& p) { return Prod{neg2(p.a), p.b}; }
+PAIR2_OP Prod2<F> operator*(const Pair2<F>& a, const Pair2<F>& b) { return {a.v, b.v}; }
+PAIR2_OP Prod2<F> operator*(const Prod2<F>& a, const Pair2<F>& b) { return {a.eval(), b.v}; }
+PAIR2_OP Prod2<F> operator*(const Pair2<F>& a, const Prod2<F>& b) { return {a.v, b.eval()}; }
+PAIR2_OP Prod2<F> operator*(const Prod2<F>& a, const Prod2<F>& b) { return {a.eval(), b.eval()}; }
+PAIR2_OP Prod2<F> operator-(const Prod2<F>& p) { return {neg2(p.a), p.b}; }
 
 // sums
-__device__ __forceinline__ f2 operator+(const f2& a, const f2& b) { return __fadd2_rn(a.v, b.v); }
-__device__ __forceinline__ f2 operator-(const f2& a, const f2& b) { return __fadd2_rn(a.v, neg2(b.v)); }
-__device__ __forceinline__ f2 operator-(const f2& a) { return neg2(a.v); }
-__device__ __forceinline__ f2 operator+(const f2& x, const Prod& p) { return __ffma2_rn(p.a, p.b, x.v); }
-__device__ __forceinline__ f2 operator+(const Prod& p, const f2& x) { return __ffma2_rn(p.a, p.b, x.v); }
-__device__ __forceinline__ f2 operator+(const Prod& p, const Prod& q) { return __ffma2_rn(q.a, q.b, p.eval()); }
-__device__ __forceinline__ f2 operator-(const f2& x, const Prod& p) { return __ffma2_rn(neg2(p.a), p.b, x.v); }
-__device__ __forceinline__ f2 operator-(const Prod& p, const f2& x) { return __ffma2_rn(p.a, p.b, neg2(x.v)); }
-__device__ __forceinline__ f2 operator-(const Prod& p, const Prod& q) { return __ffma2_rn(neg2(q.a), q.b, p.eval()); }
+PAIR2_OP Pair2<F> operator+(const Pair2<F>& a, const Pair2<F>& b) { return __fadd2_rn(a.v, b.v); }
+PAIR2_OP Pair2<F> operator-(const Pair2<F>& a, const Pair2<F>& b) { return __fadd2_rn(a.v, neg2(b.v)); }
+PAIR2_OP Pair2<F> operator-(const Pair2<F>& a) { return neg2(a.v); }
+PAIR2_OP Pair2<F> operator+(const Pair2<F>& x, const Prod2<F>& p) { return __ffma2_rn(p.a, p.b, x.v); }
+PAIR2_OP Pair2<F> operator+(const Prod2<F>& p, const Pair2<F>& x) { return __ffma2_rn(p.a, p.b, x.v); }
+PAIR2_OP Pair2<F> operator-(const Pair2<F>& x, const Prod2<F>& p) { return __ffma2_rn(neg2(p.a), p.b, x.v); }
+PAIR2_OP Pair2<F> operator-(const Prod2<F>& p, const Pair2<F>& x) { return __ffma2_rn(p.a, p.b, neg2(x.v)); }
+PAIR2_OP Pair2<F> operator+(const Prod2<F>& p, const Prod2<F>& q) {
+    return F ? __ffma2_rn(p.a, p.b, q.eval()) : __ffma2_rn(q.a, q.b, p.eval());
+}
+PAIR2_OP Pair2<F> operator-(const Prod2<F>& p, const Prod2<F>& q) {
+    return F ? __ffma2_rn(p.a, p.b, neg2(q.eval())) : __ffma2_rn(neg2(q.a), q.b, p.eval());
+}
 
 // one division per site in the physics (1/|Phi|^2): two scalar divides
-__device__ __forceinline__ f2 operator/(const f2& a, const f2& b) {
+PAIR2_OP Pair2<F> operator/(const Pair2<F>& a, const Pair2<F>& b) {
     return make_float2(a.v.x / b.v.x, a.v.y / b.v.y);
 }
-__device__ __forceinline__ f2 operator/(const f2& a, const Prod& b) { return a / f2(b); }
-
-__device__ __forceinline__ f2& f2::operator+=(const f2& b) { return *this = *this + b; }
-__device__ __forceinline__ f2& f2::operator-=(const f2& b) { return *this = *this - b; }
-__device__ __forceinline__ f2& f2::operator+=(const Prod& b) { return *this = *this + b; }
-__device__ __forceinline__ f2& f2::operator-=(const Prod& b) { return *this = *this - b; }
+PAIR2_OP Pair2<F> operator/(const Pair2<F>& a, const Prod2<F>& b) { return a / Pair2<F>(b); }
+#undef PAIR2_OP
 
 // Error-free transformations on packed pairs (Knuth's TwoSum; the product
 // error by one fused multiply-add), for the compensated stencils of the

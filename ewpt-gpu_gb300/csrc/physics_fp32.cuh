@@ -65,9 +65,9 @@ EWPT_ARITH void site_rates_fp32(const Acc& A, const PhysCoef<T>& c, Sink& out) {
             else q = p1 * pt2 - p2 * pt1 + p4 * pt3 - p3 * pt4;
             q = q - W[b][0] * Wt[cc][0] + W[cc][0] * Wt[b][0] - W[b][1] * Wt[cc][1] + W[cc][1] * Wt[b][1] -
                 W[b][2] * Wt[cc][2] + W[cc][2] * Wt[b][2];
-            out(16 + a, c.omgp2 * A.div3(24 + 3 * a) + c.gg * q);
+            out(16 + a, T(c.omgp2 * A.div3(24 + 3 * a)) + c.gg * q);
         }
-        out(19, c.omgp2 * A.div3(33) + c.ggy * (p1 * pt2 - p2 * pt1 + p3 * pt4 - p4 * pt3));
+        out(19, T(c.omgp2 * A.div3(33)) + c.ggy * (p1 * pt2 - p2 * pt1 + p3 * pt4 - p4 * pt3));
     }
 
     // ---- Higgs block: gradients, covariant derivatives, kt_phi (main_rk4.jl:337-407)

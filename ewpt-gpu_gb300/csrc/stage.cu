@@ -265,6 +265,7 @@ static void step_fp32_r(const Grid& g, const Layout& L, const Tiling& t, Fp32Buf
 cudaError_t launch_step_fp32(const Grid& g, const Layout& L, const Tiling& t, Fp32State y, Fp32Work w,
                              const ewpt_params& p, double Jex, double gam, cudaStream_t st) {
     if (L.gx == 0) return cudaErrorInvalidValue;  // the single-lattice kernels read ghost cells
+    if (t.pick && fp32_as_one(g, p)) return launch_step_fp32_as_one(g, L, y, w, p, Jex, gam, st);
     const PhysCoef<float> pc = make_phys<float>(p, Jex, gam);
     const StencilCoef<float> sc = make_stencil<float>(p.dx);
     Fp32Bufs b{y.hi, y.lo, w.kacc};

@@ -35,35 +35,39 @@ struct PairBufs {
 // The scheme of Fp32Sink (stage.cu): no stored rate sum for the fields.
 template <int STAGE, class Acc>
 struct PairSink {
+    using V = typename Acc::Value;
     const Acc& A;
     const Layout& L;
     PairBufs b;
     float* xn;
-    f2 h, w6;
+    V h, w6;
     const float *x2, *x3;  // stage 4: the inputs of stages 2 and 3
     __device__ __forceinline__ static float2* at(float* base, int64_t q) { return reinterpret_cast<float2*>(base + q); }
     __device__ __forceinline__ static float2 rd(const float* base, int64_t q) {
         return __ldg(reinterpret_cast<const float2*>(base + q));
     }
-    __device__ __forceinline__ void operator()(int a, f2 r) const {
+    __device__ __forceinline__ void operator()(int a, V r) const {
         const int64_t q = a * L.P + A.c;
         if (STAGE < 4) {
             // read then written by this thread only: read-only path is safe
-            if (a >= 16) *at(b.kacc, q) = STAGE == 1 ? r.v : (f2(rd(b.kacc, q)) + f2(2.f) * r).v;
+            if (a >= 16) *at(b.kacc, q) = STAGE == 1 ? r.v : (V(rd(b.kacc, q)) + V(2.f) * r).v;
             float* x = STAGE == 3 && a >= 20 ? b.kacc - 20 * L.P : xn;  // X4's momenta
-            *at(x, q) = ((STAGE == 1 ? A.v(a) : f2(rd(b.yhi, q))) + h * r).v;
+            *at(x, q) = ((STAGE == 1 ? A.v(a) : V(rd(b.yhi, q))) + h * r).v;
         } else {
-            f2 k;
+            V k;
             if (a < 16) {
                 const int64_t m = q + 20 * L.P;
-                k = f2(rd(b.yhi, m)) + f2(2.f) * f2(rd(x2, m));
-                k = k + f2(2.f) * f2(rd(x3, m));
+                k = V(rd(b.yhi, m)) + V(2.f) * V(rd(x2, m));
+                k = k + V(2.f) * V(rd(x3, m));
             } else {
-                k = f2(rd(b.kacc, q));
+                k = V(rd(b.kacc, q));
             }
-            const f2 s = k + r;
-            f2 hi(rd(b.yhi, q)), lo(rd(b.ylo, q));
-            acc_hilo(hi, lo, f2(w6 * s));
+            const V s = k + r;
+            V hi(rd(b.yhi, q)), lo(rd(b.ylo, q));
+            if constexpr (V::kFirst)
+                acc_hilo(hi, lo, w6 * s);
+            else
+                acc_hilo(hi, lo, V(w6 * s));
             *at(b.yhi, q) = hi.v;
             *at(b.ylo, q) = lo.v;
         }
@@ -74,15 +78,17 @@ __device__ __forceinline__ void prefetch_l2(const float* p) { asm volatile("pref
 
 // COMP: the compensated mode (gauge Laplacians and auxiliary gradients as
 // compensated pairs, accessors.cuh PairAcc); scl = the coefficients' low parts.
-template <int STAGE, bool BETA, int REG, bool COMP = false>
+// V = s2: the bits of k_stage_fp32.
+template <int STAGE, bool BETA, int REG, bool COMP, class V>
 __global__ void __launch_bounds__(PairBudget<REG>::kThreads, PairBudget<REG>::kMinBlocks)
     k_stage_fp32x2(const __grid_constant__ Grid g, const __grid_constant__ Layout L, const __grid_constant__ Ptr36 X,
-                   PairBufs b, float* xn, const float* x2, const float* x3, PhysCoef<f2> pc, StencilCoef<f2> sc,
-                   f2 h, f2 w6, Walk walk, StencilCoef<f2> scl) {
+                   PairBufs b, float* xn, const float* x2, const float* x3, PhysCoef<V> pc, StencilCoef<V> sc,
+                   V h, V w6, Walk walk, StencilCoef<V> scl) {
     int ip, j, k;  // pair index along x
     if (!walk.site(g.nx >> 1, g.ny, g.nz, ip, j, k)) return;
     const int i0 = 2 * ip;
-    PairAcc<SrcPtr36<float>, COMP> A{{X}};
+    using Acc = PairAcc<SrcPtr36<float>, COMP, V>;
+    Acc A{{X}};
     A.place_ghost(i0, j, k, g.nx, L);
     A.s = sc;
     A.sl = scl;
@@ -119,8 +125,8 @@ __global__ void __launch_bounds__(PairBudget<REG>::kThreads, PairBudget<REG>::kM
             prefetch_l2(reinterpret_cast<const float*>(X.p[q >> 1]) + (upper ? cu : cl) + kz);
         }
     }
-    PairSink<STAGE, PairAcc<SrcPtr36<float>, COMP>> out{A, L, b, xn, h, w6, x2, x3};
-    site_rates_fp32<f2, BETA>(A, pc, out);
+    PairSink<STAGE, Acc> out{A, L, b, xn, h, w6, x2, x3};
+    site_rates_fp32<V, BETA>(A, pc, out);
 }
 
 Ptr36 pack4(const void* base, int64_t S) {
@@ -129,24 +135,24 @@ Ptr36 pack4(const void* base, int64_t S) {
     return P;
 }
 
-template <bool BETA, int REG, bool COMP = false>
+template <bool BETA, int REG, bool COMP = false, class V = f2>
 void step_pair(const Grid& g, const Layout& L, const Tiling& t, PairBufs b, float* xa, float* xb,
-               const PhysCoef<f2>& pc, const StencilCoef<f2>& sc, const StencilCoef<f2>& scl, double dt,
+               const PhysCoef<V>& pc, const StencilCoef<V>& sc, const StencilCoef<V>& scl, double dt,
                cudaStream_t st) {
     dim3 gr, bl;
     const Walk walk = fp32_walk(g.nx / 2, g.ny, g.nz, t, true, gr, bl);
-    const f2 h2((float)(dt / 2.)), h1((float)dt), w6((float)(dt / 6.)), z(0.f);
+    const V h2((float)(dt / 2.)), h1((float)dt), w6((float)(dt / 6.)), z(0.f);
     float* x4m = b.kacc - 20 * L.P;  // X4's momenta
     Ptr36 X4 = pack4(xa, L.P);
     for (int a = 20; a < 36; ++a) X4.p[a] = x4m + a * L.P;
     const float* no = nullptr;
-    k_stage_fp32x2<1, BETA, REG, COMP><<<gr, bl, 0, st>>>(g, L, pack4(b.yhi, L.P), b, xa, no, no, pc, sc, h2, w6, walk, scl);
+    k_stage_fp32x2<1, BETA, REG, COMP, V><<<gr, bl, 0, st>>>(g, L, pack4(b.yhi, L.P), b, xa, no, no, pc, sc, h2, w6, walk, scl);
     launch_ghost_fill_yz(g, L, xa, xa, st);
-    k_stage_fp32x2<2, BETA, REG, COMP><<<gr, bl, 0, st>>>(g, L, pack4(xa, L.P), b, xb, no, no, pc, sc, h2, w6, walk, scl);
+    k_stage_fp32x2<2, BETA, REG, COMP, V><<<gr, bl, 0, st>>>(g, L, pack4(xa, L.P), b, xb, no, no, pc, sc, h2, w6, walk, scl);
     launch_ghost_fill_yz(g, L, xb, xb, st);
-    k_stage_fp32x2<3, BETA, REG, COMP><<<gr, bl, 0, st>>>(g, L, pack4(xb, L.P), b, xa, no, no, pc, sc, h1, w6, walk, scl);
+    k_stage_fp32x2<3, BETA, REG, COMP, V><<<gr, bl, 0, st>>>(g, L, pack4(xb, L.P), b, xa, no, no, pc, sc, h1, w6, walk, scl);
     launch_ghost_fill_yz(g, L, xa, x4m, st);
-    k_stage_fp32x2<4, BETA, REG, COMP><<<gr, bl, 0, st>>>(g, L, X4, b, nullptr, xa, xb, pc, sc, z, w6, walk, scl);
+    k_stage_fp32x2<4, BETA, REG, COMP, V><<<gr, bl, 0, st>>>(g, L, X4, b, nullptr, xa, xb, pc, sc, z, w6, walk, scl);
     launch_ghost_fill_yz(g, L, b.yhi, b.yhi, st);
 }
 
@@ -165,6 +171,15 @@ void step_pair_r(const Grid& g, const Layout& L, const Tiling& t, PairBufs b, fl
 }
 
 }  // namespace
+
+cudaError_t launch_step_fp32_as_one(const Grid& g, const Layout& L, Fp32State y, Fp32Work w, const ewpt_params& p,
+                                    double Jex, double gam, cudaStream_t st) {
+    if (!fp32_as_one(g, p) || L.gx == 0) return cudaErrorInvalidValue;
+    const StencilCoef<s2> sc = pair_stencil<s2>(make_stencil<float>(p.dx));
+    step_pair<false, 2, false, s2>(g, L, kDefaultTiling, PairBufs{y.hi, y.lo, w.kacc}, w.xa, w.xb, make_phys<s2>(p, Jex, gam), sc, sc,
+                        p.dt, st);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_step_fp32_pair(const Grid& g, const Layout& L, const Tiling& t, Fp32State y, Fp32Work w,
                                   const ewpt_params& p, double Jex, double gam, cudaStream_t st, bool comp) {
