@@ -254,9 +254,14 @@ static void step_fp32(const Grid& g, const Layout& L, const Tiling& t, Fp32Bufs 
 template <bool BETA>
 static void step_fp32_r(const Grid& g, const Layout& L, const Tiling& t, Fp32Bufs b, float* xa, float* xb,
                         const PhysCoef<float>& pc, const StencilCoef<float>& sc, double dt, cudaStream_t st) {
-    if (t.reg == 1 && !t.pick)
+    // picked: <= 168 registers, or the compiler's choice (8 warps per SM) where the
+    // lattice has no more sites than 7 warps per SM (16^3 0.049 against
+    // 0.053 ms per step, 24^3 0.051 against 0.057, 32^3 0.055 against 0.057; 33^3
+    // 0.081 against 0.076, 36^3 0.093 against 0.080)
+    const int reg = !t.pick ? t.reg : g.S > 152 * 7 * 32 ? 2 : 0;
+    if (reg == 1)
         step_fp32<BETA, 1>(g, L, t, b, xa, xb, pc, sc, dt, st);
-    else if (t.reg == 2 || t.pick)
+    else if (reg == 2)
         step_fp32<BETA, 2>(g, L, t, b, xa, xb, pc, sc, dt, st);
     else
         step_fp32<BETA, 0>(g, L, t, b, xa, xb, pc, sc, dt, st);
