@@ -7,6 +7,7 @@
 // (warp shuffle, then shared memory, then one partial row per block); a
 // second single-block kernel folds the partial rows.  Nothing N^3-sized is
 // written and nothing leaves the device but the 22 reduced values.
+#include <algorithm>
 #include <cmath>
 
 #include "ewpt_ctx.cuh"
@@ -18,10 +19,14 @@ namespace {
 constexpr int DX_ = 32, DY_ = 4, DT = DX_ * DY_;
 
 struct DiagCoef {
-    double gw, gy, hgw, hgy, lambda, vev2, sw, cw, bcoef;  // bcoef = 4 sin(th)/(gw vev^2)
-    double four_sw_gw;                                      // 4 sin(th)/gw (B_2)
-    double a[6];                                            // first-derivative weights / dx (radius R)
+    double gw, gy, lambda, vev2, sw, cw, ryw;  // ryw = g'/g
+    double a[6];                               // first-derivative weights / dx (radius R)
     double t;  // what a derivative of the accessor is multiplied by: 1, or 1 / (60 dx) (FixDiff)
+    // covariant derivatives and field strengths are kept in units of t
+    double hgw_t, gw_t;          // g/2, g over t
+    double t2, ht2;              // t^2, t^2/2
+    double sw_t, cw_t;           // sin(th) t, cos(th) t
+    double bcoef, four_sw_gw;    // 4 sin(th)/(g v^2) (B), 4 sin(th)/g (B_2), times t^2
 };
 
 // Neighbour access on an FP64 [36][S] buffer, stencil radius R.
@@ -86,8 +91,8 @@ __device__ __forceinline__ void site_diag(const DA& A, const DiagCoef& k, SiteDi
         for (int a = 0; a < 4; ++a) A.grad(a, d[a][0], d[a][1], d[a][2]);
 #pragma unroll
         for (int i = 0; i < 3; ++i)
-            cov_deriv(t * d[0][i], t * d[1][i], t * d[2][i], t * d[3][i], p1, p2, p3, p4, W1[i], W2[i], W3[i], Y[i],
-                      k.hgw, k.hgy, D[i][0], D[i][1], D[i][2], D[i][3]);
+            cov_deriv_s(d[0][i], d[1][i], d[2][i], d[3][i], p1, p2, p3, p4, W1[i], W2[i], W3[i] + k.ryw * Y[i],
+                        W3[i] - k.ryw * Y[i], k.hgw_t, D[i][0], D[i][1], D[i][2], D[i][3]);
     }
     const double mag = p1 * p1 + p2 * p2 + p3 * p3 + p4 * p4;
     const double dev = mag - k.vev2;
@@ -96,33 +101,33 @@ __device__ __forceinline__ void site_diag(const DA& A, const DiagCoef& k, SiteDi
     double ge = 0;                                                    // compute_GE!  :1498
 #pragma unroll
     for (int a = 0; a < 4; ++a) ge += D[0][a] * D[0][a] + D[1][a] * D[1][a] + D[2][a] * D[2][a];
-    o.ge = ge;
+    o.ge = k.t2 * ge;
     double eew = 0;                                                   // compute_EEW! :1817
 #pragma unroll
     for (int a = 24; a < 33; ++a) eew += A.v(a) * A.v(a);
     o.eew = 0.5 * eew;
-    const double F1_23 = t * A.curl(5, 0, 4, 1) + gw * (W22 * W33 - W23 * W32);
-    const double F1_24 = t * A.curl(6, 0, 4, 2) + gw * (W22 * W34 - W24 * W32);
-    const double F1_34 = t * A.curl(6, 1, 5, 2) + gw * (W23 * W34 - W24 * W33);
-    const double F2_23 = t * A.curl(8, 0, 7, 1) + gw * (W32 * W13 - W33 * W12);
-    const double F2_24 = t * A.curl(9, 0, 7, 2) + gw * (W32 * W14 - W34 * W12);
-    const double F2_34 = t * A.curl(9, 1, 8, 2) + gw * (W33 * W14 - W34 * W13);
-    const double F3_23 = t * A.curl(11, 0, 10, 1) + gw * (W12 * W23 - W13 * W22);
-    const double F3_24 = t * A.curl(12, 0, 10, 2) + gw * (W12 * W24 - W14 * W22);
-    const double F3_34 = t * A.curl(12, 1, 11, 2) + gw * (W13 * W24 - W14 * W23);
-    o.mew = 0.5 * (F1_23 * F1_23 + F1_24 * F1_24 + F1_34 * F1_34 + F2_23 * F2_23 + F2_24 * F2_24 +
+    const double F1_23 = A.curl(5, 0, 4, 1) + k.gw_t * (W22 * W33 - W23 * W32);
+    const double F1_24 = A.curl(6, 0, 4, 2) + k.gw_t * (W22 * W34 - W24 * W32);
+    const double F1_34 = A.curl(6, 1, 5, 2) + k.gw_t * (W23 * W34 - W24 * W33);
+    const double F2_23 = A.curl(8, 0, 7, 1) + k.gw_t * (W32 * W13 - W33 * W12);
+    const double F2_24 = A.curl(9, 0, 7, 2) + k.gw_t * (W32 * W14 - W34 * W12);
+    const double F2_34 = A.curl(9, 1, 8, 2) + k.gw_t * (W33 * W14 - W34 * W13);
+    const double F3_23 = A.curl(11, 0, 10, 1) + k.gw_t * (W12 * W23 - W13 * W22);
+    const double F3_24 = A.curl(12, 0, 10, 2) + k.gw_t * (W12 * W24 - W14 * W22);
+    const double F3_34 = A.curl(12, 1, 11, 2) + k.gw_t * (W13 * W24 - W14 * W23);
+    o.mew = k.ht2 * (F1_23 * F1_23 + F1_24 * F1_24 + F1_34 * F1_34 + F2_23 * F2_23 + F2_24 * F2_24 +
                    F2_34 * F2_34 + F3_23 * F3_23 + F3_24 * F3_24 + F3_34 * F3_34);   // compute_MEW! :1978
     const double Yt2 = A.v(33), Yt3 = A.v(34), Yt4 = A.v(35);
     o.eey = 0.5 * (Yt2 * Yt2 + Yt3 * Yt3 + Yt4 * Yt4);             // compute_EEY! :2139
-    const double Y_23 = t * A.curl(14, 0, 13, 1);
-    const double Y_24 = t * A.curl(15, 0, 13, 2);
-    const double Y_34 = t * A.curl(15, 1, 14, 2);
-    o.mey = 0.5 * (Y_23 * Y_23 + Y_24 * Y_24 + Y_34 * Y_34);       // compute_MEY! :2298
+    const double Y_23 = A.curl(14, 0, 13, 1);
+    const double Y_24 = A.curl(15, 0, 13, 2);
+    const double Y_34 = A.curl(15, 1, 14, 2);
+    o.mey = k.ht2 * (Y_23 * Y_23 + Y_24 * Y_24 + Y_34 * Y_34);       // compute_MEY! :2298
 
     // EM fields: n^a = Phi^dag sigma^a Phi / |Phi|^2 (main_rk4.jl:2455-2467)
-    double n1 = 0, n2 = 0, n3 = 0;
+    double n1 = 0, n2 = 0, n3 = 0, im = 0;
     if (mag != 0.0) {
-        const double im = 1.0 / mag;
+        im = 1.0 / mag;
         n1 = -2. * (p1 * p3 + p2 * p4) * im;
         n2 = 2. * (p2 * p3 - p1 * p4) * im;
         n3 = (-(p1 * p1) - (p2 * p2) + (p3 * p3) + (p4 * p4)) * im;
@@ -130,16 +135,16 @@ __device__ __forceinline__ void site_diag(const DA& A, const DiagCoef& k, SiteDi
     const double hx = D[1][0] * D[2][1] - D[1][1] * D[2][0] + D[1][2] * D[2][3] - D[1][3] * D[2][2];
     const double hy = D[2][0] * D[0][1] - D[2][1] * D[0][0] + D[2][2] * D[0][3] - D[2][3] * D[0][2];
     const double hz = D[0][0] * D[1][1] - D[0][1] * D[1][0] + D[0][2] * D[1][3] - D[0][3] * D[1][2];
-    const double sx = k.sw * (n1 * F1_34 + n2 * F2_34 + n3 * F3_34) + k.cw * Y_34;
-    const double sy = k.sw * (n1 * (-F1_24) + n2 * (-F2_24) + n3 * (-F3_24)) + k.cw * (-Y_24);
-    const double sz = k.sw * (n1 * F1_23 + n2 * F2_23 + n3 * F3_23) + k.cw * Y_23;
+    const double sx = k.sw_t * (n1 * F1_34 + n2 * F2_34 + n3 * F3_34) + k.cw_t * Y_34;
+    const double sy = k.sw_t * (n1 * (-F1_24) + n2 * (-F2_24) + n3 * (-F3_24)) + k.cw_t * (-Y_24);
+    const double sz = k.sw_t * (n1 * F1_23 + n2 * F2_23 + n3 * F3_23) + k.cw_t * Y_23;
     o.bx = -(sx + k.bcoef * hx);                                    // compute_Bx!  :2469
     o.by = -(sy + k.bcoef * hy);                                    // compute_By!  :2643
     o.bz = -(sz + k.bcoef * hz);                                    // compute_Bz!  :2817
     if (mag == 0.0) {                                               // compute_B_2_*! :3883
         o.b2x = o.b2y = o.b2z = 0.0;
     } else {
-        const double c2 = k.four_sw_gw / (mag * mag);
+        const double c2 = k.four_sw_gw * (im * im);
         o.b2x = -(sx + c2 * hx);
         o.b2y = -(sy + c2 * hy);
         o.b2z = -(sz + c2 * hz);
@@ -207,7 +212,7 @@ __device__ __forceinline__ void make_dacc(const Grid& g, const double* y, const 
 }
 
 template <int R>
-__global__ void __launch_bounds__(DT, R == 3 ? 3 : 1) k_diag_partial(Grid g, const double* __restrict__ y, DiagCoef kc,
+__global__ void __launch_bounds__(DT, R == 3 ? 5 : 1) k_diag_partial(Grid g, const double* __restrict__ y, DiagCoef kc,
                                                      double* __restrict__ part) {
     // the sums of each thread live in shared memory: 22 doubles less per
     // thread in registers during the stencils
@@ -250,21 +255,22 @@ __global__ void __launch_bounds__(DT, R == 3 ? 3 : 1) k_diag_partial(Grid g, con
     __syncthreads();
     // one warp per slot: four values per lane, then a shuffle reduction
     const int64_t b = blockIdx.x + (int64_t)gridDim.x * (blockIdx.y + (int64_t)gridDim.y * blockIdx.z);
+    const int64_t nb = (int64_t)gridDim.x * gridDim.y * gridDim.z;
     for (int q = threadIdx.y; q < NRED; q += DT / 32) {
         double v = acc[q][threadIdx.x];
         for (int w = 1; w < DT / 32; ++w) v = fold(q, v, acc[q][threadIdx.x + 32 * w]);
         v = fold_warp(q, v);
-        if (threadIdx.x == 0) part[b * NRED + q] = v;
+        if (threadIdx.x == 0) part[q * nb + b] = v;
     }
 }
 
-// One warp per slot folds the partial rows (one block of NRED warps).
+// One warp per slot folds its partials [NRED][nb] (one block of NRED warps).
 __global__ void __launch_bounds__(32 * NRED) k_diag_final(const double* __restrict__ part, int nb,
                                                           double* __restrict__ out) {
     const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
     double v = q == R_MIN ? (double)INFINITY : 0.0;
 #pragma unroll 8
-    for (int b = lane; b < nb; b += 32) v = fold(q, v, part[(int64_t)b * NRED + q]);
+    for (int b = lane; b < nb; b += 32) v = fold(q, v, part[(int64_t)q * nb + b]);
     v = fold_warp(q, v);
     if (lane == 0) out[q] = v;
 }
@@ -274,7 +280,7 @@ __global__ void __launch_bounds__(32 * NRED) k_diag_final(const double* __restri
 // densities (compute_PE! .. compute_MEY!).
 // A kernel per field: what the others alone need is not computed.
 template <int R, int which>
-__global__ void __launch_bounds__(DT, R == 3 && which != 2 ? 3 : 1) k_fields(Grid g, const double* __restrict__ y,
+__global__ void __launch_bounds__(DT, R == 3 ? 4 : 1) k_fields(Grid g, const double* __restrict__ y,
                                                                              DiagCoef kc, double* __restrict__ f) {
     const int i = blockIdx.x * DX_ + threadIdx.x;
     const int j = blockIdx.y * DY_ + threadIdx.y;
@@ -301,14 +307,11 @@ DiagCoef diag_coef(const ewpt_params& p) {
     DiagCoef k;
     k.gw = p.gw;
     k.gy = p.gy;
-    k.hgw = 0.5 * p.gw;
-    k.hgy = 0.5 * p.gy;
+    k.ryw = p.gy / p.gw;
     k.lambda = p.lambda;
     k.vev2 = p.vev * p.vev;
     k.sw = std::sin(p.theta_w);
     k.cw = std::cos(p.theta_w);
-    k.bcoef = 4. * k.sw / (p.gw * (p.vev * p.vev));
-    k.four_sw_gw = 4. * k.sw / p.gw;
     const int R = stencil_radius(p.stencil_order);
     for (int d = 0; d < 6; ++d) k.a[d] = 0.0;
     k.t = 1.0;
@@ -325,6 +328,14 @@ DiagCoef diag_coef(const ewpt_params& p) {
             k.t = s.a3;  // 1 / (60 dx)
         }
     }
+    k.hgw_t = 0.5 * p.gw / k.t;
+    k.gw_t = p.gw / k.t;
+    k.t2 = k.t * k.t;
+    k.ht2 = 0.5 * k.t2;
+    k.sw_t = k.sw * k.t;
+    k.cw_t = k.cw * k.t;
+    k.bcoef = 4. * k.sw / (p.gw * (p.vev * p.vev)) * k.t2;
+    k.four_sw_gw = 4. * k.sw / p.gw * k.t2;
     return k;
 }
 
@@ -340,13 +351,17 @@ void launch_partial(int R, dim3 gr, const Grid& g, const double* y, const DiagCo
     }
 }
 
+// About 8192 blocks, each over the same number of planes: ten waves and more
+// of the resident blocks, the last one small beside them.  (With 1216 blocks
+// the reduction had 2.8 waves of 13 or 12 planes each at 128^3.)  Diagnostics
+// with this grid and five blocks per SM, the B field with four: 128^3 2151 ->
+// 1768 and 972 -> 739 us, 224^3 12.9 -> 9.0 and 5.44 -> 3.98 ms, 48^3 178 -> 165
+// and 82 -> 64 us; at 224^3 three, four, five, six blocks: 10.4, 9.2, 9.0, 9.7
+// and 4.68, 3.98, 4.39, 3.94 ms.
 dim3 diag_grid(const Grid& g) {
     const int bx = (g.nx + DX_ - 1) / DX_, by = (g.ny + DY_ - 1) / DY_;
-    // about 8 resident blocks on each of the SMs, z folded into a loop
-    int bz = (152 * 8 + bx * by - 1) / (bx * by);
-    if (bz > g.nz) bz = g.nz;
-    if (bz < 1) bz = 1;
-    return dim3(bx, by, bz);
+    const int planes = (int)std::max<int64_t>((int64_t)bx * by * g.nz / 8192, 1);
+    return dim3(bx, by, (g.nz + planes - 1) / planes);
 }
 
 }  // namespace

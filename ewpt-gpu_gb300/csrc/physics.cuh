@@ -74,16 +74,6 @@ EWPT_ARITH void cov_deriv_s(T d1, T d2, T d3, T d4, T p1, T p2, T p3, T p4, T W1
     D4 = d4 - hgw * (W1 * p1 - W2 * p2 - Zm * p3);
 }
 
-// The same with Y_i and g'/2 apart (the diagnostics).
-template <typename T>
-EWPT_ARITH void cov_deriv(T d1, T d2, T d3, T d4, T p1, T p2, T p3, T p4, T W1, T W2, T W3, T Y,
-                                          T hgw, T hgy, T& D1, T& D2, T& D3, T& D4) {
-    D1 = d1 + hgw * (W1 * p4 - W2 * p3 + W3 * p2) + hgy * (Y * p2);
-    D2 = d2 - hgw * (W1 * p3 + W2 * p4 + W3 * p1) - hgy * (Y * p1);
-    D3 = d3 + hgw * (W1 * p2 + W2 * p1 - W3 * p4) + hgy * (Y * p4);
-    D4 = d4 - hgw * (W1 * p1 - W2 * p2 - W3 * p3) - hgy * (Y * p3);
-}
-
 template <typename T, bool BETA, class Acc, class Sink, int PART = 0>
 EWPT_ARITH void site_rates(const Acc& A, const PhysCoef<T>& c, Sink& out) {
     static_assert(PART == 0 || !BETA, "the beta terms couple every block: PART 0 only");
