@@ -19,7 +19,7 @@
 // Laplacian, against 37 FP64 instructions (2368 issue slots).  A step of the
 // FP64 form at 256^3 went from 144.4 to 76.1 ms (64^3: 2.41 to 1.20) with
 // these stencils and the factored physics, 1046 FP64 instructions per warp and
-// stage to 501, and to 68.4 (1.15) with four warps per 32 sites (stage_fp64.cu).
+// stage to 501, and to 66.8 (1.12) with four warps per 32 sites (stage_fp64.cu).
 //
 // Stencils whose largest magnitude lies outside [2^-895, 2^977] (denormals,
 // infinities and NaN among them) take the floating-point evaluation, a
@@ -91,125 +91,128 @@ __device__ __forceinline__ int64_t weigh_lap(int64_t t1, int64_t t2, int64_t t3)
 
 }  // namespace fix
 
-// SiteAcc's FP64 stencils on the integer pipes, first derivatives and
-// divergences times 60 dx, Laplacians times 180 dx^2.  The routines are out-of-line
-// calls: inlined 24 times they would be far larger than the instruction cache.
-struct FixAcc : SiteAcc<double, double, SrcPtr36<double>> {
-    using Base = SiteAcc<double, double, SrcPtr36<double>>;
+// FP64 stencils of the stage kernels on the integer pipes, first derivatives
+// and divergences times 60 dx, Laplacians times 180 dx^2.  The neighbours'
+// offsets are found from (i, j, k) for each stencil anew, some 50 integer
+// instructions, instead of 18 registers that live through all of them.
+struct FixAcc {
+    const Ptr36& X;
+    const Grid& g;
+    int i, j, k, c;
 
-    __device__ __noinline__ void grad_lap(int a, double& gx, double& gy, double& gz, double& lap) const {
-        const double* p = src.arr(a) + c;
-        double f[3][6];
-        const double f0 = __ldg(p);
+    __device__ __forceinline__ const double* at(int a) const { return reinterpret_cast<const double*>(X.p[a]) + c; }
+    __device__ __forceinline__ double v(int a) const { return __ldg(at(a)); }
+    // plane k of the lattice, or (g.zg > 0) interior plane k of a slab
+    __device__ __forceinline__ void place(int i_, int j_, int k_) {
+        i = i_;
+        j = j_;
+        k = k_;
+        c = i + g.nx * (j + g.ny * (k + g.zg));
+    }
+    // the neighbours [+1, +2, +3, -1, -2, -3] of *p along an axis
+    __device__ __forceinline__ void along(const double* p, int ax, double* f) const {
+        int q = ax == 0 ? i : (ax == 1 ? j : k);
+        asm volatile("" : "+r"(q));  // keeps the offsets from being hoisted out of the caller's loop
+        const int stride = ax == 0 ? 1 : (ax == 1 ? g.nx : g.nx * g.ny);
+        const int n = ax == 0 ? g.nx : (ax == 1 ? g.ny : (g.zg ? 1 << 30 : g.nz));
+        if (ax == 2 && g.zg) q = 1 << 29;  // ghost planes
 #pragma unroll
-        for (int k = 0; k < 6; ++k) {
-            f[0][k] = __ldg(p + ox[k]);
-            f[1][k] = __ldg(p + oy[k]);
-            f[2][k] = __ldg(p + oz[k]);
+        for (int d = 1; d <= 3; ++d) {
+            f[d - 1] = __ldg(p + (q + d < n ? d : d - n) * stride);
+            f[d + 2] = __ldg(p + (q >= d ? -d : n - d) * stride);
         }
-        uint32_t e = fix::exp20(f0);
+    }
+    __device__ __forceinline__ static uint32_t largest(const double (&f)[3][6]) {
+        uint32_t e = 0;
 #pragma unroll
         for (int ax = 0; ax < 3; ++ax)
 #pragma unroll
-            for (int k = 0; k < 6; ++k) e = max(e, fix::exp20(f[ax][k]));
+            for (int d = 0; d < 6; ++d) e = max(e, fix::exp20(f[ax][d]));
+        return e;
+    }
+    // the floating-point evaluation of a derivative
+    __device__ __forceinline__ static double d1(const double* f) {
+        return 45.0 * (f[0] - f[3]) - 9.0 * (f[1] - f[4]) + (f[2] - f[5]);
+    }
+    __device__ __forceinline__ static int64_t weighed(const double* f, uint32_t ep) {
+        int64_t D[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) D[d] = fix::align(f[d], ep) - fix::align(f[d + 3], ep);
+        return fix::weigh_grad(D[0], D[1], D[2]);
+    }
+
+    __device__ __forceinline__ void grad_lap(int a, double& gx, double& gy, double& gz, double& lap) const {
+        const double* p = at(a);
+        double f[3][6];
+        const double f0 = __ldg(p);
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax) along(p, ax, f[ax]);
+        const uint32_t e = max(fix::exp20(f0), largest(f));
         if (!fix::covered(e)) {
-            if (e == 0 && fix::zero_bits(f0) && fix::zero_bits(f))
+            if (e == 0 && fix::zero_bits(f0) && fix::zero_bits(f)) {
                 gx = gy = gz = lap = 0.0;
-            else {
-                Base::grad_lap(a, gx, gy, gz, lap);
-                const double T = 1.0 / s.a3;
-                gx *= T;
-                gy *= T;
-                gz *= T;
-                lap *= 2.0 / s.l3;  // 180 dx^2
+            } else {
+                gx = d1(f[0]);
+                gy = d1(f[1]);
+                gz = d1(f[2]);
+                double S[3];
+#pragma unroll
+                for (int d = 0; d < 3; ++d)
+                    S[d] = f[0][d] + f[0][d + 3] + (f[1][d] + f[1][d + 3]) + (f[2][d] + f[2][d + 3]);
+                lap = -1470.0 * f0 + 270.0 * S[0] - 27.0 * S[1] + 2.0 * S[2];
             }
             return;
         }
         const uint32_t ep = e + (7u << 20);
         const int64_t i0 = fix::align(f0, ep);
         int64_t T[3] = {-6 * i0, -6 * i0, -6 * i0};
-        double g[3];
+        double r[3];
 #pragma unroll
         for (int ax = 0; ax < 3; ++ax) {
             int64_t D[3];
 #pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                const int64_t u = fix::align(f[ax][k], ep), w = fix::align(f[ax][k + 3], ep);
-                D[k] = u - w;
-                T[k] += u + w;
+            for (int d = 0; d < 3; ++d) {
+                const int64_t u = fix::align(f[ax][d], ep), w = fix::align(f[ax][d + 3], ep);
+                D[d] = u - w;
+                T[d] += u + w;
             }
-            g[ax] = fix::to_double(fix::weigh_grad(D[0], D[1], D[2]), e, 0);
+            r[ax] = fix::to_double(fix::weigh_grad(D[0], D[1], D[2]), e, 0);
         }
-        gx = g[0];
-        gy = g[1];
-        gz = g[2];
+        gx = r[0];
+        gy = r[1];
+        gz = r[2];
         lap = fix::to_double(fix::weigh_lap(T[0], T[1], T[2]), e, 6);
     }
 
-    __device__ __noinline__ void grad(int a, double& gx, double& gy, double& gz) const {
-        const double* p = src.arr(a) + c;
+    __device__ __forceinline__ void grad(int a, double& gx, double& gy, double& gz) const {
+        const double* p = at(a);
         double f[3][6];
 #pragma unroll
-        for (int k = 0; k < 6; ++k) {
-            f[0][k] = __ldg(p + ox[k]);
-            f[1][k] = __ldg(p + oy[k]);
-            f[2][k] = __ldg(p + oz[k]);
-        }
-        uint32_t e = 0;
-#pragma unroll
-        for (int ax = 0; ax < 3; ++ax)
-#pragma unroll
-            for (int k = 0; k < 6; ++k) e = max(e, fix::exp20(f[ax][k]));
+        for (int ax = 0; ax < 3; ++ax) along(p, ax, f[ax]);
+        const uint32_t e = largest(f);
         if (!fix::covered(e)) {
-            if (e == 0 && fix::zero_bits(f))
-                gx = gy = gz = 0.0;
-            else {
-                Base::grad(a, gx, gy, gz);
-                const double T = 1.0 / s.a3;
-                gx *= T;
-                gy *= T;
-                gz *= T;
-            }
+            const bool z = e == 0 && fix::zero_bits(f);
+            gx = z ? 0.0 : d1(f[0]);
+            gy = z ? 0.0 : d1(f[1]);
+            gz = z ? 0.0 : d1(f[2]);
             return;
         }
         const uint32_t ep = e + (7u << 20);
-        double g[3];
-#pragma unroll
-        for (int ax = 0; ax < 3; ++ax) {
-            int64_t D[3];
-#pragma unroll
-            for (int k = 0; k < 3; ++k) D[k] = fix::align(f[ax][k], ep) - fix::align(f[ax][k + 3], ep);
-            g[ax] = fix::to_double(fix::weigh_grad(D[0], D[1], D[2]), e, 0);
-        }
-        gx = g[0];
-        gy = g[1];
-        gz = g[2];
+        gx = fix::to_double(weighed(f[0], ep), e, 0);
+        gy = fix::to_double(weighed(f[1], ep), e, 0);
+        gz = fix::to_double(weighed(f[2], ep), e, 0);
     }
 
-    __device__ __noinline__ double div3(int a) const {
+    // dx(a) + dy(a + 1) + dz(a + 2)
+    __device__ __forceinline__ double div3(int a) const {
         double f[3][6];
 #pragma unroll
-        for (int k = 0; k < 6; ++k) {
-            f[0][k] = __ldg(src.arr(a) + c + ox[k]);
-            f[1][k] = __ldg(src.arr(a + 1) + c + oy[k]);
-            f[2][k] = __ldg(src.arr(a + 2) + c + oz[k]);
-        }
-        uint32_t e = 0;
-#pragma unroll
-        for (int ax = 0; ax < 3; ++ax)
-#pragma unroll
-            for (int k = 0; k < 6; ++k) e = max(e, fix::exp20(f[ax][k]));
-        if (!fix::covered(e)) return e == 0 && fix::zero_bits(f) ? 0.0 : Base::div3(a) / s.a3;
+        for (int ax = 0; ax < 3; ++ax) along(at(a + ax), ax, f[ax]);
+        const uint32_t e = largest(f);
+        if (!fix::covered(e)) return e == 0 && fix::zero_bits(f) ? 0.0 : d1(f[0]) + d1(f[1]) + d1(f[2]);
         const uint32_t ep = e + (7u << 20);
-        int64_t V = 0;  // three axes: two bits more than one derivative
-#pragma unroll
-        for (int ax = 0; ax < 3; ++ax) {
-            int64_t D[3];
-#pragma unroll
-            for (int k = 0; k < 3; ++k) D[k] = fix::align(f[ax][k], ep) - fix::align(f[ax][k + 3], ep);
-            V += fix::weigh_grad(D[0], D[1], D[2]) >> 2;
-        }
-        return fix::to_double(V, e, 2);
+        // three axes: two bits more than one derivative
+        return fix::to_double((weighed(f[0], ep) >> 2) + (weighed(f[1], ep) >> 2) + (weighed(f[2], ep) >> 2), e, 2);
     }
 };
 

@@ -20,16 +20,17 @@
 // The equations are those of physics.cuh.
 //
 // Bound by the FP64 pipe (one warp instruction per 64 cycles and SM quarter):
-// 532 FP64 instructions per 32 sites and stage, the pipe 80% busy at 96^3 (ncu;
-// instruction fetch and shared-memory latency the largest stalls).  A site per
+// 532 FP64 instructions per 32 sites and stage, the pipe 82% busy at 96^3 (ncu;
+// shared-memory latency and instruction fetch the largest stalls).  A site per
 // thread took 128-255 registers through ~15 k instructions: 16 warps per SM ran
 // the pipe at 66%, and a lattice of less than a warp per SM quarter ran at the
 // latency of that one chain.  Four warps of 72 registers, 28 per SM, one such
 // chain a quarter as long.  Step at one site per thread -> four warps: 24 x 20 x
-// 28 0.171 -> 0.107 ms, 64^3 1.20 -> 1.15, 75 x 61 x 90 1.84 -> 1.77, 128^3 9.29
-// -> 8.61, 256^3 76.2 -> 68.4.  Blocks per SM (64^3): five 1.33 ms, six 1.25,
-// seven 1.23, eight 1.21 with the Higgs part in one warp; with it split by axis,
-// seven 1.15, eight 1.16.
+// 28 0.171 -> 0.0985 ms, 64^3 1.20 -> 1.12, 75 x 61 x 90 1.84 -> 1.72, 128^3 9.29
+// -> 8.40, 256^3 76.2 -> 66.8.  The Higgs part in one warp instead of split by
+// axis: 0.117 and 1.23 at 24 x 20 x 28 and 64^3.  The stencils out of line, with
+// the neighbours' offsets in local memory: 0.107 and 1.15.  Blocks per SM, six,
+// seven, eight: 24 x 20 x 28 0.098, 0.0985, 0.105; 256^3 68.8, 66.8, 66.0.
 #include <type_traits>
 
 #include "accessors.cuh"
@@ -309,19 +310,17 @@ __device__ __forceinline__ void colour_warp(const FixAcc& A, const Coef& c, Shar
 
 // sites: how many, from plane g.k0 on, x fastest
 template <int STAGE, bool BETA, class Out>
-__device__ __forceinline__ void evolve(const Grid& g, const Ptr36& X, const Coef& pc,
-                                       const StencilCoef<double>& sc, int sites, const Out& out) {
+__device__ __forceinline__ void evolve(const Grid& g, const Ptr36& X, const Coef& pc, int sites, const Out& out) {
     __shared__ SharedOf<BETA> sh;
     // The roles turn with the block: warp w of every block runs on SM quarter
-    // w % 4, and the Higgs role has half as many operations again as a colour.
+    // w % 4, and a colour has a little more to do than the Higgs warp.
     const int lane = threadIdx.x & 31, warp = ((threadIdx.x >> 5) + blockIdx.x) & (kWarps - 1);
     const int64_t q0 = (int64_t)blockIdx.x * kSites + lane;
     const bool live = q0 < sites;
     const int q = live ? (int)q0 : sites - 1;  // lanes past the end repeat the last site and write nothing
     const int row = q / g.nx, i = q - row * g.nx, pl = row / g.ny, j = row - pl * g.ny;
-    FixAcc A{{{X}}};
-    A.place(i, j, pl + g.k0, g.nx, g.ny, g.nz, g.zg);
-    A.s = sc;
+    FixAcc A{X, g};
+    A.place(i, j, pl + g.k0);
 #pragma unroll 1
     for (int n = 0; n < 4; ++n) {
         const int a = 4 * warp + n;
@@ -351,16 +350,16 @@ __device__ __forceinline__ void evolve(const Grid& g, const Ptr36& X, const Coef
 template <int STAGE, bool BETA>
 __global__ void __launch_bounds__(kSites* kWarps, 7)
     k_stage_fp64(Grid g, const __grid_constant__ Ptr36 X, const double* __restrict__ y, double* yn, double* xn,
-                 const __grid_constant__ Coef pc, const __grid_constant__ StencilCoef<double> sc, double w,
+                 const __grid_constant__ Coef pc, double w,
                  double h, int sites) {
-    evolve<STAGE, BETA>(g, X, pc, sc, sites, StageSink{y, yn, xn, g.S, w, h});
+    evolve<STAGE, BETA>(g, X, pc, sites, StageSink{y, yn, xn, g.S, w, h});
 }
 
 template <bool BETA>
 __global__ void __launch_bounds__(kSites* kWarps, 7)
     k_rates_fp64(Grid g, const __grid_constant__ Ptr36 X, const __grid_constant__ MPtr36 R,
-                 const __grid_constant__ Coef pc, const __grid_constant__ StencilCoef<double> sc, int sites) {
-    evolve<0, BETA>(g, X, pc, sc, sites, RatesOut{R});
+                 const __grid_constant__ Coef pc, int sites) {
+    evolve<0, BETA>(g, X, pc, sites, RatesOut{R});
 }
 
 unsigned blocks_for(int64_t sites) { return (unsigned)((sites + kSites - 1) / kSites); }
@@ -368,14 +367,14 @@ unsigned blocks_for(int64_t sites) { return (unsigned)((sites + kSites - 1) / kS
 // stage s over `sites` sites from plane g.k0 on
 template <bool BETA>
 void stage_fp64(const Grid& g, int stage, double* y, double* yn, double* xa, double* xb, const Coef& pc,
-                const StencilCoef<double>& sc, double dt, int sites, cudaStream_t st) {
+                double dt, int sites, cudaStream_t st) {
     const unsigned nb = blocks_for(sites);
     const int nt = kSites * kWarps;
     switch (stage) {
-        case 1: k_stage_fp64<1, BETA><<<nb, nt, 0, st>>>(g, arrays36((const double*)y, g.S), y, yn, xa, pc, sc, dt / 6., dt / 2., sites); break;
-        case 2: k_stage_fp64<2, BETA><<<nb, nt, 0, st>>>(g, arrays36((const double*)xa, g.S), y, yn, xb, pc, sc, dt / 3., dt / 2., sites); break;
-        case 3: k_stage_fp64<3, BETA><<<nb, nt, 0, st>>>(g, arrays36((const double*)xb, g.S), y, yn, xa, pc, sc, dt / 3., dt, sites); break;
-        default: k_stage_fp64<4, BETA><<<nb, nt, 0, st>>>(g, arrays36((const double*)xa, g.S), y, yn, y, pc, sc, dt / 6., 0.0, sites);
+        case 1: k_stage_fp64<1, BETA><<<nb, nt, 0, st>>>(g, arrays36((const double*)y, g.S), y, yn, xa, pc, dt / 6., dt / 2., sites); break;
+        case 2: k_stage_fp64<2, BETA><<<nb, nt, 0, st>>>(g, arrays36((const double*)xa, g.S), y, yn, xb, pc, dt / 3., dt / 2., sites); break;
+        case 3: k_stage_fp64<3, BETA><<<nb, nt, 0, st>>>(g, arrays36((const double*)xb, g.S), y, yn, xa, pc, dt / 3., dt, sites); break;
+        default: k_stage_fp64<4, BETA><<<nb, nt, 0, st>>>(g, arrays36((const double*)xa, g.S), y, yn, y, pc, dt / 6., 0.0, sites);
     }
 }
 
@@ -384,12 +383,11 @@ void stage_fp64(const Grid& g, int stage, double* y, double* yn, double* xa, dou
 cudaError_t launch_rates_fp64(const Grid& g, const Ptr36& in, const MPtr36& out, const ewpt_params& p, double Jex,
                               double gam, cudaStream_t st) {
     const Coef pc = make_coef(p, Jex, gam);
-    const StencilCoef<double> sc = make_stencil<double>(p.dx);
     const int sites = (int)((int64_t)g.nx * g.ny * g.nz);
     if (p.beta_w != 0.0 || p.beta_y != 0.0)
-        k_rates_fp64<true><<<blocks_for(sites), kSites * kWarps, 0, st>>>(g, in, out, pc, sc, sites);
+        k_rates_fp64<true><<<blocks_for(sites), kSites * kWarps, 0, st>>>(g, in, out, pc, sites);
     else
-        k_rates_fp64<false><<<blocks_for(sites), kSites * kWarps, 0, st>>>(g, in, out, pc, sc, sites);
+        k_rates_fp64<false><<<blocks_for(sites), kSites * kWarps, 0, st>>>(g, in, out, pc, sites);
     return cudaGetLastError();
 }
 
@@ -397,14 +395,13 @@ cudaError_t launch_stage_fp64_planes(const Grid& g, int stage, int k0, int k1, d
                                      double* xb, const ewpt_params& p, double Jex, double gam, cudaStream_t st) {
     if (k0 < 0 || k1 > g.nz || k0 >= k1) return k0 == k1 ? cudaSuccess : cudaErrorInvalidValue;
     const Coef pc = make_coef(p, Jex, gam);
-    const StencilCoef<double> sc = make_stencil<double>(p.dx);
     Grid gw = g;
     gw.k0 = k0;
     const int sites = (int)((int64_t)g.nx * g.ny * (k1 - k0));
     if (p.beta_w != 0.0 || p.beta_y != 0.0)
-        stage_fp64<true>(gw, stage, y, yn, xa, xb, pc, sc, p.dt, sites, st);
+        stage_fp64<true>(gw, stage, y, yn, xa, xb, pc, p.dt, sites, st);
     else
-        stage_fp64<false>(gw, stage, y, yn, xa, xb, pc, sc, p.dt, sites, st);
+        stage_fp64<false>(gw, stage, y, yn, xa, xb, pc, p.dt, sites, st);
     return cudaGetLastError();
 }
 

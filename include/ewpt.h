@@ -121,7 +121,8 @@ int ewpt_step_explicit(ewpt_ctx* ctx, int32_t nsteps, double Jex, double gamma);
 int ewpt_step_host(ewpt_ctx* ctx, const double* state_in, double* state_out, int32_t nsteps);
 /* Iterations done so far (the `it` of the reference loop). */
 int64_t ewpt_iteration(const ewpt_ctx* ctx);
-/* Launch shape of the stage kernels.  pair = 0 or 1: blocks of bx*by
+/* Launch shape of the stage kernels.  Until it is set, the library picks one
+ * for the lattice, with the results of the default below.  pair = 0 or 1: blocks of bx*by
  * threads over x and y (whole warps, at most 128 threads), reg = register-
  * budget variant (0: registers at the compiler's choice; 1: <= 128
  * registers; 2: <= 168); pair = 1 (FP32 form, even nx): each thread evolves
@@ -131,7 +132,10 @@ int64_t ewpt_iteration(const ewpt_ctx* ctx);
  * nz % 4 == 0 -- with the same arithmetic as pair = 1.  The result of a step
  * does not depend on bx, by or reg, and pair only changes FP32 rounding
  * (pair = 1 and 2 agree bit for bit); ewpt/autotune.py picks the fastest per
- * lattice size and precision.  Default 32x4, 0, 0. */
+ * lattice size and precision.  A tile that fits x and y badly is laid along
+ * the rows (FP32 form, pair = 0 or 1).  The 6th-order FP64 stages have one
+ * shape, four warps per 32 sites, and take no notice of the tile.  Default
+ * 32x4, 0, 0. */
 int ewpt_set_tiling(ewpt_ctx* ctx, int32_t bx, int32_t by, int32_t reg, int32_t pair);
 int ewpt_get_tiling(const ewpt_ctx* ctx, int32_t* bx, int32_t* by, int32_t* reg, int32_t* pair);
 /* FP32 form, compensated mode (on = 1; default 0): the gauge fields'
@@ -311,7 +315,8 @@ int32_t ewpt_slabs_count(const ewpt_slabs* slabs);
  * (set resets the iteration counter); synchronous */
 int ewpt_slabs_set_state(ewpt_slabs* slabs, const double* packed, int32_t on_device);
 int ewpt_slabs_get_state(ewpt_slabs* slabs, double* packed, int32_t on_device);
-/* launch shape of every slab's stage kernels (ewpt_set_tiling, pair = 0) */
+/* launch shape of every slab's stage kernels (ewpt_set_tiling, pair = 0; the
+ * FP64 stages have one shape) */
 int ewpt_slabs_set_tiling(ewpt_slabs* slabs, int32_t bx, int32_t by, int32_t reg);
 /* nsteps RK4 steps (the J_ext/damp schedule of ewpt_step, or explicit
  * values), asynchronous on the slabs' streams */
@@ -369,7 +374,8 @@ int ewpt_ensemble_init_thermal_gauss(ewpt_ens* ens, int32_t m, double T, double 
 int ewpt_ensemble_set_drive(ewpt_ens* ens, int32_t m, double Jex, double gamma);
 /* launch shape of every member: bx*by threads (whole warps, <= 128), at
  * most 168 registers, pair = two x-adjacent sites per thread (every member
- * needs an even nx; default when possible).  Default 16x8 threads. */
+ * needs an even nx; default when possible).  Until it is set, the shape is
+ * picked for each member (64x2 pairs, 32x4 sites). */
 int ewpt_ensemble_set_tiling(ewpt_ens* ens, int32_t bx, int32_t by, int32_t pair);
 /* launch shape of member m alone, as ewpt_set_tiling (pair 0 or 1), e.g.
  * the shape a single lattice of that size runs fastest with */
