@@ -19,7 +19,7 @@
 // Laplacian, against 37 FP64 instructions (2368 issue slots).  A step of the
 // FP64 form at 256^3 went from 144.4 to 76.1 ms (64^3: 2.41 to 1.20) with
 // these stencils and the factored physics, 1046 FP64 instructions per warp and
-// stage to 501, and to 66.8 (1.12) with four warps per 32 sites (stage_fp64.cu).
+// stage to 501, and to 60.2 (1.01) with four warps per 32 sites (stage_fp64.cu).
 //
 // Stencils whose largest magnitude lies outside [2^-895, 2^977] (denormals,
 // infinities and NaN among them) take the floating-point evaluation, a

@@ -16,18 +16,21 @@
 // memory, 80 doubles per site.  Then warp 1 + a evaluates colour a -- W^a_i,
 // Gamma^a and one component of Y -- and the covariant Higgs derivatives along
 // axis a, and warp 0 the momentum rates, the local Higgs terms and Sigma, with
-// the axes' parts added when they are there: some 115 and 130 FP64 instructions.
+// the axes' parts added when they are there: some 100 and 120 FP64 instructions.
 // The equations are those of physics.cuh.
 //
 // Bound by the FP64 pipe (one warp instruction per 64 cycles and SM quarter):
-// 532 FP64 instructions per 32 sites and stage, the pipe 82% busy at 96^3 (ncu;
-// shared-memory latency and instruction fetch the largest stalls).  A site per
+// 487 FP64 instructions per 32 sites and stage, the pipe 83-85% busy at 96^3 (ncu;
+// chains of independent FMAs reach 84%; shared-memory latency and instruction
+// fetch the largest stalls).  A site per
 // thread took 128-255 registers through ~15 k instructions: 16 warps per SM ran
 // the pipe at 66%, and a lattice of less than a warp per SM quarter ran at the
 // latency of that one chain.  Four warps of 72 registers, 28 per SM, one such
 // chain a quarter as long.  Step at one site per thread -> four warps: 24 x 20 x
 // 28 0.171 -> 0.0985 ms, 64^3 1.20 -> 1.12, 75 x 61 x 90 1.84 -> 1.72, 128^3 9.29
-// -> 8.40, 256^3 76.2 -> 66.8.  The Higgs part in one warp instead of split by
+// -> 8.40, 256^3 76.2 -> 66.8 (532 FP64 instructions); with the units of the
+// momentum rates in the sink's weights, negations folded and no division
+// without damping (487) 64^3 1.01, 128^3 7.59, 256^3 60.2.  The Higgs part in one warp instead of split by
 // axis: 0.117 and 1.23 at 24 x 20 x 28 and 64^3.  The stencils out of line, with
 // the neighbours' offsets in local memory: 0.107 and 1.15.  Blocks per SM, six,
 // seven, eight: 24 x 20 x 28 0.098, 0.0985, 0.105; 256^3 68.8, 66.8, 66.0.
@@ -100,36 +103,41 @@ template <bool BETA>
 using SharedOf = std::conditional_t<BETA, SharedBeta, Shared>;
 
 struct StageSink {
-    const double* __restrict__ y;
+    const double* y;
     double* yn;
     double* xn;  // next stage input, or the new y (stage 4)
     int64_t S;
-    double w, h;
+    double w[3], h[3];  // by unit
 };
 
+// Units of the rates handed over: 1, Coef::hgw_o and Coef::gw_o.  The last two
+// are in the sink's weights, one multiplication less for 13 arrays.
+enum Unit { kOne, kHiggs, kGauge };
+
 // the rate of array a at the site c; x: the stage input's value (stage 1)
-template <int STAGE>
+template <int STAGE, Unit U = kOne>
 __device__ __forceinline__ void put(const StageSink& o, int a, int c, bool live, double x, double r) {
     if (!live) return;
     const int64_t q = a * o.S + c;
     if (STAGE == 1) {  // X1 == y
-        o.yn[q] = fma(r, o.w, x);
-        o.xn[q] = fma(r, o.h, x);
+        o.yn[q] = fma(r, o.w[U], x);
+        o.xn[q] = fma(r, o.h[U], x);
     } else if (STAGE < 4) {
         // read then written by this thread only: the read-only path lets these
         // loads issue ahead of earlier stores
-        o.yn[q] = fma(r, o.w, __ldg(o.yn + q));
-        o.xn[q] = fma(r, o.h, __ldg(o.y + q));
+        o.yn[q] = fma(r, o.w[U], __ldg(o.yn + q));
+        o.xn[q] = fma(r, o.h[U], __ldg(o.y + q));
     } else {
-        o.xn[q] = fma(r, o.w, __ldg(o.yn + q));
+        o.xn[q] = fma(r, o.w[U], __ldg(o.yn + q));
     }
 }
 struct RatesOut {
-    const MPtr36& R;
+    MPtr36 R;
+    double unit[3];
 };
-template <int STAGE>
+template <int STAGE, Unit U = kOne>
 __device__ __forceinline__ void put(const RatesOut& o, int a, int c, bool live, double, double r) {
-    if (live) reinterpret_cast<double*>(o.R.p[a])[c] = r;
+    if (live) reinterpret_cast<double*>(o.R.p[a])[c] = U == kOne ? r : o.unit[U] * r;
 }
 
 // Named barriers.  1: the colour warps' parts of the Higgs rates are in shared
@@ -153,20 +161,21 @@ __device__ __forceinline__ void strengths(Shared& sh, int lane, int a, const dou
         const int i = m == 2 ? 1 : 0, j = m == 0 ? 1 : 2;
         double &dij = sh.s[3 * (4 + 3 * a + i) + j][lane], &dji = sh.s[3 * (4 + 3 * a + j) + i][lane];
         F[m] = dji - dij + gw * (u[i] * v[j] - u[j] * v[i]);  // d_i W_j - d_j W_i + g (...)
-        const double e = -(F[m] + dji);
+        const double e = -F[m] - dji;
         dij = F[m] - dij;
         dji = e;
     }
 }
 
-// Q_i += sum_j f_j E^b_ij (E_ii = -d_i W_i)
+// Q_i += sum_j f_j E^b_ij (E_ii = -d_i W_i), or -= with NEG
+template <bool NEG>
 __device__ __forceinline__ void add_strengths(const Shared& sh, int lane, int b, const double* f, double* Q) {
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
             const double e = sh.s[3 * (4 + 3 * b + i) + j][lane];
-            Q[i] = i == j ? fma(-f[j], e, Q[i]) : fma(f[j], e, Q[i]);
+            Q[i] = (i == j) != NEG ? fma(-f[j], e, Q[i]) : fma(f[j], e, Q[i]);
         }
 }
 
@@ -191,7 +200,7 @@ __device__ __forceinline__ void axis_part(const FixAcc& A, const Coef& c, Shared
     d3 += D3;
     d4 += D4;
     sh.part(0, i, lane) = W1 * d4 - W2 * d3 + Zp * d2;
-    sh.part(1, i, lane) = -(W1 * d3 + W2 * d4 + Zp * d1);
+    sh.part(1, i, lane) = -W1 * d3 - W2 * d4 - Zp * d1;
     sh.part(2, i, lane) = W1 * d2 + W2 * d1 - Zm * d4;
     sh.part(3, i, lane) = W2 * d2 - W1 * d1 + Zm * d3;
 }
@@ -209,7 +218,10 @@ __device__ __forceinline__ void higgs_warp(const FixAcc& A, const Coef& c, Share
     double a[4];
     {
         const double mag = p[0] * p[0] + p[1] * p[1] + p[2] * p[2] + p[3] * p[3];
-        const double potg = c.lam2h * (mag - c.vev2) + c.hJexh, damp = c.gamh / mag;
+        const double potg = c.lam2h * (mag - c.vev2) + c.hJexh;
+        // gamma / |Phi|^2, its 0/0 at |Phi| = 0 kept; no division without damping
+        double damp = fix::zero_bits(mag) ? __longlong_as_double(0x7ff8000000000000LL) : 0.0;
+        if (!fix::zero_bits(c.gamh)) damp = c.gamh / mag;
         const double G1 = c.it * A.v(16), G2 = c.it * A.v(17), G3 = c.it * A.v(18), S = c.it * A.v(19);
         const double q12 = G3 + c.ryw * S, q34 = c.ryw * S - G3;
         a[0] = q12 * p[1] - G2 * p[2] + G1 * p[3] - p[0] * (potg + damp * (p[0] * pt[0]));
@@ -236,9 +248,11 @@ __device__ __forceinline__ void higgs_warp(const FixAcc& A, const Coef& c, Share
     }
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
-        double r = c.hgw_o * (a[b] + (sh.part(b, 0, lane) + sh.part(b, 1, lane) + sh.part(b, 2, lane)));
-        if (BETA) r += bsum * p[b];
-        put<STAGE>(out, 20 + b, A.c, live, pt[b], r);
+        const double r = a[b] + (sh.part(b, 0, lane) + sh.part(b, 1, lane) + sh.part(b, 2, lane));
+        if (BETA)
+            put<STAGE>(out, 20 + b, A.c, live, pt[b], c.hgw_o * r + bsum * p[b]);
+        else
+            put<STAGE, kHiggs>(out, 20 + b, A.c, live, pt[b], r);
     }
 }
 
@@ -273,10 +287,8 @@ __device__ __forceinline__ void colour_warp(const FixAcc& A, const Coef& c, Shar
     for (int i = 0; i < 3; ++i)
         Q[i] = Wc[i] * Gb - Wb[i] * Gc + sh.s[60 + 4 + 3 * a + i][lane] * c.lap_w - sh.s[3 * (16 + a) + i][lane] * c.igw;
     colours_ready();
-    add_strengths(sh, lane, b, Wc, Q);
-#pragma unroll
-    for (int i = 0; i < 3; ++i) Wb[i] = -Wb[i];
-    add_strengths(sh, lane, cc, Wb, Q);
+    add_strengths<false>(sh, lane, b, Wc, Q);
+    add_strengths<true>(sh, lane, cc, Wb, Q);
     double kY = c.lap_y * sh.s[60 + 13 + a][lane] - c.t * sh.s[3 * 19 + a][lane];
     double kb[3] = {};  // beta terms
     if (BETA) {
@@ -301,9 +313,11 @@ __device__ __forceinline__ void colour_warp(const FixAcc& A, const Coef& c, Shar
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         const int arr = 24 + 3 * a + i;
-        double r = c.gw_o * (Q[i] + sh.j[3 * a + i][lane]);
-        if (BETA) r += kb[i];
-        put<STAGE>(out, arr, A.c, live, STAGE == 1 ? A.v(arr) : 0.0, r);
+        const double r = Q[i] + sh.j[3 * a + i][lane];
+        if (BETA)
+            put<STAGE>(out, arr, A.c, live, STAGE == 1 ? A.v(arr) : 0.0, c.gw_o * r + kb[i]);
+        else
+            put<STAGE, kGauge>(out, arr, A.c, live, STAGE == 1 ? A.v(arr) : 0.0, r);
     }
     put<STAGE>(out, 33 + a, A.c, live, STAGE == 1 ? A.v(33 + a) : 0.0, kY + c.gy_o * sh.j[9 + a][lane]);
 }
@@ -349,17 +363,16 @@ __device__ __forceinline__ void evolve(const Grid& g, const Ptr36& X, const Coef
 
 template <int STAGE, bool BETA>
 __global__ void __launch_bounds__(kSites* kWarps, 7)
-    k_stage_fp64(Grid g, const __grid_constant__ Ptr36 X, const double* __restrict__ y, double* yn, double* xn,
-                 const __grid_constant__ Coef pc, double w,
-                 double h, int sites) {
-    evolve<STAGE, BETA>(g, X, pc, sites, StageSink{y, yn, xn, g.S, w, h});
+    k_stage_fp64(Grid g, const __grid_constant__ Ptr36 X, const __grid_constant__ StageSink out,
+                 const __grid_constant__ Coef pc, int sites) {
+    evolve<STAGE, BETA>(g, X, pc, sites, out);
 }
 
 template <bool BETA>
 __global__ void __launch_bounds__(kSites* kWarps, 7)
-    k_rates_fp64(Grid g, const __grid_constant__ Ptr36 X, const __grid_constant__ MPtr36 R,
+    k_rates_fp64(Grid g, const __grid_constant__ Ptr36 X, const __grid_constant__ RatesOut out,
                  const __grid_constant__ Coef pc, int sites) {
-    evolve<0, BETA>(g, X, pc, sites, RatesOut{R});
+    evolve<0, BETA>(g, X, pc, sites, out);
 }
 
 unsigned blocks_for(int64_t sites) { return (unsigned)((sites + kSites - 1) / kSites); }
@@ -370,11 +383,15 @@ void stage_fp64(const Grid& g, int stage, double* y, double* yn, double* xa, dou
                 double dt, int sites, cudaStream_t st) {
     const unsigned nb = blocks_for(sites);
     const int nt = kSites * kWarps;
+    auto sink = [&](double* xn, double w, double h) {
+        return StageSink{y, yn, xn, g.S, {w, w * pc.hgw_o, w * pc.gw_o}, {h, h * pc.hgw_o, h * pc.gw_o}};
+    };
+    auto in = [&](const double* x) { return arrays36(x, g.S); };
     switch (stage) {
-        case 1: k_stage_fp64<1, BETA><<<nb, nt, 0, st>>>(g, arrays36((const double*)y, g.S), y, yn, xa, pc, dt / 6., dt / 2., sites); break;
-        case 2: k_stage_fp64<2, BETA><<<nb, nt, 0, st>>>(g, arrays36((const double*)xa, g.S), y, yn, xb, pc, dt / 3., dt / 2., sites); break;
-        case 3: k_stage_fp64<3, BETA><<<nb, nt, 0, st>>>(g, arrays36((const double*)xb, g.S), y, yn, xa, pc, dt / 3., dt, sites); break;
-        default: k_stage_fp64<4, BETA><<<nb, nt, 0, st>>>(g, arrays36((const double*)xa, g.S), y, yn, y, pc, dt / 6., 0.0, sites);
+        case 1: k_stage_fp64<1, BETA><<<nb, nt, 0, st>>>(g, in(y), sink(xa, dt / 6., dt / 2.), pc, sites); break;
+        case 2: k_stage_fp64<2, BETA><<<nb, nt, 0, st>>>(g, in(xa), sink(xb, dt / 3., dt / 2.), pc, sites); break;
+        case 3: k_stage_fp64<3, BETA><<<nb, nt, 0, st>>>(g, in(xb), sink(xa, dt / 3., dt), pc, sites); break;
+        default: k_stage_fp64<4, BETA><<<nb, nt, 0, st>>>(g, in(xa), sink(y, dt / 6., 0.0), pc, sites);
     }
 }
 
@@ -383,11 +400,12 @@ void stage_fp64(const Grid& g, int stage, double* y, double* yn, double* xa, dou
 cudaError_t launch_rates_fp64(const Grid& g, const Ptr36& in, const MPtr36& out, const ewpt_params& p, double Jex,
                               double gam, cudaStream_t st) {
     const Coef pc = make_coef(p, Jex, gam);
+    const RatesOut o{out, {1.0, pc.hgw_o, pc.gw_o}};
     const int sites = (int)((int64_t)g.nx * g.ny * g.nz);
     if (p.beta_w != 0.0 || p.beta_y != 0.0)
-        k_rates_fp64<true><<<blocks_for(sites), kSites * kWarps, 0, st>>>(g, in, out, pc, sites);
+        k_rates_fp64<true><<<blocks_for(sites), kSites * kWarps, 0, st>>>(g, in, o, pc, sites);
     else
-        k_rates_fp64<false><<<blocks_for(sites), kSites * kWarps, 0, st>>>(g, in, out, pc, sites);
+        k_rates_fp64<false><<<blocks_for(sites), kSites * kWarps, 0, st>>>(g, in, o, pc, sites);
     return cudaGetLastError();
 }
 
