@@ -104,7 +104,12 @@ __global__ void __launch_bounds__(PairBudget<REG>::kThreads, PairBudget<REG>::kM
     // their lanes 0 and 16 (a warp's 64 sites where it lies in one row, its two
     // rows of 32 in tiles 16 wide): 72 lines of 128 bytes per buffer, two
     // or three per lane.  Plane k+2 <= nz+1 lies inside the ghosted box.
-    if (blockDim.x >= 16 && __activemask() == 0xffffffffu) {
+    // Only for 2^19 sites and more: ms per step without / with, 48^3 0.109 / 0.116,
+    // 96^3 0.618 / 0.619, 128^3 1.300 / 1.285, 160^3 2.45 / 2.39, 256^3 9.70 / 9.37
+    // (a smaller lattice has more of the lines in L2 already).  The compensated
+    // mode, bound by its instructions, is faster without at every size: 64^3 0.314 /
+    // 0.339, 128^3 1.77 / 1.88, 256^3 13.41 / 14.05.
+    if (!COMP && g.S >= 1 << 19 && blockDim.x >= 16 && __activemask() == 0xffffffffu) {
         const int lane = (threadIdx.y * blockDim.x + threadIdx.x) & 31;
         const int cl = __shfl_sync(0xffffffffu, A.c, 0), cu = __shfl_sync(0xffffffffu, A.c, 16);
         const int kz = 2 * L.px * L.py;
