@@ -28,6 +28,8 @@ roofline HBM roofline of the stage kernels: algorithmic bytes per
 roofline_compute  the FP64 form's own bound, the FP64 pipe: counted FLOPs
          per site-update x site-updates/s over the FP64 peak measured in
          this run (ewpt_fp64_peak, fused multiply-add chains on every SM).
+         The stencils' FLOPs are done in 64-bit integers, so this passes 1;
+         `pipe` has the FP64 instructions that are executed.
 --impl reference  times the CPU restatement of the reference's routines (the
          oracle) on the host cores on a bounded sample lattice.
 With --gpus N > 1 (torchrun), each rank evolves its own replica; value is the
@@ -52,22 +54,23 @@ BYTES_FP64 = 3744  # 468 FP64 values per site-update (k-storage RK4)
 BYTES_FP32 = 2592  # y in FP64 width, stage rates in FP32
 # DRAM bytes per site-update (sum over the 4 stage launches) from one ncu
 # capture of the stage kernels (dram__bytes_read.sum + dram__bytes_write.sum):
-# FP64 at 80^3, 32x2 threads; FP32 form at 128^3, the tuned paired kernel
+# FP64 at 96^3; FP32 form at 128^3, the tuned paired kernel
 # (64x2 pair-threads, <= 168 registers, with its L2 prefetches).  Traffic grows with the site count,
 # so a 256^3 launch moves this x S / 4.
-TRAFFIC_FP64 = 4383
-TRAFFIC_FP32 = 2973
+TRAFFIC_FP64 = 4632
+TRAFFIC_FP32 = 2682
 # FP64 operations of one site-update of the FP64 stage kernels (4 stages of
 # site_rates + the RK4 epilogue), counted exactly by compiling the kernels'
 # own per-site templates with an operator-counting scalar type
 # (tests/test_devphys.py checks these figures against that count): FLOPs with
-# an FMA as 2, and FP64 pipe instructions with single-use products fused.
+# an FMA as 2, and FP64 pipe instructions with single-use products fused, the
+# stencils in floating point (the 6th-order stages do theirs in integers).
 FLOPS_FP64 = 6820
 FP64_INST_EST = 4704
 # FP64 instructions per site-update the stage kernels execute (ncu
-# smsp__sass_thread_inst_executed_op_{dadd,dmul,dfma}_pred_on.sum over the 4
-# launches at 80^3, per site): 3 x (454 + 126 + 604) + (454 + 126 + 568).
-FP64_INST_NCU = 4700
+# smsp__inst_executed_pipe_fp64.sum x 32 lanes over the 4 launches at 96^3, per
+# site).
+FP64_INST_NCU = 1912
 N_BUBBLES = 64
 
 
@@ -308,7 +311,7 @@ def run_ours(args, ws, rank, local):
                      "traffic": TRAFFIC_FP64 * S / 4, "peak_kind": peak_kind,
                      "kernel": "k_stage_fp64 (4 launches/step, the whole step)",
                      "launch_ms": t64 / args.steps / 4 * 1e3,
-                     "traffic_source": "ncu dram bytes per site-update at 80^3 x sites / 4",
+                     "traffic_source": "ncu dram bytes per site-update at 96^3 x sites / 4",
                      "algorithmic_bytes_per_site_update": BYTES_FP64,
                      "limiter": "the FP64 pipe, not HBM: see roofline_compute"},
         "roofline_compute": {"bound": "fp64", "achieved": S * args.steps / t64 * FLOPS_FP64 / 1e12,
@@ -319,12 +322,13 @@ def run_ours(args, ws, rank, local):
                              "flops_source": "exact count of the kernels' per-site source (oracle/devphys.cu), "
                                              "FMA = 2 FLOPs",
                              "pipe": {"fp64_inst_per_site_update": FP64_INST_NCU,
-                                      "source": "ncu DADD+DMUL+DFMA thread instructions at 80^3",
+                                      "source": "ncu FP64 pipe instructions at 96^3, 32 lanes each",
                                       "achieved_ginst_s": S * args.steps / t64 * FP64_INST_NCU / 1e9,
                                       "peak_ginst_s": res["fp64"]["peak"] / 2 / 1e9,
                                       "frac": S * args.steps / t64 * FP64_INST_NCU / (res["fp64"]["peak"] / 2)},
-                             "note": "FLOP frac < 1 by construction: DADD and DMUL take a pipe slot for 1 FLOP; "
-                                     "the pipe frac is the FP64 instruction rate over the probe's",
+                             "note": "the FLOP count holds the stencils, which run in 64-bit integers: frac "
+                                     "may pass 1; the pipe frac is the FP64 instruction rate over the "
+                                     "probe's",
                              "kernel": "k_stage_fp64 (4 launches/step)"},
         "gpu_launches": 4 * args.steps,
         "clocks": clocks,
