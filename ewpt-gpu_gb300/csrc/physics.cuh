@@ -1,6 +1,8 @@
 // physics.cuh -- per-site right-hand side of the temporal-gauge SU(2)xU(1)
-// Higgs system, templated on the arithmetic type T (double for the FP64
-// form, float for the FP32 stencil/flux form).
+// Higgs system, templated on the arithmetic type T: double (the FP64 form's
+// alternative stencil orders; its 6th-order stages spread the same equations
+// over four warps, stage_fp64.cu), double-float and pairs of it (DF64).  The
+// FP32 forms keep an order of operations of their own (physics_fp32.cuh).
 //
 // Same equations as rk4_step! (gpu-kernels-rk4/main_rk4.jl:52-661):
 //   covariant derivatives  cov_derivs_temporal.jl:23-130

@@ -5,6 +5,8 @@
 // per site and stage) round differently, by a few 1e-8 of the fields per
 // step, for 2% of the step time at 256^3: the FP32 stage waits on memory.
 #pragma once
+#include <type_traits>
+
 #include "physics.cuh"
 
 // Accessors that declare kCompGauge = true give the gauge fields'

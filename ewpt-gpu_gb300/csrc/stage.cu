@@ -1,19 +1,21 @@
-// stage.cu -- fused RK4 stage kernels.
+// stage.cu -- fused RK4 stage kernels of the FP32 form, one site per thread, and
+// the conversions and ghost cells of its buffers.
 //
 // One launch = one stage of classical RK4 (gpu-kernels-rk4/main_rk4.jl:
 // 6146-6437): the stage kernel rk4_step! (main_rk4.jl:52-661) with the
 // reference's broadcast combination fused into its epilogue, so the 144
 // broadcast kernels and ~72 temporary N^3 arrays of a reference step become
 // four launches and no temporaries.  The stage input X is written once per
-// stage by the previous launch; the periodic halo is a wrap of the neighbour
-// offsets inside the kernel (no ghost cells, no halo exchange).
+// stage by the previous launch; the periodic images along y and z lie in ghost
+// cells, along x the neighbour offsets wrap.
 //
 // FP32 form (FP32 stencils and fluxes, compensated float hi/lo state):
 //   stage 1:     kacc = k1;           X2 = y_hi + k1 dt/2
 //   stage 2, 3:  kacc += 2 k_s;       X3 = y_hi + k2 dt/2,  X4 = y_hi + k3 dt
 //   stage 4:     (y_hi, y_lo) += dt/6 (kacc + k4), compensated, in place
 // (X_1 is y_hi itself; kacc of the fields is not stored, see Fp32Bufs).
-// Bytes per site-update: FP64 4608, FP32 2480.
+// Bytes per site-update: 2480.  Bound by the latency of its loads (12 warps per
+// SM; 128^3: issue slots 41% active, 3.5 TB/s).
 #include <algorithm>
 
 #include "accessors.cuh"

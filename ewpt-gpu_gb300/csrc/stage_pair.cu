@@ -1,14 +1,14 @@
 // stage_pair.cu -- FP32-form RK4 stage kernels with two sites per thread.
 //
-// Same stage structure and arithmetic as k_stage_fp32 (stage.cu), but each
-// thread owns the x-adjacent sites (i0, i0+1), i0 even, and runs the physics
+// Same stage structure and arithmetic as k_stage_fp32 (stage.cu; with s2 its
+// roundings too), but each thread owns the x-adjacent sites (i0, i0+1), i0 even, and runs the physics
 // on packed float pairs (f32x2.cuh): every flux operation is one FFMA2 /
 // FADD2 / FMUL2 for both sites, and every neighbour access is a float2 load.
 // For the x stencil the pairs at i0-4, i0-2, i0, i0+2, i0+4 (five aligned
 // float2 loads) are re-paired into the +-1, +-2, +-3 neighbour pairs; y and z
 // neighbours are aligned float2 loads of the same x pair.  The buffers use
 // the ghosted layout (ewpt_internal.cuh), so neighbours past a face are read
-// from the ghost cells along y and z (refreshed by k_ghost_fill after each
+// from the ghost cells along y and z (refreshed by k_ghost_fill_yz after each
 // stage) and wrapped in the offsets along x.  Needs nx even.
 #include <algorithm>
 
