@@ -23,9 +23,16 @@
 // these stencils and the factored physics, 1046 FP64 instructions per warp and
 // stage to 501, and to 60.2 (1.01) with four warps per 32 sites (stage_fp64.cu).
 //
+// Every stencil of -v is minus the stencil of v to the bit, as IEEE sums are, and
+// does not see the signs of zeros: a start that is symmetric under Phi -> -Phi
+// or a reflection stays so.  Step times with all of this: 64^3 1.04 ms, 128^3
+// 7.83, 256^3 63.4, 1 to 3% above those of sums rounded downwards.  Values with exact
+// zeros among them cost more: 64^3 1.38 ms where every array but one is odd in x.
+//
 // Stencils whose largest magnitude lies outside [2^-895, 2^977] (denormals,
-// infinities and NaN among them) take the floating-point evaluation, a
-// stencil of zeros gives zero.
+// infinities and NaN among them) take the floating-point evaluation, as do
+// gradients and divergences with a zero among their values; a stencil of zeros
+// gives zero.
 #pragma once
 #include "accessors.cuh"
 
@@ -53,17 +60,21 @@ __device__ __forceinline__ bool zero_bits(const double (&f)[N][6]) {
     return z;
 }
 
-// v in units of 2^(E - 1023 - 55), rounded towards minus infinity (a
-// negative value one unit lower: stencil weights sum to zero, and the unit is
-// an eighth of the largest value's last place); e20p = e20 + (7 << 20)
-__device__ __forceinline__ int64_t align(double v, uint32_t e20p) {
+// v in units of 2^(E - 1023 - 55).  Rounded towards minus infinity where no value
+// of a stencil is zero: align(-v) = -align(v) - 1, and the weights sum to zero, so
+// a stencil of -v is minus that of v to the bit.  A zero has no such image, and
+// its sign is not to matter: NEAREST, ties away from zero, takes four
+// instructions more.
+template <bool NEAREST = false>
+__device__ __forceinline__ int64_t align(double v, uint32_t e20) {
     const uint32_t h = (uint32_t)__double2hiint(v), l = (uint32_t)__double2loint(v);
     const uint32_t s = (uint32_t)((int32_t)h >> 31);
-    const uint32_t sh = (e20p - (h & 0x7ff00000u)) >> 20;  // 7 + the distance to the largest exponent
-    // 1.mantissa at bits 62..10
+    const uint32_t sh = (e20 + ((NEAREST ? 6u : 7u) << 20) - (h & 0x7ff00000u)) >> 20;  // and the distance to the largest exponent
+    // 1.mantissa at bits 62..10, the one's complement of a negative value's
     const uint32_t mh = ((__funnelshift_l(l, h, 10) & 0x3fffffffu) | 0x40000000u) ^ s;
     const uint32_t ml = (l << 10) ^ s;
-    return i64(ml, mh) >> min(sh, 63u);
+    const int64_t q = i64(ml, mh) >> min(sh, 63u);
+    return NEAREST ? (q + 1) >> 1 : q;  // q half units, or -q - 1
 }
 
 // V * 2^(E - 1023 - 55 + up) rounded to nearest, |V| < 2^63
@@ -87,29 +98,32 @@ __device__ __forceinline__ int64_t weigh_grad(int64_t d1, int64_t d2, int64_t d3
 __device__ __forceinline__ double d1(const double* f) {
     return 45.0 * (f[0] - f[3]) - 9.0 * (f[1] - f[4]) + (f[2] - f[5]);
 }
-__device__ __forceinline__ uint32_t largest(const double* f) {
+// the largest of the values' exponents; lo: down to the smallest
+__device__ __forceinline__ uint32_t largest(const double* f, uint32_t& lo) {
     uint32_t e = 0;
 #pragma unroll
-    for (int d = 0; d < 6; ++d) e = max(e, exp20(f[d]));
+    for (int d = 0; d < 6; ++d) {
+        e = max(e, exp20(f[d]));
+        lo = min(lo, exp20(f[d]));
+    }
     return e;
 }
 // The weighted sums V of N lines of neighbours, each on the line's own exponent e.
-// False: a line is not covered.
+// False: a line is not covered or holds a zero.
 template <int N>
 __device__ __forceinline__ bool weighed(const double (&f)[N][6], int64_t* V, uint32_t* e) {
-    bool all = true;
+    uint32_t lo = ~0u;
 #pragma unroll
-    for (int ax = 0; ax < N; ++ax) {
-        e[ax] = largest(f[ax]);
-        all = all && covered(e[ax]);
-    }
+    for (int ax = 0; ax < N; ++ax) e[ax] = largest(f[ax], lo);
+    bool all = lo != 0u;
+#pragma unroll
+    for (int ax = 0; ax < N; ++ax) all = all && covered(e[ax]);
     if (!all) return false;
 #pragma unroll
     for (int ax = 0; ax < N; ++ax) {
-        const uint32_t ep = e[ax] + (7u << 20);
         int64_t D[3];
 #pragma unroll
-        for (int d = 0; d < 3; ++d) D[d] = align(f[ax][d], ep) - align(f[ax][d + 3], ep);
+        for (int d = 0; d < 3; ++d) D[d] = align(f[ax][d], e[ax]) - align(f[ax][d + 3], e[ax]);
         V[ax] = weigh_grad(D[0], D[1], D[2]);
     }
     return true;
@@ -167,13 +181,55 @@ __device__ __forceinline__ double div(const double (&f)[3][6]) {
     return (e[0] | e[1] | e[2]) == 0u && zero_bits(f) ? 0.0 : d1(f[0]) + d1(f[1]) + d1(f[2]);
 }
 
-// (270 t1 - 27 t2 + 2 t3) >> 6, |t| < 2^60, without overflow
+// (270 t1 - 27 t2 + 2 t3) / 64, |t| < 2^60, without overflow; where that is no
+// whole number, the odd one next to it (odd in t, and the rounding to 53 bits that
+// follows is that of the fraction)
 __device__ __forceinline__ int64_t weigh_lap(int64_t t1, int64_t t2, int64_t t3) {
     const int64_t lo = (int64_t)((uint64_t)(uint32_t)t1 * 270u + (uint64_t)(uint32_t)t3 * 2u) -
                        (int64_t)((uint64_t)(uint32_t)t2 * 27u);
     const int64_t hi = (int64_t)(int32_t)(t1 >> 32) * 270 + (int64_t)(int32_t)(t3 >> 32) * 2 -
                        (int64_t)(int32_t)(t2 >> 32) * 27 + (lo >> 32);
-    return (hi << 26) | (int64_t)((uint32_t)lo >> 6);
+    return (hi << 26) | (int64_t)((uint32_t)lo >> 6) | (int64_t)(((uint32_t)lo & 63u) != 0u);
+}
+
+// gradient and Laplacian, all values aligned to one exponent
+template <bool NEAREST>
+__device__ __forceinline__ void grad_lap(double f0, const double (&f)[3][6], uint32_t e, double* r) {
+    const int64_t i0 = align<NEAREST>(f0, e);
+    int64_t T[3] = {-6 * i0, -6 * i0, -6 * i0};
+#pragma unroll
+    for (int ax = 0; ax < 3; ++ax) {
+        int64_t D[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const int64_t u = align<NEAREST>(f[ax][d], e), w = align<NEAREST>(f[ax][d + 3], e);
+            D[d] = u - w;
+            T[d] += u + w;
+        }
+        r[ax] = to_double(weigh_grad(D[0], D[1], D[2]), e, 0);
+    }
+    r[3] = to_double(weigh_lap(T[0], T[1], T[2]), e, 6);
+}
+
+// the neighbours [+1, +2, +3, -1, -2, -3] of *p, index q of n
+__device__ __forceinline__ void line(const double* p, int q, int n, int stride, double* f) {
+#pragma unroll
+    for (int d = 1; d <= 3; ++d) {
+        f[d - 1] = __ldg(p + (q + d < n ? d : d - n) * stride);
+        f[d + 2] = __ldg(p + (q >= d ? -d : n - d) * stride);
+    }
+}
+
+// Where the stencil holds a zero, at (i, j, k) of nx, ny, nz: out of line, so that
+// its instructions do not lie between those of the other sites (in line: 3%
+// more per step at 256^3).
+static __device__ __noinline__ void grad_lap_zero(const double* p, int i, int j, int k, int nx, int ny, int nz,
+                                                  uint32_t e, double* r) {
+    double f[3][6];
+    line(p, i, nx, 1, f[0]);
+    line(p, j, ny, nx, f[1]);
+    line(p, k, nz, nx * ny, f[2]);
+    grad_lap<true>(__ldg(p), f, e, r);
 }
 
 }  // namespace fix
@@ -196,18 +252,14 @@ struct FixAcc {
         k = k_;
         c = i + g.nx * (j + g.ny * (k + g.zg));
     }
-    // the neighbours [+1, +2, +3, -1, -2, -3] of *p along an axis
+    // index and side along z; in a slab none that wrap (ghost planes)
+    __device__ __forceinline__ int kz() const { return g.zg ? 1 << 29 : k; }
+    __device__ __forceinline__ int nz() const { return g.zg ? 1 << 30 : g.nz; }
+    // the neighbours of *p along an axis
     __device__ __forceinline__ void along(const double* p, int ax, double* f) const {
-        int q = ax == 0 ? i : (ax == 1 ? j : k);
+        int q = ax == 0 ? i : (ax == 1 ? j : kz());
         asm volatile("" : "+r"(q));  // keeps the offsets from being hoisted out of the caller's loop
-        const int stride = ax == 0 ? 1 : (ax == 1 ? g.nx : g.nx * g.ny);
-        const int n = ax == 0 ? g.nx : (ax == 1 ? g.ny : (g.zg ? 1 << 30 : g.nz));
-        if (ax == 2 && g.zg) q = 1 << 29;  // ghost planes
-#pragma unroll
-        for (int d = 1; d <= 3; ++d) {
-            f[d - 1] = __ldg(p + (q + d < n ? d : d - n) * stride);
-            f[d + 2] = __ldg(p + (q >= d ? -d : n - d) * stride);
-        }
+        fix::line(p, q, ax == 0 ? g.nx : (ax == 1 ? g.ny : nz()), ax == 0 ? 1 : (ax == 1 ? g.nx : g.nx * g.ny), f);
     }
     __device__ __forceinline__ void grad_lap(int a, double& gx, double& gy, double& gz, double& lap) const {
         const double* p = at(a);
@@ -215,7 +267,9 @@ struct FixAcc {
         const double f0 = __ldg(p);
 #pragma unroll
         for (int ax = 0; ax < 3; ++ax) along(p, ax, f[ax]);
-        const uint32_t e = max(fix::exp20(f0), max(fix::largest(f[0]), max(fix::largest(f[1]), fix::largest(f[2]))));
+        uint32_t e = fix::exp20(f0), lo = e;
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax) e = max(e, fix::largest(f[ax], lo));
         if (!fix::covered(e)) {
             if (e == 0 && fix::zero_bits(f0) && fix::zero_bits(f)) {
                 gx = gy = gz = lap = 0.0;
@@ -231,25 +285,15 @@ struct FixAcc {
             }
             return;
         }
-        const uint32_t ep = e + (7u << 20);
-        const int64_t i0 = fix::align(f0, ep);
-        int64_t T[3] = {-6 * i0, -6 * i0, -6 * i0};
-        double r[3];
-#pragma unroll
-        for (int ax = 0; ax < 3; ++ax) {
-            int64_t D[3];
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                const int64_t u = fix::align(f[ax][d], ep), w = fix::align(f[ax][d + 3], ep);
-                D[d] = u - w;
-                T[d] += u + w;
-            }
-            r[ax] = fix::to_double(fix::weigh_grad(D[0], D[1], D[2]), e, 0);
-        }
+        double r[4];
+        if (lo != 0u)
+            fix::grad_lap<false>(f0, f, e, r);
+        else
+            fix::grad_lap_zero(p, i, j, kz(), g.nx, g.ny, nz(), e, r);
         gx = r[0];
         gy = r[1];
         gz = r[2];
-        lap = fix::to_double(fix::weigh_lap(T[0], T[1], T[2]), e, 6);
+        lap = r[3];
     }
 
     __device__ __forceinline__ void grad(int a, double& gx, double& gy, double& gz) const {

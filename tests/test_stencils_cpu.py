@@ -56,3 +56,19 @@ def test_divergence_and_curl_of_arrays_far_apart(big, eps):
     assert close(out[3], div)
     for i in range(3):
         assert close(out[4 + i], curl[i])
+
+
+@pytest.mark.parametrize("kind", ["random", "wide", "zeros"])
+def test_stencils_are_odd(kind):
+    """Those of -y are minus those of y, bit for bit, as with IEEE sums: wherever
+    the values' bits are dropped, and where zeros keep their sign."""
+    shape = (11, 8, 9)
+    rng = np.random.default_rng(2)
+    y = rng.normal(size=(36, int(np.prod(shape))))
+    if kind == "wide":
+        y *= 2.0 ** rng.integers(-60, 60, y.shape)
+    if kind == "zeros":
+        y[rng.random(y.shape) < 0.3] = 0.0
+    minus = np.where(y == 0.0, 0.0, -y)
+    for f in (devstage.stencils, devstage.diffs):
+        np.testing.assert_array_equal(f(shape, minus, 4), -f(shape, y, 4))
