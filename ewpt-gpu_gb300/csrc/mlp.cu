@@ -37,7 +37,8 @@ struct GemmArgs {
     float* C;
     int M, N, K, lda, ldb, ldc;
     int transA, transB;
-    long spin;  // polls before the commit wait gives up
+    long spin;  // polls before the commit wait gives up, which sets
+    int* err;   // (device memory)
 };
 
 __device__ __forceinline__ __nv_bfloat16 ldA(const GemmArgs& g, int m, int k) {
@@ -63,12 +64,11 @@ __device__ __forceinline__ __nv_bfloat16 ldB(const GemmArgs& g, int k, int n) {
 // tcgen05.ld and writes C.  Every wait is bounded (g.spin polls, host-set
 // by ewpt_mlp_set_wait_limit, default kTcSpin).  A wait that runs out in any
 // thread ends the slab loop for the whole CTA (a block-wide vote, so every
-// thread leaves the loop at the same barrier), sets g_tc_err and skips the
+// thread leaves the loop at the same barrier), sets the net's flag and skips the
 // remaining tensor-core work; before the TMEM columns are freed the CTA waits
 // again, with the full kTcSpin limit, for the MMAs already committed.
 constexpr int TC_M = 128, TC_N = 64, TC_K = 64;
 constexpr long kTcSpin = 1L << 22;
-__device__ int g_tc_err = 0;
 
 __device__ __forceinline__ uint32_t tc_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(128) k_gemm_tc(GemmArgs g) {
             // let them finish before the CTA leaves the loop
             tc_wait(ubar, ks & 1, kTcSpin);
             ok = false;
-            if (tid == 0) atomicExch(&g_tc_err, 1);
+            if (tid == 0) atomicExch(g.err, 1);
         }
     }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -261,8 +261,10 @@ __global__ void k_colsum(const float* __restrict__ dz, float* db, int B, int N) 
     db[n] = s;
 }
 
+// No step where a wait of the call's GEMMs ran out (all of them have ended).
 __global__ void k_adamw(float* w, const float* __restrict__ g, float* m, float* v, int64_t n, float lr, float b1,
-                        float b2, float eps, float wd, float c1, float c2) {
+                        float b2, float eps, float wd, float c1, float c2, const int* __restrict__ err) {
+    if (*err) return;
     for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x) {
         const float gq = g[q];
         const float mq = b1 * m[q] + (1.f - b1) * gq;
@@ -284,7 +286,9 @@ __global__ void k_sum_partials(const float* __restrict__ part, int n, float* out
 struct ewpt_mlp {
     int nin = 0, width = 0, nout = 0, maxb = 0, device = 0;
     cudaStream_t st = nullptr;
-    int64_t wait_polls = -1;  // limit of the GEMM's tensor-core waits in polls (< 0: default)
+    int* tc_err = nullptr;      // set by a GEMM whose wait ran out
+    int64_t wait_polls = -1;    // limit of the GEMM's tensor-core waits in polls (< 0: default)
+    int64_t weight_polls = -1;  // the same in k_weights alone (< 0: wait_polls)
     int64_t np = 0;
     int64_t oW1 = 0, ob1 = 0, oW2 = 0, ob2 = 0, oW3 = 0, ob3 = 0;
     float *p = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;
@@ -328,9 +332,8 @@ int mlp_cuda(ewpt_mlp* n, cudaError_t e, const char* what) {
     if (e == cudaSuccess) {
         // a bounded tensor-core wait that ran out (k_gemm_tc) invalidates the results
         int h = 0;
-        if (cudaMemcpyFromSymbol(&h, g_tc_err, sizeof h) == cudaSuccess && h) {
-            const int z = 0;
-            cudaMemcpyToSymbol(g_tc_err, &z, sizeof z);
+        if (n && cudaMemcpy(&h, n->tc_err, sizeof h, cudaMemcpyDeviceToHost) == cudaSuccess && h) {
+            cudaMemsetAsync(n->tc_err, 0, sizeof h, n->st);
             return mlp_fail(n, EWPT_ERR_TIMEOUT, "a tensor-core wait in the MLP GEMM ran out (results invalid)");
         }
         return EWPT_OK;
@@ -342,7 +345,7 @@ int mlp_cuda(ewpt_mlp* n, cudaError_t e, const char* what) {
 cudaError_t gemm(const ewpt_mlp* n, const __nv_bfloat16* A, int lda, int transA, const __nv_bfloat16* B, int ldb,
                  int transB, float* C, int ldc, int M, int N, int K) {
     const cudaStream_t st = n->st;
-    GemmArgs g{A, B, C, M, N, K, lda, ldb, ldc, transA, transB, n->wait_polls < 0 ? kTcSpin : (long)n->wait_polls};
+    GemmArgs g{A, B, C, M, N, K, lda, ldb, ldc, transA, transB, n->wait_polls < 0 ? kTcSpin : (long)n->wait_polls, n->tc_err};
     const dim3 gr((N + TC_N - 1) / TC_N, (M + TC_M - 1) / TC_M);
     k_gemm_tc<<<gr, 128, 0, st>>>(g);
     return cudaGetLastError();
@@ -523,17 +526,25 @@ cudaError_t layers_run(ewpt_mlp* n, int B, bool train, bool adam, float lr, floa
     if (e == cudaSuccess) e = launch(n, k_layer<kBackward>, dim3(W / LN, my), smem(W), b1, true);
     WeightArgs w{};
     const int tw = round_up(W, LM) / LM, n1 = round_up(I, LN) / LN, nW = W / LN;
-    w.w[0] = WeightGrad{n->dz2T, n->a1T, n->dz2, W, W, nW, 0, n->oW2, n->ob2, n->W2i, n->W2t, W, W};
-    w.w[1] = WeightGrad{n->dz1T, n->x0T, n->dz1, W, I, n1, tw * nW, n->oW1, n->ob1, n->W1i, nullptr, n->K1, 0};
-    w.w[2] = WeightGrad{n->dz3T, n->a2T, n->dz3, O, W, nW, tw * (nW + n1), n->oW3, n->ob3, n->W3i, n->W3t, W, n->N3};
-    w.batch = B, w.Bp = Bp, w.adam = adam, w.nloss = (int)my * (n->N3 / LN) * (LT / 32), w.loss_part = n->lpart;
+    w.w[0] = WeightGrad{n->dz2T, n->a1T, n->dz2, W, W, nW, 0, n->oW2, n->ob2};
+    w.w[1] = WeightGrad{n->dz1T, n->x0T, n->dz1, W, I, n1, tw * nW, n->oW1, n->ob1};
+    w.w[2] = WeightGrad{n->dz3T, n->a2T, n->dz3, O, W, nW, tw * (nW + n1), n->oW3, n->ob3};
+    w.batch = B, w.Bp = Bp, w.nloss = (int)my * (n->N3 / LN) * (LT / 32), w.loss_part = n->lpart;
     w.loss = n->mapped;
-    w.p = n->p, w.g = n->g, w.m = n->m, w.v = n->v, w.pb = n->pb;
-    w.lr = lr, w.b1 = 0.9f, w.b2 = 0.999f, w.eps = 1e-8f, w.wd = wd, w.c1 = c1, w.c2 = c2;
+    w.g = n->g;
     w.st = st;
+    if (n->weight_polls >= 0) w.st.spin = (long)n->weight_polls;
     if (e == cudaSuccess)
         e = launch(n, k_weights, dim3(tw * (nW + n1) + nW), std::max(smem(Bp), LM * (LN + 1) * 4), w, true);
-    return e;
+    if (!adam || e != cudaSuccess) return e;
+    StepArgs s{};
+    s.w[0] = StepWeights{n->oW1, W, I, n->W1i, nullptr, n->K1, 0};
+    s.w[1] = StepWeights{n->oW2, W, W, n->W2i, n->W2t, W, W};
+    s.w[2] = StepWeights{n->oW3, O, W, n->W3i, n->W3t, W, n->N3};
+    s.np = n->np, s.g = n->g, s.p = n->p, s.m = n->m, s.v = n->v, s.pb = n->pb;
+    s.lr = lr, s.b1 = 0.9f, s.b2 = 0.999f, s.eps = 1e-8f, s.wd = wd, s.c1 = c1, s.c2 = c2;
+    s.st = st;
+    return launch(n, k_step, dim3((unsigned)std::min<int64_t>((n->np + LT - 1) / LT, 1216)), 0, s, true);
 }
 
 // after the stream has been waited for
@@ -605,6 +616,7 @@ int ewpt_mlp_create(int32_t n_in, int32_t width, int32_t n_out, int32_t max_batc
     A((void**)&n->dzb, (size_t)max_batch * wa * 2);
     A((void**)&n->part, 64 * 4);
     A((void**)&n->loss, 4);
+    A((void**)&n->tc_err, 4);
     n->layers = layers_fit(n);
     if (e == cudaSuccess && n->layers) e = layers_alloc(n);
     if (e == cudaSuccess) e = cudaStreamSynchronize(n->st);
@@ -622,7 +634,7 @@ int ewpt_mlp_destroy(ewpt_mlp* n) {
     cudaSetDevice(n->device);
     if (n->st) cudaStreamSynchronize(n->st);
     void* bufs[] = {n->p, n->g, n->m, n->v, n->pb, n->xf, n->yf, n->x0, n->z1, n->z2, n->z3,
-                    n->a1, n->a2, n->da, n->dzf, n->dzb, n->part, n->loss};
+                    n->a1, n->a2, n->da, n->dzf, n->dzb, n->part, n->loss, n->tc_err};
     for (void* b : bufs) cudaFree(b);
     cudaFree(n->images);
     cudaFreeHost(n->host);
@@ -638,6 +650,12 @@ int64_t ewpt_mlp_num_params(const ewpt_mlp* n) { return n ? n->np : -1; }
 int ewpt_mlp_set_wait_limit(ewpt_mlp* n, int64_t polls) {
     if (!n) return ewpt_fail(nullptr, EWPT_ERR_ARG, "net is NULL");
     n->wait_polls = polls < 0 ? -1 : polls;
+    return EWPT_OK;
+}
+
+int ewpt_mlp_set_weight_wait_limit(ewpt_mlp* n, int64_t polls) {
+    if (!n) return ewpt_fail(nullptr, EWPT_ERR_ARG, "net is NULL");
+    n->weight_polls = polls < 0 ? -1 : polls;
     return EWPT_OK;
 }
 
@@ -719,22 +737,24 @@ int ewpt_mlp_train_step(ewpt_mlp* n, const float* x, const float* y, int32_t bat
     if (n->layers && batch <= kLayerMaxK) {
         std::memcpy(n->hx, x, (size_t)batch * n->nin * 4);
         std::memcpy(n->hy, y, (size_t)batch * n->nout * 4);
-        n->t += 1;
-        cudaError_t e = layers_run(n, batch, true, true, lr, weight_decay, 1.f - std::pow(0.9f, (float)n->t),
-                                   1.f - std::pow(0.999f, (float)n->t));
+        const int64_t t = n->t + 1;
+        cudaError_t e = layers_run(n, batch, true, true, lr, weight_decay, 1.f - std::pow(0.9f, (float)t),
+                                   1.f - std::pow(0.999f, (float)t));
         if (e == cudaSuccess) e = cudaStreamSynchronize(n->st);
         if (loss) *loss = n->host[0] / ((float)batch * n->nout);
-        return layers_done(n, e, "mlp train_step");
+        rc = layers_done(n, e, "mlp train_step");
+        if (!rc) n->t = t;
+        return rc;
     }
     cudaError_t e = upload(n, n->xf, x, (int64_t)batch * n->nin);
     if (e == cudaSuccess) e = upload(n, n->yf, y, (int64_t)batch * n->nout);
     if (e == cudaSuccess) e = forward(n, batch);
     if (e == cudaSuccess) e = backward(n, batch);
-    n->t += 1;
+    const int64_t t = n->t + 1;
     const float b1 = 0.9f, b2 = 0.999f;
-    const float c1 = 1.f - std::pow(b1, (float)n->t), c2 = 1.f - std::pow(b2, (float)n->t);
+    const float c1 = 1.f - std::pow(b1, (float)t), c2 = 1.f - std::pow(b2, (float)t);
     if (e == cudaSuccess) {
-        k_adamw<<<kEW, 256, 0, n->st>>>(n->p, n->g, n->m, n->v, n->np, lr, b1, b2, 1e-8f, weight_decay, c1, c2);
+        k_adamw<<<kEW, 256, 0, n->st>>>(n->p, n->g, n->m, n->v, n->np, lr, b1, b2, 1e-8f, weight_decay, c1, c2, n->tc_err);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = refresh_bf16(n);
@@ -743,7 +763,9 @@ int ewpt_mlp_train_step(ewpt_mlp* n, const float* x, const float* y, int32_t bat
     if (e == cudaSuccess && loss) e = cudaMemcpyAsync(&l, n->loss, 4, cudaMemcpyDeviceToHost, n->st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(n->st);
     if (loss) *loss = l / ((float)batch * n->nout);
-    return mlp_cuda(n, e, "mlp train_step");
+    rc = mlp_cuda(n, e, "mlp train_step");
+    if (!rc) n->t = t;
+    return rc;
 }
 
 }  // extern "C"

@@ -4,11 +4,12 @@
 // A training step at the surrogate's size (84-256-256-40, batches of 128) is
 // bound by latency: 0.06 GFLOP, 1 MB.  As 11 general GEMMs (k_gemm_tc, 25 us
 // each, most of it the scalar gather of the operands) and 13 element-wise
-// launches it took 282 us.  Here it is six launches:
+// launches it took 282 us.  Here it is seven launches:
 //   layer 1, layer 2    Z = A W^T + b, A' = gelu(Z)
 //   layer 3             Z3, the loss and dZ3
 //   back 2, back 1      dZ = (dZ' W) gelu'(Z)
-//   weights             all three dW = dZ^T A with the bias sums and AdamW
+//   weights             all three dW = dZ^T A with the bias sums
+//   AdamW               unless a wait of the call ran out
 // Every operand lies in global memory as the tensor cores read it (K-major
 // core matrices of 8 rows x 16 bytes, no swizzle), written by the kernel that
 // makes it: an epilogue stores the activations once with K along the features,
@@ -21,7 +22,9 @@
 // The accumulation order along K is k_gemm_tc's (K = 16 per MMA, in order).
 //
 // Waits are bounded as in k_gemm_tc: one that runs out ends the CTA's work
-// after its copies and MMAs in flight have landed, and marks the call.
+// after its copies and MMAs in flight have landed, and marks the call.  The
+// parameters are stepped by a kernel of their own, which reads the mark after the
+// last of the waits: a step is taken whole or not at all.
 #pragma once
 #include <cuda_bf16.h>
 
@@ -263,40 +266,25 @@ __global__ void __launch_bounds__(LT) k_layer(const __grid_constant__ LayerArgs 
     tile_end(t);
 }
 
-// One weight matrix of the last kernel: dW [M][N] = dZ^T A, K along the batch.
+// One weight matrix: dW [M][N] = dZ^T A, K along the batch.
 struct WeightGrad {
     const __nv_bfloat16 *dzT, *aT;  // images [M][Bp], [N][Bp]
     const float* dz;                // [batch][M]: the bias gradient's terms
     int M, N, tiles_n, first;       // first CTA
     int64_t oW, ob;                 // of the weights and biases in the parameter vector
-    __nv_bfloat16 *img, *imgT;      // weight images [M][Kp], [N][KpT] (imgT may be null)
-    int Kp, KpT;
 };
 struct WeightArgs {
     WeightGrad w[3];
-    int batch, Bp, adam, nloss;
+    int batch, Bp, nloss;
     const float* loss_part;
     volatile float* loss;  // mapped
-    float *p, *g, *m, *v;
-    __nv_bfloat16* pb;
-    float lr, b1, b2, eps, wd, c1, c2;
+    float* g;
     Status st;
 };
 
-// parameter q after AdamW's step with gradient gq, from its moments and value;
-// k_adamw's operations with its fused multiply-adds written out, so that both
-// train to the same bits
-__device__ __forceinline__ float weight_step(const WeightArgs& a, int64_t q, float gq, float m, float v, float w) {
-    const float mq = fmaf(1.f - a.b1, gq, __fmul_rn(a.b1, m));
-    const float vq = fmaf(__fmul_rn(1.f - a.b2, gq), gq, __fmul_rn(a.b2, v));
-    a.m[q] = mq;
-    a.v[q] = vq;
-    const float r = fmaf(-a.lr, fmaf(a.wd, w, (mq / a.c1) / (sqrtf(vq / a.c2) + a.eps)), w);
-    a.p[q] = r;
-    return r;
-}
-
-__global__ void __launch_bounds__(LT) k_weights(const __grid_constant__ WeightArgs a) {
+// One block per SM: registers for 32 loads of the bias sums in flight (without it
+// the compiler takes 32 registers and a step at a batch of 512 11 us more).
+__global__ void __launch_bounds__(LT, 1) k_weights(const __grid_constant__ WeightArgs a) {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ Tile t;
     const int tid = threadIdx.x;
@@ -305,8 +293,8 @@ __global__ void __launch_bounds__(LT) k_weights(const __grid_constant__ WeightAr
     const int tile = blockIdx.x - w.first, m0 = tile / w.tiles_n * LM, n0 = tile % w.tiles_n * LN;
     uint8_t *sa = smem, *sb = smem + LM * a.Bp * 2;
     tile_begin(t);
+    dep_launch();
     dep_wait();
-    const bool dead = *a.st.dev == a.st.gen;  // an earlier kernel of the call gave up: leave the weights alone
     if (tid == 0) {
         tile_expect(t, (LM + LN) * a.Bp * 2);
         tile_copy(t, sa, w.dzT + img(m0, 0, a.Bp), LM * a.Bp * 2);
@@ -323,9 +311,9 @@ __global__ void __launch_bounds__(LT) k_weights(const __grid_constant__ WeightAr
     }
     bool ok = tile_wait(t.ld, a.st);
     if (ok) ok = tile_mma(t, sa, sb, a.Bp, a.st);
-    if (ok && !dead) {
+    if (ok) {
         // through shared memory (the operand tiles are done with), so that the
-        // parameters are read and written along their rows
+        // gradients are written along their rows
         float* c = reinterpret_cast<float*>(smem);
         {
             float v[8];
@@ -336,40 +324,12 @@ __global__ void __launch_bounds__(LT) k_weights(const __grid_constant__ WeightAr
         __syncthreads();
         const int n = n0 + (tid & (LN - 1));
         constexpr int kRows = LM * LN / LT;  // rows of this thread: tid / 16, + 16, ...
-        float pm[kRows], pv[kRows], pp[kRows];
-        if (a.adam)
-#pragma unroll
-            for (int i = 0; i < kRows; ++i) {
-                const int m = m0 + tid / LN + i * (LT / LN);
-                if (m < w.M && n < w.N) {
-                    const int64_t q = w.oW + (int64_t)m * w.N + n;
-                    pm[i] = a.m[q];
-                    pv[i] = a.v[q];
-                    pp[i] = a.p[q];
-                }
-            }
 #pragma unroll
         for (int i = 0; i < kRows; ++i) {
             const int r = tid / LN + i * (LT / LN), m = m0 + r;
-            if (m >= w.M || n >= w.N) continue;
-            const int64_t q = w.oW + (int64_t)m * w.N + n;
-            const float gq = c[r * (LN + 1) + (tid & (LN - 1))];
-            if (a.adam) {
-                const __nv_bfloat16 h = __float2bfloat16(weight_step(a, q, gq, pm[i], pv[i], pp[i]));
-                a.pb[q] = h;
-                w.img[img(m, n, w.Kp)] = h;
-                if (w.imgT) w.imgT[img(n, m, w.KpT)] = h;
-            } else {
-                a.g[q] = gq;
-            }
+            if (m < w.M && n < w.N) a.g[w.oW + (int64_t)m * w.N + n] = c[r * (LN + 1) + (tid & (LN - 1))];
         }
-        if (bias) {
-            const int64_t q = w.ob + mb;
-            if (a.adam)
-                a.pb[q] = __float2bfloat16(weight_step(a, q, db, a.m[q], a.v[q], a.p[q]));
-            else
-                a.g[q] = db;
-        }
+        if (bias) a.g[w.ob + mb] = db;
         if (blockIdx.x == 0 && tid == 0) {
             float s = 0.f;
             for (int i = 0; i < a.nloss; ++i) s += a.loss_part[i];
@@ -377,6 +337,49 @@ __global__ void __launch_bounds__(LT) k_weights(const __grid_constant__ WeightAr
         }
     }
     tile_end(t);
+}
+
+// AdamW on all parameters, and the images of the stepped weights.
+struct StepWeights {
+    int64_t oW;  // weights [M][N] in the parameter vector
+    int M, N;
+    __nv_bfloat16 *im, *imT;  // images [M][Kp], [N][KpT] (imT may be null)
+    int Kp, KpT;
+};
+struct StepArgs {
+    StepWeights w[3];
+    int64_t np;
+    const float* g;
+    float *p, *m, *v;
+    __nv_bfloat16* pb;
+    float lr, b1, b2, eps, wd, c1, c2;
+    Status st;
+};
+
+// k_adamw's operations with its fused multiply-adds written out, so that both
+// train to the same bits
+__global__ void __launch_bounds__(LT) k_step(const __grid_constant__ StepArgs a) {
+    dep_wait();
+    if (*a.st.dev == a.st.gen) return;  // every kernel that could set it has ended
+    for (int64_t q = blockIdx.x * LT + threadIdx.x; q < a.np; q += (int64_t)gridDim.x * LT) {
+        const float gq = a.g[q], w = a.p[q];
+        const float mq = fmaf(1.f - a.b1, gq, __fmul_rn(a.b1, a.m[q]));
+        const float vq = fmaf(__fmul_rn(1.f - a.b2, gq), gq, __fmul_rn(a.b2, a.v[q]));
+        a.m[q] = mq;
+        a.v[q] = vq;
+        const float r = fmaf(-a.lr, fmaf(a.wd, w, (mq / a.c1) / (sqrtf(vq / a.c2) + a.eps)), w);
+        a.p[q] = r;
+        const __nv_bfloat16 h = __float2bfloat16(r);
+        a.pb[q] = h;
+#pragma unroll
+        for (int l = 0; l < 3; ++l) {
+            const StepWeights& s = a.w[l];
+            if (q < s.oW || q >= s.oW + (int64_t)s.M * s.N) continue;
+            const int e = (int)(q - s.oW), m = e / s.N, n = e - m * s.N;
+            s.im[img(m, n, s.Kp)] = h;
+            if (s.imT) s.imT[img(n, m, s.KpT)] = h;
+        }
+    }
 }
 
 // the weight images of the FP32 parameters

@@ -146,6 +146,7 @@ def _sig(L):
     L.ewpt_slab_unpack.argtypes = [V, C.c_int32, C.c_void_p, C.c_void_p]
     L.ewpt_slab_stage.argtypes = [V, C.c_int32, C.c_double, C.c_double]
     L.ewpt_mlp_set_wait_limit.argtypes = [V, C.c_int64]
+    L.ewpt_mlp_set_weight_wait_limit.argtypes = [V, C.c_int64]
 
 
 def load():

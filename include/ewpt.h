@@ -406,6 +406,9 @@ int64_t ewpt_mlp_num_params(const ewpt_mlp* net);
  * default 2^22; 0: every wait gives up at once, the call returns
  * EWPT_ERR_TIMEOUT and the net stays usable).  For testing. */
 int ewpt_mlp_set_wait_limit(ewpt_mlp* net, int64_t polls);
+/* The same for the weight-gradient kernel of a training step alone, the last
+ * that waits (< 0: the limit above; nets with layer kernels). */
+int ewpt_mlp_set_weight_wait_limit(ewpt_mlp* net, int64_t polls);
 /* set (resets the optimizer state) / get the FP32 parameters */
 int ewpt_mlp_set_params(ewpt_mlp* net, const float* params);
 int ewpt_mlp_get_params(ewpt_mlp* net, float* params);
@@ -413,7 +416,8 @@ int ewpt_mlp_get_params(ewpt_mlp* net, float* params);
 int ewpt_mlp_forward(ewpt_mlp* net, const float* x, int32_t batch, float* y);
 /* loss and d loss / d params (same layout as the parameters) at the current parameters */
 int ewpt_mlp_gradients(ewpt_mlp* net, const float* x, const float* y, int32_t batch, float* grads, float* loss);
-/* one AdamW step (beta1 0.9, beta2 0.999, eps 1e-8, decoupled weight decay); loss may be NULL */
+/* one AdamW step (beta1 0.9, beta2 0.999, eps 1e-8, decoupled weight decay); loss may be NULL.
+ * A call that returns EWPT_ERR_TIMEOUT has taken no step. */
 int ewpt_mlp_train_step(ewpt_mlp* net, const float* x, const float* y, int32_t batch, float lr, float weight_decay,
                         float* loss);
 

@@ -106,3 +106,34 @@ def test_a_wait_that_runs_out_leaves_the_weights_alone():
     f = mo.forward(p.astype(np.float64), x.astype(np.float64), *dims)["z3"]
     assert np.linalg.norm(net.forward(x) - f) / np.linalg.norm(f) < 2e-3
     net.close()
+
+
+@pytest.mark.parametrize("dims,B", [((84, 256, 40), 128), ((17, 96, 33), 37), ((84, 40, 40), 40), ((84, 256, 40), 600)])
+@pytest.mark.parametrize("last", [False, True])
+def test_a_step_whose_wait_runs_out_is_not_taken(dims, B, last):
+    """Neither where the first kernel gives up nor where only the weight
+    gradients' does (last; networks with layer kernels): parameters, moments
+    and the step count are as before, so the net then trains as a fresh one
+    does, bit for bit."""
+    from ewpt import _lib
+
+    layers = dims[1] % 16 == 0 and B <= 512
+    if last and not layers:
+        pytest.skip("no layer kernels")
+    net, fresh = make(dims, 600), make(dims, 600)
+    x, y = data(dims, B, 3)
+    p = net.get_params()
+    limit = net.L.ewpt_mlp_set_weight_wait_limit if last else net.L.ewpt_mlp_set_wait_limit
+    assert limit(net.h, 0) == 0
+    for _ in range(3):
+        with pytest.raises(_lib.EwptError) as ei:
+            net.train_step(x, y, 1e-3, 1e-2)
+        assert ei.value.code == _lib.ERR_TIMEOUT
+        assert np.array_equal(net.get_params(), p)
+    assert limit(net.h, -1) == 0
+    for _ in range(2):
+        assert net.train_step(x, y, 1e-3, 1e-2) == fresh.train_step(x, y, 1e-3, 1e-2)
+        assert np.array_equal(net.get_params(), fresh.get_params())
+    assert np.array_equal(net.forward(x), fresh.forward(x))
+    net.close()
+    fresh.close()
