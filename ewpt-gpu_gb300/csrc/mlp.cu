@@ -316,6 +316,7 @@ struct ewpt_mlp {
     float *dz1 = nullptr, *dz2 = nullptr, *dz3 = nullptr, *lpart = nullptr;
     int* flag = nullptr;
     int gen = 0;
+    int hrows = 0;          // rows of x and z3 in
     float* host = nullptr;  // [0] loss, [1] status, then x, y, z3
     float *hx = nullptr, *hy = nullptr, *hz = nullptr;
     float* mapped = nullptr;  // device address of host
@@ -404,6 +405,13 @@ cudaError_t backward(ewpt_mlp* n, int B) {
 
 // ---- layer kernels
 constexpr int kMappedHead = 32;  // floats before x in the mapped buffer
+// Layer 1 reads a batch's inputs once for each of its width / 16 column tiles:
+// from the mapped buffer while that is at most so many floats, else from a copy
+// in device memory.  Forward pass, us, mapped / copied: 84-256-40 128 rows 41 / 42,
+// 256 rows 46 / 48, 512 rows 67 / 51, 8192 rows 567 / 183; 512-512-128 32 rows 53 / 54,
+// 128 rows 89 / 66, 8192 rows 4146 / 748 (element-wise kernels and general GEMM: 299
+// and 899 at 8192).
+constexpr int64_t kHostReads = 3 << 17;
 
 bool layers_fit(const ewpt_mlp* n) {
     return n->width % LN == 0 && n->width <= kLayerMaxK && n->nin <= kLayerMaxK && n->nout <= LM;
@@ -448,13 +456,15 @@ cudaError_t layers_alloc(ewpt_mlp* n) {
         *q.p = static_cast<char*>(n->images) + off;
         off += (q.bytes + 127) / 128 * 128;
     }
-    const int64_t rows = n->maxb;
+    n->hrows = (int)std::min<int64_t>(std::max<int64_t>(kHostReads / ((int64_t)n->nin * (W / LN)), 1), n->maxb);
+    const int64_t targets = (int64_t)std::min(n->maxb, kLayerMaxK) * n->nout;
     if (e == cudaSuccess)
-        e = cudaHostAlloc((void**)&n->host, (kMappedHead + rows * (n->nin + 2 * n->nout)) * 4, cudaHostAllocMapped);
+        e = cudaHostAlloc((void**)&n->host, (kMappedHead + targets + (int64_t)n->hrows * (n->nin + n->nout)) * 4,
+                          cudaHostAllocMapped);
     if (e == cudaSuccess) e = cudaHostGetDevicePointer((void**)&n->mapped, n->host, 0);
     n->hx = n->host + kMappedHead;
-    n->hy = n->hx + rows * n->nin;
-    n->hz = n->hy + rows * n->nout;
+    n->hy = n->hx + (int64_t)n->hrows * n->nin;
+    n->hz = n->hy + targets;
     const int smem = (LM + LN) * kLayerMaxK * 2;
     const void* kernels[] = {(const void*)k_layer<kForward>, (const void*)k_layer<kOutput>,
                              (const void*)k_layer<kBackward>, (const void*)k_weights};
@@ -488,9 +498,16 @@ cudaError_t launch(const ewpt_mlp* n, void (*k)(Args), dim3 grid, int smem, cons
     return cudaLaunchKernelEx(&c, k, a);
 }
 
-// The layers on the batch in the mapped buffer; train: loss and weight
-// gradients into n->g, or (adam) one AdamW step instead.
-cudaError_t layers_run(ewpt_mlp* n, int B, bool train, bool adam, float lr, float wd, float c1, float c2) {
+// The layers on the inputs x and the targets in the mapped buffer; train: loss
+// and weight gradients into n->g, and (adam) one AdamW step.
+cudaError_t layers_run(ewpt_mlp* n, const float* x, int B, bool train, bool adam, float lr, float wd, float c1,
+                       float c2) {
+    cudaError_t e = cudaSuccess;
+    if (B <= n->hrows)
+        std::memcpy(n->hx, x, (size_t)B * n->nin * 4);
+    else
+        e = cudaMemcpyAsync(n->xf, x, (size_t)B * n->nin * 4, cudaMemcpyHostToDevice, n->st);
+    if (e != cudaSuccess) return e;
     const int W = n->width, I = n->nin, O = n->nout, Bp = round_up(B, 16);
     const unsigned my = (unsigned)((B + LM - 1) / LM);
     n->host[0] = 0.f;
@@ -505,7 +522,7 @@ cudaError_t layers_run(ewpt_mlp* n, int B, bool train, bool adam, float lr, floa
     b.train = train;
     b.st = st;
     LayerArgs f1 = b, f2 = b, f3 = b, b2 = b, b1 = b;
-    f1.x = n->mapped + kMappedHead;
+    f1.x = B <= n->hrows ? n->mapped + kMappedHead : n->xf;
     f1.W = n->W1i, f1.bias = n->p + n->ob1, f1.N = W, f1.Kp = n->K1, f1.z = n->z1, f1.out = n->a1i, f1.outK = W;
     f2.A = n->a1i, f2.W = n->W2i, f2.bias = n->p + n->ob2, f2.N = W, f2.Kp = W, f2.z = n->z2, f2.out = n->a2i, f2.outK = W;
     f3.A = n->a2i, f3.W = n->W3i, f3.bias = n->p + n->ob3, f3.N = O, f3.Kp = W, f3.zo = n->z3;
@@ -515,7 +532,7 @@ cudaError_t layers_run(ewpt_mlp* n, int B, bool train, bool adam, float lr, floa
         f3.out = n->dz3i, f3.outK = n->N3, f3.outT = n->dz3T;
     }
     auto smem = [](int K) { return (LM + LN) * K * 2; };
-    cudaError_t e = launch(n, k_layer<kForward>, dim3(W / LN, my), smem(f1.Kp), f1, false);
+    e = launch(n, k_layer<kForward>, dim3(W / LN, my), smem(f1.Kp), f1, false);
     if (e == cudaSuccess) e = launch(n, k_layer<kForward>, dim3(W / LN, my), smem(W), f2, true);
     if (e == cudaSuccess) e = launch(n, k_layer<kOutput>, dim3(n->N3 / LN, my), smem(W), f3, true);
     if (!train || e != cudaSuccess) return e;
@@ -688,12 +705,12 @@ int ewpt_mlp_forward(ewpt_mlp* n, const float* x, int32_t batch, float* y) {
     if (!x || !y) return mlp_fail(n, EWPT_ERR_ARG, "NULL argument");
     if (n->layers) {
         const size_t out = (size_t)batch * n->nout * 4;
-        std::memcpy(n->hx, x, (size_t)batch * n->nin * 4);
-        cudaError_t e = layers_run(n, batch, false, false, 0.f, 0.f, 1.f, 1.f);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(n->hz, n->z3, out, cudaMemcpyDeviceToHost, n->st);
+        const bool staged = batch <= n->hrows;
+        cudaError_t e = layers_run(n, x, batch, false, false, 0.f, 0.f, 1.f, 1.f);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(staged ? n->hz : y, n->z3, out, cudaMemcpyDeviceToHost, n->st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(n->st);
         rc = layers_done(n, e, "mlp forward");
-        if (!rc) std::memcpy(y, n->hz, out);
+        if (!rc && staged) std::memcpy(y, n->hz, out);
         return rc;
     }
     cudaError_t e = upload(n, n->xf, x, (int64_t)batch * n->nin);
@@ -708,9 +725,8 @@ int ewpt_mlp_gradients(ewpt_mlp* n, const float* x, const float* y, int32_t batc
     if (rc) return rc;
     if (!x || !y || !grads) return mlp_fail(n, EWPT_ERR_ARG, "NULL argument");
     if (n->layers && batch <= kLayerMaxK) {
-        std::memcpy(n->hx, x, (size_t)batch * n->nin * 4);
         std::memcpy(n->hy, y, (size_t)batch * n->nout * 4);
-        cudaError_t e = layers_run(n, batch, true, false, 0.f, 0.f, 1.f, 1.f);
+        cudaError_t e = layers_run(n, x, batch, true, false, 0.f, 0.f, 1.f, 1.f);
         if (e == cudaSuccess) e = cudaMemcpyAsync(grads, n->g, n->np * 4, cudaMemcpyDeviceToHost, n->st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(n->st);
         if (loss) *loss = n->host[0] / ((float)batch * n->nout);
@@ -735,10 +751,9 @@ int ewpt_mlp_train_step(ewpt_mlp* n, const float* x, const float* y, int32_t bat
     if (!x || !y) return mlp_fail(n, EWPT_ERR_ARG, "NULL argument");
     if (!std::isfinite(lr) || !std::isfinite(weight_decay)) return mlp_fail(n, EWPT_ERR_ARG, "non-finite lr/wd");
     if (n->layers && batch <= kLayerMaxK) {
-        std::memcpy(n->hx, x, (size_t)batch * n->nin * 4);
         std::memcpy(n->hy, y, (size_t)batch * n->nout * 4);
         const int64_t t = n->t + 1;
-        cudaError_t e = layers_run(n, batch, true, true, lr, weight_decay, 1.f - std::pow(0.9f, (float)t),
+        cudaError_t e = layers_run(n, x, batch, true, true, lr, weight_decay, 1.f - std::pow(0.9f, (float)t),
                                    1.f - std::pow(0.999f, (float)t));
         if (e == cudaSuccess) e = cudaStreamSynchronize(n->st);
         if (loss) *loss = n->host[0] / ((float)batch * n->nout);
