@@ -3,10 +3,13 @@
 // A context owns the device state of one periodic lattice and one CUDA
 // stream.  Host <-> device copies are explicit (ewpt_set_state /
 // ewpt_get_state); stepping, diagnostics and spectra run on the stream.
+#include <cuda.h>
+
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
 
 #include "ewpt_ctx.cuh"
@@ -34,14 +37,39 @@ int ewpt_cuda_check(ewpt_ctx* ctx, cudaError_t e, const char* what) {
     return ewpt_fail(ctx, EWPT_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
 }
 
-bool ewpt_kernel_reads(const void* p, int device) {
+// cuMemGetAddressRange: the allocation that holds an address
+using RangeFn = CUresult (*)(CUdeviceptr*, size_t*, CUdeviceptr);
+static RangeFn range_fn() {
+    static RangeFn fn = nullptr;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            fn = reinterpret_cast<RangeFn>(p);
+    });
+    return fn;
+}
+
+cudaError_t ewpt_kernel_reads(const void* p, size_t bytes, int device, bool* direct) {
+    *direct = false;
     cudaPointerAttributes a{};
-    if ((uintptr_t)p % sizeof(double) != 0) return false;
+    const RangeFn range = range_fn();
+    if (!range || (uintptr_t)p % sizeof(double) != 0) return cudaSuccess;
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         cudaGetLastError();  // not a sticky error: clear it
-        return false;
+        return cudaSuccess;
     }
-    return a.type == cudaMemoryTypeDevice && a.device == device;
+    if (a.type != cudaMemoryTypeDevice || a.device != device) return cudaSuccess;
+    const CUdeviceptr lo = (CUdeviceptr)p, hi = lo + bytes;
+    CUdeviceptr base = 0;
+    size_t size = 0;
+    if (range(&base, &size, lo) != CUDA_SUCCESS) return cudaSuccess;
+    *direct = base + size >= hi;
+    for (CUdeviceptr end = base + size; end < hi; end = base + size)
+        if (range(&base, &size, end) != CUDA_SUCCESS) return cudaErrorInvalidValue;
+    return cudaSuccess;
 }
 
 int ewpt_validate_params(const ewpt_params* p, ewpt_ctx* ctx) {
@@ -277,12 +305,19 @@ static cudaError_t copy_runs(ewpt_ctx* c, double* dev, const double* const* arra
 
 // A device state of the FP32 and DF64 forms is converted from / to the
 // caller's arrays themselves, without a pass through a staging buffer (at
-// 256^3 set + get of the FP32 form took 14.5 ms with it).
-static bool converts_in_place(const ewpt_ctx* c, const double* const* arrays) {
-    if (c->p.precision == EWPT_FP64) return false;
-    for (int a = 0; a < 36; ++a)
-        if ((a == 0 || arrays[a] != arrays[a - 1] + c->g.S) && !ewpt_kernel_reads(arrays[a], c->p.device)) return false;
-    return true;
+// 256^3 set + get of the FP32 form took 14.5 ms with it).  Error: arrays that
+// reach past the end of their allocation.
+static cudaError_t converts_in_place(const ewpt_ctx* c, const double* const* arrays, bool* yes) {
+    *yes = false;
+    if (c->p.precision == EWPT_FP64) return cudaSuccess;
+    for (int a = 0; a < 36;) {  // runs of arrays that lie back to back
+        int b = a + 1;
+        while (b < 36 && arrays[b] == arrays[b - 1] + c->g.S) ++b;
+        const cudaError_t e = ewpt_kernel_reads(arrays[a], (size_t)(b - a) * c->g.S * 8, c->p.device, yes);
+        if (e != cudaSuccess || !*yes) return e;
+        a = b;
+    }
+    return cudaSuccess;
 }
 
 int ewpt_set_state(ewpt_ctx* c, const double* const arrays[EWPT_NARR], int32_t on_device) {
@@ -292,8 +327,10 @@ int ewpt_set_state(ewpt_ctx* c, const double* const arrays[EWPT_NARR], int32_t o
     for (int a = 0; a < 36; ++a)
         if (!arrays[a]) return ewpt_fail(c, EWPT_ERR_ARG, "arrays[%d] is NULL", a);
     cudaSetDevice(c->p.device);
-    cudaError_t e;
-    if (on_device && converts_in_place(c, arrays)) {
+    bool direct = false;
+    cudaError_t e = on_device ? converts_in_place(c, arrays, &direct) : cudaSuccess;
+    if (e != cudaSuccess) return ewpt_cuda_check(c, e, "set_state");
+    if (direct) {
         Ptr36 src;
         for (int a = 0; a < 36; ++a) src.p[a] = arrays[a];
         e = c->p.precision == EWPT_FP32 ? launch_fp32_split(c->g, c->lay, src, c->y32, c->st, c->tile.pair == 2)
@@ -323,13 +360,14 @@ int ewpt_get_state(ewpt_ctx* c, double* const arrays[EWPT_NARR], int32_t on_devi
     for (int a = 0; a < 36; ++a)
         if (!arrays[a]) return ewpt_fail(c, EWPT_ERR_ARG, "arrays[%d] is NULL", a);
     cudaSetDevice(c->p.device);
-    const bool direct = on_device && converts_in_place(c, arrays);
+    bool direct = false;
+    cudaError_t e = on_device ? converts_in_place(c, arrays, &direct) : cudaSuccess;
+    if (e != cudaSuccess) return ewpt_cuda_check(c, e, "get_state");
     double* src = nullptr;
     int rc = direct ? EWPT_OK : ewpt_staging64(c, &src, false);
     if (rc) return rc;
     MPtr36 dst;
     for (int a = 0; a < 36; ++a) dst.p[a] = direct ? arrays[a] : src + a * c->g.S;
-    cudaError_t e = cudaSuccess;
     if (c->p.precision == EWPT_FP32) e = launch_fp32_join(c->g, c->lay, c->y32, dst, c->st);
     if (c->p.precision == EWPT_DF64) e = launch_from_dd(c->g.S, dd_in_pairs(c->g, c->p), c->y, dst, c->st);
     if (e == cudaSuccess && !direct) e = copy_runs(c, src, arrays, c->g.S, false, on_device);

@@ -200,9 +200,11 @@ int ewpt_ensemble_set_state(ewpt_ens* e, int32_t m, const double* packed, int32_
     if (!packed) return ens_fail(e, EWPT_ERR_ARG, "state is NULL");
     cudaSetDevice(e->device);
     ewpt_ctx* c = e->mem[m];
-    cudaError_t ce = cudaSuccess;
+    bool direct = false;
+    cudaError_t ce = on_device ? ewpt_kernel_reads(packed, (size_t)36 * c->g.S * 8, e->device, &direct) : cudaSuccess;
+    if (ce != cudaSuccess) return ens_cuda(e, ce, "ensemble set_state");
     const double* src = packed;
-    if (!on_device || !ewpt_kernel_reads(packed, e->device)) {
+    if (!direct) {
         ewpt_ctx* v;
         rc = ens_view(e, m, &v, 0);
         if (rc) return rc;
@@ -220,15 +222,17 @@ int ewpt_ensemble_get_state(ewpt_ens* e, int32_t m, double* packed, int32_t on_d
     if (rc) return rc;
     if (!packed) return ens_fail(e, EWPT_ERR_ARG, "state is NULL");
     cudaSetDevice(e->device);
-    cudaError_t ce;
-    if (on_device && ewpt_kernel_reads(packed, e->device)) {
-        const ewpt_ctx* c = e->mem[m];
+    const ewpt_ctx* c = e->mem[m];
+    bool direct = false;
+    cudaError_t ce = on_device ? ewpt_kernel_reads(packed, (size_t)36 * c->g.S * 8, e->device, &direct) : cudaSuccess;
+    if (ce != cudaSuccess) return ens_cuda(e, ce, "ensemble get_state");
+    if (direct) {
         ce = launch_fp32_join(c->g, c->lay, c->y32, arrays36(packed, c->g.S), e->st);
     } else {
         ewpt_ctx* v;
         rc = ens_view(e, m, &v);
         if (rc) return rc;
-        ce = cudaMemcpyAsync(packed, v->y, (size_t)36 * e->mem[m]->g.S * 8,
+        ce = cudaMemcpyAsync(packed, v->y, (size_t)36 * c->g.S * 8,
                              on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, e->st);
     }
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->st);

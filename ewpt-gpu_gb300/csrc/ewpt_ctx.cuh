@@ -68,9 +68,11 @@ int ewpt_ensure_scratch64(ewpt_ctx* c);
 // context's form (FP32 split with ghost faces, DF64 pairs), on c->st.
 extern "C" int ewpt_staging64(ewpt_ctx* c, double** out, bool in);
 extern "C" cudaError_t ewpt_commit_staged(ewpt_ctx* c, const double* staged);
-// Whether a kernel on `device` may take p's memory as it is (memory of that
-// device, 8-byte aligned); other memory goes through a copy.
-bool ewpt_kernel_reads(const void* p, int device);
+// Whether a kernel on `device` may take the bytes from p on as they are (within
+// one allocation of that device, 8-byte aligned); other memory goes through a
+// copy.  Error: they reach past the end of device memory, which a copy refuses
+// and a kernel would fault on.
+cudaError_t ewpt_kernel_reads(const void* p, size_t bytes, int device, bool* direct);
 // Interior of a slab context <-> a packed [36][nx ny nz] buffer (slab.cu).
 cudaError_t ewpt_slab_copy(ewpt_ctx* c, double* packed, bool to_dev, int32_t on_device);
 // Thermal IC (thermal.cu) into an FP64 [36][S] device state y, synchronous

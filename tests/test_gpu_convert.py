@@ -89,3 +89,48 @@ def test_ensemble_device_states():
         ens.set_state(0, y)
         np.testing.assert_array_equal(bits(out.cpu().numpy()), bits(ens.get_state(0)))
         np.testing.assert_array_equal(bits(ens.get_state(1)), bits(ens.get_state(0)))
+
+
+@pytest.mark.parametrize("form", [ewpt.FP32, ewpt.DF64, "ensemble"])
+def test_a_state_past_the_end_of_its_memory_is_refused(form):
+    """An error before anything is queued, and the context stays usable."""
+    import torch
+
+    from ewpt import _lib
+
+    shape = (64, 48, 48)
+    n = int(np.prod(shape))
+    p = ewpt.baseline_couplings(shape=shape, N=64, precision=ewpt.FP32 if form == "ensemble" else form)
+    y = torch.randn(36, n, dtype=torch.float64, device="cuda")
+    cu = C.CDLL("libcuda.so.1")
+    half, base, size = C.c_uint64(), C.c_uint64(), C.c_size_t()
+    assert cu.cuMemAlloc_v2(C.byref(half), C.c_size_t(18 * n * 8)) == 0
+    try:
+        end = half.value  # of the allocations that lie back to back
+        while cu.cuMemGetAddressRange_v2(C.byref(base), C.byref(size), C.c_uint64(end)) == 0:
+            end = base.value + size.value
+        short = end - 18 * n * 8
+        torch.cuda.synchronize()
+        lat = ewpt.Ensemble([p]) if form == "ensemble" else ewpt.Lattice(p)
+        with lat:
+            if form == "ensemble":
+                def put(ptr):
+                    return lat.L.ewpt_ensemble_set_state(lat.h, 0, C.c_void_p(ptr), 1)
+
+                def get(ptr):
+                    return lat.L.ewpt_ensemble_get_state(lat.h, 0, C.c_void_p(ptr), 1)
+            else:
+                def put(ptr):
+                    return lat.L.ewpt_set_state_packed(lat.h, C.c_void_p(ptr), 1)
+
+                def get(ptr):
+                    return lat.L.ewpt_get_state_packed(lat.h, C.c_void_p(ptr), 1)
+            assert put(y.data_ptr()) == 0
+            assert put(short) == _lib.ERR_CUDA
+            assert get(short) == _lib.ERR_CUDA
+            out = torch.zeros_like(y)
+            torch.cuda.synchronize()
+            assert get(out.data_ptr()) == 0
+            assert torch.allclose(out, y, rtol=1e-13, atol=0)
+    finally:
+        cu.cuMemFree_v2(half)
