@@ -43,9 +43,9 @@
 #pragma once
 
 // Qualifier of the per-site arithmetic (here and in accessors.cuh).  The
-// library compiles it for the device only; the operation counter of the test
-// suite (oracle/opcount.cu) defines it as __host__ __device__ to run the same
-// templates on the host with an operator-counting scalar type.
+// library compiles it for the device only; the test suite (oracle/devphys.cu,
+// oracle/devstage.cc) defines it as inline to run the same templates on the
+// host, with an operator-counting scalar type among others.
 #ifndef EWPT_ARITH
 #define EWPT_ARITH __device__ __forceinline__
 #endif

@@ -1,19 +1,19 @@
-// devphys.cu -- the stage kernels' per-site arithmetic compiled for the host
+// devphys.cu -- the equations of csrc/physics.cuh compiled for the host
 // (test and measurement infrastructure, never linked into libewpt).
 //
-// The per-site arithmetic of the stage kernels is the template site_rates
-// (csrc/physics.cuh) over the accessor SiteAcc (csrc/accessors.cuh).  This
-// file compiles those same templates for the host (EWPT_ARITH = inline) and
-// instantiates them twice:
+// site_rates (csrc/physics.cuh) over the accessor SiteAcc (csrc/accessors.cuh) is
+// what the stages of the alternative stencil orders evaluate in FP64 and those
+// of the DF64 form in double-float.  The 6th-order FP64 stages and the FP32 forms
+// have code of their own, which devstage.cc compiles.  Two instantiations:
 //
 //  * with double: dp_rates() evaluates all 36 rates at every site of a
-//    periodic lattice, so the tests compare the kernels' own equations with
-//    the oracle's restatement of rk4_step! on the CPU;
+//    periodic lattice, for a comparison with the oracle's restatement of
+//    rk4_step!;
 //  * with an operator-counting scalar type: dp_count() counts every
-//    addition, subtraction, multiplication and division the kernels' source
-//    performs for one site, exactly.  The epilogue of each stage (the RK4
-//    combination of stage.cu's Fp64Sink: two fused multiply-adds per array in
-//    stages 1-3, one in stage 4) is counted from its formulas.
+//    addition, subtraction, multiplication and division of one site, exactly:
+//    the work of a site-update whose stencils are in floating point.  The
+//    epilogue of each stage (the RK4 combination: two fused multiply-adds per
+//    array in stages 1-3, one in stage 4) is counted from its formulas.
 //
 // FLOPs are counted as the source writes them: an addition, subtraction or
 // multiplication is 1 FLOP and a fused multiply-add 2, so the total does not

@@ -1,9 +1,9 @@
-"""ctypes binding of oracle/devphys.cu: the stage kernels' per-site
-arithmetic (csrc/physics.cuh, csrc/accessors.cuh) compiled for the host.
+"""ctypes binding of oracle/devphys.cu: the equations of csrc/physics.cuh over
+csrc/accessors.cuh compiled for the host (devstage.py has the other stages').
 
 TEST AND MEASUREMENT INFRASTRUCTURE ONLY: the tests use it to compare the
-kernels' own equations with the oracle on the CPU and to count the FP64
-operations of one site-update exactly; the product library never links it.
+equations with the oracle on the CPU and to count the FP64 operations of one
+site-update exactly; the product library never links it.
 """
 from __future__ import annotations
 

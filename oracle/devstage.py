@@ -36,7 +36,7 @@ def build(force: bool = False) -> str:
         return LIB
     os.makedirs(os.path.dirname(LIB), exist_ok=True)
     tmp = f"{LIB}.{os.getpid()}"
-    subprocess.check_call([os.environ.get("CXX", "g++"), "-shared", "-fPIC", "-O2", "-std=c++17", "-ffp-contract=off",
+    subprocess.check_call([os.environ.get("CXX", "g++"), "-shared", "-fPIC", "-O2", "-std=c++17", "-ffp-contract=off", "-pthread",
                            "-I", HERE, "-I", os.path.join(ROOT, "include"), "-I", CSRC, "-I", _cuda_include(), SRC,
                            "-o", tmp])
     os.replace(tmp, LIB)
@@ -55,6 +55,8 @@ def lib():
         for f in (L.ds_stencils, L.ds_diffs):
             f.argtypes = [C.c_int, C.c_int, C.c_int, dp, C.c_int, dp]
             f.restype = None
+        L.ds_rates.argtypes = [C.c_int, C.c_int, C.c_int, dp, dp, dp, C.c_double, C.c_double, C.c_int]
+        L.ds_rates.restype = None
         _lib = L
     return _lib
 
@@ -79,3 +81,17 @@ def stencils(shape, y, a):
 def diffs(shape, y, a):
     """The diagnostics' rows: grad (3) of array a, divergence and curl (3) of a, a + 1, a + 2."""
     return _call(lib().ds_diffs, 7, shape, y, a)
+
+
+FORMS = {"fp64": 0, "fp32": 1, "orders": 2}
+
+
+def rates(shape, coef, y, Jex=0.0, gamma=0.0, form="fp64"):
+    """Rates of every site.  coef: (gw, gy, gp2, lambda, vev, beta_w, beta_y, dx);
+    form: the code of the FP64 stages, the equations of the FP32 forms, or those
+    of the DF64 form and the alternative stencil orders."""
+    y = np.ascontiguousarray(y, dtype=np.float64)
+    cp = np.ascontiguousarray(coef, dtype=np.float64)
+    r = np.full_like(y, np.nan)
+    lib().ds_rates(*shape, _ptr(cp), _ptr(y), _ptr(r), Jex, gamma, FORMS[form])
+    return r
