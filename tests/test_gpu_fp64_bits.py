@@ -63,3 +63,31 @@ def test_a_mirror_image_evolves_to_the_mirror_image():
 
     a = evolve(shape, y)
     np.testing.assert_array_equal(evolve(shape, mirror(y)), mirror(a))
+
+
+# 32-site blocks that straddle the edges of planes, of the host step's windows
+# and of slabs, where a whole lattice's blocks lie otherwise
+@pytest.mark.parametrize("shape", [(7, 9, 40), (11, 13, 37), (33, 7, 33)])
+@pytest.mark.parametrize("beta", [0.0, 0.3])
+def test_windows_and_slabs_of_ragged_planes(shape, beta):
+    import torch
+
+    from ewpt.slabs import SlabGroup
+
+    p = ewpt.baseline_couplings(shape=shape, N=shape[0], beta_w=beta, beta_y=-beta)
+    y = state(shape, 5)
+    ref = evolve(shape, y, steps=2, beta_w=beta, beta_y=-beta)
+    for cut in ([3, shape[2] - 3], [5, 7, shape[2] - 12]):
+        with SlabGroup(p, len(cut), nz_local=cut) as g:
+            g.set_state(y)
+            g.step(2, Jex=0.0, gamma=0.01)
+            np.testing.assert_array_equal(g.get_state(), ref)
+    with ewpt.Lattice(p) as lat:
+        lat.set_state(y)
+        lat.step(2)
+        ref = lat.get_state()
+    with ewpt.Lattice(p) as lat:
+        src = torch.from_numpy(y).pin_memory()
+        dst = torch.empty_like(src).pin_memory()
+        lat.step_host(src, dst, 2)
+    np.testing.assert_array_equal(dst.numpy(), ref)
