@@ -60,3 +60,26 @@ def test_register_variants_agree(tile):
     shape = (64, 48, 40)
     y = state(shape, 2)
     assert torch.equal(evolve(shape, ewpt.DF64, y, steps=3), evolve(shape, ewpt.DF64, y, tile, steps=3))
+
+
+@pytest.mark.parametrize("shape", [(50, 50, 50), (64, 48, 40)])
+def test_bubbles_match_fp64(shape):
+    """From a start in which most arrays are zero, and set by the device
+    initialiser, whose conversion is in place."""
+    import torch
+
+    p = ewpt.baseline_couplings(shape=shape, N=shape[0])
+    R, w = ewpt.ic.tanh_profile_params(p.lam, p.vev)
+    bubbles = ewpt.ic.tanh_bubble_list(shape, p.dx, 4, seed=3)
+    got = []
+    for form in (ewpt.DF64, ewpt.FP64):
+        with ewpt.Lattice(ewpt.baseline_couplings(shape=shape, N=shape[0], precision=form)) as lat:
+            lat.init_bubbles(bubbles, "tanh", R, w)
+            start = torch.from_numpy(lat.get_state())
+            lat.step(10, Jex=0.0, gamma=0.0)
+            got.append((start, torch.from_numpy(lat.get_state())))
+    assert torch.all((got[0][0] - got[1][0]).abs() <= 2.0 ** -47 * got[1][0].abs())
+    top = got[1][1].abs().amax(dim=1)
+    err = (got[0][1] - got[1][1]).abs().amax(dim=1)
+    assert torch.all(err <= 1e-11 * top)
+    assert (top > 0).sum() > 20
