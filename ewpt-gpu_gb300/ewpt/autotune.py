@@ -3,9 +3,10 @@
 Times every candidate launch shape (block bx x by over x-y, register-budget
 variant reg; see ewpt_set_tiling in include/ewpt.h) on a scratch lattice of
 the same size and precision, with CUDA events on the library's stream, and
-caches the fastest per (lattice shape, precision, beta on/off, GPU name) in a
-JSON file (default ~/.cache/ewpt/autotune.json, or $EWPT_AUTOTUNE_CACHE).
-The result does not change any number the kernels compute, only their speed.
+caches the fastest per (lattice shape, precision, stencil order, beta on/off,
+GPU name) in a JSON file (default ~/.cache/ewpt/autotune.json, or
+$EWPT_AUTOTUNE_CACHE).  A shape changes the kernels' speed and, in the FP32 form,
+whether a thread evolves one site or two, which round differently.
 """
 from __future__ import annotations
 
@@ -38,7 +39,17 @@ def _key(p: Params) -> str:
 
     nx, ny, nz = p.dims
     beta = int(p.beta_w != 0.0 or p.beta_y != 0.0)
-    return f"{nx}x{ny}x{nz}:p{int(p.precision)}:b{beta}:{torch.cuda.get_device_name(p.device)}"
+    order = "" if _order(p) == 6 else f":o{_order(p)}"
+    return f"{nx}x{ny}x{nz}:p{int(p.precision)}{order}:b{beta}:{torch.cuda.get_device_name(p.device)}"
+
+
+def _order(p: Params) -> int:
+    return int(p.stencil_order) or 6
+
+
+def _one_shape(p: Params) -> bool:
+    """The 6th-order FP64 stages take no notice of the tile."""
+    return int(p.precision) == _lib.FP64 and _order(p) == 6
 
 
 def _load_cache() -> dict:
@@ -106,6 +117,8 @@ def sweep(p: Params, steps: int = 2, candidates=None) -> list:
 
 
 def best_tiling(p: Params, steps: int = 2, use_cache: bool = True) -> tuple:
+    if _one_shape(p):
+        return CANDIDATES[0]
     key = _key(p)
     cache = _load_cache() if use_cache else {}
     if key in cache:

@@ -52,3 +52,20 @@ def test_member_tilings_sweep_once_per_size(tmp_path, monkeypatch):
     assert not any(t[3] for t in odd)  # odd nx: one site per thread only
     assert (8, 16, 2, 1) in dict(swept)[(48, 48, 48)]
     assert autotune.member_tilings(ps) == tiles and len(swept) == 2  # from the cache
+
+
+def test_nothing_is_swept_where_the_tile_changes_nothing(tmp_path, monkeypatch):
+    """The 6th-order FP64 stages have one launch shape; the other stencil orders
+    are swept, and cached apart from each other."""
+    import types
+
+    monkeypatch.setenv("EWPT_AUTOTUNE_CACHE", str(tmp_path / "tune.json"))
+    monkeypatch.setitem(__import__("sys").modules, "torch", types.SimpleNamespace(
+        cuda=types.SimpleNamespace(get_device_name=lambda d: "test-gpu")))
+    swept = []
+    monkeypatch.setattr(autotune, "sweep", lambda p, steps=2, candidates=None: swept.append(p.stencil_order) or
+                        [((32, 4, 0, 0), 2.0), ((64, 2, 2, 0), 1.0)])
+    for order in (6, 0, 8, 10, 8):
+        tile = autotune.best_tiling(ewpt.baseline_couplings(N=64, stencil_order=order))
+        assert tile == ((32, 4, 0, 0) if order in (6, 0) else (64, 2, 2, 0))
+    assert swept == [8, 10]
