@@ -533,7 +533,6 @@ extern "C" int ewpt_diagnostics(ewpt_ctx* c, double out[EWPT_NDIAG]) {
     int rc = ewpt_state64(c, &y);
     if (rc) return rc;
     if (!c->red) {
-        c->red_blocks = (int)(diag_partial_count(c->g) / NRED);
         rc = ewpt_cuda_check(c, cudaMalloc(&c->red, (size_t)diag_partial_count(c->g) * 8), "diag scratch");
         if (rc) return rc;
         rc = ewpt_cuda_check(c, cudaMalloc(&c->dres, 64 * 8), "diag result");

@@ -40,7 +40,6 @@ struct ewpt_ctx {
     double* scratch64 = nullptr;
     // diagnostics / spectra scratch (diag.cu, spectrum.cu)
     double* red = nullptr;      // per-block partial sums
-    int red_blocks = 0;
     double* dres = nullptr;     // device result row
     double* field3 = nullptr;   // [3 or 4][S] real fields for the FFT
     void* fft_out = nullptr;    // complex half-spectrum buffers
