@@ -25,11 +25,10 @@ e2e      the same metric through the C ABI with host buffers, as a drop-in
 roofline HBM roofline of the stage kernels: algorithmic bytes per
          site-update (3744 B FP64, 2592 B FP32 form) x site-updates/s over
          the measured copy bandwidth.
-roofline_compute  the FP64 form's own bound, the FP64 pipe: counted FLOPs
-         per site-update x site-updates/s over the FP64 peak measured in
-         this run (ewpt_fp64_peak, fused multiply-add chains on every SM).
-         The stencils' FLOPs are done in 64-bit integers, so this passes 1;
-         `pipe` has the FP64 instructions that are executed.
+roofline_compute  the FP64 form's own bound, the FP64 pipe: FP64 instructions
+         executed per site-update (ncu) x site-updates/s over the rate of
+         fused multiply-adds measured in this run (ewpt_fp64_peak, chains on
+         every SM).  The stencils run in 64-bit integers and are not in it.
 --impl reference  times the CPU restatement of the reference's routines (the
          oracle) on the host cores on a bounded sample lattice.
 With --gpus N > 1 (torchrun), each rank evolves its own replica; value is the
@@ -57,14 +56,14 @@ BYTES_FP32 = 2592  # y in FP64 width, stage rates in FP32
 # FP64 at 96^3; FP32 form at 128^3, the tuned paired kernel
 # (64x2 pair-threads, <= 168 registers, with its L2 prefetches).  Traffic grows with the site count,
 # so a 256^3 launch moves this x S / 4.
-TRAFFIC_FP64 = 4632
-TRAFFIC_FP32 = 2682
-# FP64 operations of one site-update of the FP64 stage kernels (4 stages of
-# site_rates + the RK4 epilogue), counted exactly by compiling the kernels'
-# own per-site templates with an operator-counting scalar type
-# (tests/test_devphys.py checks these figures against that count): FLOPs with
-# an FMA as 2, and FP64 pipe instructions with single-use products fused, the
-# stencils in floating point (the 6th-order stages do theirs in integers).
+TRAFFIC_FP64 = 4562
+TRAFFIC_FP32 = 2684
+# Operations of one site-update with the stencils in floating point (4 stages
+# of csrc/physics.cuh + the RK4 epilogue), counted exactly by compiling it with
+# an operator-counting scalar type (tests/test_devphys.py checks these figures
+# against that count): FLOPs with an FMA as 2, and FP64 pipe instructions with
+# single-use products fused.  The 6th-order FP64 stages execute fewer
+# (FP64_INST_NCU): their stencils are integers, their physics is csrc/stage_fp64.cuh.
 FLOPS_FP64 = 6820
 FP64_INST_EST = 4704
 # FP64 instructions per site-update the stage kernels execute (ncu
@@ -314,21 +313,15 @@ def run_ours(args, ws, rank, local):
                      "traffic_source": "ncu dram bytes per site-update at 96^3 x sites / 4",
                      "algorithmic_bytes_per_site_update": BYTES_FP64,
                      "limiter": "the FP64 pipe, not HBM: see roofline_compute"},
-        "roofline_compute": {"bound": "fp64", "achieved": S * args.steps / t64 * FLOPS_FP64 / 1e12,
-                             "peak": res["fp64"]["peak"] / 1e12, "unit": "TFLOP/s",
-                             "frac": S * args.steps / t64 * FLOPS_FP64 / res["fp64"]["peak"],
+        "roofline_compute": {"bound": "fp64 pipe", "achieved": S * args.steps / t64 * FP64_INST_NCU / 1e9,
+                             "peak": res["fp64"]["peak"] / 2 / 1e9, "unit": "Ginst/s",
+                             "frac": S * args.steps / t64 * FP64_INST_NCU / (res["fp64"]["peak"] / 2),
                              "peak_kind": "measured in this run: ewpt_fp64_peak (DFMA chains on every SM)",
+                             "fp64_inst_per_site_update": FP64_INST_NCU,
+                             "inst_source": "ncu FP64 pipe instructions at 96^3, 32 lanes each",
                              "flops_per_site_update": FLOPS_FP64,
-                             "flops_source": "exact count of the kernels' per-site source (oracle/devphys.cu), "
-                                             "FMA = 2 FLOPs",
-                             "pipe": {"fp64_inst_per_site_update": FP64_INST_NCU,
-                                      "source": "ncu FP64 pipe instructions at 96^3, 32 lanes each",
-                                      "achieved_ginst_s": S * args.steps / t64 * FP64_INST_NCU / 1e9,
-                                      "peak_ginst_s": res["fp64"]["peak"] / 2 / 1e9,
-                                      "frac": S * args.steps / t64 * FP64_INST_NCU / (res["fp64"]["peak"] / 2)},
-                             "note": "the FLOP count holds the stencils, which run in 64-bit integers: frac "
-                                     "may pass 1; the pipe frac is the FP64 instruction rate over the "
-                                     "probe's",
+                             "flops_source": "exact count of the same equations with floating-point stencils "
+                                             "(oracle/devphys.cu), FMA = 2 FLOPs; no part of frac",
                              "kernel": "k_stage_fp64 (4 launches/step)"},
         "gpu_launches": 4 * args.steps,
         "clocks": clocks,
