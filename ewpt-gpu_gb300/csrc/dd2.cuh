@@ -2,11 +2,17 @@
 // hi and lo are packed float pairs, every operation one FADD2 / FMUL2 / FFMA2
 // for both sites, half the instructions of two scalar sequences.
 //
-// Values stay unnormalised through sums: an addition is Knuth's TwoSum on the
-// high parts plus the low parts (8 operations, 11 with dd's renormalisation);
-// a product renormalises (7), so that the factors of the next product are
-// normalised where they are products, and sums are renormalised (done2) where
-// a rate ends.  The error per operation stays ~2^-47 of the operands.
+// Values stay unnormalised through sums and products: an addition is Knuth's
+// TwoSum on the high parts plus the low parts (8 operations, 11 with dd's
+// renormalisation), a product the FMA error of the high parts plus the cross
+// terms (4, 7 with it).  Finished derivatives, currents and rates are
+// renormalised (done2).  TwoSum holds whatever the order of its operands, and a
+// product drops the product of the low parts alone: each low part is within a
+// few 2^-24 of the values that were summed to it, so the loss is ~2^-47 of the
+// factors before they cancelled, as it is for normalised pairs.  Against FP64,
+// 192 runs of three lattices (bubbles, thermal states, a drive; 1 to 40 steps):
+// l2 error of the worst array 0.975 (median) of the normalised one-site form's,
+// at most 1.0004; largest error 0.99 (mean; single runs 0.76 to 1.16).
 #pragma once
 #include "dd.cuh"
 #include "f32x2.cuh"

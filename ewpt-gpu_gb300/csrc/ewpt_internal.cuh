@@ -253,8 +253,8 @@ cudaError_t launch_step_fp32(const Grid& g, const Layout& L, const Tiling& t, Fp
 // the compiler orders otherwise), of more sites than one wave of the one-site
 // kernel (152 SMs x 12 warps).  Below that a step costs one thread's chain of
 // operations, which two sites lengthen.  ms per step, one site -> two: 32^3
-// 0.050 -> 0.068, 48^3 0.123 -> 0.113, 64^3 0.260 -> 0.250, 128^3 1.63 -> 1.28,
-// 256^3 12.6 -> 9.29.
+// 0.055 -> 0.068, 48^3 0.123 -> 0.107, 64^3 0.260 -> 0.241, 128^3 1.63 -> 1.28,
+// 256^3 12.6 -> 9.31.
 inline bool fp32_as_one(const Grid& g, const ewpt_params& p) {
     return g.nx % 2 == 0 && g.S > 152 * 12 * 32 && p.beta_w == 0.0 && p.beta_y == 0.0;
 }

@@ -8,12 +8,13 @@
 // exactly with the integer weights 45, -9, 1 (60 dx times the derivative) and
 // 270, -27, 2 (180 dx^2 times the Laplacian, on differences from the centre
 // value), and each finished sum is rounded once to FP64; the factors stay in
-// the coefficients of the physics.  A derivative carries that rounding and
-// the bits below 2^-55 of the largest value on its line of neighbours (of the
-// whole stencil where a Laplacian comes with it), where the
-// floating-point evaluation rounds every partial sum at 2^-53 and every
-// weight (3/20, 1/90, 49/6 ... are no FP64 numbers) once.  Divergences and curls
-// add such sums of different arrays, each aligned by itself.
+// the coefficients of the physics.  A value that is aligned loses less than one
+// unit, 2^-55 of the largest value on its line of neighbours (of the whole
+// stencil where a Laplacian comes with it): at most 55 units in a derivative and
+// 1794 in a Laplacian by the weights, and 63/64 of 64 more where the Laplacian's
+// sum is cut to 64 bits.  The floating-point evaluation rounds every partial sum
+// at 2^-53 and every weight (3/20, 1/90, 49/6 ... are no FP64 numbers) once.
+// Divergences and curls add such sums of different arrays, each aligned by itself.
 //
 // A value goes to an integer by bit operations (about 12), the sums are
 // add/multiply pairs, a finished sum goes back by a count of leading zeros
@@ -26,8 +27,9 @@
 // Every stencil of -v is minus the stencil of v to the bit, as IEEE sums are, and
 // does not see the signs of zeros: a start that is symmetric under Phi -> -Phi
 // or a reflection stays so.  Step times with all of this: 64^3 1.04 ms, 128^3
-// 7.83, 256^3 63.4, 1 to 3% above those of sums rounded downwards.  Values with exact
-// zeros among them cost more: 64^3 1.38 ms where every array but one is odd in x.
+// 7.83, 256^3 62.0, 3% above those of sums rounded downwards on one exponent.  Values
+// with exact zeros among them cost more: 64^3 1.38 ms where every array but one is
+// odd in x (2.37 with floating-point stencils).
 //
 // Stencils whose largest magnitude lies outside [2^-895, 2^977] (denormals,
 // infinities and NaN among them) take the floating-point evaluation, as do
@@ -135,7 +137,7 @@ __device__ __forceinline__ bool weighed(const double (&f)[N][6], int64_t* V, uin
 // must not cost the others their last bits (values aligned to the largest of
 // all lines: error 3e-11 of the divergence where one array is 1 and constant, the
 // others waves of 1e-6; now 1e-16).  About 70 integer instructions more than
-// that: a step 0.8% at 64^3, 1.3% at 256^3, a snapshot at 128^3 2.7%.
+// that: a step 0.8% longer at 64^3, 1.3% at 256^3, a snapshot at 128^3 2.7%.
 template <int N>
 __device__ __forceinline__ double sum(const int64_t* V, const uint32_t* e20) {
     uint64_t u[N];

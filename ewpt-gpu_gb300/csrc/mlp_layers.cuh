@@ -4,7 +4,8 @@
 // A training step at the surrogate's size (84-256-256-40, batches of 128) is
 // bound by latency: 0.06 GFLOP, 1 MB.  As 11 general GEMMs (k_gemm_tc, 25 us
 // each, most of it the scalar gather of the operands) and 13 element-wise
-// launches it took 282 us.  Here it is seven launches:
+// launches it took 267 us, and takes 55 now (forward pass 137 and 41).  Here it is
+// seven launches:
 //   layer 1, layer 2    Z = A W^T + b, A' = gelu(Z)
 //   layer 3             Z3, the loss and dZ3
 //   back 2, back 1      dZ = (dZ' W) gelu'(Z)

@@ -258,7 +258,7 @@ static void step_fp32_r(const Grid& g, const Layout& L, const Tiling& t, Fp32Buf
                         const PhysCoef<float>& pc, const StencilCoef<float>& sc, double dt, cudaStream_t st) {
     // picked: <= 168 registers, or the compiler's choice (8 warps per SM) where the
     // lattice has no more sites than 7 warps per SM (16^3 0.049 against
-    // 0.053 ms per step, 24^3 0.051 against 0.057, 32^3 0.055 against 0.057; 33^3
+    // 0.053 ms per step, 24^3 0.051 against 0.057, 32^3 0.056 against 0.059; 33^3
     // 0.081 against 0.076, 36^3 0.093 against 0.080)
     const int reg = !t.pick ? t.reg : g.S > 152 * 7 * 32 ? 2 : 0;
     if (reg == 1)

@@ -419,7 +419,7 @@ void step_dd_r(const Grid& g, const Tiling& t, float2* y, float2* yn, float2* xa
 cudaError_t launch_step_dd(const Grid& g, const Tiling& t, double* y, double* yn, double* xa, double* xb,
                            double* cur, const ewpt_params& p, double Jex, double gam, cudaStream_t st) {
     if (dd_in_pairs(g, p)) {
-        // 128 registers run fastest (256^3: 46.9 ms per step against 48.2 with
+        // 128 registers run fastest (256^3: 45.8 ms per step against 48.2 with
         // 168 and 55.9 with 255)
         if (t.reg == 0 && !t.pick)
             step_dd2<0>(g, t, y, yn, xa, xb, cur, p, Jex, gam, st);

@@ -20,7 +20,7 @@
 // The equations are those of physics.cuh.
 //
 // Bound by the FP64 pipe (one warp instruction per 64 cycles and SM quarter):
-// 487 FP64 instructions per 32 sites and stage, the pipe 83-85% busy at 96^3 (ncu;
+// 487 FP64 instructions per 32 sites and stage, the pipe 81-83% busy at 96^3 (ncu;
 // chains of independent FMAs reach 84%; shared-memory latency and instruction
 // fetch the largest stalls).  A site per
 // thread took 128-255 registers through ~15 k instructions: 16 warps per SM ran
@@ -30,7 +30,9 @@
 // 28 0.171 -> 0.0985 ms, 64^3 1.20 -> 1.12, 75 x 61 x 90 1.84 -> 1.72, 128^3 9.29
 // -> 8.40, 256^3 76.2 -> 66.8 (532 FP64 instructions); with the units of the
 // momentum rates in the sink's weights, negations folded and no division
-// without damping (487) 64^3 1.01, 128^3 7.59, 256^3 60.2.  The Higgs part in one warp instead of split by
+// without damping (487) 64^3 1.01, 128^3 7.58, 256^3 60.2; with stencils that are
+// odd to the bit and an exponent per line (fixstencil.cuh) 24 x 20 x 28 0.097,
+// 64^3 1.04, 75 x 61 x 90 1.59, 128^3 7.83, 256^3 62.0.  The Higgs part in one warp instead of split by
 // axis: 0.117 and 1.23 at 24 x 20 x 28 and 64^3.  The stencils out of line, with
 // the neighbours' offsets in local memory: 0.107 and 1.15.  Blocks per SM, six,
 // seven, eight: 24 x 20 x 28 0.098, 0.0985, 0.105; 256^3 68.8, 66.8, 66.0.
